@@ -128,6 +128,7 @@ phr_status cuda_status(Ctx* ctx, cudaError_t e, const char* what) {
 namespace {
 
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
+constexpr uint32_t kTileSeg = 6;   // key segment of the register-tile pairs (log2 lanes is 0..5)
 
 __device__ __forceinline__ int next_pow2_cap32(int v) {
     int g = 1;
@@ -225,6 +226,7 @@ struct PackParams {
     int wfa_g_short, wfa_g_long;
     int wfa_long_min;   // qn + tn from which a WFA pair gets wfa_g_long lanes
     int band_base;      // Myers band half-width base
+    int big_min;        // qn + tn from which a linear WFA pair runs in register tiles
 };
 
 // 2-bit packing (16 bases per word) of both suffixes; a pair holding any byte other
@@ -360,7 +362,8 @@ __global__ void pack_kernel(PackParams P) {
             G = (d.qn + d.tn < P.wfa_long_min) ? P.wfa_g_short : P.wfa_g_long;
             len = static_cast<uint32_t>(d.qn + d.tn);
         }
-        const uint32_t glog = static_cast<uint32_t>(__ffs(G) - 1);
+        // register-tile pairs form a segment of their own after the warp-group ones
+        const uint32_t glog = tile_pair(P.engine, P.big_min, d.qn, d.tn) ? kTileSeg : static_cast<uint32_t>(__ffs(G) - 1);
         const uint32_t lk = 0x0FFFFFFFu - min(len, 0x0FFFFFFFu);  // longest first within a bucket
         P.keys[i] = (static_cast<uint32_t>(d.mode) << 31) | (glog << 28) | lk;
         P.vals[i] = static_cast<uint32_t>(i);
@@ -389,9 +392,13 @@ struct TaskBuild {
     int32_t big_min;              // linear WFA pairs for the CTA-per-pair kernel (not in the
     uint32_t big_smem;            // main pass, so not in its slot statistics)
     int32_t lane_ckpt;            // lane kernel mode (its scratch need)
+    uint32_t* tile_min;           // [2] first register-tile task of each symbol mode
+    uint32_t* tile_ranges;        // {begin, end} of the register-tile tasks of each mode
+    unsigned long long* tile_need;   // scratch wanted by the register-tile pairs
 };
 
-__device__ __forceinline__ int key_group(uint32_t k) { return 1 << ((k >> 28) & 7); }
+__device__ __forceinline__ bool key_tile(uint32_t k) { return ((k >> 28) & 7u) == kTileSeg; }
+__device__ __forceinline__ int key_group(uint32_t k) { return key_tile(k) ? 32 : 1 << ((k >> 28) & 7); }
 __device__ __forceinline__ uint32_t key_seg(uint32_t k) { return k >> 28; }
 
 __global__ void task_head_kernel(TaskBuild T) {
@@ -424,8 +431,8 @@ __global__ void task_fill_kernel(TaskBuild T) {
     // every lane stays to the warp-level reductions at the end; lanes without a task
     // contribute nothing to them
     const bool has_task = p < T.n && T.flag[p];
-    uint64_t need = 0;
-    uint32_t t_split = 0xFFFFFFFFu, t_g1 = 0xFFFFFFFFu;
+    uint64_t need = 0, tile_need = 0;
+    uint32_t t_split = 0xFFFFFFFFu, t_g1 = 0xFFFFFFFFu, t_tile[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
     if (has_task) {
         const uint32_t k = T.keys[p];
         const int G = key_group(k);
@@ -447,6 +454,9 @@ __global__ void task_fill_kernel(TaskBuild T) {
                 m_max = max(m_max, d.qn);
             } else if (T.engine == PHR_ENGINE_MYERS_FIT || T.engine == PHR_ENGINE_MYERS_GLOBAL)
                 need += myers_need_est(d.qn, d.tn, G, T.band_base);
+            else if (key_tile(k))
+                tile_need = tile_fixed_bytes(d.qn, d.tn) +
+                            tile_align(tile_hist_bytes(d.qn, d.tn, tile_score_est(d.qn, d.mode))) + kTileChunk;
             else if (!big_pair(T.engine, T.big_min, T.big_smem, d.qn, d.tn, d.mode))
                 region = max(region, wfa_region_est(d.qn, d.tn, T.engine == PHR_ENGINE_WFA_AFFINE));
             ++cnt;
@@ -460,6 +470,7 @@ __global__ void task_fill_kernel(TaskBuild T) {
         T.task_need[t] = need;
         if ((k >> 31) & 1) t_split = t;
         else if (G > 1) t_g1 = t;
+        if (key_tile(k)) t_tile[(k >> 31) & 1] = t;
     }
     // one atomic per warp and value instead of one per task (a million tasks would
     // otherwise queue on the same three addresses)
@@ -468,6 +479,16 @@ __global__ void task_fill_kernel(TaskBuild T) {
     for (int o = 16; o > 0; o >>= 1) nmax = max(nmax, __shfl_xor_sync(PHR_FULL_MASK, nmax, o));
     t_split = __reduce_min_sync(PHR_FULL_MASK, t_split);
     t_g1 = __reduce_min_sync(PHR_FULL_MASK, t_g1);
+    if (__any_sync(PHR_FULL_MASK, tile_need != 0)) {
+        uint64_t sum = tile_need;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(PHR_FULL_MASK, sum, o);
+        for (int m = 0; m < 2; ++m) {
+            const uint32_t f = __reduce_min_sync(PHR_FULL_MASK, t_tile[m]);
+            if ((threadIdx.x & 31) == 0 && f != 0xFFFFFFFFu) atomicMin(T.tile_min + m, f);
+        }
+        if ((threadIdx.x & 31) == 0) atomicAdd(T.tile_need, static_cast<unsigned long long>(sum));
+    }
     const int bucket = need ? 64 - __clzll(need) : 64;   // 64: no histogram entry
     const uint32_t same = __match_any_sync(PHR_FULL_MASK, bucket);
     const int lane = threadIdx.x & 31;
@@ -483,10 +504,15 @@ __global__ void task_finalize_kernel(TaskBuild T) {
     uint32_t nt = 0;
     if (T.n > 0) nt = T.tidx[T.n - 1] + T.flag[T.n - 1];
     const uint32_t split = min(*T.split_min, nt);
+    const uint32_t b0 = min(T.tile_min[0], split), b1 = min(T.tile_min[1], nt);
     T.ranges[0] = 0;
-    T.ranges[1] = split;
+    T.ranges[1] = b0;
     T.ranges[2] = split;
-    T.ranges[3] = nt;
+    T.ranges[3] = b1;
+    T.tile_ranges[0] = b0;
+    T.tile_ranges[1] = split;
+    T.tile_ranges[2] = b1;
+    T.tile_ranges[3] = nt;
     // lane-kernel range {0, g1} and warp-group 2-bit range {g1, split} (global Myers)
     const uint32_t g1 = min(*T.g1_min, split);
     T.ranges[28] = 0;
@@ -516,7 +542,7 @@ __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* red
     task_first[t] = t;
     task_count[t] = 1;
     task_group[t] = static_cast<uint8_t>(G);
-    if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode)) task_group[t] = kBigTask | 32;
+    if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode) || tile_pair(engine, big_min, d.qn, d.tn)) task_group[t] = kBigTask | 32;
 }
 
 struct FinishParams {
@@ -705,7 +731,9 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // counters: [0..3] ranges, [4] split_min, [5] queue head 0, [6] queue head 1,
     // [7] redo count, [8..9] need max (u64), [10] error flag, [12..13] total (u64), [14..17] redo ranges,
     // [20] first multi-lane 2-bit task, [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
-    // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64)
+    // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64),
+    // [40..41] first register-tile task of each mode, [42..45] register-tile ranges, [46..47] their
+    // scratch need (u64), [48..49] pool bytes taken (u64)
     uint32_t* cnt = static_cast<uint32_t*>(take(256));
     if (!cnt) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted");
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
@@ -713,6 +741,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 256, st));
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 4, 0xFF, 4, st));
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 20, 0xFF, 4, st));
+    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 40, 0xFF, 8, st));
 
     // CUB temp sizes
     size_t t_sort = 0, t_scan = 0, t_max = 0;
@@ -742,7 +771,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
 
     PackParams pk{in, engine, costs, desc, pout, w2o, wbo, tbo, arena2, arenab, text, keys, vals,
                   g_short, ctx->tune.wfa_group_long, ctx->tune.wfa_long_min,
-                  ctx->tune.myers_band_base};
+                  ctx->tune.myers_band_base, ctx->tune.wfa_big_min};
     {
         KernelScope ks(ctx, "pack");
         pack_kernel<<<blocks_for(n * 32, T), T, 0, st>>>(pk);
@@ -753,7 +782,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(need_hist, 0, 64 * 4, st));
     TaskBuild tbp{keys_s, order, n, head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4, cnt + 20, desc,
                   engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
-                  ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt};
+                  ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt,
+                  cnt + 40, cnt + 42, reinterpret_cast<unsigned long long*>(cnt + 46)};
     {
         KernelScope ks(ctx, "task_head");
         task_head_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
@@ -781,13 +811,17 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // are deferred to the redo passes, which size scratch per task.
     uint64_t h_need = 0;
     unsigned int h_hist[64];
-    uint32_t h_ranges[4];
+    uint32_t h_cnt[48];   // the counter block up to the register-tile need
+    const uint32_t* h_ranges = h_cnt;
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_need, need_max, 8, cudaMemcpyDeviceToHost, st));
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_hist, need_hist, sizeof(h_hist), cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_ranges, cnt, sizeof(h_ranges), cudaMemcpyDeviceToHost, st));
+    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
     PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     PHR_CUDA_TRY(ctx, cudaGetLastError());
     hs_setup.stop();
+    const uint32_t n_tile[2] = {h_cnt[43] - h_cnt[42], h_cnt[45] - h_cnt[44]};
+    uint64_t tile_need = 0;
+    std::memcpy(&tile_need, h_cnt + 46, 8);
     {
         uint64_t n_tasks = 0;  // tasks of the main pass with a scratch need
         for (int b = 0; b < 64; ++b) n_tasks += h_hist[b];
@@ -838,12 +872,19 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                            uint64_t n_tasks_hint = 0) -> phr_status {
         const uint64_t warps_per_block = block / 32;
         uint64_t grid = static_cast<uint64_t>(ctx->sm_count) * ctx->tune.max_blocks_per_sm;
+        uint64_t pool = 0;
         if (!per_task) {
             slot = std::max<uint64_t>((slot + 255) & ~255ull, 4096);
             // grid: resident blocks per SM, no more warps than tasks, shrunk to the scratch budget
             grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (h_ranges[3] + warps_per_block - 1) / warps_per_block));
             while (grid > 1 && grid * warps_per_block * slot > ctx->scratch_budget) grid = (grid + 1) / 2;
-            PHR_CUDA_TRY(ctx, ctx->scratch.reserve(grid * warps_per_block * slot));
+            // the register-tile pairs run after the group kernels and reuse the buffer from
+            // its start; a small batch gets room for pairs of any divergence
+            pool = 0;
+            if (n_tile[0] + n_tile[1] > 0)
+                pool = std::min<uint64_t>(std::max<uint64_t>(tile_need, std::min<uint64_t>(16 * tile_need, 1ull << 30)),
+                                          ctx->scratch_budget);
+            PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
         } else {
             grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (n_tasks_hint + warps_per_block - 1) / warps_per_block));
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(per_task_total));
@@ -900,27 +941,34 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             else
                 launch_wfa_affine_bytes(P, static_cast<int>(grid), block, st);
         }
-        if (per_task && (engine == PHR_ENGINE_WFA_LINEAR || engine == PHR_ENGINE_WFA_AFFINE) && P.big_min > 0 &&
-            n_tasks_hint > 0) {
-            // long pairs of this redo list, one CTA each
-            // linear: two CTAs of kBigThreads per SM (one when the tune keeps fewer blocks
-            // resident); gap-affine: kBigAffineThreads / wfa_affine_big_threads CTAs per SM
+        if (engine == PHR_ENGINE_WFA_LINEAR && P.big_min > 0 && (per_task ? n_tasks_hint : n_tile[0] + n_tile[1]) > 0) {
+            // long pairs in register tiles, one CTA each: two CTAs per SM (one when the tune
+            // keeps fewer blocks resident)
+            const uint64_t per_sm = ctx->tune.max_blocks_per_sm >= 4 ? 2 : 1;
+            PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 24, 0, 8, st));
+            if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 48, 0, 8, st));
+            const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 48), pool, kTileChunk};
+            for (int mode = 0; mode < 2; ++mode) {
+                const uint64_t nt = per_task ? n_tasks_hint : n_tile[mode];
+                if (nt == 0) continue;
+                P.tasks.range = per_task ? (mode ? range1 : range0) : cnt + 42 + 2 * mode;
+                P.queue_head = cnt + 24 + mode;
+                KernelScope ks(ctx, mode ? "wfa_linear_big_bytes" : "wfa_linear_big");
+                launch_wfa_linear_big(P, tl, static_cast<int>(std::min<uint64_t>(nt, ctx->sm_count * per_sm)), mode, st);
+            }
+        }
+        if (per_task && engine == PHR_ENGINE_WFA_AFFINE && P.big_min > 0 && n_tasks_hint > 0) {
+            // long gap-affine pairs of this redo list, one CTA each: kBigAffineThreads /
+            // wfa_affine_big_threads CTAs per SM
             const int aff_threads = ctx->tune.wfa_affine_big_threads;
-            const uint64_t big_per_sm = engine == PHR_ENGINE_WFA_AFFINE
-                                            ? static_cast<uint64_t>(kBigAffineThreads / aff_threads)
-                                            : (ctx->tune.max_blocks_per_sm >= 4 ? 2 : 1);
-            const int big_grid = static_cast<int>(std::min<uint64_t>(n_tasks_hint, ctx->sm_count * big_per_sm));
+            const int big_grid = static_cast<int>(std::min<uint64_t>(
+                n_tasks_hint, ctx->sm_count * static_cast<uint64_t>(kBigAffineThreads / aff_threads)));
             PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 24, 0, 8, st));
             for (int mode = 0; mode < 2; ++mode) {
                 P.tasks.range = mode ? range1 : range0;
                 P.queue_head = cnt + 24 + mode;
-                if (engine == PHR_ENGINE_WFA_LINEAR) {
-                    KernelScope ks(ctx, mode ? "wfa_linear_big_bytes" : "wfa_linear_big");
-                    launch_wfa_linear_big(P, big_grid, mode, st);
-                } else {
-                    KernelScope ks(ctx, mode ? "wfa_affine_big_bytes" : "wfa_affine_big");
-                    launch_wfa_affine_big(P, big_grid, aff_threads, mode, st);
-                }
+                KernelScope ks(ctx, mode ? "wfa_affine_big_bytes" : "wfa_affine_big");
+                launch_wfa_affine_big(P, big_grid, aff_threads, mode, st);
             }
         }
         PHR_CUDA_TRY(ctx, cudaGetLastError());

@@ -65,13 +65,13 @@ __host__ __device__ __forceinline__ uint64_t big_seq_words(int qn, int tn, int m
     return static_cast<uint64_t>((qn + per - 1) / per) + static_cast<uint64_t>((tn + per - 1) / per) + 16;
 }
 
-// A WFA pair (linear or gap-affine) long enough that one warp would be latency-bound on
-// it: it runs one per CTA.
+// A gap-affine WFA pair long enough that one warp would be latency-bound on it: it runs
+// one per CTA (linear pairs: tile_pair below).
 __host__ __device__ __forceinline__ bool big_pair(int32_t engine, int32_t big_min, uint32_t big_smem, int qn, int tn,
                                                   int mode) {
     (void)big_smem;
     (void)mode;
-    return big_min > 0 && (engine == PHR_ENGINE_WFA_LINEAR || engine == PHR_ENGINE_WFA_AFFINE) && qn + tn >= big_min;
+    return big_min > 0 && engine == PHR_ENGINE_WFA_AFFINE && qn + tn >= big_min;
 }
 
 // Whether the CTA kernel stages a big pair's sequences in its shared memory (with room
@@ -169,6 +169,56 @@ __host__ __device__ __forceinline__ uint64_t myers_full_need(int m, int n) {
     return need;
 }
 
+// ---------------------------------------------------------------------------
+// Linear WFA in register tiles, one CTA per long pair (wfa_tile.cu).
+// ---------------------------------------------------------------------------
+constexpr int kTileSteps = 8;                                  // scores a tile advances between barriers
+constexpr int kTileRegs = 8;                                   // most diagonals per lane
+constexpr int kTileMax = 32 * kTileRegs;                       // most diagonals of a tile
+constexpr uint32_t kTileCtlBytes = 128;                         // a team's control block in shared memory
+
+__host__ __device__ __forceinline__ uint64_t tile_align(uint64_t v) { return (v + 255) & ~255ull; }
+__host__ __device__ __forceinline__ uint64_t tile_runs_bytes(int qn, int tn) {
+    return tile_align(4 * (static_cast<uint64_t>(qn) + tn + 2));
+}
+__host__ __device__ __forceinline__ uint64_t tile_table_bytes(int qn, int tn) {
+    return tile_align(4 * ((static_cast<uint64_t>(qn) + tn) / kTileSteps + 3));
+}
+// What a pair takes before its first record: match runs, CIGAR runs and three tables.
+__host__ __device__ __forceinline__ uint64_t tile_fixed_bytes(int qn, int tn) {
+    return 2 * tile_runs_bytes(qn, tn) + 3 * tile_table_bytes(qn, tn);
+}
+// Upper bound of the records of scores up to s: block u holds 16 (u + 1) diagonals of 4
+// bytes of value and at most 8 / 3 of ops, plus rounding to tiles and the narrow tiles of
+// small bands.
+__host__ __device__ __forceinline__ uint64_t tile_hist_bytes(int qn, int tn, int64_t s) {
+    (void)qn;
+    (void)tn;
+    const uint64_t u = static_cast<uint64_t>(s) / kTileSteps + 1;
+    return u * 6144 + 54 * u * (u + 1);
+}
+// Score a pair is given room for at first: a quarter of the query for DNA, half for bytes
+// (protein). Records come from a pool, so one pair may take more.
+__host__ __device__ __forceinline__ int64_t tile_score_est(int qn, int mode) {
+    return 64 + static_cast<int64_t>(qn) / (mode == 0 ? 4 : 2);
+}
+constexpr uint32_t kTileChunk = 64 << 10;   // bytes a team takes from the pool at a time
+
+// The pool of a main-pass launch: bytes [0, pool_end) of the scratch buffer, taken by
+// atomicAdd on pool_used. pool_used NULL (redo passes): every pair has its own region.
+struct TileLaunch {
+    unsigned long long* pool_used;
+    uint64_t pool_end;
+    uint32_t chunk;
+};
+
+// Pairs the register-tile kernel takes: long linear pairs. Offsets are kept times 256 in 32
+// bits, hence the upper limit; longer queries stay in the warp-group kernel.
+__host__ __device__ __forceinline__ bool tile_pair(int32_t engine, int32_t big_min, int qn, int tn) {
+    return big_min > 0 && engine == PHR_ENGINE_WFA_LINEAR && static_cast<int64_t>(qn) + tn >= big_min &&
+           qn < (1 << 22) && tn < (1 << 28);
+}
+
 void launch_myers(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_myers_lane(const ExtendParams& p, int grid, cudaStream_t st);
 // Resident blocks per SM of the lane kernel in each mode (its shared memory per warp).
@@ -176,7 +226,7 @@ int myers_lane_blocks_per_sm(int ckpt);
 constexpr int kLaneThreads = 256;
 void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
-void launch_wfa_linear_big(const ExtendParams& p, int grid, int mode, cudaStream_t st);
+void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st);
 
 }  // namespace phr

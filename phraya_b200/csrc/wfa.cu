@@ -350,17 +350,6 @@ __device__ void wfa_linear_group(const ExtendParams& P, const PairDesc& d, uint3
     }
 }
 
-// ===========================================================================
-// Linear WFA, one CTA per pair (long pairs)
-// ===========================================================================
-// A warp-per-pair wavefront on a long, divergent pair is latency-bound: every cell is a
-// chain of dependent loads (previous frame, both sequences) and one warp cannot hide
-// them. Here a CTA of kBigThreads threads takes one pair; both sequences and, while they
-// fit, the two value frames live in shared memory; the history (hr) goes to the pair's
-// scratch region with coalesced stores (consecutive diagonals on consecutive threads).
-// Frames that outgrow shared memory move to the region's global frames, the same layout
-// the warp kernel uses, so scratch needs and the redo rule are identical.
-
 // Bulk asynchronous copies (the TMA unit's untiled cp.async.bulk, no multicast) of the
 // pair's sequences into shared memory, completing on an mbarrier.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -399,33 +388,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     for (int it = 0; it < (1 << 22); ++it)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
-}
-
-// 32 bits holding symbols [pos, pos + kPerWord) of a sequence staged in shared memory.
-template <class S>
-__device__ __forceinline__ uint32_t window_sm(const uint32_t* base, int32_t pos) {
-    const uint32_t w = static_cast<uint32_t>(pos) / S::kPerWord;
-    const uint32_t sh = (static_cast<uint32_t>(pos) % S::kPerWord) * S::kBits;
-    return __funnelshift_r(base[w], base[w + 1], sh);
-}
-
-template <class S>
-__device__ __forceinline__ int32_t extend_sm(const uint32_t* q, int32_t qn, const uint32_t* t, int32_t tn,
-                                             int32_t q_pos, int32_t k, uint32_t& words) {
-    const int32_t j = q_pos - k;
-    if (q_pos < 0 || q_pos >= qn || j < 0 || j >= tn) return q_pos;
-    const int32_t lim = min(qn - q_pos, tn - j);
-    int32_t n = 0;
-    while (n < lim) {
-        ++words;
-        const uint32_t x = window_sm<S>(q, q_pos + n) ^ window_sm<S>(t, j + n);
-        if (x != 0) {
-            n += (__ffs(x) - 1) / S::kBits;
-            return q_pos + (n < lim ? n : lim);
-        }
-        n += S::kPerWord;
-    }
-    return q_pos + lim;
 }
 
 // Stages a pair's two sequences in the CTA's shared memory `sm`, each followed by one
@@ -477,275 +439,6 @@ __device__ uint32_t stage_pair_cta(const ExtendParams& P, const PairDesc& d, uin
     *sq_out = sq;
     *st_out = st;
     return (t_base + static_cast<uint32_t>(lead_t + tw + 1) + 3) & ~3u;
-}
-
-template <class S>
-__device__ void wfa_linear_cta(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
-                               uint64_t region_bytes, uint32_t* sm, uint32_t sm_words, int* sh_end, uint64_t* bar,
-                               uint32_t& phase) {
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    const int qn = d.qn, tn = d.tn;
-    const bool fitting = tn > qn + qn / 2 + 10;
-
-    // ---- stage both sequences (plus one zero word each) in shared memory ----
-    uint32_t *sq, *st;
-    const uint32_t fr_off = stage_pair_cta<S>(P, d, sm, bar, phase, &sq, &st);
-    const int qw = (qn + S::kPerWord - 1) / S::kPerWord;
-    const int tw = (tn + S::kPerWord - 1) / S::kPerWord;
-    const uint32_t fcap = sm_words > fr_off ? (sm_words - fr_off) / 2 : 0;  // cells per shared frame
-    int32_t* sfr = reinterpret_cast<int32_t*>(sm + fr_off);
-
-    // ---- region layout, as in wfa_linear_group ----
-    uint32_t* runs = reinterpret_cast<uint32_t*>(region);
-    const uint64_t runs_bytes = align16(static_cast<uint64_t>(qn + tn + 2) * 4);
-    const uint64_t frame_bytes = align16(static_cast<uint64_t>(qn + tn + 1) * 4);
-    const uint64_t fixed = runs_bytes + 2 * frame_bytes;
-    const uint64_t cell_cap = region_bytes > fixed ? (region_bytes - fixed) / 4 : 0;
-    int32_t* gfr = reinterpret_cast<int32_t*>(region + runs_bytes);
-    uint32_t* hr = reinterpret_cast<uint32_t*>(region + fixed);
-    bool global_frames = false;
-    auto frame = [&](int sc) -> int32_t* {
-        return global_frames ? gfr + (sc & 1) * (frame_bytes / 4) : sfr + (sc & 1) * fcap;
-    };
-
-    if (tid < 3) sh_end[tid] = INT32_MAX;
-    const int max_s = qn + tn;
-    bool done = false, overflow = false;
-    uint64_t wf_cells = 0;   // band diagonals of the scores computed
-    uint32_t lcp_words = 0;  // this thread's word compares of match extension
-    int s_end = 0, t_end = 0, s = 1;
-    if (lin_base(1, qn, tn) > cell_cap) overflow = true;
-    if (fcap < 1) global_frames = true;
-    __syncthreads();
-    if (!overflow) {
-        if (tid == 0) {
-            frame(0)[0] = extend_sm<S>(sq, qn, st, tn, 0, 0, lcp_words);
-            hr[0] = 0;
-        }
-        __syncthreads();
-        const int32_t v0 = frame(0)[0];
-        if (!fitting) {
-            if (qn - tn == 0 && v0 == qn) {  // wfa_simd.rs:277-283
-                done = true;
-                t_end = tn;
-            }
-        } else if (qn <= tn && v0 >= qn) {
-            done = true;
-            t_end = qn;
-        }
-        for (; !done && s <= max_s; ++s) {
-            const int lo = -min(s, tn), hi = min(s, qn);
-            const int plo = -min(s - 1, tn), phi = min(s - 1, qn);
-            const uint64_t base = lin_base(s, qn, tn);
-            const int width = hi - lo + 1;
-            if (base + static_cast<uint64_t>(width) > cell_cap) {
-                overflow = true;
-                break;
-            }
-            wf_cells += static_cast<uint64_t>(width);
-            if (!global_frames && static_cast<uint32_t>(width) > fcap) {
-                // frames outgrow shared memory: continue on the region's global frames
-                const int32_t* src = frame(s - 1);
-                int32_t* dst = gfr + ((s - 1) & 1) * (frame_bytes / 4);
-                for (int i = tid; i < phi - plo + 1; i += nthr) dst[i] = src[i];
-                global_frames = true;
-                __syncthreads();
-            }
-            const int32_t* pv_frame = frame(s - 1);
-            int32_t* cur_frame = frame(s);
-            if (tid == 0) sh_end[(s + 1) % 3] = INT32_MAX;
-            int my_end = INT32_MAX;
-            for (int k = lo + tid; k <= hi; k += nthr) {
-                int32_t best_pos = UNSET;
-                uint32_t best_op = 0;
-                bool have = false;
-                // candidates in order [mismatch, ins, del]; the LAST maximal one wins
-                if (k >= plo && k <= phi) {
-                    const int32_t pv = pv_frame[k - plo];
-                    if (pv != UNSET) {
-                        best_pos = pv + 1;
-                        best_op = 1;
-                        have = true;
-                    }
-                }
-                if (k > -tn && k - 1 >= plo && k - 1 <= phi) {
-                    const int32_t pv = pv_frame[k - 1 - plo];
-                    if (pv != UNSET) {
-                        const int32_t c = pv + 1;
-                        if (!have || c >= best_pos) {
-                            best_pos = c;
-                            best_op = 2;
-                            have = true;
-                        }
-                    }
-                }
-                if (k < qn && k + 1 >= plo && k + 1 <= phi) {
-                    const int32_t pv = pv_frame[k + 1 - plo];
-                    if (pv != UNSET) {
-                        if (!have || pv >= best_pos) {
-                            best_pos = pv;
-                            best_op = 3;
-                            have = true;
-                        }
-                    }
-                }
-                int32_t val = UNSET;
-                uint32_t aux = 0;
-                if (have) {
-                    const int32_t j = best_pos - k;
-                    if (!(best_pos < 0 || best_pos > qn || j < 0 || j > tn)) {
-                        val = extend_sm<S>(sq, qn, st, tn, best_pos, k, lcp_words);
-                        aux = (static_cast<uint32_t>(best_pos) << 2) | best_op;
-                    }
-                }
-                cur_frame[k - lo] = val;
-                hr[base + (k - lo)] = aux;
-                if (val != UNSET) {
-                    if (!fitting) {
-                        if (k == qn - tn && val >= qn) my_end = k;
-                    } else if (k >= qn - tn && k <= qn && val >= qn) {
-                        my_end = min(my_end, k);
-                    }
-                }
-            }
-            my_end = __reduce_min_sync(PHR_FULL_MASK, my_end);
-            if ((tid & 31) == 0 && my_end != INT32_MAX) atomicMin(&sh_end[s % 3], my_end);
-            __syncthreads();
-            const int kk = sh_end[s % 3];
-            if (kk != INT32_MAX) {
-                done = true;
-                s_end = s;
-                t_end = qn - kk;
-            }
-        }
-    }
-    if (done && s_end == 0) s = 0;
-    if (P.work) {  // work counters: band diagonals (the same in every thread), LCP word compares
-        if (tid == 0) atomicAdd(P.work + 2, static_cast<unsigned long long>(wf_cells));
-        if (lcp_words) atomicAdd(P.work + 3, static_cast<unsigned long long>(lcp_words));
-    }
-    const bool failed = !done && !overflow;
-    if (overflow) {  // CTA-uniform
-        // Scratch for the redo: extrapolate the final score from the progress so far (the
-        // furthest query offset the last score reached; the wavefront advances about in
-        // proportion to the score), plus a quarter as margin, so that one redo usually
-        // suffices; at least twice the scores reached, at most the whole search.
-        int vm = 0;
-        if (s >= 2) {
-            const int32_t* pf = frame(s - 1);
-            const int plo = -min(s - 1, tn), phi = min(s - 1, qn);
-            for (int k = plo + tid; k <= phi; k += nthr) vm = max(vm, pf[k - plo]);
-        }
-        vm = __reduce_max_sync(PHR_FULL_MASK, vm);
-        __syncthreads();  // every thread is done with the end flags
-        if (tid == 0) sh_end[0] = 0;
-        __syncthreads();
-        if ((tid & 31) == 0) atomicMax(&sh_end[0], vm);
-        __syncthreads();
-        if (tid == 0) {
-            const int64_t reach = sh_end[0];
-            int64_t s2 = 2LL * s + 64;
-            if (reach > 0) {
-                int64_t est = static_cast<int64_t>(s) * qn / reach;
-                est += est / 4 + 64;
-                s2 = ::max(s2, est);
-            }
-            s2 = ::min(static_cast<int64_t>(max_s) + 1, s2);
-            report_redo(P, pid, fixed + lin_base(s2, qn, tn) * 4 + 64);
-        }
-    }
-
-    // ---- traceback (wfa_simd.rs:959-1041) by thread 0, formatting by warp 0 ----
-    if (tid < 32) {
-        RunWriter rw;
-        rw.init(runs, static_cast<uint32_t>(qn + tn + 2));
-        if (done && tid == 0) {
-            int qi = qn, ti = t_end, k = qi - ti, ss = s_end;
-            while (qi > 0 || ti > 0) {
-                if (ss < 0) break;
-                if (ss == 0) {
-                    const int mm = min(qi, ti);
-                    rw.push(0, static_cast<uint32_t>(mm));
-                    qi -= mm;
-                    ti -= mm;
-                    break;
-                }
-                const int lo = -min(ss, tn);
-                const uint32_t aux = hr[lin_base(ss, qn, tn) + (k - lo)];
-                const uint32_t op = aux & 3;
-                const int32_t edit_start = static_cast<int32_t>(aux >> 2);
-                const int mc = qi - edit_start;
-                if (mc > 0) {
-                    rw.push(0, static_cast<uint32_t>(mc));
-                    qi -= mc;
-                    ti -= mc;
-                }
-                if (op == 1) {
-                    rw.push(1, 1);
-                    --qi;
-                    --ti;
-                } else if (op == 2) {
-                    rw.push(3, 1);
-                    --qi;
-                    k -= 1;
-                } else if (op == 3) {
-                    rw.push(2, 1);
-                    --ti;
-                    k += 1;
-                }
-                --ss;
-            }
-            rw.flush();
-        }
-        const uint32_t nr = __shfl_sync(PHR_FULL_MASK, rw.n, 0);
-        const bool ovf = __shfl_sync(PHR_FULL_MASK, rw.overflow ? 1 : 0, 0) != 0;
-        __syncwarp();
-        const uint32_t tl = format_group(runs, (done && !ovf) ? nr : 0, P.text + P.text_off[pid], 32);
-        if (tid == 0) {
-            if (done && !ovf) {
-                PairOut o;
-                o.status = PHR_OK;
-                o.ed = s_end;
-                o.t_consumed = t_end;
-                o.affine_score = 0;
-                o.n_runs = nr;
-                o.text_len = tl;
-                P.out[pid] = o;
-            } else if (failed) {
-                PairOut o = {};
-                o.status = PHR_ALIGNMENT_FAILED;
-                P.out[pid] = o;
-            } else if (done && ovf) {
-                atomicOr(P.error_flag, 2u);
-            }
-        }
-    }
-    __syncthreads();  // shared memory and the task slot are reused by the next pair
-}
-
-template <class S>
-__global__ void __launch_bounds__(kBigThreads, 2) wfa_linear_big_kernel(ExtendParams P) {
-    extern __shared__ __align__(16) uint32_t big_sm[];
-    __shared__ uint32_t sh_task;
-    __shared__ int sh_end[3];
-    __shared__ __align__(8) uint64_t sh_bar;
-    const uint32_t sm_words = P.big_smem / 4;
-    uint32_t phase = 0;  // parity of sh_bar's current phase, the same in every thread
-    if (threadIdx.x == 0) mbar_init(&sh_bar, 1);
-    __syncthreads();
-    for (;;) {
-        if (threadIdx.x == 0) sh_task = P.tasks.range[0] + atomicAdd(P.queue_head, 1u);
-        __syncthreads();
-        const uint32_t task = sh_task;
-        __syncthreads();
-        if (task >= P.tasks.range[1]) break;
-        if (!(P.tasks.task_group[task] & kBigTask)) continue;
-        const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
-        const PairDesc d = P.desc[pid];
-        if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
-        wfa_linear_cta<S>(P, d, pid, P.scratch + P.task_off[task], P.task_len[task] & ~15ull, big_sm, sm_words,
-                          sh_end, &sh_bar, phase);
-    }
 }
 
 // ===========================================================================
@@ -1838,17 +1531,6 @@ void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t 
 }
 void launch_wfa_linear_bytes(const ExtendParams& p, int grid, int block, cudaStream_t st) {
     wfa_kernel<SeqB, false><<<grid, block, 0, st>>>(p);
-}
-void launch_wfa_linear_big(const ExtendParams& p, int grid, int mode, cudaStream_t st) {
-    if (mode == 0) {
-        cudaFuncSetAttribute(wfa_linear_big_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
-        wfa_linear_big_kernel<Seq2><<<grid, kBigThreads, p.big_smem, st>>>(p);
-    } else {
-        cudaFuncSetAttribute(wfa_linear_big_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
-        wfa_linear_big_kernel<SeqB><<<grid, kBigThreads, p.big_smem, st>>>(p);
-    }
 }
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st) {
     if (mode == 0) {

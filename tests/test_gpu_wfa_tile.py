@@ -1,0 +1,88 @@
+"""Linear WFA in register tiles (wfa_tile.cu) against the oracle where it can go wrong:
+bands that end at, cross and leave tile edges, both end rules, both symbol modes, paths
+along the band's rim, sequences and frames that do not fit shared memory, and a scratch
+pool that runs out."""
+import numpy as np
+import pytest
+
+import oracle as O
+from phraya_b200 import _abi as A
+from phraya_b200 import api as P
+
+pytestmark = pytest.mark.gpu
+
+DNA, AA = b"ACGT", b"ACDEFGHIKLMNPQRSTVWY"
+
+
+def rand(rng, n, alphabet=DNA):
+    return bytes(rng.choice(list(alphabet), n).tolist())
+
+
+def mutate(rng, s, rate, alphabet=DNA):
+    out = bytearray()
+    for c in s:
+        x = rng.random()
+        if x < rate * 0.6:
+            out.append(alphabet[int(rng.integers(len(alphabet)))])
+        elif x < rate * 0.8:
+            out += rand(rng, int(rng.integers(1, 4)), alphabet) + bytes([c])
+        elif x < rate:
+            pass
+        else:
+            out.append(c)
+    return bytes(out)
+
+
+def edge_pairs(rng, alphabet):
+    """Similar, unrelated and rim pairs with lengths and scores around the tile sizes
+    (8 scores, 240 kept diagonals of 256)."""
+    pairs = []
+    for n in (31, 64, 119, 120, 121, 127, 128, 239, 240, 241, 256, 257, 500):
+        q = rand(rng, n, alphabet)
+        pairs += [(q, q), (q, mutate(rng, q, 0.08, alphabet) or q), (q, rand(rng, n, alphabet)),
+                  (q, q[: n // 2] or q), (q, rand(rng, 7, alphabet) + q),
+                  (q, mutate(rng, q, 0.05, alphabet) + rand(rng, n, alphabet)),     # fitting: the target runs on
+                  (q, rand(rng, 2 * n + 20, alphabet)), (q[:17], rand(rng, n, alphabet))]
+    a, c = alphabet[:1], alphabet[1:2]
+    for n in (7, 8, 9, 112, 120, 128, 240, 250):   # one gap of n: the path follows the band's rim
+        core = rand(rng, 60, alphabet)
+        pairs += [(core + a * n + core, core + core), (core + core, core + c * n + core), (a * (n + 30), c * (n + 30))]
+    return pairs
+
+
+@pytest.mark.parametrize("alphabet", [DNA, AA], ids=["2bit", "bytes"])
+@pytest.mark.parametrize("smem", [16 << 10, 100 << 10])
+def test_tile_edges(alphabet, smem):
+    rng = np.random.default_rng(41)
+    pairs = edge_pairs(rng, alphabet)
+    with P.Engine(0) as eng:
+        eng.set_tune("wfa_big_min", 32)
+        eng.set_tune("wfa_big_smem", smem)
+        got = eng.extend(A.ENGINE_WFA_LINEAR, pairs)
+    assert got == O.extend(A.ENGINE_WFA_LINEAR, pairs)
+
+
+@pytest.mark.parametrize("alphabet", [DNA, AA], ids=["2bit", "bytes"])
+def test_bands_beyond_shared_memory(alphabet):
+    """Unrelated pairs: wavefronts of thousands of diagonals, frames in global memory."""
+    rng = np.random.default_rng(42)
+    pairs = [(rand(rng, n, alphabet), rand(rng, m, alphabet)) for n, m in ((3000, 3100), (2500, 2900), (2100, 2000))]
+    q = rand(rng, 9000, alphabet)
+    pairs += [(q, mutate(rng, q, 0.1, alphabet)), (q[:5000], mutate(rng, q, 0.03, alphabet))]
+    with P.Engine(0) as eng:
+        eng.set_tune("wfa_big_smem", 24 << 10)
+        got = eng.extend(A.ENGINE_WFA_LINEAR, pairs)
+    assert got == O.extend(A.ENGINE_WFA_LINEAR, pairs)
+
+
+@pytest.mark.parametrize("budget", [1 << 20, 4 << 20])
+def test_pool_runs_out(budget):
+    """More records than the workspace holds at once: pairs are redone with their own
+    scratch and give the same results."""
+    rng = np.random.default_rng(43)
+    q = [rand(rng, n) for n in (4000, 4100, 5000, 2300, 2050, 3000)]
+    pairs = [(s, mutate(rng, s, 0.04)) for s in q] + [(rand(rng, 1500), rand(rng, 2600)) for _ in range(4)]
+    with P.Engine(0, workspace_bytes=budget) as eng:
+        got = eng.extend(A.ENGINE_WFA_LINEAR, pairs)
+        assert eng.counter("scratch_oom_pairs") == 0
+    assert got == O.extend(A.ENGINE_WFA_LINEAR, pairs)
