@@ -128,7 +128,8 @@ phr_status cuda_status(Ctx* ctx, cudaError_t e, const char* what) {
 namespace {
 
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
-constexpr uint32_t kTileSeg = 6;   // key segment of the register-tile pairs (log2 lanes is 0..5)
+// key segments of the register-tile pairs (log2 lanes is 0..5): one warp, one CTA per pair
+constexpr uint32_t kWarpTileSeg = 6, kTileSeg = 7;
 
 __device__ __forceinline__ int next_pow2_cap32(int v) {
     int g = 1;
@@ -362,8 +363,9 @@ __global__ void pack_kernel(PackParams P) {
             G = (d.qn + d.tn < P.wfa_long_min) ? P.wfa_g_short : P.wfa_g_long;
             len = static_cast<uint32_t>(d.qn + d.tn);
         }
-        // register-tile pairs form a segment of their own after the warp-group ones
-        const uint32_t glog = tile_pair(P.engine, P.big_min, d.qn, d.tn) ? kTileSeg : static_cast<uint32_t>(__ffs(G) - 1);
+        // register-tile pairs form segments of their own after the warp-group ones
+        const int tw = tile_warps(P.engine, P.big_min, P.wfa_long_min, d.qn, d.tn, d.mode);
+        const uint32_t glog = tw == 0 ? static_cast<uint32_t>(__ffs(G) - 1) : tw == 1 ? kWarpTileSeg : kTileSeg;
         const uint32_t lk = 0x0FFFFFFFu - min(len, 0x0FFFFFFFu);  // longest first within a bucket
         P.keys[i] = (static_cast<uint32_t>(d.mode) << 31) | (glog << 28) | lk;
         P.vals[i] = static_cast<uint32_t>(i);
@@ -392,12 +394,12 @@ struct TaskBuild {
     int32_t big_min;              // linear WFA pairs for the CTA-per-pair kernel (not in the
     uint32_t big_smem;            // main pass, so not in its slot statistics)
     int32_t lane_ckpt;            // lane kernel mode (its scratch need)
-    uint32_t* tile_min;           // [2] first register-tile task of each symbol mode
-    uint32_t* tile_ranges;        // {begin, end} of the register-tile tasks of each mode
+    uint32_t* tile_min;           // [4] first one-warp register-tile task of each symbol mode, first CTA one
+    uint32_t* tile_ranges;        // {begin, end} of each of the four
     unsigned long long* tile_need;   // scratch wanted by the register-tile pairs
 };
 
-__device__ __forceinline__ bool key_tile(uint32_t k) { return ((k >> 28) & 7u) == kTileSeg; }
+__device__ __forceinline__ bool key_tile(uint32_t k) { return ((k >> 28) & 7u) >= kWarpTileSeg; }
 __device__ __forceinline__ int key_group(uint32_t k) { return key_tile(k) ? 32 : 1 << ((k >> 28) & 7); }
 __device__ __forceinline__ uint32_t key_seg(uint32_t k) { return k >> 28; }
 
@@ -432,7 +434,7 @@ __global__ void task_fill_kernel(TaskBuild T) {
     // contribute nothing to them
     const bool has_task = p < T.n && T.flag[p];
     uint64_t need = 0, tile_need = 0;
-    uint32_t t_split = 0xFFFFFFFFu, t_g1 = 0xFFFFFFFFu, t_tile[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
+    uint32_t t_split = 0xFFFFFFFFu, t_g1 = 0xFFFFFFFFu, t_tile = 0xFFFFFFFFu;
     if (has_task) {
         const uint32_t k = T.keys[p];
         const int G = key_group(k);
@@ -456,7 +458,8 @@ __global__ void task_fill_kernel(TaskBuild T) {
                 need += myers_need_est(d.qn, d.tn, G, T.band_base);
             else if (key_tile(k))
                 tile_need = tile_fixed_bytes(d.qn, d.tn) +
-                            tile_align(tile_hist_bytes(d.qn, d.tn, tile_score_est(d.qn, d.mode))) + kTileChunk;
+                            tile_align(tile_hist_bytes(d.qn, d.tn, tile_score_est(d.qn, d.mode))) +
+                            ((k >> 28 & 7u) == kTileSeg ? kTileChunk : kWarpTileChunk);
             else if (!big_pair(T.engine, T.big_min, T.big_smem, d.qn, d.tn, d.mode))
                 region = max(region, wfa_region_est(d.qn, d.tn, T.engine == PHR_ENGINE_WFA_AFFINE));
             ++cnt;
@@ -470,7 +473,7 @@ __global__ void task_fill_kernel(TaskBuild T) {
         T.task_need[t] = need;
         if ((k >> 31) & 1) t_split = t;
         else if (G > 1) t_g1 = t;
-        if (key_tile(k)) t_tile[(k >> 31) & 1] = t;
+        if (key_tile(k)) t_tile = t;
     }
     // one atomic per warp and value instead of one per task (a million tasks would
     // otherwise queue on the same three addresses)
@@ -483,8 +486,10 @@ __global__ void task_fill_kernel(TaskBuild T) {
         uint64_t sum = tile_need;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(PHR_FULL_MASK, sum, o);
-        for (int m = 0; m < 2; ++m) {
-            const uint32_t f = __reduce_min_sync(PHR_FULL_MASK, t_tile[m]);
+        const uint32_t kind = has_task ? key_seg(T.keys[p]) : 0u;   // mode << 3 | segment
+        for (int m = 0; m < 4; ++m) {
+            const bool mine = kind == ((m & 1) << 3 | (m < 2 ? kWarpTileSeg : kTileSeg));
+            const uint32_t f = __reduce_min_sync(PHR_FULL_MASK, mine ? t_tile : 0xFFFFFFFFu);
             if ((threadIdx.x & 31) == 0 && f != 0xFFFFFFFFu) atomicMin(T.tile_min + m, f);
         }
         if ((threadIdx.x & 31) == 0) atomicAdd(T.tile_need, static_cast<unsigned long long>(sum));
@@ -504,15 +509,17 @@ __global__ void task_finalize_kernel(TaskBuild T) {
     uint32_t nt = 0;
     if (T.n > 0) nt = T.tidx[T.n - 1] + T.flag[T.n - 1];
     const uint32_t split = min(*T.split_min, nt);
-    const uint32_t b0 = min(T.tile_min[0], split), b1 = min(T.tile_min[1], nt);
-    T.ranges[0] = 0;
-    T.ranges[1] = b0;
-    T.ranges[2] = split;
-    T.ranges[3] = b1;
-    T.tile_ranges[0] = b0;
-    T.tile_ranges[1] = split;
-    T.tile_ranges[2] = b1;
-    T.tile_ranges[3] = nt;
+    // segments of each mode in key order: warp groups, one-warp tiles, CTA tiles
+    for (int m = 0; m < 2; ++m) {
+        const uint32_t begin = m ? split : 0, end = m ? nt : split;
+        const uint32_t cta = min(T.tile_min[2 + m], end), warp = min(T.tile_min[m], cta);
+        T.ranges[2 * m] = begin;
+        T.ranges[2 * m + 1] = warp;
+        T.tile_ranges[2 * m] = warp;
+        T.tile_ranges[2 * m + 1] = cta;
+        T.tile_ranges[4 + 2 * m] = cta;
+        T.tile_ranges[4 + 2 * m + 1] = end;
+    }
     // lane-kernel range {0, g1} and warp-group 2-bit range {g1, split} (global Myers)
     const uint32_t g1 = min(*T.g1_min, split);
     T.ranges[28] = 0;
@@ -542,7 +549,9 @@ __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* red
     task_first[t] = t;
     task_count[t] = 1;
     task_group[t] = static_cast<uint8_t>(G);
-    if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode) || tile_pair(engine, big_min, d.qn, d.tn)) task_group[t] = kBigTask | 32;
+    const int tw = tile_warps(engine, big_min, wfa_long_min, d.qn, d.tn, d.mode);
+    if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode) || tw > 1) task_group[t] = kBigTask | 32;
+    else if (tw == 1) task_group[t] = kWarpTileTask | 32;
 }
 
 struct FinishParams {
@@ -558,6 +567,7 @@ struct FinishParams {
     uint64_t cigar_capacity;
     uint32_t* error_flag;
     uint64_t cigar_base;
+    int per_warp;            // pairs a warp writes (1..32)
 };
 
 __global__ void text_len_kernel(const PairOut* out, uint64_t n, uint64_t* len) {
@@ -567,18 +577,47 @@ __global__ void text_len_kernel(const PairOut* out, uint64_t n, uint64_t* len) {
     len[i] = (o.status == PHR_OK) ? o.text_len : 0;
 }
 
-// Packs CIGAR text and writes the phr_alignment records. One warp per 32 consecutive
-// pairs: lane l writes pair first + l's record (the warp's records are contiguous), then
-// the lanes copy the pairs' texts one pair after the other.
+// Copies len bytes with one warp: words at the destination's 4-byte boundaries, funnelled
+// from the source's, single bytes at both ends (and for short texts). Reads stay within the
+// source's aligned words.
+__device__ __forceinline__ void copy_text(char* dst, const char* src, uint32_t len, int lane) {
+    if (len < 96) {
+        for (uint32_t c = lane; c < len; c += 32) dst[c] = src[c];
+        return;
+    }
+    const uint32_t head = static_cast<uint32_t>(-reinterpret_cast<intptr_t>(dst)) & 3u;
+    if (static_cast<uint32_t>(lane) < head) dst[lane] = src[lane];
+    const char* s = src + head;
+    uint32_t* d = reinterpret_cast<uint32_t*>(dst + head);
+    const uint32_t words = (len - head) / 4;
+    const uint32_t sh = (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s)) & 3u) * 8;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s) & ~static_cast<uintptr_t>(3));
+    if (sh == 0) {
+#pragma unroll 4
+        for (uint32_t i = lane; i < words; i += 32) d[i] = w[i];
+    } else {
+#pragma unroll 4
+        for (uint32_t i = lane; i < words; i += 32) d[i] = __funnelshift_r(w[i], w[i + 1], sh);
+    }
+    const uint32_t done = head + 4 * words;
+    if (done + lane < len) dst[done + lane] = src[done + lane];
+}
+
+// Packs CIGAR text and writes the phr_alignment records. One warp per F.per_warp
+// consecutive pairs: lane l writes pair first + l's record (the warp's records are
+// contiguous), then the lanes copy the pairs' texts one pair after the other. 32 pairs per
+// warp in a large batch; fewer when there are few pairs, whose texts then are copied side
+// by side (500 texts of ~3 kB: 0.60 ms with 32 per warp and byte copies, below 0.01 ms now).
 __global__ void finish_kernel(FinishParams F) {
-    const uint64_t first = ((blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5) * 32;
+    const uint64_t first =
+        ((blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5) * static_cast<uint64_t>(F.per_warp);
     const int lane = threadIdx.x & 31;
     if (first >= F.n) return;
     const uint64_t i = first + lane;
     uint64_t off = 0, toff = 0;
     uint32_t len = 0;
     bool copy = false;
-    if (i < F.n) {
+    if (lane < F.per_warp && i < F.n) {
         const PairOut o = F.out[i];
         if (o.status == -1) {
             atomicOr(F.error_flag, 8u);
@@ -617,7 +656,7 @@ __global__ void finish_kernel(FinishParams F) {
         const uint32_t lj = __shfl_sync(PHR_FULL_MASK, len, j);
         const uint64_t oj = __shfl_sync(PHR_FULL_MASK, off, j);
         const uint64_t tj = __shfl_sync(PHR_FULL_MASK, toff, j);
-        for (uint32_t c = lane; c < lj; c += 32) F.cigar[oj + c] = F.text[tj + c];
+        copy_text(F.cigar + oj, F.text + tj, lj, lane);
     }
 }
 
@@ -732,8 +771,9 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // [7] redo count, [8..9] need max (u64), [10] error flag, [12..13] total (u64), [14..17] redo ranges,
     // [20] first multi-lane 2-bit task, [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
     // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64),
-    // [40..41] first register-tile task of each mode, [42..45] register-tile ranges, [46..47] their
-    // scratch need (u64), [48..49] pool bytes taken (u64)
+    // [40..43] first register-tile task of each kind (one warp 2-bit / bytes, CTA 2-bit / bytes),
+    // [44..51] their ranges, [52..53] their scratch need (u64), [54..55] pool bytes taken (u64),
+    // [56..59] their queue heads
     uint32_t* cnt = static_cast<uint32_t*>(take(256));
     if (!cnt) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted");
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
@@ -741,7 +781,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 256, st));
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 4, 0xFF, 4, st));
     PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 20, 0xFF, 4, st));
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 40, 0xFF, 8, st));
+    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 40, 0xFF, 16, st));
 
     // CUB temp sizes
     size_t t_sort = 0, t_scan = 0, t_max = 0;
@@ -783,7 +823,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     TaskBuild tbp{keys_s, order, n, head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4, cnt + 20, desc,
                   engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
                   ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt,
-                  cnt + 40, cnt + 42, reinterpret_cast<unsigned long long*>(cnt + 46)};
+                  cnt + 40, cnt + 44, reinterpret_cast<unsigned long long*>(cnt + 52)};
     {
         KernelScope ks(ctx, "task_head");
         task_head_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
@@ -811,7 +851,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // are deferred to the redo passes, which size scratch per task.
     uint64_t h_need = 0;
     unsigned int h_hist[64];
-    uint32_t h_cnt[48];   // the counter block up to the register-tile need
+    uint32_t h_cnt[54];   // the counter block up to the register-tile need
     const uint32_t* h_ranges = h_cnt;
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_need, need_max, 8, cudaMemcpyDeviceToHost, st));
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_hist, need_hist, sizeof(h_hist), cudaMemcpyDeviceToHost, st));
@@ -819,9 +859,10 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     PHR_CUDA_TRY(ctx, cudaGetLastError());
     hs_setup.stop();
-    const uint32_t n_tile[2] = {h_cnt[43] - h_cnt[42], h_cnt[45] - h_cnt[44]};
+    uint32_t n_tile[4], n_tiles = 0;
+    for (int i = 0; i < 4; ++i) n_tiles += n_tile[i] = h_cnt[45 + 2 * i] - h_cnt[44 + 2 * i];
     uint64_t tile_need = 0;
-    std::memcpy(&tile_need, h_cnt + 46, 8);
+    std::memcpy(&tile_need, h_cnt + 52, 8);
     {
         uint64_t n_tasks = 0;  // tasks of the main pass with a scratch need
         for (int b = 0; b < 64; ++b) n_tasks += h_hist[b];
@@ -881,7 +922,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             // the register-tile pairs run after the group kernels and reuse the buffer from
             // its start; a small batch gets room for pairs of any divergence
             pool = 0;
-            if (n_tile[0] + n_tile[1] > 0)
+            if (n_tiles > 0)
                 pool = std::min<uint64_t>(std::max<uint64_t>(tile_need, std::min<uint64_t>(16 * tile_need, 1ull << 30)),
                                           ctx->scratch_budget);
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
@@ -941,20 +982,28 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             else
                 launch_wfa_affine_bytes(P, static_cast<int>(grid), block, st);
         }
-        if (engine == PHR_ENGINE_WFA_LINEAR && P.big_min > 0 && (per_task ? n_tasks_hint : n_tile[0] + n_tile[1]) > 0) {
-            // long pairs in register tiles, one CTA each: two CTAs per SM (one when the tune
-            // keeps fewer blocks resident)
-            const uint64_t per_sm = ctx->tune.max_blocks_per_sm >= 4 ? 2 : 1;
-            PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 24, 0, 8, st));
-            if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 48, 0, 8, st));
-            const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 48), pool, kTileChunk};
-            for (int mode = 0; mode < 2; ++mode) {
-                const uint64_t nt = per_task ? n_tasks_hint : n_tile[mode];
+        if (engine == PHR_ENGINE_WFA_LINEAR && P.big_min > 0 && (per_task ? n_tasks_hint : n_tiles) > 0) {
+            // register tiles: long pairs one CTA each (one per SM), the others a warp each
+            PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 56, 0, 16, st));
+            if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 54, 0, 8, st));
+            static const char* const tile_names[4] = {"wfa_linear_tile", "wfa_linear_tile_bytes", "wfa_linear_big",
+                                                      "wfa_linear_big_bytes"};
+            for (int i = 3; i >= 0; --i) {   // the longest first
+                const uint64_t nt = per_task ? n_tasks_hint : n_tile[i];
                 if (nt == 0) continue;
-                P.tasks.range = per_task ? (mode ? range1 : range0) : cnt + 42 + 2 * mode;
-                P.queue_head = cnt + 24 + mode;
-                KernelScope ks(ctx, mode ? "wfa_linear_big_bytes" : "wfa_linear_big");
-                launch_wfa_linear_big(P, tl, static_cast<int>(std::min<uint64_t>(nt, ctx->sm_count * per_sm)), mode, st);
+                const bool cta = i >= 2;
+                const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 54), pool,
+                                    cta ? kTileChunk : kWarpTileChunk};
+                const uint64_t most = static_cast<uint64_t>(ctx->sm_count) *
+                                      (cta ? 1 : std::min(ctx->tune.max_blocks_per_sm, 2));
+                const uint64_t ctas = cta ? nt : (nt + kWarpTileThreads / 32 - 1) / (kWarpTileThreads / 32);
+                P.tasks.range = per_task ? ((i & 1) ? range1 : range0) : cnt + 44 + 2 * i;
+                P.queue_head = cnt + 56 + i;
+                KernelScope ks(ctx, tile_names[i]);
+                if (cta)
+                    launch_wfa_linear_big(P, tl, static_cast<int>(std::min(ctas, most)), i & 1, st);
+                else
+                    launch_wfa_linear_tile(P, tl, static_cast<int>(std::min(ctas, most)), i & 1, st);
             }
         }
         if (per_task && engine == PHR_ENGINE_WFA_AFFINE && P.big_min > 0 && n_tasks_hint > 0) {
@@ -1117,10 +1166,12 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     if (h_total > res->cigar_capacity)
         return set_error(ctx, PHR_ERR_CAPACITY, "CIGAR arena too small: need " + std::to_string(h_total) + " bytes");
     FinishParams F{n,           engine,     desc,       pout,    tbo, text, cigoff, res->aln, res->cigar,
-                   res->cigar_capacity, cnt + 10, res->cigar_base};
+                   res->cigar_capacity, cnt + 10, res->cigar_base, 32};
+    // at least 16 warps per SM before a warp takes more than one pair
+    while (F.per_warp > 1 && (n + F.per_warp - 1) / F.per_warp < 16ull * ctx->sm_count) F.per_warp /= 2;
     {
         KernelScope ks(ctx, "finish");
-        finish_kernel<<<blocks_for((n + 31) / 32 * 32, T), T, 0, st>>>(F);
+        finish_kernel<<<blocks_for((n + F.per_warp - 1) / F.per_warp * 32, T), T, 0, st>>>(F);
     }
     uint32_t h_err = 0;
     unsigned long long h_work[4] = {0, 0, 0, 0};

@@ -47,8 +47,9 @@ struct ExtendParams {
                                 // or every column's records (0)
 };
 
-// task_group bit marking a redo task for the CTA-per-pair kernel
+// task_group bits marking a redo task for a CTA-per-pair kernel / the one-warp register tiles
 constexpr uint8_t kBigTask = 0x80;
+constexpr uint8_t kWarpTileTask = 0x40;
 constexpr int kBigThreads = 512;         // threads of the linear CTA-per-pair kernel (two CTAs per SM)
 // most threads per CTA of the gap-affine CTA-per-pair kernel, and its default (one CTA
 // per SM; the "wfa_affine_big_threads" setting launches 512 or 256, two or four per SM)
@@ -195,14 +196,17 @@ __host__ __device__ __forceinline__ uint64_t tile_hist_bytes(int qn, int tn, int
     (void)qn;
     (void)tn;
     const uint64_t u = static_cast<uint64_t>(s) / kTileSteps + 1;
-    return u * 6144 + 54 * u * (u + 1);
+    return u * 3200 + 54 * u * (u + 1);
 }
 // Score a pair is given room for at first: a quarter of the query for DNA, half for bytes
 // (protein). Records come from a pool, so one pair may take more.
 __host__ __device__ __forceinline__ int64_t tile_score_est(int qn, int mode) {
     return 64 + static_cast<int64_t>(qn) / (mode == 0 ? 4 : 2);
 }
-constexpr uint32_t kTileChunk = 64 << 10;   // bytes a team takes from the pool at a time
+constexpr uint32_t kTileChunk = 64 << 10;   // bytes a CTA takes from the pool at a time
+constexpr uint32_t kWarpTileChunk = 16 << 10;   // the same for a one-warp team
+constexpr int kWarpTileThreads = 256;           // threads per CTA of the one-warp teams' kernel
+constexpr uint32_t kWarpTileSmem = 12 << 10;    // shared memory of a one-warp team
 
 // The pool of a main-pass launch: bytes [0, pool_end) of the scratch buffer, taken by
 // atomicAdd on pool_used. pool_used NULL (redo passes): every pair has its own region.
@@ -212,11 +216,19 @@ struct TileLaunch {
     uint32_t chunk;
 };
 
-// Pairs the register-tile kernel takes: long linear pairs. Offsets are kept times 256 in 32
-// bits, hence the upper limit; longer queries stay in the warp-group kernel.
-__host__ __device__ __forceinline__ bool tile_pair(int32_t engine, int32_t big_min, int qn, int tn) {
-    return big_min > 0 && engine == PHR_ENGINE_WFA_LINEAR && static_cast<int64_t>(qn) + tn >= big_min &&
-           qn < (1 << 22) && tn < (1 << 28);
+// How many warps a linear pair's register tiles get: 0 (the warp-group kernel), 1, or
+// kBigThreads / 32 (one CTA, long pairs). One warp: pairs from long_min on, and byte pairs
+// (protein, which mostly differ a lot) from kWarpTileBytesMin on, where the warp-group
+// kernel's frames in global memory cost more than a warp per pair: 5,000 protein pairs of
+// 200-800 at 30 % measured 1.9 + 1.6 ms (two passes) before and 0.96 ms now. Offsets are kept times 256 in 32 bits, hence the upper
+// limit; longer queries stay in the warp-group kernel.
+constexpr int kWarpTileBytesMin = 128;
+__host__ __device__ __forceinline__ int tile_warps(int32_t engine, int32_t big_min, int32_t long_min, int qn, int tn,
+                                                   int mode) {
+    const int64_t len = static_cast<int64_t>(qn) + tn;
+    if (big_min <= 0 || engine != PHR_ENGINE_WFA_LINEAR || qn >= (1 << 22) || tn >= (1 << 28)) return 0;
+    if (len >= big_min) return kBigThreads / 32;
+    return len >= (mode == 0 ? long_min : kWarpTileBytesMin) ? 1 : 0;
 }
 
 void launch_myers(const ExtendParams& p, int grid, int block, cudaStream_t st);
@@ -227,6 +239,7 @@ constexpr int kLaneThreads = 256;
 void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st);
 
 }  // namespace phr

@@ -1468,7 +1468,7 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
         uint8_t* slot = P.task_off ? P.scratch + P.task_off[task] : P.scratch + warp_global * P.slot_bytes;
         const uint64_t slot_bytes = P.task_off ? P.task_len[task] : P.slot_bytes;
         const uint8_t tg = P.tasks.task_group[task];
-        if (tg & kBigTask) continue;  // a redo task of a CTA-per-pair kernel
+        if (tg & (kBigTask | kWarpTileTask)) continue;  // a redo task of another kernel
         const int G = tg;
         const int count = P.tasks.task_count[task];
         const int grp = lane / G;

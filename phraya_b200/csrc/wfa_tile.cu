@@ -175,7 +175,12 @@ template <int W>
 __device__ __forceinline__ int tile_regs(int s_hi, int qn, int tn) {
     const int width = min(s_hi, qn) + min(s_hi, tn) + 1;
     if constexpr (W == 1) {
-        return width <= tile_use(1) ? 1 : width <= tile_use(2) ? 2 : width <= tile_use(4) ? 4 : 8;
+        // one warp does a block's tiles one after the other: the fewest diagonals computed
+        // (tiles grow to both sides of diagonal 0: five of R = 4 beat three of R = 8)
+        return width <= tile_use(1) ? 1
+               : width <= tile_use(2) ? 2
+               : width <= tile_use(4) ? 4
+               : width <= tile_use(8) || width > 5 * tile_use(4) ? 8 : 4;
     } else {
         return width <= kTeamTiles * tile_use(1) ? 1
                : width <= kTeamTiles * tile_use(2) ? 2
@@ -789,7 +794,7 @@ __device__ __forceinline__ void tile_team(const ExtendParams& P, const TileLaunc
         const uint32_t task = sh->task;
         team_sync<W>();
         if (task >= P.tasks.range[1]) break;
-        if (P.task_off && !(P.tasks.task_group[task] & kBigTask)) continue;
+        if (P.task_off && !(P.tasks.task_group[task] & (W == 1 ? kWarpTileTask : kBigTask))) continue;
         const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
         const PairDesc d = P.desc[pid];
         if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
@@ -848,7 +853,24 @@ __global__ void __launch_bounds__(kBigThreads, 1) wfa_linear_big_kernel(ExtendPa
     tile_team<S, kBigThreads / 32>(P, A, 0, P.big_smem);
 }
 
+// One warp per pair: kWarpTileThreads / 32 teams per CTA, two CTAs per SM.
+template <class S>
+__global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_linear_tile_kernel(ExtendParams P, TileLaunch A) {
+    tile_team<S, 1>(P, A, (threadIdx.x >> 5) * kWarpTileSmem, kWarpTileSmem);
+}
+
 }  // namespace
+
+void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
+    constexpr int smem = kWarpTileThreads / 32 * static_cast<int>(kWarpTileSmem);
+    if (mode == 0) {
+        cudaFuncSetAttribute(wfa_linear_tile_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        wfa_linear_tile_kernel<Seq2><<<grid, kWarpTileThreads, smem, st>>>(p, a);
+    } else {
+        cudaFuncSetAttribute(wfa_linear_tile_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        wfa_linear_tile_kernel<SeqB><<<grid, kWarpTileThreads, smem, st>>>(p, a);
+    }
+}
 
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
     if (mode == 0) {

@@ -51,19 +51,22 @@ def edge_pairs(rng, alphabet):
 
 
 @pytest.mark.parametrize("alphabet", [DNA, AA], ids=["2bit", "bytes"])
-@pytest.mark.parametrize("smem", [16 << 10, 100 << 10])
-def test_tile_edges(alphabet, smem):
+@pytest.mark.parametrize("tune", [{"wfa_big_min": 32, "wfa_big_smem": 16 << 10}, {"wfa_big_min": 32},
+                                  {"wfa_big_min": 1 << 20, "wfa_long_min": 32}], ids=["cta16k", "cta", "warp"])
+def test_tile_edges(alphabet, tune):
+    """Every pair on one CTA (with and without room for its frames), or one warp."""
     rng = np.random.default_rng(41)
     pairs = edge_pairs(rng, alphabet)
     with P.Engine(0) as eng:
-        eng.set_tune("wfa_big_min", 32)
-        eng.set_tune("wfa_big_smem", smem)
+        for key, value in tune.items():
+            eng.set_tune(key, value)
         got = eng.extend(A.ENGINE_WFA_LINEAR, pairs)
     assert got == O.extend(A.ENGINE_WFA_LINEAR, pairs)
 
 
 @pytest.mark.parametrize("alphabet", [DNA, AA], ids=["2bit", "bytes"])
-def test_bands_beyond_shared_memory(alphabet):
+@pytest.mark.parametrize("big_min", [4096, 1 << 20], ids=["cta", "warp"])
+def test_bands_beyond_shared_memory(alphabet, big_min):
     """Unrelated pairs: wavefronts of thousands of diagonals, frames in global memory."""
     rng = np.random.default_rng(42)
     pairs = [(rand(rng, n, alphabet), rand(rng, m, alphabet)) for n, m in ((3000, 3100), (2500, 2900), (2100, 2000))]
@@ -71,6 +74,7 @@ def test_bands_beyond_shared_memory(alphabet):
     pairs += [(q, mutate(rng, q, 0.1, alphabet)), (q[:5000], mutate(rng, q, 0.03, alphabet))]
     with P.Engine(0) as eng:
         eng.set_tune("wfa_big_smem", 24 << 10)
+        eng.set_tune("wfa_big_min", big_min)
         got = eng.extend(A.ENGINE_WFA_LINEAR, pairs)
     assert got == O.extend(A.ENGINE_WFA_LINEAR, pairs)
 
