@@ -364,7 +364,7 @@ __global__ void pack_kernel(PackParams P) {
             len = static_cast<uint32_t>(d.qn + d.tn);
         }
         // register-tile pairs form segments of their own after the warp-group ones
-        const int tw = tile_warps(P.engine, P.big_min, P.wfa_long_min, d.qn, d.tn, d.mode);
+        const int tw = tile_warps(P.engine, aff_tile_open(P.costs), P.big_min, P.wfa_long_min, d.qn, d.tn, d.mode);
         const uint32_t glog = tw == 0 ? static_cast<uint32_t>(__ffs(G) - 1) : tw == 1 ? kWarpTileSeg : kTileSeg;
         const uint32_t lk = 0x0FFFFFFFu - min(len, 0x0FFFFFFFu);  // longest first within a bucket
         P.keys[i] = (static_cast<uint32_t>(d.mode) << 31) | (glog << 28) | lk;
@@ -396,7 +396,7 @@ struct TaskBuild {
     int32_t lane_ckpt;            // lane kernel mode (its scratch need)
     uint32_t* tile_min;           // [4] first one-warp register-tile task of each symbol mode, first CTA one
     uint32_t* tile_ranges;        // {begin, end} of each of the four
-    unsigned long long* tile_need;   // scratch wanted by the register-tile pairs
+    unsigned long long* tile_need;   // scratch wanted by the register-tile pairs: sum, largest
 };
 
 __device__ __forceinline__ bool key_tile(uint32_t k) { return ((k >> 28) & 7u) >= kWarpTileSeg; }
@@ -457,9 +457,10 @@ __global__ void task_fill_kernel(TaskBuild T) {
             } else if (T.engine == PHR_ENGINE_MYERS_FIT || T.engine == PHR_ENGINE_MYERS_GLOBAL)
                 need += myers_need_est(d.qn, d.tn, G, T.band_base);
             else if (key_tile(k))
-                tile_need = tile_fixed_bytes(d.qn, d.tn) +
-                            tile_align(tile_hist_bytes(d.qn, d.tn, tile_score_est(d.qn, d.mode))) +
-                            ((k >> 28 & 7u) == kTileSeg ? kTileChunk : kWarpTileChunk);
+                tile_need = T.engine == PHR_ENGINE_WFA_AFFINE
+                                ? aff_tile_fixed_bytes(d.qn, d.tn) +
+                                      tile_align(aff_tile_hist_bytes(tile_score_est(d.qn, d.mode)))
+                                : tile_fixed_bytes(d.qn, d.tn) + tile_align(tile_hist_bytes(tile_score_est(d.qn, d.mode)));
             else if (!big_pair(T.engine, T.big_min, T.big_smem, d.qn, d.tn, d.mode))
                 region = max(region, wfa_region_est(d.qn, d.tn, T.engine == PHR_ENGINE_WFA_AFFINE));
             ++cnt;
@@ -492,7 +493,13 @@ __global__ void task_fill_kernel(TaskBuild T) {
             const uint32_t f = __reduce_min_sync(PHR_FULL_MASK, mine ? t_tile : 0xFFFFFFFFu);
             if ((threadIdx.x & 31) == 0 && f != 0xFFFFFFFFu) atomicMin(T.tile_min + m, f);
         }
-        if ((threadIdx.x & 31) == 0) atomicAdd(T.tile_need, static_cast<unsigned long long>(sum));
+        uint64_t most = tile_need;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(PHR_FULL_MASK, most, o));
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(T.tile_need, static_cast<unsigned long long>(sum));
+            atomicMax(T.tile_need + 1, static_cast<unsigned long long>(most));
+        }
     }
     const int bucket = need ? 64 - __clzll(need) : 64;   // 64: no histogram entry
     const uint32_t same = __match_any_sync(PHR_FULL_MASK, bucket);
@@ -530,7 +537,7 @@ __global__ void task_finalize_kernel(TaskBuild T) {
 
 // Redo pass task list: one pair per task, in redo order.
 __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* redo_count, const PairDesc* desc,
-                                  int32_t engine, int wfa_g_short, int wfa_g_long, int wfa_long_min, int32_t big_min,
+                                  int32_t engine, int aff_open, int wfa_g_short, int wfa_g_long, int wfa_long_min, int32_t big_min,
                                   uint32_t big_smem, uint32_t* task_first, uint8_t* task_count,
                                   uint8_t* task_group, uint32_t* ranges) {
     const uint32_t n = *redo_count;
@@ -549,9 +556,10 @@ __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* red
     task_first[t] = t;
     task_count[t] = 1;
     task_group[t] = static_cast<uint8_t>(G);
-    const int tw = tile_warps(engine, big_min, wfa_long_min, d.qn, d.tn, d.mode);
-    if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode) || tw > 1) task_group[t] = kBigTask | 32;
+    const int tw = tile_warps(engine, aff_open, big_min, wfa_long_min, d.qn, d.tn, d.mode);
+    if (tw > 1) task_group[t] = kCtaTileTask | 32;
     else if (tw == 1) task_group[t] = kWarpTileTask | 32;
+    else if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode)) task_group[t] = kBigTask | 32;
 }
 
 struct FinishParams {
@@ -772,8 +780,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // [20] first multi-lane 2-bit task, [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
     // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64),
     // [40..43] first register-tile task of each kind (one warp 2-bit / bytes, CTA 2-bit / bytes),
-    // [44..51] their ranges, [52..53] their scratch need (u64), [54..55] pool bytes taken (u64),
-    // [56..59] their queue heads
+    // [44..51] their ranges, [52..55] their scratch need: sum, largest (u64), [56..59] their queue
+    // heads, [60..61] pool bytes taken (u64)
     uint32_t* cnt = static_cast<uint32_t*>(take(256));
     if (!cnt) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted");
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
@@ -851,7 +859,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // are deferred to the redo passes, which size scratch per task.
     uint64_t h_need = 0;
     unsigned int h_hist[64];
-    uint32_t h_cnt[54];   // the counter block up to the register-tile need
+    uint32_t h_cnt[56];   // the counter block up to the register-tile need
     const uint32_t* h_ranges = h_cnt;
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_need, need_max, 8, cudaMemcpyDeviceToHost, st));
     PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_hist, need_hist, sizeof(h_hist), cudaMemcpyDeviceToHost, st));
@@ -861,8 +869,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     hs_setup.stop();
     uint32_t n_tile[4], n_tiles = 0;
     for (int i = 0; i < 4; ++i) n_tiles += n_tile[i] = h_cnt[45 + 2 * i] - h_cnt[44 + 2 * i];
-    uint64_t tile_need = 0;
-    std::memcpy(&tile_need, h_cnt + 52, 8);
+    uint64_t tile_need[2];   // sum, largest
+    std::memcpy(tile_need, h_cnt + 52, 16);
     {
         uint64_t n_tasks = 0;  // tasks of the main pass with a scratch need
         for (int b = 0; b < 64; ++b) n_tasks += h_hist[b];
@@ -919,12 +927,16 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             // grid: resident blocks per SM, no more warps than tasks, shrunk to the scratch budget
             grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (h_ranges[3] + warps_per_block - 1) / warps_per_block));
             while (grid > 1 && grid * warps_per_block * slot > ctx->scratch_budget) grid = (grid + 1) / 2;
-            // the register-tile pairs run after the group kernels and reuse the buffer from
-            // its start; a small batch gets room for pairs of any divergence
+            // The register-tile pairs run after the group kernels and reuse the buffer from its
+            // start. Teams keep their chunks from pair to pair and chunks grow by doubling:
+            // twice what the pairs in flight want; a small batch gets room for any divergence.
             pool = 0;
-            if (n_tiles > 0)
-                pool = std::min<uint64_t>(std::max<uint64_t>(tile_need, std::min<uint64_t>(16 * tile_need, 1ull << 30)),
-                                          ctx->scratch_budget);
+            if (n_tiles > 0) {
+                const uint64_t teams = n_tile[0] + n_tile[1] > 0 ? 16ull * ctx->sm_count : ctx->sm_count;
+                pool = std::min<uint64_t>(2 * tile_need[0], 2 * teams * tile_need[1]);
+                pool = std::max<uint64_t>(pool, std::min<uint64_t>(16 * tile_need[0], 1ull << 30)) + (1 << 20);
+                pool = std::min<uint64_t>(pool, ctx->scratch_budget);
+            }
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
         } else {
             grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (n_tasks_hint + warps_per_block - 1) / warps_per_block));
@@ -982,33 +994,38 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             else
                 launch_wfa_affine_bytes(P, static_cast<int>(grid), block, st);
         }
-        if (engine == PHR_ENGINE_WFA_LINEAR && P.big_min > 0 && (per_task ? n_tasks_hint : n_tiles) > 0) {
+        const bool tiles = engine == PHR_ENGINE_WFA_LINEAR ||
+                           (engine == PHR_ENGINE_WFA_AFFINE && aff_tile_open(costs) != 0);
+        if (tiles && P.big_min > 0 && (per_task ? n_tasks_hint : n_tiles) > 0) {
             // register tiles: long pairs one CTA each (one per SM), the others a warp each
             PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 56, 0, 16, st));
-            if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 54, 0, 8, st));
-            static const char* const tile_names[4] = {"wfa_linear_tile", "wfa_linear_tile_bytes", "wfa_linear_big",
-                                                      "wfa_linear_big_bytes"};
+            static const char* const tile_names[2][4] = {
+                {"wfa_linear_tile", "wfa_linear_tile_bytes", "wfa_linear_big", "wfa_linear_big_bytes"},
+                {"wfa_affine_tile", "wfa_affine_tile_bytes", "wfa_affine_big", "wfa_affine_big_bytes"}};
+            const bool affine = engine == PHR_ENGINE_WFA_AFFINE;
             for (int i = 3; i >= 0; --i) {   // the longest first
                 const uint64_t nt = per_task ? n_tasks_hint : n_tile[i];
                 if (nt == 0) continue;
                 const bool cta = i >= 2;
-                const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 54), pool,
+                if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 60, 0, 8, st));
+                const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 60), pool,
                                     cta ? kTileChunk : kWarpTileChunk};
                 const uint64_t most = static_cast<uint64_t>(ctx->sm_count) *
                                       (cta ? 1 : std::min(ctx->tune.max_blocks_per_sm, 2));
                 const uint64_t ctas = cta ? nt : (nt + kWarpTileThreads / 32 - 1) / (kWarpTileThreads / 32);
                 P.tasks.range = per_task ? ((i & 1) ? range1 : range0) : cnt + 44 + 2 * i;
                 P.queue_head = cnt + 56 + i;
-                KernelScope ks(ctx, tile_names[i]);
-                if (cta)
-                    launch_wfa_linear_big(P, tl, static_cast<int>(std::min(ctas, most)), i & 1, st);
+                const int tile_grid = static_cast<int>(std::min(ctas, most));
+                KernelScope ks(ctx, tile_names[affine][i]);
+                if (affine)
+                    (cta ? launch_wfa_affine_cta_tiles : launch_wfa_affine_warp_tiles)(P, tl, tile_grid, i & 1, st);
                 else
-                    launch_wfa_linear_tile(P, tl, static_cast<int>(std::min(ctas, most)), i & 1, st);
+                    (cta ? launch_wfa_linear_big : launch_wfa_linear_tile)(P, tl, tile_grid, i & 1, st);
             }
         }
         if (per_task && engine == PHR_ENGINE_WFA_AFFINE && P.big_min > 0 && n_tasks_hint > 0) {
-            // long gap-affine pairs of this redo list, one CTA each: kBigAffineThreads /
-            // wfa_affine_big_threads CTAs per SM
+            // long gap-affine pairs the register tiles do not take, one CTA each:
+            // kBigAffineThreads / wfa_affine_big_threads CTAs per SM
             const int aff_threads = ctx->tune.wfa_affine_big_threads;
             const int big_grid = static_cast<int>(std::min<uint64_t>(
                 n_tasks_hint, ctx->sm_count * static_cast<uint64_t>(kBigAffineThreads / aff_threads)));
@@ -1110,7 +1127,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             {
                 KernelScope ks(ctx, "redo_tasks");
                 redo_tasks_kernel<<<blocks_for(m, T), T, 0, st>>>(rlist2, cnt + 18, desc, engine,
-                                                                 g_short, ctx->tune.wfa_group_long,
+                                                                 aff_tile_open(costs), g_short, ctx->tune.wfa_group_long,
                                                                  ctx->tune.wfa_long_min,
                                                                  P.big_min, P.big_smem, task_first, task_count,
                                                                  task_group, cnt + 14);

@@ -47,9 +47,12 @@ struct ExtendParams {
                                 // or every column's records (0)
 };
 
-// task_group bits marking a redo task for a CTA-per-pair kernel / the one-warp register tiles
+// task_group values marking a redo task for wfa.cu's CTA-per-pair kernel, the register tiles
+// of one CTA and those of one warp (added to the lanes per pair, at most 32)
 constexpr uint8_t kBigTask = 0x80;
+constexpr uint8_t kCtaTileTask = 0xC0;
 constexpr uint8_t kWarpTileTask = 0x40;
+constexpr uint8_t kOtherKernel = 0xC0;   // mask of the three
 constexpr int kBigThreads = 512;         // threads of the linear CTA-per-pair kernel (two CTAs per SM)
 // most threads per CTA of the gap-affine CTA-per-pair kernel, and its default (one CTA
 // per SM; the "wfa_affine_big_threads" setting launches 512 or 256, two or four per SM)
@@ -67,7 +70,7 @@ __host__ __device__ __forceinline__ uint64_t big_seq_words(int qn, int tn, int m
 }
 
 // A gap-affine WFA pair long enough that one warp would be latency-bound on it: it runs
-// one per CTA (linear pairs: tile_pair below).
+// one per CTA of wfa.cu's kernel unless the register tiles take it (tile_warps below).
 __host__ __device__ __forceinline__ bool big_pair(int32_t engine, int32_t big_min, uint32_t big_smem, int qn, int tn,
                                                   int mode) {
     (void)big_smem;
@@ -176,7 +179,7 @@ __host__ __device__ __forceinline__ uint64_t myers_full_need(int m, int n) {
 constexpr int kTileSteps = 8;                                  // scores a tile advances between barriers
 constexpr int kTileRegs = 8;                                   // most diagonals per lane
 constexpr int kTileMax = 32 * kTileRegs;                       // most diagonals of a tile
-constexpr uint32_t kTileCtlBytes = 128;                         // a team's control block in shared memory
+constexpr uint32_t kTileCtlBytes = 768;                         // a team's control block in shared memory
 
 __host__ __device__ __forceinline__ uint64_t tile_align(uint64_t v) { return (v + 255) & ~255ull; }
 __host__ __device__ __forceinline__ uint64_t tile_runs_bytes(int qn, int tn) {
@@ -185,25 +188,48 @@ __host__ __device__ __forceinline__ uint64_t tile_runs_bytes(int qn, int tn) {
 __host__ __device__ __forceinline__ uint64_t tile_table_bytes(int qn, int tn) {
     return tile_align(4 * ((static_cast<uint64_t>(qn) + tn) / kTileSteps + 3));
 }
-// What a pair takes before its first record: match runs, CIGAR runs and three tables.
+// What a pair takes before its first record: edits, CIGAR runs and two tables.
 __host__ __device__ __forceinline__ uint64_t tile_fixed_bytes(int qn, int tn) {
-    return 2 * tile_runs_bytes(qn, tn) + 3 * tile_table_bytes(qn, tn);
+    return 2 * tile_runs_bytes(qn, tn) + 2 * tile_table_bytes(qn, tn);
 }
 // Upper bound of the records of scores up to s: block u holds 16 (u + 1) diagonals of 4
 // bytes of value and at most 8 / 3 of ops, plus rounding to tiles and the narrow tiles of
 // small bands.
-__host__ __device__ __forceinline__ uint64_t tile_hist_bytes(int qn, int tn, int64_t s) {
-    (void)qn;
-    (void)tn;
+__host__ __device__ __forceinline__ uint64_t tile_hist_bytes(int64_t s) {
     const uint64_t u = static_cast<uint64_t>(s) / kTileSteps + 1;
     return u * 3200 + 54 * u * (u + 1);
 }
+// The gap-affine tiles' counterparts. Steps are scores over g = gcd of the costs; an edit
+// costs at least one, a mismatch two.
+__host__ __device__ __forceinline__ uint64_t aff_tile_steps(int qn, int tn) {
+    return 2 * (static_cast<uint64_t>(qn) + tn) + 16;
+}
+__host__ __device__ __forceinline__ uint64_t aff_tile_table_bytes(int qn, int tn) {
+    return tile_align(4 * (aff_tile_steps(qn, tn) / kTileSteps + 3));
+}
+__host__ __device__ __forceinline__ uint64_t aff_tile_fixed_bytes(int qn, int tn) {
+    return 2 * tile_runs_bytes(qn, tn) + 4 * aff_tile_table_bytes(qn, tn);
+}
+// Block u: up to 16 (u + 1) diagonals at 28 bytes of values and at most 8 of ops.
+__host__ __device__ __forceinline__ uint64_t aff_tile_hist_bytes(int64_t steps) {
+    const uint64_t u = static_cast<uint64_t>(steps) / kTileSteps + 1;
+    return u * 8192 + 288 * u * (u + 1);
+}
+// Costs the gap-affine tiles are specialised for, as (O + E) / g; 0: none. (2, 4, 1) gives 5,
+// (4, 6, 2) gives 4.
+__host__ __device__ __forceinline__ int aff_tile_open(phr_affine_costs c) {
+    const int E = c.gap_extend;
+    if (E <= 0 || c.mismatch != 2 * E || c.gap_open <= 0 || c.gap_open > (1 << 20)) return 0;
+    const int oe = c.gap_open / E + 1;
+    return c.gap_open % E == 0 && (oe == 4 || oe == 5) ? oe : 0;
+}
+
 // Score a pair is given room for at first: a quarter of the query for DNA, half for bytes
 // (protein). Records come from a pool, so one pair may take more.
 __host__ __device__ __forceinline__ int64_t tile_score_est(int qn, int mode) {
     return 64 + static_cast<int64_t>(qn) / (mode == 0 ? 4 : 2);
 }
-constexpr uint32_t kTileChunk = 64 << 10;   // bytes a CTA takes from the pool at a time
+constexpr uint32_t kTileChunk = 64 << 10;   // first chunk a CTA takes from the pool, bytes
 constexpr uint32_t kWarpTileChunk = 16 << 10;   // the same for a one-warp team
 constexpr int kWarpTileThreads = 256;           // threads per CTA of the one-warp teams' kernel
 constexpr uint32_t kWarpTileSmem = 12 << 10;    // shared memory of a one-warp team
@@ -216,17 +242,23 @@ struct TileLaunch {
     uint32_t chunk;
 };
 
-// How many warps a linear pair's register tiles get: 0 (the warp-group kernel), 1, or
-// kBigThreads / 32 (one CTA, long pairs). One warp: pairs from long_min on, and byte pairs
-// (protein, which mostly differ a lot) from kWarpTileBytesMin on, where the warp-group
-// kernel's frames in global memory cost more than a warp per pair: 5,000 protein pairs of
-// 200-800 at 30 % measured 1.9 + 1.6 ms (two passes) before and 0.96 ms now. Offsets are kept times 256 in 32 bits, hence the upper
-// limit; longer queries stay in the warp-group kernel.
+// How many warps a WFA pair's register tiles get: 0 (the warp-group kernels, or wfa.cu's
+// CTA kernel), 1, or kBigThreads / 32 (one CTA, long pairs). One warp: pairs from long_min
+// on, and byte pairs (protein, which mostly differ a lot) from kWarpTileBytesMin on, where
+// the warp-group kernel's frames in global memory cost more than a warp per pair: 5,000
+// protein pairs of 200-800 at 30 % measured 1.9 + 1.6 ms (two passes) before and 0.78 ms
+// now (linear). `open` is aff_tile_open for gap-affine pairs. Offsets are kept times 256
+// (linear) or 1024 in 32 bits, hence the upper limits; longer queries stay where they were.
 constexpr int kWarpTileBytesMin = 128;
-__host__ __device__ __forceinline__ int tile_warps(int32_t engine, int32_t big_min, int32_t long_min, int qn, int tn,
-                                                   int mode) {
+__host__ __device__ __forceinline__ int tile_warps(int32_t engine, int open, int32_t big_min, int32_t long_min, int qn,
+                                                   int tn, int mode) {
     const int64_t len = static_cast<int64_t>(qn) + tn;
-    if (big_min <= 0 || engine != PHR_ENGINE_WFA_LINEAR || qn >= (1 << 22) || tn >= (1 << 28)) return 0;
+    if (big_min <= 0 || tn >= (1 << 27)) return 0;
+    if (engine == PHR_ENGINE_WFA_LINEAR) {
+        if (qn >= (1 << 22)) return 0;
+    } else if (engine != PHR_ENGINE_WFA_AFFINE || open == 0 || qn >= (1 << 20)) {
+        return 0;
+    }
     if (len >= big_min) return kBigThreads / 32;
     return len >= (mode == 0 ? long_min : kWarpTileBytesMin) ? 1 : 0;
 }
@@ -239,6 +271,8 @@ constexpr int kLaneThreads = 256;
 void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+void launch_wfa_affine_cta_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+void launch_wfa_affine_warp_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st);
 

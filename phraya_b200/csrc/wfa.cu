@@ -1173,7 +1173,7 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
         const uint32_t task = sh_task;
         __syncthreads();
         if (task >= P.tasks.range[1]) break;
-        if (!(P.tasks.task_group[task] & kBigTask)) continue;
+        if ((P.tasks.task_group[task] & kOtherKernel) != kBigTask) continue;
         const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
         const PairDesc d = P.desc[pid];
         if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
@@ -1468,7 +1468,7 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
         uint8_t* slot = P.task_off ? P.scratch + P.task_off[task] : P.scratch + warp_global * P.slot_bytes;
         const uint64_t slot_bytes = P.task_off ? P.task_len[task] : P.slot_bytes;
         const uint8_t tg = P.tasks.task_group[task];
-        if (tg & (kBigTask | kWarpTileTask)) continue;  // a redo task of another kernel
+        if (tg & kOtherKernel) continue;  // a redo task of another kernel
         const int G = tg;
         const int count = P.tasks.task_count[task];
         const int grp = lane / G;

@@ -30,177 +30,22 @@
 // the longest common prefix again. Records come from a pool shared by the pairs of a
 // launch, so a divergent pair uses what the others leave (a pair that still runs out is
 // redone with scratch of its own).
-#include <type_traits>
-
-#include "kernels.cuh"
+#include "wfa_tile.cuh"
 
 namespace phr {
 namespace {
 
-constexpr int kTeamTiles = 16;     // tiles a 16-warp team spreads a band over before they widen
 // A value word: offset << 8 | op << 6 | diagonals moved since the block's start + kStay.
-// An unset cell is negative.
-constexpr int kNeg = -(1 << 30);
-constexpr int kStay = 16;
-constexpr uint64_t kNoBase = ~0ull;
+constexpr int kLinRegs = 8;   // most diagonals per lane
 
-template <class S>
-constexpr int sym_shift() {  // log2 of the bits per symbol
-    return S::kBits == 2 ? 1 : 3;
-}
-
-// Symbols before the first set bit of x (kPerWord when x is zero): the bits below it are
-// counted, one operation of the slow pipe instead of a reversal and a leading-zero count.
-template <class S>
-__device__ __forceinline__ int first_diff(uint32_t x) {
-    return __popc((x - 1) & ~x) >> sym_shift<S>();
-}
-
-// Symbols before the first difference of three consecutive words.
-template <class S>
-__device__ __forceinline__ int first_diff3(uint32_t d0, uint32_t d1, uint32_t d2) {
-    int n = first_diff<S>(d0);
-    n += d0 == 0 ? first_diff<S>(d1) : 0;
-    n += (d0 | d1) == 0 ? first_diff<S>(d2) : 0;
-    return n;
-}
-
-// The CTA's dynamic shared memory: every access names it, so that loads through a call
-// stay shared-memory loads.
-extern __shared__ __align__(16) uint8_t tile_sm[];
-
-// A pair's sequences: in shared memory as overlapping word pairs (entry i holds words i and
-// i + 1, so one 64-bit load gives the 32 bits at any offset), or in global memory.
-template <class S, bool STAGED>
-struct PairSeq {
-    uint32_t q2, t2;      // byte offsets in tile_sm (staged)
-    const uint32_t* q;    // global words (otherwise)
-    const uint32_t* t;
-    __device__ __forceinline__ static uint64_t entry(uint32_t w2, uint32_t i) {
-        return *reinterpret_cast<const uint64_t*>(tile_sm + w2 + i * 8);
-    }
-    __device__ __forceinline__ static uint32_t win(uint32_t w2, const uint32_t* w, int pos) {
-        const uint32_t i = static_cast<uint32_t>(pos) / S::kPerWord;
-        if constexpr (STAGED) {
-            const uint64_t e = entry(w2, i);
-            return __funnelshift_r(static_cast<uint32_t>(e), static_cast<uint32_t>(e >> 32),
-                                   static_cast<uint32_t>(pos) << sym_shift<S>());
-        } else {
-            return __funnelshift_r(w[i], w[i + 1], static_cast<uint32_t>(pos) << sym_shift<S>());
-        }
-    }
-    // XOR of the symbols from query position p and target position j on
-    __device__ __forceinline__ uint32_t diff(int p, int j) const { return win(q2, q, p) ^ win(t2, t, j); }
-    // three consecutive words from position pos on
-    __device__ __forceinline__ static void win3(uint32_t w2, const uint32_t* w, int pos, uint32_t (&o)[3]) {
-        const uint32_t i = static_cast<uint32_t>(pos) / S::kPerWord;
-        const uint32_t sh = static_cast<uint32_t>(pos) << sym_shift<S>();
-        uint32_t a, b, c, d;
-        if constexpr (STAGED) {
-            const uint64_t e = entry(w2, i), f = entry(w2, i + 2);
-            a = static_cast<uint32_t>(e), b = static_cast<uint32_t>(e >> 32);
-            c = static_cast<uint32_t>(f), d = static_cast<uint32_t>(f >> 32);
-        } else {
-            a = w[i], b = w[i + 1], c = w[i + 2], d = w[i + 3];
-        }
-        o[0] = __funnelshift_r(a, b, sh);
-        o[1] = __funnelshift_r(b, c, sh);
-        o[2] = __funnelshift_r(c, d, sh);
-    }
-    // symbols query and target share from (p, j) on, at most three words
-    __device__ __forceinline__ int run3(int p, int j) const {
-        uint32_t a[3], b[3];
-        win3(q2, q, p, a);
-        win3(t2, t, j, b);
-        return first_diff3<S>(a[0] ^ b[0], a[1] ^ b[1], a[2] ^ b[2]);
-    }
-};
-
-// Offset where the match run of diagonal k ends that goes on at offset v, at most hi. Three
-// words a round, loaded together: runs between two edits mostly end in the first.
-template <class S, bool STAGED>
-__device__ __forceinline__ int extend_run(const PairSeq<S, STAGED>& sq, int v, int k, int hi, uint32_t& words) {
-    while (v < hi) {
-        ++words;
-        const int n = sq.run3(v, v - k);
-        v += n;
-        if (n < 3 * S::kPerWord) break;
-    }
-    return min(v, hi);
-}
-
-// Longest common prefix from (p, j), at most lim, by the whole warp (warp-uniform
-// arguments): one word first, then 32 words per round.
-template <class S, bool STAGED>
-__device__ __forceinline__ int warp_lcp(const PairSeq<S, STAGED>& sq, int p, int j, int lim) {
-    if (lim <= 0) return 0;
-    const uint32_t x0 = sq.diff(p, j);
-    if (x0 != 0 || lim <= S::kPerWord) return min(first_diff<S>(x0), lim);
-    const int lane = lane_id();
-    for (int n = S::kPerWord; n < lim; n += 32 * S::kPerWord) {
-        const int o = n + lane * S::kPerWord;
-        const uint32_t x = o < lim ? sq.diff(p + o, j + o) : 0u;
-        const unsigned b = __ballot_sync(PHR_FULL_MASK, x != 0);
-        if (b) {
-            const int src = __ffs(b) - 1;
-            const int f = __shfl_sync(PHR_FULL_MASK, first_diff<S>(x), src);
-            return min(n + src * S::kPerWord + f, lim);
-        }
-    }
-    return lim;
-}
-
-// Diagonals a tile of R per lane keeps, and the words of its records of kTileSteps scores.
-__host__ __device__ constexpr int tile_use(int R) { return 32 * R - 2 * kTileSteps; }
+// Record words of a tile's kTileSteps scores (two bits a cell), and the scores per word.
 __host__ __device__ constexpr int rec_words(int R) { return R < 2 ? 1 : R * kTileSteps / 16; }
-__host__ __device__ constexpr int rec_steps(int R) { return kTileSteps / rec_words(R); }  // scores per word
-
-// Tiles of R diagonals per lane over a pair: diagonal 0 sits in the middle of tile nb.
-template <int R>
-struct TileGeom {
-    static constexpr int use = tile_use(R);
-    int qn, tn, nb;
-    __device__ __forceinline__ TileGeom(int q, int t) : qn(q), tn(t), nb(t / use + 2) {}
-    __device__ __forceinline__ int tile_of(int k) const { return static_cast<int>(static_cast<uint32_t>(k + use / 2 + nb * use) / use); }
-    __device__ __forceinline__ int first(int g) const { return (g - nb) * use - use / 2; }   // first kept diagonal
-    // first / last tile with a reachable diagonal at score s
-    __device__ __forceinline__ int lo(int s) const { return tile_of(-min(s, tn)); }
-    __device__ __forceinline__ int hi(int s) const { return tile_of(min(s, qn)); }
-};
-
-// Diagonals per lane for the scores up to s_hi: few while the band is narrow, so that a
-// team's warps share it and a score's chain is short; more as it widens, since the
-// overlap of 16 diagonals per tile weighs less.
-template <int W>
-__device__ __forceinline__ int tile_regs(int s_hi, int qn, int tn) {
-    const int width = min(s_hi, qn) + min(s_hi, tn) + 1;
-    if constexpr (W == 1) {
-        // one warp does a block's tiles one after the other: the fewest diagonals computed
-        // (tiles grow to both sides of diagonal 0: five of R = 4 beat three of R = 8)
-        return width <= tile_use(1) ? 1
-               : width <= tile_use(2) ? 2
-               : width <= tile_use(4) ? 4
-               : width <= tile_use(8) || width > 5 * tile_use(4) ? 8 : 4;
-    } else {
-        return width <= kTeamTiles * tile_use(1) ? 1
-               : width <= kTeamTiles * tile_use(2) ? 2
-               : width <= kTeamTiles * tile_use(4) ? 4 : 8;
-    }
-}
+__host__ __device__ constexpr int rec_steps(int R) { return kTileSteps / rec_words(R); }
 
 // Value words of a block of n tiles.
 template <int R>
 __device__ __forceinline__ uint64_t frame_bytes(int n) {
     return (static_cast<uint64_t>(n) * tile_use(R) * 4 + 127) & ~127ull;
-}
-
-// Calls f with R (1, 2, 4 or 8) as a compile-time constant.
-template <class F>
-__device__ __forceinline__ void with_regs(int R, F&& f) {
-    if (R == 1) f(std::integral_constant<int, 1>{});
-    else if (R == 2) f(std::integral_constant<int, 2>{});
-    else if (R == 4) f(std::integral_constant<int, 4>{});
-    else f(std::integral_constant<int, 8>{});
 }
 
 // Advances tile g of one warp by kTileSteps scores, s0 + 1 .. s0 + kTileSteps. `cur` holds
@@ -229,7 +74,7 @@ __device__ __forceinline__ unsigned long long lin_tile(const PairSeq<S, STAGED>&
     const int up_src = (lane + 31) & 31, dn_src = (lane + 1) & 31;
     unsigned long long best_key = ~0ull;
     uint32_t ops = 0;
-#pragma unroll(8 / R)
+#pragma unroll(R < 4 ? 4 / R : 1)
     for (int h = 0; h < kTileSteps; ++h) {
         uint32_t more = 0, acc = 0;
         int prev_up = kNeg;   // lane 31 of the slot below
@@ -317,10 +162,9 @@ __device__ __forceinline__ uint64_t tile_band_cells(int qn, int tn, int64_t s) {
 
 // A team's share of the launch's scratch.
 struct TileScratch {
-    uint32_t* runs;     // match run after every score of the path, then the CIGAR runs
+    uint32_t* edits;    // the path's edits (one per score), each with the match run after it
     uint32_t* cigar;    // forward-order CIGAR runs
     int32_t* kpath;     // diagonal of the path after score kTileSteps u
-    uint16_t* ops;      // ops of the path's block u, two bits per score
     uint32_t* table;    // record block u, in 16-byte units of P.scratch
 };
 
@@ -365,27 +209,6 @@ __device__ __forceinline__ uint32_t block_ops(const BlockAt& b, const TileGeom<R
     return ops;
 }
 
-// One team's pair. W warps; `sh` is the team's control block, `frames` its shared memory
-// for value frames (fcap cells each).
-struct TileCtl {
-    unsigned long long end_key[2];   // smallest end cell, by parity of the score block
-    unsigned long long base[2];      // record block of this / the next kTileSteps scores
-    unsigned long long cursor, chunk_end;   // free part of the record chunk in hand, bytes of P.scratch
-    int32_t reach;
-    uint32_t task;
-    uint32_t n_runs;
-    uint32_t text_len[kBigThreads / 32];
-};
-static_assert(sizeof(TileCtl) <= kTileCtlBytes, "control block");
-
-template <int W>
-__device__ __forceinline__ void team_sync() {
-    if constexpr (W == 1)
-        __syncwarp();
-    else
-        __syncthreads();
-}
-
 // Follows the path back from block u_top's start (kpath[u_top]) block by block: the value
 // word of the path's cell after block u says how far it moved in it. The words of the next
 // blocks are fetched ahead for the 64 diagonals the path can have reached by then, so that
@@ -399,7 +222,7 @@ __device__ void walk_blocks(const uint8_t* scratch, const TileScratch& sc, int q
     auto fetch = [&](int u, int c, int& a, int& b) {   // words of diagonals c - 32 + lane, c + lane
         a = b = 0;
         if (u < 0) return;
-        with_regs(tile_regs<W>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
+        with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
             constexpr int R = decltype(rc)::value;
             const TileGeom<R> G(qn, tn);
             const int s_hi = (u + 1) * kTileSteps;
@@ -433,7 +256,7 @@ __device__ void walk_blocks(const uint8_t* scratch, const TileScratch& sc, int q
 }
 
 // Expands the path's blocks, one per thread of the team: their ops, and from the block's
-// start offset the match run after every score (runs[s]).
+// start offset the match run after every score.
 template <class S, bool STAGED, int W>
 __device__ void expand_blocks(const PairSeq<S, STAGED>& sq, const uint8_t* scratch, const TileScratch& sc, int qn, int tn,
                               int s_end, int k_end, int v0) {
@@ -443,14 +266,13 @@ __device__ void expand_blocks(const PairSeq<S, STAGED>& sq, const uint8_t* scrat
         const int h_top = u == u_top ? (s_end - 1) % kTileSteps : kTileSteps - 1;
         int k = u == u_top ? k_end : sc.kpath[u + 1];
         uint32_t ops = 0;
-        with_regs(tile_regs<W>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
+        with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
             constexpr int R = decltype(rc)::value;
             ops = block_ops<R>(block_at<R>(scratch, sc.table, qn, tn, u), TileGeom<R>(qn, tn), h_top, k);
         });
-        sc.ops[u] = static_cast<uint16_t>(ops);
         int p = v0;
         if (u > 0)
-            with_regs(tile_regs<W>(u * kTileSteps, qn, tn), [&](auto rc) {
+            with_regs<kLinRegs>(tile_regs<W, kLinRegs>(u * kTileSteps, qn, tn), [&](auto rc) {
                 const BlockAt b = block_at<decltype(rc)::value>(scratch, sc.table, qn, tn, u - 1);
                 p = b.frame[k - b.lo] >> 8;
             });
@@ -460,99 +282,10 @@ __device__ void expand_blocks(const PairSeq<S, STAGED>& sq, const uint8_t* scrat
             p += op != 3;
             k += op == 2 ? 1 : op == 3 ? -1 : 0;
             const int e = extend_run<S, STAGED>(sq, p, k, min(qn, tn + k), words);
-            sc.runs[u * kTileSteps + h + 1] = static_cast<uint32_t>(max(e - p, 0));
+            sc.edits[u * kTileSteps + h + 1] = static_cast<uint32_t>(max(e - p, 0)) << 2 | op;
             p = max(e, p);
         }
     }
-}
-
-// Forward-order CIGAR runs from the path's ops and match runs, 32 scores at a time; returns
-// their number. One warp.
-__device__ uint32_t path_runs(const TileScratch& sc, int s_end, int v0) {
-    const int lane = lane_id();
-    uint32_t nr = 0;
-    if (v0 > 0) {
-        if (lane == 0) sc.cigar[0] = static_cast<uint32_t>(v0) << 2;
-        nr = 1;
-    }
-    auto op_of = [&](int s) -> uint32_t {
-        return s <= s_end ? (sc.ops[(s - 1) / kTileSteps] >> (2 * ((s - 1) % kTileSteps))) & 3u : 0u;
-    };
-    auto run_of = [&](int s) -> uint32_t { return s <= s_end ? sc.runs[s] : 0u; };
-    uint32_t ops = op_of(1 + lane), my_n = run_of(1 + lane);
-    uint32_t last_op = 0;   // op and length so far of an edit run that goes on into this chunk (0: none)
-    uint32_t open = 0;
-    for (int base = 1; base <= s_end; base += 32) {
-        const uint32_t next_ops = op_of(base + 32 + lane), next_n = run_of(base + 32 + lane);
-        // an edit run starts where a match came before or the op changes
-        const uint32_t prev_op = __shfl_up_sync(PHR_FULL_MASK, ops, 1);
-        const uint32_t prev_n = __shfl_up_sync(PHR_FULL_MASK, my_n, 1);
-        const uint32_t first_next = __shfl_sync(PHR_FULL_MASK, next_ops, 0);
-        uint32_t next_op = __shfl_down_sync(PHR_FULL_MASK, ops, 1);
-        if (lane == 31) next_op = first_next;
-        const bool in = base + lane <= s_end;
-        const bool start = lane == 0 ? ops != last_op : (prev_n > 0 || prev_op != ops);
-        const bool end = in && (my_n > 0 || base + lane == s_end || next_op != ops);
-        const unsigned starts = __ballot_sync(PHR_FULL_MASK, in && start);
-        const unsigned ends = __ballot_sync(PHR_FULL_MASK, end);
-        const unsigned match = __ballot_sync(PHR_FULL_MASK, in && my_n > 0);
-        const unsigned below = (1u << lane) - 1u;
-        const unsigned mine = starts & (below | (1u << lane));   // starts at or below this lane
-        const uint32_t len = mine ? static_cast<uint32_t>(lane - (31 - __clz(mine)) + 1) : open + lane + 1;
-        uint32_t at = nr + __popc(ends & below) + __popc(match & below);
-        if (end) sc.cigar[at++] = (len << 2) | (ops == 1 ? 1u : ops == 2 ? 3u : 2u);
-        if (in && my_n > 0) sc.cigar[at] = my_n << 2;
-        nr += __popc(ends) + __popc(match);
-        const bool closed = (ends >> 31) & 1u;
-        open = closed ? 0u : __shfl_sync(PHR_FULL_MASK, len, 31);
-        last_op = closed ? 0u : __shfl_sync(PHR_FULL_MASK, ops, 31);
-        ops = next_ops;
-        my_n = next_n;
-    }
-    return nr;
-}
-
-// Writes the runs as CIGAR text, a contiguous share per warp of the team; returns the
-// text's length. `sh_len` holds a length per warp.
-template <int W>
-__device__ uint32_t format_runs(const uint32_t* runs, uint32_t nr, char* out, uint32_t* sh_len) {
-    const int lane = lane_id();
-    const int warp = W == 1 ? 0 : static_cast<int>(threadIdx.x) >> 5;
-    const uint32_t share = (nr + W - 1) / W;
-    const uint32_t from = min(nr, warp * share), to = min(nr, from + share);
-    uint32_t base = 0, total = 0;
-    if constexpr (W > 1) {
-        uint32_t mine = 0;
-        for (uint32_t c = from + lane; c < to; c += 32) mine += ndigits(runs[c] >> 2) + 1;
-        mine = __reduce_add_sync(PHR_FULL_MASK, mine);
-        if (lane == 0) sh_len[warp] = mine;
-        team_sync<W>();
-        for (int i = 0; i < W; ++i) {
-            const uint32_t l = sh_len[i];
-            if (i < warp) base += l;
-            total += l;
-        }
-    }
-    for (uint32_t c0 = from; c0 < to; c0 += 32) {
-        const uint32_t c = c0 + lane;
-        uint32_t len = 0, run = 0;
-        if (c < to) {
-            run = runs[c];
-            len = ndigits(run >> 2) + 1;
-        }
-        const uint32_t incl = group_incl_scan(len, 32);
-        if (c < to) {
-            char* p = out + base + incl - len;
-            uint32_t v = run >> 2;
-            for (int dd = static_cast<int>(len) - 2; dd >= 0; --dd) {
-                p[dd] = static_cast<char>('0' + v % 10);
-                v /= 10;
-            }
-            p[len - 1] = op_char(run & 3);
-        }
-        base += __shfl_sync(PHR_FULL_MASK, incl, 31);
-    }
-    return W == 1 ? base : total;
 }
 
 // The wavefront of a team's pair between two score blocks.
@@ -564,21 +297,6 @@ struct TileWave {
     unsigned long long end;
     uint32_t extra;           // word compares beyond a cell's first
 };
-
-// Record space for `bytes`, kNoBase when there is none (the team's allocating thread).
-__device__ __forceinline__ unsigned long long grab_records(const TileLaunch& A, TileCtl* sh, uint64_t bytes) {
-    if (sh->cursor + bytes > sh->chunk_end) {
-        if (!A.pool_used) return kNoBase;
-        const uint64_t want = bytes > A.chunk ? bytes : A.chunk;
-        const uint64_t o = atomicAdd(A.pool_used, static_cast<unsigned long long>(want));
-        if (o + want > A.pool_end) return kNoBase;
-        sh->cursor = o;
-        sh->chunk_end = o + want;
-    }
-    const uint64_t o = sh->cursor;
-    sh->cursor = o + bytes;
-    return o;
-}
 
 template <int R>
 __device__ __forceinline__ uint64_t block_bytes(const TileGeom<R>& G, int u) {
@@ -607,21 +325,21 @@ __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaun
         }
         // the next score's values: in shared memory while they fit, else only in the record
         int32_t* saved = reinterpret_cast<int32_t*>(P.scratch + base);
-        int32_t* nxt = nxt_hi - nxt_lo <= fcap ? frames + ((w.u + 1) & 1) * fcap : saved;
+        int32_t* nxt = nxt_hi - nxt_lo <= fcap / 2 ? frames + ((w.u + 1) & 1) * (fcap / 2) : saved;
         uint32_t* rec = reinterpret_cast<uint32_t*>(P.scratch + base + frame_bytes<R>(ghi - glo + 1));
         unsigned long long key = ~0ull;
         for (int g = glo + warp; g <= ghi; g += W)
             key = min(key, lin_tile<S, STAGED, R>(sq, G, g, w.s0, fitting, w.cur, w.cur_lo, w.cur_hi, nxt, saved, nxt_lo,
                                                   rec + (g - glo) * rec_words(R) * 32, w.extra));
         if (key != ~0ull) atomicMin(&sh->end_key[w.u & 1], key);
-        const bool more = tile_regs<W>(s_hi + kTileSteps, qn, tn) == R;
+        const bool more = tile_regs<W, kLinRegs>(s_hi + kTileSteps, qn, tn) == R;
         if (tid == 32 * (W - 1)) {
             table[w.u] = static_cast<uint32_t>(base / 16);
             uint64_t bytes = 0;
             if (more)
                 bytes = block_bytes<R>(G, w.u + 1);
             else
-                with_regs(tile_regs<W>(s_hi + kTileSteps, qn, tn),
+                with_regs<kLinRegs>(tile_regs<W, kLinRegs>(s_hi + kTileSteps, qn, tn),
                           [&](auto rc) { bytes = block_bytes(TileGeom<decltype(rc)::value>(qn, tn), w.u + 1); });
             sh->base[(w.u + 1) & 1] = grab_records(A, sh, bytes);
         }
@@ -642,8 +360,7 @@ __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaun
 
 template <class S, bool STAGED, int W>
 __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32_t pid, const PairDesc& d,
-                              const PairSeq<S, STAGED>& sq, uint8_t* region, uint64_t region_bytes, int32_t* frames,
-                              int fcap, TileCtl* sh) {
+                              const PairSeq<S, STAGED>& sq, uint8_t* region, int32_t* frames, int fcap, TileCtl* sh) {
     const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
     const int warp = W == 1 ? 0 : tid >> 5;
     const int qn = d.qn, tn = d.tn;
@@ -652,16 +369,13 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
 
     TileScratch sc;
     uint64_t at = 0;
-    sc.runs = reinterpret_cast<uint32_t*>(region);
+    sc.edits = reinterpret_cast<uint32_t*>(region);
     at += tile_runs_bytes(qn, tn);
     sc.cigar = reinterpret_cast<uint32_t*>(region + at);
     at += tile_runs_bytes(qn, tn);
     sc.kpath = reinterpret_cast<int32_t*>(region + at);
     at += tile_table_bytes(qn, tn);
     sc.table = reinterpret_cast<uint32_t*>(region + at);
-    at += tile_table_bytes(qn, tn);
-    sc.ops = reinterpret_cast<uint16_t*>(region + at);
-    at += tile_table_bytes(qn, tn);
 
     // ---- s = 0 ----
     const int v0 = warp_lcp<S, STAGED>(sq, 0, 0, min(qn, tn));
@@ -672,17 +386,11 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
         if (tid == 32 * (W - 1)) {
             frames[0] = v0 << 8;
             sh->end_key[0] = sh->end_key[1] = ~0ull;
-            // records come from the launch's pool, or (redo) from the rest of the pair's region
-            sh->cursor = sh->chunk_end = 0;
-            if (!A.pool_used) {
-                sh->cursor = static_cast<uint64_t>(region - P.scratch) + at;
-                sh->chunk_end = static_cast<uint64_t>(region - P.scratch) + region_bytes;
-            }
             sh->base[0] = grab_records(A, sh, block_bytes(TileGeom<1>(qn, tn), 0));
         }
         team_sync<W>();
         while (w.state == 0)
-            with_regs(tile_regs<W>(w.s0 + kTileSteps, qn, tn), [&](auto rc) {
+            with_regs<kLinRegs>(tile_regs<W, kLinRegs>(w.s0 + kTileSteps, qn, tn), [&](auto rc) {
                 lin_blocks<S, STAGED, W, decltype(rc)::value>(P, A, sq, qn, tn, fitting, sc.table, frames, fcap, sh, w);
             });
         if (w.state == 1) {
@@ -709,11 +417,7 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                     s2 = ::max(s2, est);
                 }
                 s2 = ::min(static_cast<int64_t>(max_s) + 1, s2);
-                const uint64_t need = tile_fixed_bytes(qn, tn) + tile_hist_bytes(qn, tn, s2);
-                const uint32_t i = atomicAdd(P.redo_count, 1u);
-                P.redo_list[i] = pid;
-                atomicMax(P.redo_need_max, static_cast<unsigned long long>(need));
-                if (P.redo_need) P.redo_need[i] = need;
+                tile_redo(P, pid, tile_fixed_bytes(qn, tn) + tile_hist_bytes(s2));
             }
         }
     }
@@ -737,7 +441,7 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                     // the last block is walked score by score, those below block by block
                     const int u_top = (s_end - 1) / kTileSteps;
                     int k = k_end;
-                    with_regs(tile_regs<W>((u_top + 1) * kTileSteps, qn, tn), [&](auto rc) {
+                    with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u_top + 1) * kTileSteps, qn, tn), [&](auto rc) {
                         constexpr int R = decltype(rc)::value;
                         block_ops<R>(block_at<R>(P.scratch, sc.table, qn, tn, u_top), TileGeom<R>(qn, tn),
                                      (s_end - 1) % kTileSteps, k);
@@ -751,7 +455,7 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
             if (s_end > 0) expand_blocks<S, STAGED, W>(sq, P.scratch, sc, qn, tn, s_end, k_end, v0);
             team_sync<W>();
             if (warp == 0) {
-                const uint32_t n = path_runs(sc, s_end, v0);
+                const uint32_t n = path_runs(sc.edits, sc.cigar, s_end, v0);
                 if (tid == 0) sh->n_runs = n;
             }
             team_sync<W>();
@@ -773,90 +477,26 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
     team_sync<W>();   // shared memory is reused by the team's next pair
 }
 
-// Stages a sequence as overlapping word pairs.
-__device__ __forceinline__ void stage_pairs(uint64_t* dst, const uint32_t* src, int words, int tid, int nthr) {
-    for (int i = tid; i < words; i += nthr) {
-        const uint32_t a = __ldg(src + i), b = __ldg(src + i + 1);
-        dst[i] = (static_cast<uint64_t>(b) << 32) | a;
+struct LinearTiles {
+    __device__ static uint64_t fixed_bytes(int qn, int tn) { return tile_fixed_bytes(qn, tn); }
+    __device__ static uint64_t hist_bytes(int64_t s) { return tile_hist_bytes(s); }
+    __device__ static int64_t score_est(int qn, int mode) { return tile_score_est(qn, mode); }
+    template <class S, bool STAGED, int W>
+    __device__ static void pair(const ExtendParams& P, const TileLaunch& A, uint32_t pid, const PairDesc& d,
+                                const PairSeq<S, STAGED>& sq, uint8_t* region, int32_t* frames, int fcap, TileCtl* sh) {
+        lin_tile_pair<S, STAGED, W>(P, A, pid, d, sq, region, frames, fcap, sh);
     }
-}
-
-template <class S, int W>
-__device__ __forceinline__ void tile_team(const ExtendParams& P, const TileLaunch& A, uint32_t sm_off, uint32_t sm_bytes) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
-    TileCtl* sh = reinterpret_cast<TileCtl*>(tile_sm + sm_off);
-    const uint32_t body_off = sm_off + kTileCtlBytes;
-    uint8_t* body = tile_sm + body_off;
-    const uint32_t body_bytes = sm_bytes - kTileCtlBytes;
-    for (;;) {
-        if (tid == 0) sh->task = P.tasks.range[0] + atomicAdd(P.queue_head, 1u);
-        team_sync<W>();
-        const uint32_t task = sh->task;
-        team_sync<W>();
-        if (task >= P.tasks.range[1]) break;
-        if (P.task_off && !(P.tasks.task_group[task] & (W == 1 ? kWarpTileTask : kBigTask))) continue;
-        const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
-        const PairDesc d = P.desc[pid];
-        if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
-        uint8_t* region;
-        uint64_t region_bytes;
-        if (P.task_off) {
-            region = P.scratch + P.task_off[task];
-            region_bytes = P.task_len[task] & ~15ull;
-        } else {
-            // main pass: the pair's fixed part comes from the pool, which the host sized for it
-            const uint64_t fixed = tile_fixed_bytes(d.qn, d.tn);
-            if (tid == 0) sh->base[0] = atomicAdd(A.pool_used, static_cast<unsigned long long>(fixed));
-            team_sync<W>();
-            const uint64_t o = sh->base[0];
-            team_sync<W>();
-            if (o + fixed > A.pool_end) {
-                if (tid == 0) {
-                    const uint64_t need = fixed + tile_hist_bytes(d.qn, d.tn, tile_score_est(d.qn, d.mode));
-                    const uint32_t i = atomicAdd(P.redo_count, 1u);
-                    P.redo_list[i] = pid;
-                    atomicMax(P.redo_need_max, static_cast<unsigned long long>(need));
-                    if (P.redo_need) P.redo_need[i] = need;
-                }
-                continue;
-            }
-            region = P.scratch + o;
-            region_bytes = fixed;
-        }
-        const uint32_t* gq = (S::kBits == 2 ? P.packed2 : P.bytes) + d.q_word;
-        const uint32_t* gt = (S::kBits == 2 ? P.packed2 : P.bytes) + d.t_word;
-        const int qw = (d.qn + S::kPerWord - 1) / S::kPerWord, tw = (d.tn + S::kPerWord - 1) / S::kPerWord;
-        // lanes on diagonals outside [-tn, qn] read up to a tile past a sequence's end
-        constexpr int pad = kTileMax / S::kPerWord + 2;
-        const uint64_t seq_bytes = (static_cast<uint64_t>(qw) + tw + 2 * pad) * 8;
-        if (seq_bytes + 4 * kTileMax * 4 <= body_bytes) {
-            uint64_t* q2 = reinterpret_cast<uint64_t*>(body);
-            uint64_t* t2 = q2 + qw + pad;
-            stage_pairs(q2, gq, qw, tid, 32 * W);
-            stage_pairs(t2, gt, tw, tid, 32 * W);
-            team_sync<W>();
-            const PairSeq<S, true> sq{body_off, body_off + (qw + pad) * 8, gq, gt};
-            const int fcap = static_cast<int>((body_bytes - seq_bytes) / 8);
-            lin_tile_pair<S, true, W>(P, A, pid, d, sq, region, region_bytes,
-                                      reinterpret_cast<int32_t*>(body + seq_bytes), fcap, sh);
-        } else {
-            const PairSeq<S, false> sq{0, 0, gq, gt};
-            const int fcap = static_cast<int>(body_bytes / 8);
-            lin_tile_pair<S, false, W>(P, A, pid, d, sq, region, region_bytes, reinterpret_cast<int32_t*>(body), fcap,
-                                       sh);
-        }
-    }
-}
+};
 
 template <class S>
 __global__ void __launch_bounds__(kBigThreads, 1) wfa_linear_big_kernel(ExtendParams P, TileLaunch A) {
-    tile_team<S, kBigThreads / 32>(P, A, 0, P.big_smem);
+    tile_team<S, kBigThreads / 32, LinearTiles>(P, A, 0, P.big_smem);
 }
 
 // One warp per pair: kWarpTileThreads / 32 teams per CTA, two CTAs per SM.
 template <class S>
 __global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_linear_tile_kernel(ExtendParams P, TileLaunch A) {
-    tile_team<S, 1>(P, A, (threadIdx.x >> 5) * kWarpTileSmem, kWarpTileSmem);
+    tile_team<S, 1, LinearTiles>(P, A, (threadIdx.x >> 5) * kWarpTileSmem, kWarpTileSmem);
 }
 
 }  // namespace
