@@ -781,7 +781,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64),
     // [40..43] first register-tile task of each kind (one warp 2-bit / bytes, CTA 2-bit / bytes),
     // [44..51] their ranges, [52..55] their scratch need: sum, largest (u64), [56..59] their queue
-    // heads, [60..61] pool bytes taken (u64)
+    // heads, [60..61] pool bytes taken (u64), [62] deferred register-tile pairs, [63] their queue head
     uint32_t* cnt = static_cast<uint32_t*>(take(256));
     if (!cnt) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted");
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
@@ -915,6 +915,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // main pass (per_task false): per-warp slots of `slot` bytes; redo passes: per-task
     // scratch (P.task_off / P.task_len set by the caller, `per_task_total` bytes in all,
     // `n_tasks_hint` tasks)
+    uint64_t tile_pool = 0;   // of the main pass
     auto launch_pass = [&](const uint32_t* ord, const uint32_t* tfirst, const uint8_t* tcount, const uint8_t* tgroup,
                            const uint32_t* range0, const uint32_t* range1, uint64_t slot, int full_band,
                            bool per_task = false, uint64_t per_task_total = 0,
@@ -936,6 +937,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 pool = std::min<uint64_t>(2 * tile_need[0], 2 * teams * tile_need[1]);
                 pool = std::max<uint64_t>(pool, std::min<uint64_t>(16 * tile_need[0], 1ull << 30)) + (1 << 20);
                 pool = std::min<uint64_t>(pool, ctx->scratch_budget);
+                tile_pool = pool;
             }
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
         } else {
@@ -1007,9 +1009,10 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 const uint64_t nt = per_task ? n_tasks_hint : n_tile[i];
                 if (nt == 0) continue;
                 const bool cta = i >= 2;
-                if (!per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 60, 0, 8, st));
                 const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 60), pool,
-                                    cta ? kTileChunk : kWarpTileChunk};
+                                    cta ? kTileChunk : kWarpTileChunk,
+                                    per_task || !cta ? 0 : kTileDeferStep, ctx->sm_count,
+                                    cnt + 62, reinterpret_cast<unsigned long long*>(rtask_off)};
                 const uint64_t most = static_cast<uint64_t>(ctx->sm_count) *
                                       (cta ? 1 : std::min(ctx->tune.max_blocks_per_sm, 2));
                 const uint64_t ctas = cta ? nt : (nt + kWarpTileThreads / 32 - 1) / (kWarpTileThreads / 32);
@@ -1043,6 +1046,27 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
 
     phr_status s = launch_pass(order, task_first, task_count, task_group, cnt + 0, cnt + 2, h_need, 0);
     if (s != PHR_OK) return s;
+    if (n_tile[2] + n_tile[3] > 0) {
+        // long pairs left by the CTA kernels when most SMs had run out of pairs: a cluster each
+        uint32_t h_defer = 0;
+        PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_defer, cnt + 62, 4, cudaMemcpyDeviceToHost, st));
+        PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        if (h_defer > 0) {
+            const TileLaunch tl{reinterpret_cast<unsigned long long*>(cnt + 60), tile_pool, kTileChunk, 0, ctx->sm_count, cnt + 62,
+                                reinterpret_cast<unsigned long long*>(rtask_off)};
+            const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
+            const int ctas = h_defer <= sms / 16 ? 16 : h_defer <= sms / 8 ? 8 : 4;
+            for (int mode = 0; mode < 2; ++mode) {
+                if (n_tile[2 + mode] == 0) continue;
+                PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 63, 0, 4, st));
+                P.queue_head = cnt + 63;
+                const bool affine = engine == PHR_ENGINE_WFA_AFFINE;
+                KernelScope ks(ctx, affine ? "wfa_affine_resume" : "wfa_linear_resume");
+                (affine ? launch_wfa_affine_resume : launch_wfa_linear_resume)(P, tl, static_cast<int>(h_defer), ctas, mode, st);
+            }
+            PHR_CUDA_TRY(ctx, cudaGetLastError());
+        }
+    }
 
     // Redo passes: each pair that did not fit its slot (or, for Myers, whose edit distance
     // left the stored band) runs again alone, with scratch sized for it: pairs are packed

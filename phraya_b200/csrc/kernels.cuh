@@ -181,6 +181,34 @@ constexpr int kTileRegs = 8;                                   // most diagonals
 constexpr int kTileMax = 32 * kTileRegs;                       // most diagonals of a tile
 constexpr uint32_t kTileCtlBytes = 768;                         // a team's control block in shared memory
 
+// The pool of a main-pass launch: bytes [0, pool_end) of the scratch buffer, taken by
+// atomicAdd on pool_used. pool_used NULL (redo passes): every pair has its own region.
+// A launch of one CTA per pair leaves a pair past step `defer_at` (0: never) where it is once
+// no more than a quarter of the SMs have a pair, and lists it; a second launch with a
+// cluster of CTAs per pair (resume) takes it up. One SM per pair to the end measured, for
+// 1,000 long reads with a few unrelated windows of 10-40 kb among them, 50.7 ms, with
+// clusters 22.8 ms; 200 gap-affine pairs of 4-16 kb 14.1 against 8.8 ms; one 10 kb
+// pair (score 1,143, linear) 0.85 against 0.49 ms.
+struct TileLaunch {
+    unsigned long long* pool_used;
+    uint64_t pool_end;
+    uint32_t chunk;
+    int32_t defer_at;
+    int32_t sm_count;
+    uint32_t* defer_count;
+    unsigned long long* defer_list;   // region / 256 << 32 | pair
+};
+
+// Below this step a band is too narrow for more than one SM (one pair alone: left at step 96
+// 0.49 ms, at 256 0.49, at 512 0.55).
+constexpr int32_t kTileDeferStep = 256;
+
+// How far a deferred pair got, kept in the last kTileHeadBytes of its fixed part.
+struct TileHead {
+    int32_t u, step, v0;   // block to go on with, its first step less one, the match run at score 0
+};
+constexpr uint64_t kTileHeadBytes = 256;
+
 __host__ __device__ __forceinline__ uint64_t tile_align(uint64_t v) { return (v + 255) & ~255ull; }
 __host__ __device__ __forceinline__ uint64_t tile_runs_bytes(int qn, int tn) {
     return tile_align(4 * (static_cast<uint64_t>(qn) + tn + 2));
@@ -190,7 +218,7 @@ __host__ __device__ __forceinline__ uint64_t tile_table_bytes(int qn, int tn) {
 }
 // What a pair takes before its first record: edits, CIGAR runs and two tables.
 __host__ __device__ __forceinline__ uint64_t tile_fixed_bytes(int qn, int tn) {
-    return 2 * tile_runs_bytes(qn, tn) + 2 * tile_table_bytes(qn, tn);
+    return 2 * tile_runs_bytes(qn, tn) + 2 * tile_table_bytes(qn, tn) + kTileHeadBytes;
 }
 // Upper bound of the records of scores up to s: block u holds 16 (u + 1) diagonals of 4
 // bytes of value and at most 8 / 3 of ops, plus rounding to tiles and the narrow tiles of
@@ -208,7 +236,7 @@ __host__ __device__ __forceinline__ uint64_t aff_tile_table_bytes(int qn, int tn
     return tile_align(4 * (aff_tile_steps(qn, tn) / kTileSteps + 3));
 }
 __host__ __device__ __forceinline__ uint64_t aff_tile_fixed_bytes(int qn, int tn) {
-    return 2 * tile_runs_bytes(qn, tn) + 4 * aff_tile_table_bytes(qn, tn);
+    return 2 * tile_runs_bytes(qn, tn) + 4 * aff_tile_table_bytes(qn, tn) + kTileHeadBytes;
 }
 // Block u: up to 16 (u + 1) diagonals at 28 bytes of values and at most 8 of ops.
 __host__ __device__ __forceinline__ uint64_t aff_tile_hist_bytes(int64_t steps) {
@@ -233,14 +261,6 @@ constexpr uint32_t kTileChunk = 64 << 10;   // first chunk a CTA takes from the 
 constexpr uint32_t kWarpTileChunk = 16 << 10;   // the same for a one-warp team
 constexpr int kWarpTileThreads = 256;           // threads per CTA of the one-warp teams' kernel
 constexpr uint32_t kWarpTileSmem = 12 << 10;    // shared memory of a one-warp team
-
-// The pool of a main-pass launch: bytes [0, pool_end) of the scratch buffer, taken by
-// atomicAdd on pool_used. pool_used NULL (redo passes): every pair has its own region.
-struct TileLaunch {
-    unsigned long long* pool_used;
-    uint64_t pool_end;
-    uint32_t chunk;
-};
 
 // How many warps a WFA pair's register tiles get: 0 (the warp-group kernels, or wfa.cu's
 // CTA kernel), 1, or kBigThreads / 32 (one CTA, long pairs). One warp: pairs from long_min
@@ -271,6 +291,9 @@ constexpr int kLaneThreads = 256;
 void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+// Deferred pairs of both symbol modes' launches, `ctas` (4, 8 or 16) CTAs per pair.
+void launch_wfa_linear_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st);
+void launch_wfa_affine_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st);
 void launch_wfa_affine_cta_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_warp_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);

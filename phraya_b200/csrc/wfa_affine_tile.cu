@@ -47,9 +47,10 @@ __device__ __forceinline__ uint64_t aff_frame_bytes(int tiles) {
 
 // Advances tile g of one warp by kTileSteps steps, t0 + 1 .. t0 + kTileSteps. `cur` holds
 // the rows of step t0; the kept diagonals' rows go to `nxt` and `saved` (one array when
-// they are the same) and the ops, eight steps of four bits per diagonal, to `rec`. Returns
+// they are the same) and the ops, eight steps of four bits per diagonal, to `rec`. FAR:
+// `cur` was written by other SMs. Returns
 // the smallest (step << 32 | (k + tn) << 2 | layer) of a kept end cell, ~0 without one.
-template <class S, bool STAGED, int R, int OES>
+template <class S, bool STAGED, int R, int OES, bool FAR>
 __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>& sq, const TileGeom<R>& G, int g, int t0,
                                                        bool fitting, const AffRows& cur, int32_t* nxt, int32_t* saved,
                                                        int nxt_lo, int nxt_w, uint32_t* rec, uint32_t& extra) {
@@ -64,7 +65,8 @@ __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>&
         const int i = k0 + 32 * r - cur.lo;
         const bool in = i >= 0 && i < cur.width;
         auto row = [&](int a) -> int {
-            const int v = in ? cur.base[static_cast<int64_t>(a) * cur.width + i] : kUnset;
+            const int32_t* at = cur.base + static_cast<int64_t>(a) * cur.width + i;
+            const int v = in ? (FAR ? __ldcg(at) : *at) : kUnset;
             return v < 0 ? kUnset : (v & ~1023) | (a << 5) | kStay;
         };
 #pragma unroll
@@ -197,7 +199,7 @@ struct AffScratch {
     int32_t* entry;     // diagonal and state the path enters block u with: (k + tn) << 3 | state
     uint32_t* list;     // block u's edits in path order, three bits each (op, match run follows), count << 24
     uint32_t* start;    // edits before block u
-    uint32_t* table;    // record block u, in 16-byte units of P.scratch
+    uint32_t* table;    // record block u (table_entry)
 };
 
 // Where block u of a pair keeps its rows and ops.
@@ -213,7 +215,7 @@ struct AffBlock {
         const int half = aff_half((u + 1) * kTileSteps, OES);
         b.glo = b.G.lo(half);
         const int ghi = b.G.hi(half);
-        const uint8_t* base = scratch + static_cast<uint64_t>(table[u]) * 16;
+        const uint8_t* base = scratch + entry_base(table[u]);
         b.rows.base = reinterpret_cast<const int32_t*>(base);
         b.rows.lo = b.G.first(b.glo);
         b.rows.width = b.G.first(ghi + 1) - b.rows.lo;
@@ -266,25 +268,27 @@ __device__ __forceinline__ uint32_t aff_block_edits(const AffBlock<R>& b, int h,
 struct AffWave {
     AffRows cur;              // rows of step t0
     int u, t0;                // block, its first step less one
-    int state;                // 0 running, 1 end found, 2 out of records, 3 every score done
+    int state;                // 0 running, 1 end found, 2 out of records, 3 every score done, 4 deferred
     unsigned long long end;
     uint32_t extra;           // word compares beyond a cell's first
 };
+
+template <int OES, int R>
+__device__ __forceinline__ uint64_t aff_block_bytes(const TileGeom<R>& G, int u) {
+    const int half = aff_half((u + 1) * kTileSteps, OES);
+    const int n = G.hi(half) - G.lo(half) + 1;
+    return aff_frame_bytes<R, OES>(n) + static_cast<uint64_t>(n) * R * 128;
+}
 
 // Blocks of a pair while its tiles hold R diagonals per lane (see lin_blocks).
 template <class S, bool STAGED, int W, int R, int OES>
 __device__ __forceinline__ void aff_blocks(const ExtendParams& P, const TileLaunch& A, const PairSeq<S, STAGED>& sq,
                                            int qn, int tn, bool fitting, int64_t max_t, uint32_t* table, int32_t* frames,
-                                           int fcap, TileCtl* sh, AffWave& w) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
+                                           int fcap, TileCtl* sh, TileMin* tm, AffWave& w) {
+    constexpr bool kFar = W > kCtaWarps;   // a cluster's rows go through L2
+    const int tid = team_tid<W>();
     const int warp = W == 1 ? 0 : tid >> 5;
     const TileGeom<R> G(qn, tn);
-    auto block_bytes = [](const auto& geom, int u) -> uint64_t {
-        constexpr int kR = (std::remove_reference_t<decltype(geom)>::use + 2 * kTileSteps) / 32;
-        const int half = aff_half((u + 1) * kTileSteps, OES);
-        const int n = geom.hi(half) - geom.lo(half) + 1;
-        return aff_frame_bytes<kR, OES>(n) + static_cast<uint64_t>(n) * kR * 128;
-    };
     do {
         const int half = aff_half(w.t0 + kTileSteps, OES);
         const int glo = G.lo(half), ghi = G.hi(half);
@@ -296,34 +300,37 @@ __device__ __forceinline__ void aff_blocks(const ExtendParams& P, const TileLaun
         }
         // the next rows: in shared memory while they fit, else only in the record
         int32_t* saved = reinterpret_cast<int32_t*>(P.scratch + base);
-        int32_t* nxt = nxt_w * (OES + 2) <= fcap / 2 ? frames + ((w.u + 1) & 1) * (fcap / 2) : saved;
+        int32_t* nxt = !kFar && nxt_w * (OES + 2) <= fcap / 2 ? frames + ((w.u + 1) & 1) * (fcap / 2) : saved;
         uint32_t* rec = reinterpret_cast<uint32_t*>(P.scratch + base + aff_frame_bytes<R, OES>(ghi - glo + 1));
         unsigned long long key = ~0ull;
         for (int g = glo + warp; g <= ghi; g += W)
-            key = min(key, aff_tile<S, STAGED, R, OES>(sq, G, g, w.t0, fitting, w.cur, nxt, saved, nxt_lo, nxt_w,
+            key = min(key, aff_tile<S, STAGED, R, OES, kFar>(sq, G, g, w.t0, fitting, w.cur, nxt, saved, nxt_lo, nxt_w,
                                                        rec + (g - glo) * R * 32, w.extra));
-        if (key != ~0ull) atomicMin(&sh->end_key[w.u & 1], key);
+        if (key != ~0ull) atomicMin(&tm->end_key[w.u & 1], key);
         const int next_R = tile_regs<W, kAffRegs>(aff_half(w.t0 + 2 * kTileSteps, OES), qn, tn);
-        if (tid == 32 * (W - 1)) {
-            table[w.u] = static_cast<uint32_t>(base / 16);
+        if (tid == alloc_tid<W>()) {
+            table[w.u] = table_entry(base, R);
             uint64_t bytes = 0;
             if (next_R == R)
-                bytes = block_bytes(G, w.u + 1);
+                bytes = aff_block_bytes<OES>(G, w.u + 1);
             else
                 with_regs<kAffRegs>(next_R, [&](auto rc) {
-                    bytes = block_bytes(TileGeom<decltype(rc)::value>(qn, tn), w.u + 1);
+                    bytes = aff_block_bytes<OES>(TileGeom<decltype(rc)::value>(qn, tn), w.u + 1);
                 });
             sh->base[(w.u + 1) & 1] = grab_records(A, sh, bytes);
+            if (W == kCtaWarps && A.defer_at > 0) sh->defer[w.u & 1] = tile_sms_idle(P, A);
         }
         team_sync<W>();
         w.cur = AffRows{nxt, nxt_lo, nxt_w};
         w.t0 += kTileSteps;
-        w.end = sh->end_key[w.u & 1];
+        w.end = kFar ? __ldcg(&tm->end_key[w.u & 1]) : tm->end_key[w.u & 1];
         ++w.u;
         if (w.end != ~0ull)
             w.state = 1;
         else if (w.t0 >= max_t)
             w.state = 3;
+        else if (W == kCtaWarps && A.defer_at > 0 && w.t0 >= A.defer_at && sh->defer[(w.u - 1) & 1])
+            w.state = 4;
         if (next_R != R) return;
     } while (w.state == 0);
 }
@@ -331,7 +338,9 @@ __device__ __forceinline__ void aff_blocks(const ExtendParams& P, const TileLaun
 template <class S, bool STAGED, int W, int OES>
 __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32_t pid, const PairDesc& d,
                               const PairSeq<S, STAGED>& sq, uint8_t* region, int32_t* frames, int fcap, TileCtl* sh) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
+    constexpr bool kResume = W > kCtaWarps;
+    constexpr int W1 = W < kCtaWarps ? W : kCtaWarps;   // the traceback is the first CTA's
+    const int tid = team_tid<W>();
     const int warp = W == 1 ? 0 : tid >> 5;
     const int qn = d.qn, tn = d.tn;
     const bool fitting = tn > qn + qn / 2 + 10;
@@ -349,25 +358,37 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
     sc.start = reinterpret_cast<uint32_t*>(tables + 2 * tab);
     sc.table = reinterpret_cast<uint32_t*>(tables + 3 * tab);
 
-    // ---- s = 0: endpoint (wfa_simd.rs:618-650) on diagonal 0 alone ----
-    const int v0 = warp_lcp<S, STAGED>(sq, 0, 0, min(qn, tn));
-    bool done = v0 == qn && (fitting ? qn <= tn : qn == tn);
+    // ---- s = 0: endpoint (wfa_simd.rs:618-650) on diagonal 0 alone; or where the pair was left ----
+    const uint64_t fixed = aff_tile_fixed_bytes(qn, tn);
+    const TileHead head = kResume ? *reinterpret_cast<const TileHead*>(region + fixed - kTileHeadBytes) : TileHead{};
+    const int v0 = kResume ? head.v0 : warp_lcp<S, STAGED>(sq, 0, 0, min(qn, tn));
+    bool done = !kResume && v0 == qn && (fitting ? qn <= tn : qn == tn);
+    TileMin* tm = team_min<W>(sh, region, fixed);
     int t_end = 0, k_end = 0, layer_end = 0;
     AffWave w = {{frames, 0, 1}, 0, 0, 0, ~0ull, 0u};
+    if (kResume) {
+        w.u = head.u;
+        w.t0 = head.step;
+        with_regs<kAffRegs>(entry_regs(sc.table[w.u - 1]), [&](auto rc) {
+            w.cur = AffBlock<decltype(rc)::value>::template at<OES>(P.scratch, sc.table, qn, tn, w.u - 1).rows;
+        });
+    }
     if (!done) {
-        if (tid == 32 * (W - 1)) {
-            for (int a = 0; a < OES + 2; ++a) frames[a] = a == 0 ? v0 << 10 : kUnset;
-            sh->end_key[0] = sh->end_key[1] = ~0ull;
-            const TileGeom<1> G(qn, tn);
-            const int half = aff_half(kTileSteps, OES);
-            const int n = G.hi(half) - G.lo(half) + 1;
-            sh->base[0] = grab_records(A, sh, aff_frame_bytes<1, OES>(n) + static_cast<uint64_t>(n) * 128);
+        if (tid == alloc_tid<W>()) {
+            tm->end_key[0] = tm->end_key[1] = ~0ull;
+            if (!kResume)
+                for (int a = 0; a < OES + 2; ++a) frames[a] = a == 0 ? v0 << 10 : kUnset;
+            uint64_t bytes = 0;
+            with_regs<kAffRegs>(tile_regs<W, kAffRegs>(aff_half(w.t0 + kTileSteps, OES), qn, tn), [&](auto rc) {
+                bytes = aff_block_bytes<OES>(TileGeom<decltype(rc)::value>(qn, tn), w.u);
+            });
+            sh->base[w.u & 1] = grab_records(A, sh, bytes);
         }
         team_sync<W>();
         while (w.state == 0)
             with_regs<kAffRegs>(tile_regs<W, kAffRegs>(aff_half(w.t0 + kTileSteps, OES), qn, tn), [&](auto rc) {
                 aff_blocks<S, STAGED, W, decltype(rc)::value, OES>(P, A, sq, qn, tn, fitting, max_t, sc.table, frames,
-                                                                  fcap, sh, w);
+                                                                  fcap, sh, tm, w);
             });
         if (w.state == 1) {
             t_end = static_cast<int>(w.end >> 32);
@@ -375,24 +396,31 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
             layer_end = static_cast<int>(w.end & 3u);
             done = t_end <= max_t;
         }
+        if (w.state == 4) {   // uniform over the team
+            if (tid == alloc_tid<W>()) tile_defer(P, A, sh, pid, region, fixed, TileHead{w.u, w.t0, v0});
+            if (P.work && w.extra) atomicAdd(P.work + 3, static_cast<unsigned long long>(w.extra));
+            team_sync<W>();
+            return;
+        }
         if (w.state == 2) {   // uniform over the team
             // Scratch for the redo from the furthest query offset so far, as in wfa_tile.cu.
-            if (tid == 0) sh->reach = 0;
+            if (tid == 0) tm->reach = 0;
             team_sync<W>();
             int vm = 0;
             for (int i = tid; i < w.cur.width; i += 32 * W) vm = max(vm, w.cur.base[i] >> 10);
             vm = __reduce_max_sync(PHR_FULL_MASK, vm);
-            if ((tid & 31) == 0) atomicMax(&sh->reach, vm);
+            if ((tid & 31) == 0) atomicMax(&tm->reach, vm);
             team_sync<W>();
             if (tid == 0) {
                 int64_t s2 = 2LL * w.t0 + 64;
-                if (sh->reach > 0) {
-                    int64_t est = static_cast<int64_t>(w.t0) * qn / sh->reach;
+                const int64_t reach = kResume ? __ldcg(&tm->reach) : tm->reach;
+                if (reach > 0) {
+                    int64_t est = static_cast<int64_t>(w.t0) * qn / reach;
                     est += est / 4 + 64;
                     s2 = ::max(s2, est);
                 }
                 s2 = ::min(max_t + 1, s2);
-                tile_redo(P, pid, aff_tile_fixed_bytes(qn, tn) + aff_tile_hist_bytes(s2));
+                tile_redo(P, pid, fixed + aff_tile_hist_bytes(s2));
             }
         }
     }
@@ -409,12 +437,12 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
         }
         if (w.extra) atomicAdd(P.work + 3, static_cast<unsigned long long>(w.extra));
     }
-    if (!overflow) {   // uniform over the team
+    if (!overflow && team_rank<W>() == 0) {   // uniform over each CTA
         uint32_t nr = 0, tl = 0, n_edits = 0;
         if (done) {
             const int u_top = (t_end - 1) / kTileSteps;
             const int h_end = t_end - u_top * kTileSteps;
-            auto regs_of = [&](int u) { return tile_regs<W, kAffRegs>(aff_half((u + 1) * kTileSteps, OES), qn, tn); };
+            auto regs_of = [&](int u) { return entry_regs(sc.table[u]); };
             if (t_end > 0) {
                 if (tid == 0) {
                     // the entry of every block: the last one step by step, those below by their
@@ -438,9 +466,9 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                         sc.entry[u] = (k + tn) << 3 | state;
                     }
                 }
-                team_sync<W>();
+                team_sync<W1>();
                 // the edits of every block, one block per thread
-                for (int u = tid; u <= u_top; u += 32 * W) {
+                for (int u = tid; u <= u_top; u += 32 * W1) {
                     int k = k_end, h = h_end, layer = layer_end, state = 0;
                     if (u < u_top) {
                         const int e = sc.entry[u + 1];
@@ -455,7 +483,7 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                         sc.list[u] = aff_block_edits<R, OES>(b, h, layer, k, state);
                     });
                 }
-                team_sync<W>();
+                team_sync<W1>();
                 if (warp == 0) {   // edits before each block
                     uint32_t total = 0;
                     for (int c = 0; c <= u_top; c += 32) {
@@ -467,10 +495,10 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                     }
                     if (tid == 0) sh->n_runs = total;
                 }
-                team_sync<W>();
+                team_sync<W1>();
                 n_edits = sh->n_runs;
                 // from each block's entry offset, the match runs after its edits
-                for (int u = tid; u <= u_top; u += 32 * W) {
+                for (int u = tid; u <= u_top; u += 32 * W1) {
                     const int e = sc.entry[u];
                     int k = (e >> 3) - tn, p = v0;
                     if (u > 0)
@@ -496,14 +524,14 @@ __device__ void aff_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                     }
                 }
             }
-            team_sync<W>();
+            team_sync<W1>();
             if (warp == 0) {
                 const uint32_t n = path_runs(sc.edits, sc.cigar, static_cast<int>(n_edits), v0);
                 if (tid == 0) sh->n_runs = n;
             }
-            team_sync<W>();
+            team_sync<W1>();
             nr = sh->n_runs;
-            tl = format_runs<W>(sc.cigar, nr, P.text + P.text_off[pid], sh->text_len);
+            tl = format_runs<W1>(sc.cigar, nr, P.text + P.text_off[pid], sh->text_len);
         }
         if (tid == 0) {
             PairOut o = {};
@@ -538,6 +566,12 @@ __global__ void __launch_bounds__(kBigThreads, 1) wfa_affine_big_tile_kernel(Ext
     tile_team<S, kBigThreads / 32, AffineTiles<OES>>(P, A, 0, P.big_smem);
 }
 
+// Deferred pairs, a cluster of C CTAs per pair.
+template <class S, int OES, int C>
+__global__ void __launch_bounds__(kBigThreads, 1) wfa_affine_resume_kernel(ExtendParams P, TileLaunch A) {
+    tile_team<S, C * kCtaWarps, AffineTiles<OES>>(P, A, 0, P.big_smem);
+}
+
 // One warp per pair: kWarpTileThreads / 32 teams per CTA, two CTAs per SM.
 template <class S, int OES>
 __global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_affine_tile_kernel(ExtendParams P, TileLaunch A) {
@@ -560,6 +594,20 @@ void launch_warps(const ExtendParams& p, const TileLaunch& a, int grid, cudaStre
 
 }  // namespace
 
+void launch_wfa_affine_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st) {
+    auto go = [&](auto kernel) { launch_clusters(kernel, p, a, pairs, ctas, st); };
+    auto by_size = [&](auto sc, auto oc) {
+        using S = decltype(sc);
+        constexpr int kO = decltype(oc)::value;
+        ctas == 16 ? go(wfa_affine_resume_kernel<S, kO, 16>) : ctas == 8 ? go(wfa_affine_resume_kernel<S, kO, 8>) : go(wfa_affine_resume_kernel<S, kO, 4>);
+    };
+    const std::integral_constant<int, 4> o4;
+    const std::integral_constant<int, 5> o5;
+    if (aff_tile_open(p.costs) == 4)
+        mode == 0 ? by_size(Seq2{}, o4) : by_size(SeqB{}, o4);
+    else
+        mode == 0 ? by_size(Seq2{}, o5) : by_size(SeqB{}, o5);
+}
 void launch_wfa_affine_cta_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
     const bool four = aff_tile_open(p.costs) == 4;
     if (mode == 0)

@@ -51,9 +51,9 @@ __device__ __forceinline__ uint64_t frame_bytes(int n) {
 // Advances tile g of one warp by kTileSteps scores, s0 + 1 .. s0 + kTileSteps. `cur` holds
 // the value words of score s0 for diagonals [cur_lo, cur_hi); the kept diagonals' words go
 // to `nxt` and `saved` (from diagonal nxt_lo on; one array when they are the same) and the
-// ops to `rec`. Returns the smallest (score << 32 | k + tn) of a kept end cell, ~0 when
-// there is none.
-template <class S, bool STAGED, int R>
+// ops to `rec`. FAR: `cur` was written by other SMs. Returns the smallest (score << 32 |
+// k + tn) of a kept end cell, ~0 when there is none.
+template <class S, bool STAGED, int R, bool FAR>
 __device__ __forceinline__ unsigned long long lin_tile(const PairSeq<S, STAGED>& sq, const TileGeom<R>& G, int g, int s0,
                                                        bool fitting, const int32_t* cur, int cur_lo, int cur_hi,
                                                        int32_t* nxt, int32_t* saved, int nxt_lo, uint32_t* rec,
@@ -66,7 +66,7 @@ __device__ __forceinline__ unsigned long long lin_tile(const PairSeq<S, STAGED>&
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int k = k0 + 32 * r;
-        x[r] = (k >= cur_lo && k < cur_hi) ? (cur[k - cur_lo] & ~255) | kStay : kNeg;
+        x[r] = (k >= cur_lo && k < cur_hi) ? ((FAR ? __ldcg(cur + (k - cur_lo)) : cur[k - cur_lo]) & ~255) | kStay : kNeg;
     }
     // end cells: diagonal qn - tn alone (global), or any from there on (fitting)
     const int kend = qn - tn;
@@ -165,7 +165,7 @@ struct TileScratch {
     uint32_t* edits;    // the path's edits (one per score), each with the match run after it
     uint32_t* cigar;    // forward-order CIGAR runs
     int32_t* kpath;     // diagonal of the path after score kTileSteps u
-    uint32_t* table;    // record block u, in 16-byte units of P.scratch
+    uint32_t* table;    // record block u (table_entry)
 };
 
 // Where block u of a pair keeps its value words and ops.
@@ -181,7 +181,7 @@ __device__ __forceinline__ BlockAt block_at(const uint8_t* scratch, const uint32
     BlockAt b;
     b.glo = G.lo(s_hi);
     b.lo = G.first(b.glo);
-    const uint8_t* base = scratch + static_cast<uint64_t>(table[u]) * 16;
+    const uint8_t* base = scratch + entry_base(table[u]);
     b.frame = reinterpret_cast<const int32_t*>(base);
     b.rec = reinterpret_cast<const uint32_t*>(base + frame_bytes<R>(G.hi(s_hi) - b.glo + 1));
     return b;
@@ -213,7 +213,6 @@ __device__ __forceinline__ uint32_t block_ops(const BlockAt& b, const TileGeom<R
 // word of the path's cell after block u says how far it moved in it. The words of the next
 // blocks are fetched ahead for the 64 diagonals the path can have reached by then, so that
 // the chain is a lookup per block and not a memory round trip. One warp; leaves kpath.
-template <int W>
 __device__ void walk_blocks(const uint8_t* scratch, const TileScratch& sc, int qn, int tn, int u_top) {
     constexpr int kAhead = 4;
     const int lane = lane_id();
@@ -222,12 +221,13 @@ __device__ void walk_blocks(const uint8_t* scratch, const TileScratch& sc, int q
     auto fetch = [&](int u, int c, int& a, int& b) {   // words of diagonals c - 32 + lane, c + lane
         a = b = 0;
         if (u < 0) return;
-        with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
+        const uint32_t e = sc.table[u];
+        with_regs<kLinRegs>(entry_regs(e), [&](auto rc) {
             constexpr int R = decltype(rc)::value;
             const TileGeom<R> G(qn, tn);
             const int s_hi = (u + 1) * kTileSteps;
             const int glo = G.lo(s_hi), lo = G.first(glo), hi = G.first(G.hi(s_hi) + 1);
-            const int32_t* f = reinterpret_cast<const int32_t*>(scratch + static_cast<uint64_t>(sc.table[u]) * 16);
+            const int32_t* f = reinterpret_cast<const int32_t*>(scratch + entry_base(e));
             const int ka = c - 32 + lane, kb = c + lane;
             if (ka >= lo && ka < hi) a = f[ka - lo];
             if (kb >= lo && kb < hi) b = f[kb - lo];
@@ -266,13 +266,13 @@ __device__ void expand_blocks(const PairSeq<S, STAGED>& sq, const uint8_t* scrat
         const int h_top = u == u_top ? (s_end - 1) % kTileSteps : kTileSteps - 1;
         int k = u == u_top ? k_end : sc.kpath[u + 1];
         uint32_t ops = 0;
-        with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u + 1) * kTileSteps, qn, tn), [&](auto rc) {
+        with_regs<kLinRegs>(entry_regs(sc.table[u]), [&](auto rc) {
             constexpr int R = decltype(rc)::value;
             ops = block_ops<R>(block_at<R>(scratch, sc.table, qn, tn, u), TileGeom<R>(qn, tn), h_top, k);
         });
         int p = v0;
         if (u > 0)
-            with_regs<kLinRegs>(tile_regs<W, kLinRegs>(u * kTileSteps, qn, tn), [&](auto rc) {
+            with_regs<kLinRegs>(entry_regs(sc.table[u - 1]), [&](auto rc) {
                 const BlockAt b = block_at<decltype(rc)::value>(scratch, sc.table, qn, tn, u - 1);
                 p = b.frame[k - b.lo] >> 8;
             });
@@ -293,7 +293,7 @@ struct TileWave {
     const int32_t* cur;       // values of score s0, diagonals [cur_lo, cur_hi)
     int cur_lo, cur_hi;
     int u, s0;                // score block, its first score less one
-    int state;                // 0 running, 1 end found, 2 out of records, 3 every score done
+    int state;                // 0 running, 1 end found, 2 out of records, 3 every score done, 4 deferred
     unsigned long long end;
     uint32_t extra;           // word compares beyond a cell's first
 };
@@ -310,8 +310,9 @@ __device__ __forceinline__ uint64_t block_bytes(const TileGeom<R>& G, int u) {
 template <class S, bool STAGED, int W, int R>
 __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaunch& A, const PairSeq<S, STAGED>& sq,
                                            int qn, int tn, bool fitting, uint32_t* table, int32_t* frames, int fcap,
-                                           TileCtl* sh, TileWave& w) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
+                                           TileCtl* sh, TileMin* tm, TileWave& w) {
+    constexpr bool kFar = W > kCtaWarps;   // a cluster's values go through L2
+    const int tid = team_tid<W>();
     const int warp = W == 1 ? 0 : tid >> 5;
     const TileGeom<R> G(qn, tn);
     do {
@@ -325,16 +326,16 @@ __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaun
         }
         // the next score's values: in shared memory while they fit, else only in the record
         int32_t* saved = reinterpret_cast<int32_t*>(P.scratch + base);
-        int32_t* nxt = nxt_hi - nxt_lo <= fcap / 2 ? frames + ((w.u + 1) & 1) * (fcap / 2) : saved;
+        int32_t* nxt = !kFar && nxt_hi - nxt_lo <= fcap / 2 ? frames + ((w.u + 1) & 1) * (fcap / 2) : saved;
         uint32_t* rec = reinterpret_cast<uint32_t*>(P.scratch + base + frame_bytes<R>(ghi - glo + 1));
         unsigned long long key = ~0ull;
         for (int g = glo + warp; g <= ghi; g += W)
-            key = min(key, lin_tile<S, STAGED, R>(sq, G, g, w.s0, fitting, w.cur, w.cur_lo, w.cur_hi, nxt, saved, nxt_lo,
+            key = min(key, lin_tile<S, STAGED, R, kFar>(sq, G, g, w.s0, fitting, w.cur, w.cur_lo, w.cur_hi, nxt, saved, nxt_lo,
                                                   rec + (g - glo) * rec_words(R) * 32, w.extra));
-        if (key != ~0ull) atomicMin(&sh->end_key[w.u & 1], key);
+        if (key != ~0ull) atomicMin(&tm->end_key[w.u & 1], key);
         const bool more = tile_regs<W, kLinRegs>(s_hi + kTileSteps, qn, tn) == R;
-        if (tid == 32 * (W - 1)) {
-            table[w.u] = static_cast<uint32_t>(base / 16);
+        if (tid == alloc_tid<W>()) {
+            table[w.u] = table_entry(base, R);
             uint64_t bytes = 0;
             if (more)
                 bytes = block_bytes<R>(G, w.u + 1);
@@ -342,18 +343,21 @@ __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaun
                 with_regs<kLinRegs>(tile_regs<W, kLinRegs>(s_hi + kTileSteps, qn, tn),
                           [&](auto rc) { bytes = block_bytes(TileGeom<decltype(rc)::value>(qn, tn), w.u + 1); });
             sh->base[(w.u + 1) & 1] = grab_records(A, sh, bytes);
+            if (W == kCtaWarps && A.defer_at > 0) sh->defer[w.u & 1] = tile_sms_idle(P, A);
         }
         team_sync<W>();
         w.cur = nxt;
         w.cur_lo = nxt_lo;
         w.cur_hi = nxt_hi;
         w.s0 = s_hi;
-        w.end = sh->end_key[w.u & 1];
+        w.end = kFar ? __ldcg(&tm->end_key[w.u & 1]) : tm->end_key[w.u & 1];
         ++w.u;
         if (w.end != ~0ull)
             w.state = 1;
         else if (s_hi >= qn + tn)
             w.state = 3;
+        else if (W == kCtaWarps && A.defer_at > 0 && s_hi >= A.defer_at && sh->defer[(w.u - 1) & 1])
+            w.state = 4;
         if (!more) return;
     } while (w.state == 0);
 }
@@ -361,7 +365,9 @@ __device__ __forceinline__ void lin_blocks(const ExtendParams& P, const TileLaun
 template <class S, bool STAGED, int W>
 __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32_t pid, const PairDesc& d,
                               const PairSeq<S, STAGED>& sq, uint8_t* region, int32_t* frames, int fcap, TileCtl* sh) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
+    constexpr bool kResume = W > kCtaWarps;
+    constexpr int W1 = W < kCtaWarps ? W : kCtaWarps;   // the traceback is the first CTA's
+    const int tid = team_tid<W>();
     const int warp = W == 1 ? 0 : tid >> 5;
     const int qn = d.qn, tn = d.tn;
     const bool fitting = tn > qn + qn / 2 + 10;
@@ -377,47 +383,75 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
     at += tile_table_bytes(qn, tn);
     sc.table = reinterpret_cast<uint32_t*>(region + at);
 
-    // ---- s = 0 ----
-    const int v0 = warp_lcp<S, STAGED>(sq, 0, 0, min(qn, tn));
-    bool done = fitting ? v0 >= qn : qn == tn && v0 == qn;   // wfa_simd.rs:277-283
+    // ---- s = 0, or where the pair was left ----
+    const uint64_t fixed = tile_fixed_bytes(qn, tn);
+    const TileHead head = kResume ? *reinterpret_cast<const TileHead*>(region + fixed - kTileHeadBytes) : TileHead{};
+    const int v0 = kResume ? head.v0 : warp_lcp<S, STAGED>(sq, 0, 0, min(qn, tn));
+    bool done = !kResume && (fitting ? v0 >= qn : qn == tn && v0 == qn);   // wfa_simd.rs:277-283
+    TileMin* tm = team_min<W>(sh, region, fixed);
     int s_end = 0, k_end = 0;
     TileWave w = {frames, 0, 1, 0, 0, 0, ~0ull, 0u};
+    if (kResume) {
+        w.u = head.u;
+        w.s0 = head.step;
+        with_regs<kLinRegs>(entry_regs(sc.table[w.u - 1]), [&](auto rc) {
+            const TileGeom<decltype(rc)::value> G(qn, tn);
+            w.cur_lo = G.first(G.lo(w.s0));
+            w.cur_hi = G.first(G.hi(w.s0) + 1);
+        });
+        w.cur = reinterpret_cast<const int32_t*>(P.scratch + entry_base(sc.table[w.u - 1]));
+    }
     if (!done) {
-        if (tid == 32 * (W - 1)) {
-            frames[0] = v0 << 8;
-            sh->end_key[0] = sh->end_key[1] = ~0ull;
-            sh->base[0] = grab_records(A, sh, block_bytes(TileGeom<1>(qn, tn), 0));
+        if (tid == alloc_tid<W>()) {
+            tm->end_key[0] = tm->end_key[1] = ~0ull;
+            if (kResume) {
+                // block u's space was taken for the narrower team's tiles
+                uint64_t bytes = 0;
+                with_regs<kLinRegs>(tile_regs<W, kLinRegs>(w.s0 + kTileSteps, qn, tn),
+                                    [&](auto rc) { bytes = block_bytes(TileGeom<decltype(rc)::value>(qn, tn), w.u); });
+                sh->base[w.u & 1] = grab_records(A, sh, bytes);
+            } else {
+                frames[0] = v0 << 8;
+                sh->base[0] = grab_records(A, sh, block_bytes(TileGeom<1>(qn, tn), 0));
+            }
         }
         team_sync<W>();
         while (w.state == 0)
             with_regs<kLinRegs>(tile_regs<W, kLinRegs>(w.s0 + kTileSteps, qn, tn), [&](auto rc) {
-                lin_blocks<S, STAGED, W, decltype(rc)::value>(P, A, sq, qn, tn, fitting, sc.table, frames, fcap, sh, w);
+                lin_blocks<S, STAGED, W, decltype(rc)::value>(P, A, sq, qn, tn, fitting, sc.table, frames, fcap, sh, tm, w);
             });
         if (w.state == 1) {
             s_end = static_cast<int>(w.end >> 32);
             k_end = static_cast<int>(w.end & 0xffffffffu) - tn;
             done = s_end <= max_s;
         }
+        if (w.state == 4) {   // uniform over the team
+            if (tid == alloc_tid<W>()) tile_defer(P, A, sh, pid, region, fixed, TileHead{w.u, w.s0, v0});
+            if (P.work && w.extra) atomicAdd(P.work + 3, static_cast<unsigned long long>(w.extra));
+            team_sync<W>();
+            return;
+        }
         if (w.state == 2) {   // uniform over the team
             // Scratch for the redo: the final score from the furthest query offset reached
             // so far (the wavefront advances about in proportion to the score) plus a
             // quarter, at least twice the scores reached, at most the whole search.
-            if (tid == 0) sh->reach = 0;
+            if (tid == 0) tm->reach = 0;
             team_sync<W>();
             int vm = 0;
             for (int i = tid; i < w.cur_hi - w.cur_lo; i += 32 * W) vm = max(vm, w.cur[i] >> 8);
             vm = __reduce_max_sync(PHR_FULL_MASK, vm);
-            if ((tid & 31) == 0) atomicMax(&sh->reach, vm);
+            if ((tid & 31) == 0) atomicMax(&tm->reach, vm);
             team_sync<W>();
             if (tid == 0) {
                 int64_t s2 = 2LL * w.s0 + 64;
-                if (sh->reach > 0) {
-                    int64_t est = static_cast<int64_t>(w.s0) * qn / sh->reach;
+                const int64_t reach = kResume ? __ldcg(&tm->reach) : tm->reach;
+                if (reach > 0) {
+                    int64_t est = static_cast<int64_t>(w.s0) * qn / reach;
                     est += est / 4 + 64;
                     s2 = ::max(s2, est);
                 }
                 s2 = ::min(static_cast<int64_t>(max_s) + 1, s2);
-                tile_redo(P, pid, tile_fixed_bytes(qn, tn) + tile_hist_bytes(s2));
+                tile_redo(P, pid, fixed + tile_hist_bytes(s2));
             }
         }
     }
@@ -433,7 +467,7 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
         }
         if (extra) atomicAdd(P.work + 3, static_cast<unsigned long long>(extra));
     }
-    if (!overflow) {   // uniform over the team
+    if (!overflow && team_rank<W>() == 0) {   // uniform over each CTA
         uint32_t nr = 0, tl = 0;
         if (done) {
             if (warp == 0) {
@@ -441,26 +475,26 @@ __device__ void lin_tile_pair(const ExtendParams& P, const TileLaunch& A, uint32
                     // the last block is walked score by score, those below block by block
                     const int u_top = (s_end - 1) / kTileSteps;
                     int k = k_end;
-                    with_regs<kLinRegs>(tile_regs<W, kLinRegs>((u_top + 1) * kTileSteps, qn, tn), [&](auto rc) {
+                    with_regs<kLinRegs>(entry_regs(sc.table[u_top]), [&](auto rc) {
                         constexpr int R = decltype(rc)::value;
                         block_ops<R>(block_at<R>(P.scratch, sc.table, qn, tn, u_top), TileGeom<R>(qn, tn),
                                      (s_end - 1) % kTileSteps, k);
                     });
                     if (tid == 0) sc.kpath[u_top] = k;
                     __syncwarp();
-                    walk_blocks<W>(P.scratch, sc, qn, tn, u_top);
+                    walk_blocks(P.scratch, sc, qn, tn, u_top);
                 }
             }
-            team_sync<W>();
-            if (s_end > 0) expand_blocks<S, STAGED, W>(sq, P.scratch, sc, qn, tn, s_end, k_end, v0);
-            team_sync<W>();
+            team_sync<W1>();
+            if (s_end > 0) expand_blocks<S, STAGED, W1>(sq, P.scratch, sc, qn, tn, s_end, k_end, v0);
+            team_sync<W1>();
             if (warp == 0) {
                 const uint32_t n = path_runs(sc.edits, sc.cigar, s_end, v0);
                 if (tid == 0) sh->n_runs = n;
             }
-            team_sync<W>();
+            team_sync<W1>();
             nr = sh->n_runs;
-            tl = format_runs<W>(sc.cigar, nr, P.text + P.text_off[pid], sh->text_len);
+            tl = format_runs<W1>(sc.cigar, nr, P.text + P.text_off[pid], sh->text_len);
         }
         if (tid == 0) {
             PairOut o = {};
@@ -493,6 +527,12 @@ __global__ void __launch_bounds__(kBigThreads, 1) wfa_linear_big_kernel(ExtendPa
     tile_team<S, kBigThreads / 32, LinearTiles>(P, A, 0, P.big_smem);
 }
 
+// Deferred pairs, a cluster of C CTAs per pair.
+template <class S, int C>
+__global__ void __launch_bounds__(kBigThreads, 1) wfa_linear_resume_kernel(ExtendParams P, TileLaunch A) {
+    tile_team<S, C * kCtaWarps, LinearTiles>(P, A, 0, P.big_smem);
+}
+
 // One warp per pair: kWarpTileThreads / 32 teams per CTA, two CTAs per SM.
 template <class S>
 __global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_linear_tile_kernel(ExtendParams P, TileLaunch A) {
@@ -501,6 +541,13 @@ __global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_linear_tile_kernel(Ex
 
 }  // namespace
 
+void launch_wfa_linear_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st) {
+    auto go = [&](auto kernel) { launch_clusters(kernel, p, a, pairs, ctas, st); };
+    if (mode == 0)
+        ctas == 16 ? go(wfa_linear_resume_kernel<Seq2, 16>) : ctas == 8 ? go(wfa_linear_resume_kernel<Seq2, 8>) : go(wfa_linear_resume_kernel<Seq2, 4>);
+    else
+        ctas == 16 ? go(wfa_linear_resume_kernel<SeqB, 16>) : ctas == 8 ? go(wfa_linear_resume_kernel<SeqB, 8>) : go(wfa_linear_resume_kernel<SeqB, 4>);
+}
 void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
     constexpr int smem = kWarpTileThreads / 32 * static_cast<int>(kWarpTileSmem);
     if (mode == 0) {

@@ -3,6 +3,8 @@
 // (wfa_tile.cu linear, wfa_affine_tile.cu gap-affine; the method is described there).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -10,7 +12,6 @@
 namespace phr {
 namespace {
 
-constexpr int kTeamTiles = 16;     // tiles a 16-warp team spreads a band over before they widen
 constexpr int kNeg = -(1 << 30);   // an unset value word (any negative word is)
 constexpr int kStay = 16;          // a block's diagonals moved are kept plus this
 constexpr uint64_t kNoBase = ~0ull;
@@ -151,9 +152,10 @@ __device__ __forceinline__ int tile_regs(int half, int qn, int tn) {
                : RMAX == 4 || width <= tile_use(4) ? 4
                : width <= tile_use(8) || width > 5 * tile_use(4) ? 8 : 4;
     } else {
-        return width <= kTeamTiles * tile_use(1) ? 1
-               : width <= kTeamTiles * tile_use(2) ? 2
-               : RMAX == 4 || width <= kTeamTiles * tile_use(4) ? 4 : 8;
+        // a tile per warp before tiles widen
+        return width <= W * tile_use(1) ? 1
+               : width <= W * tile_use(2) ? 2
+               : RMAX == 4 || width <= W * tile_use(4) ? 4 : 8;
     }
 }
 
@@ -169,27 +171,69 @@ __device__ __forceinline__ void with_regs(int R, F&& f) {
 // A team's control block in shared memory. Its record chunks, of growing size, are taken from
 // the launch's pool once and used again for each of the team's pairs.
 constexpr int kMaxChunks = 40;
-struct TileCtl {
+struct TileMin {   // what all of a team's warps reduce into
     unsigned long long end_key[2];   // smallest end cell, by parity of the score block
+    int32_t reach;                   // furthest query offset
+};
+struct TileCtl {
+    TileMin min;
     unsigned long long base[2];      // record block of this / the next kTileSteps scores
     unsigned long long cursor, chunk_end;   // free part of the record chunk in hand, bytes of P.scratch
     unsigned long long chunk[kMaxChunks];   // where the team's chunks start
     uint32_t chunk_size[kMaxChunks];        // in units of 256 bytes
     int32_t n_chunks, cur_chunk;
-    int32_t reach;
     uint32_t task;
+    uint32_t defer[2];   // leave the pair to a cluster, by parity of the block
     uint32_t n_runs;
     uint32_t text_len[kBigThreads / 32];
 };
 static_assert(sizeof(TileCtl) <= kTileCtlBytes, "control block");
 
+// Teams: one warp, the warps of one CTA (W = kCtaWarps), or those of a cluster of CTAs, whose
+// control block is the first CTA's.
+constexpr int kCtaWarps = kBigThreads / 32;
+
 template <int W>
 __device__ __forceinline__ void team_sync() {
-    if constexpr (W == 1)
+    if constexpr (W == 1) {
         __syncwarp();
-    else
+    } else if constexpr (W == kCtaWarps) {
         __syncthreads();
+    } else {
+        cooperative_groups::this_cluster().sync();
+    }
 }
+template <int W>
+__device__ __forceinline__ int team_rank() {   // CTA within the cluster
+    return W <= kCtaWarps ? 0 : static_cast<int>(cooperative_groups::this_cluster().block_rank());
+}
+template <int W>
+__device__ __forceinline__ int team_tid() {
+    return W == 1 ? lane_id() : team_rank<W>() * kBigThreads + static_cast<int>(threadIdx.x);
+}
+// The thread that takes record space: the first CTA's last warp, which has a tile least often.
+template <int W>
+constexpr int alloc_tid() {
+    return 32 * ((W < kCtaWarps ? W : kCtaWarps) - 1);
+}
+
+// Where a team reduces: its shared memory; a cluster in global memory (64-bit atomic minima
+// on another CTA's shared memory lost updates), behind the pair's head.
+template <int W>
+__device__ __forceinline__ TileMin* team_min(TileCtl* sh, uint8_t* region, uint64_t fixed) {
+    if constexpr (W <= kCtaWarps)
+        return &sh->min;
+    else
+        return reinterpret_cast<TileMin*>(region + fixed - kTileHeadBytes / 2);
+}
+
+// Record block u of a pair: where it starts, in units of 128 bytes of P.scratch, and log2 of
+// its tiles' diagonals per lane.
+__device__ __forceinline__ uint32_t table_entry(uint64_t base, int R) {
+    return static_cast<uint32_t>(base / 128) << 3 | static_cast<uint32_t>(31 - __clz(R));
+}
+__device__ __forceinline__ uint64_t entry_base(uint32_t e) { return static_cast<uint64_t>(e >> 3) * 128; }
+__device__ __forceinline__ int entry_regs(uint32_t e) { return 1 << (e & 7u); }
 
 // Record space for `bytes`, kNoBase when there is none (one thread of the team). New chunks
 // double from A.chunk up to 256 times that.
@@ -317,38 +361,50 @@ __device__ __forceinline__ void stage_pairs(uint64_t* dst, const uint32_t* src, 
     }
 }
 
-// Persistent loop of one team of W warps over the launch's tasks; Algo aligns a pair.
+// Persistent loop of one team of W warps over the launch's tasks (W > kCtaWarps: over the
+// deferred pairs); Algo aligns a pair.
 template <class S, int W, class Algo>
 __device__ __forceinline__ void tile_team(const ExtendParams& P, const TileLaunch& A, uint32_t sm_off, uint32_t sm_bytes) {
-    const int tid = W == 1 ? lane_id() : static_cast<int>(threadIdx.x);
+    constexpr bool kResume = W > kCtaWarps;
+    const int tid = team_tid<W>();
     TileCtl* sh = reinterpret_cast<TileCtl*>(tile_sm + sm_off);
+    if constexpr (kResume) sh = cooperative_groups::this_cluster().map_shared_rank(sh, 0);
     const uint32_t body_off = sm_off + kTileCtlBytes;
     uint8_t* body = tile_sm + body_off;
     const uint32_t body_bytes = sm_bytes - kTileCtlBytes;
+    const uint32_t first = kResume ? 0u : P.tasks.range[0], last = kResume ? *A.defer_count : P.tasks.range[1];
     if (tid == 0) sh->n_chunks = 0;
     for (;;) {
-        if (tid == 0) sh->task = P.tasks.range[0] + atomicAdd(P.queue_head, 1u);
+        if (tid == 0) sh->task = first + atomicAdd(P.queue_head, 1u);
         team_sync<W>();
         const uint32_t task = sh->task;
         team_sync<W>();
-        if (task >= P.tasks.range[1]) break;
-        if (P.task_off && (P.tasks.task_group[task] & kOtherKernel) != (W == 1 ? kWarpTileTask : kCtaTileTask)) continue;
-        const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
+        if (task >= last) break;
+        uint32_t pid;
+        if constexpr (kResume) {
+            pid = static_cast<uint32_t>(A.defer_list[task]);
+        } else {
+            if (P.task_off && (P.tasks.task_group[task] & kOtherKernel) != (W == 1 ? kWarpTileTask : kCtaTileTask)) continue;
+            pid = P.tasks.order[P.tasks.task_first[task]];
+        }
         const PairDesc d = P.desc[pid];
         if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
-        // the pair's fixed part and records: its own region (redo), or the team's chunks
+        // the pair's fixed part and records: its own region (redo), or the team's chunks. A
+        // cluster takes new chunks for every pair: what one of its CTAs has read before, and
+        // may hold in its L1, is never written again.
         const uint64_t fixed = Algo::fixed_bytes(d.qn, d.tn);
         if (tid == 0) {
             sh->cur_chunk = -1;
             sh->cursor = sh->chunk_end = 0;
+            if (kResume) sh->n_chunks = 0;
             if (P.task_off) {
                 sh->cursor = P.task_off[task];
                 sh->chunk_end = sh->cursor + (P.task_len[task] & ~15ull);
             }
-            sh->base[0] = grab_records(A, sh, fixed);
+            if (!kResume) sh->base[0] = grab_records(A, sh, fixed);
         }
         team_sync<W>();
-        const unsigned long long at = sh->base[0];
+        const unsigned long long at = kResume ? (A.defer_list[task] >> 32) * 256 : sh->base[0];
         team_sync<W>();
         if (at == kNoBase) {   // uniform over the team
             if (tid == 0) tile_redo(P, pid, fixed + Algo::hist_bytes(Algo::score_est(d.qn, d.mode)));
@@ -364,8 +420,10 @@ __device__ __forceinline__ void tile_team(const ExtendParams& P, const TileLaunc
         if (seq_bytes + 4 * kTileMax * 4 <= body_bytes) {
             uint64_t* q2 = reinterpret_cast<uint64_t*>(body);
             uint64_t* t2 = q2 + qw + pad;
-            stage_pairs(q2, gq, qw, tid, 32 * W);
-            stage_pairs(t2, gt, tw, tid, 32 * W);
+            constexpr int nthr = W == 1 ? 32 : kBigThreads;   // each CTA of a cluster stages both
+            const int t = W == 1 ? tid : static_cast<int>(threadIdx.x);
+            stage_pairs(q2, gq, qw, t, nthr);
+            stage_pairs(t2, gt, tw, t, nthr);
             team_sync<W>();
             const PairSeq<S, true> sq{body_off, body_off + (qw + pad) * 8, gq, gt};
             const int fcap = static_cast<int>((body_bytes - seq_bytes) / 4);
@@ -376,6 +434,45 @@ __device__ __forceinline__ void tile_team(const ExtendParams& P, const TileLaunc
             Algo::template pair<S, false, W>(P, A, pid, d, sq, region, reinterpret_cast<int32_t*>(body), fcap, sh);
         }
     }
+}
+
+// Whether most SMs have run out of pairs (one thread): each CTA that found the queue empty
+// has moved its head past the end.
+__device__ __forceinline__ bool tile_sms_idle(const ExtendParams& P, const TileLaunch& A) {
+    const int past = static_cast<int>(*reinterpret_cast<const volatile uint32_t*>(P.queue_head) + P.tasks.range[0] -
+                                      P.tasks.range[1]);
+    const int busy = static_cast<int>(gridDim.x) - max(past, 0);
+    return busy * 4 <= A.sm_count;
+}
+
+// Leaves a pair for the cluster launch: what it has stays where it is, so the team starts
+// over with new chunks (one thread).
+__device__ __forceinline__ void tile_defer(const ExtendParams& P, const TileLaunch& A, TileCtl* sh, uint32_t pid,
+                                           uint8_t* region, uint64_t fixed, const TileHead& head) {
+    *reinterpret_cast<TileHead*>(region + fixed - kTileHeadBytes) = head;
+    const uint32_t i = atomicAdd(A.defer_count, 1u);
+    A.defer_list[i] = static_cast<unsigned long long>((region - P.scratch) / 256) << 32 | pid;
+    sh->n_chunks = 0;
+}
+
+// Launches a cluster kernel, `ctas` CTAs per team, at most as many teams as fit at once.
+template <class K>
+inline void launch_clusters(K kernel, const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, cudaStream_t st) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.big_smem));
+    if (ctas > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    const int most = a.sm_count / ctas > 0 ? a.sm_count / ctas : 1;
+    cfg.gridDim = dim3(static_cast<unsigned>((pairs < most ? pairs : most) * ctas));
+    cfg.blockDim = dim3(kBigThreads);
+    cfg.dynamicSmemBytes = p.big_smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, p, a);
 }
 
 }  // namespace
