@@ -135,31 +135,35 @@ __host__ __device__ __forceinline__ int lane_slots(int dmin, int dmax, int nb) {
 }
 
 // Columns per traceback segment of the checkpointed lane kernel: the forward pass keeps
-// the window's {VP, VN} after every kSegCols-th column, the traceback recomputes one
-// segment of columns at a time into the task's scratch slot and walks it. Per 1,000,000
-// pairs of 64-2048 bp: 8 columns 13.43 ms, 4 columns 13.76 ms, 2 columns 15.90 ms (the
-// recompute is the same work; fewer checkpoints are fewer stores and dependent loads).
+// the window's {VP, VN} after every kSegCols-th column and the horizontal deltas that
+// entered each block, the traceback recomputes one segment's columns of the two blocks its
+// path is in. (Recomputing every block of the window, 8 columns took 13.43 ms per 1,000,000
+// pairs of 64-2048 bp, 4 columns 13.76, 2 columns 15.90.)
 constexpr int kSegCols = 8;
 
 // Scratch of one lane task, then one reverse-run list of (m_max + n_max + 2) words per
 // lane. Record mode: 16-byte {VP, HP} records [column group][slot][lane][column in
 // group] of every column. Checkpoint mode: 16-byte {VP, VN} states [checkpoint][slot]
-// [lane] after columns kSegCols, 2 kSegCols, ... below n_max, then the traceback's
-// segment buffer: the {VP, HP} records of one segment [column][slot][lane] (rewritten
-// every segment, so it stays in the caches).
+// [lane] after columns kSegCols, 2 kSegCols, ... below n_max, then the deltas that
+// entered each block, two bits a column, [segment][slot][lane], and the query blocks' two
+// bit planes [block][lane].
 __host__ __device__ __forceinline__ uint64_t lane_ckpt_bytes(int n_max, int P) {
     const uint64_t nck = n_max > 0 ? static_cast<uint64_t>((n_max - 1) / kSegCols) : 0;
     return (nck * P * 512 + 255) & ~255ull;
 }
 
-__host__ __device__ __forceinline__ uint64_t lane_rec_bytes(int n_max, int P, int ckpt) {
+__host__ __device__ __forceinline__ uint64_t lane_hin_bytes(int n_max, int P) {
+    return (static_cast<uint64_t>((n_max + kSegCols - 1) / kSegCols) * P * 64 + 255) & ~255ull;
+}
+
+__host__ __device__ __forceinline__ uint64_t lane_rec_bytes(int n_max, int m_max, int P, int ckpt) {
     const uint64_t ng = static_cast<uint64_t>((n_max + kLaneColGroup - 1) / kLaneColGroup);
-    return ckpt ? lane_ckpt_bytes(n_max, P) + static_cast<uint64_t>(kSegCols) * P * 512
+    return ckpt ? lane_ckpt_bytes(n_max, P) + lane_hin_bytes(n_max, P) + static_cast<uint64_t>((m_max + 63) / 64) * 512
                 : ((ng * kLaneColGroup * P * 512 + 255) & ~255ull);
 }
 
 __host__ __device__ __forceinline__ uint64_t lane_task_need(int n_max, int m_max, int P, int ckpt = 0) {
-    const uint64_t rec = lane_rec_bytes(n_max, P, ckpt);
+    const uint64_t rec = lane_rec_bytes(n_max, m_max, P, ckpt);
     const uint64_t runs = (32ull * static_cast<uint64_t>(m_max + n_max + 2) * 4 + 255) & ~255ull;
     return rec + runs;
 }

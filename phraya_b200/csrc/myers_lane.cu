@@ -135,14 +135,33 @@ __device__ __forceinline__ uint64_t ck_off(int c, int k, int lane) {
     return ((static_cast<uint64_t>(c) * P + k) * 32 + lane) * 16;
 }
 
+// Byte offset of the horizontal deltas that entered slot k in the columns of segment sg.
+template <int P>
+__device__ __forceinline__ uint64_t hin_off(int sg, int k, int lane) {
+    return ((static_cast<uint64_t>(sg) * P + k) * 32 + lane) * 2;
+}
+
 // Forward pass of one lane's pair. CK = false: every column's {VP, HP} records go to
 // `rec`; CK = true: only the window's {VP, VN} after every kSegCols-th column below
-// n_max (the traceback recomputes the columns in between).
+// n_max, and per segment of kSegCols columns the horizontal deltas (two bits a column,
+// the latest lowest) that entered each block of the window at the segment's end, to
+// `hin`. The traceback recomputes from those the two blocks a lane's path is in.
 template <int P, bool CK>
 __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb, int n,
-                                             int nb, const LaneGeom& g, uint64_t* sp, uint8_t* rec) {
+                                             int nb, const LaneGeom& g, uint64_t* sp, uint8_t* rec, uint8_t* hin,
+                                             uint4* planes) {
     const int lane = lane_id();
+    // a block's two bit planes, from its match masks, for the traceback
+    auto keep_planes = [&](int b, const uint64_t e[4]) {
+        if (CK && b < nb) {
+            const uint64_t p0 = e[1] | e[3], p1 = e[2] | e[3];
+            planes[b * 32 + lane] = make_uint4(lo32(p0), hi32(p0), lo32(p1), hi32(p1));
+        }
+    };
     uint64_t vp[P], vn[P];
+    uint32_t ha[P];   // deltas that entered each slot's block
+#pragma unroll
+    for (int k = 0; k < P; ++k) ha[k] = 0;
 #pragma unroll
     for (int k = 0; k < P; ++k) {
         uint64_t e[4] = {0, 0, 0, 0};
@@ -153,6 +172,7 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) sp[(k * 4 + c) * 32 + lane] = e[c];
+        keep_planes(k, e);
         vp[k] = ~0ull;
         vn[k] = 0;
     }
@@ -179,6 +199,7 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
             for (int k = 0; k + 1 < P; ++k) {
                 vp[k] = vp[k + 1];
                 vn[k] = vn[k + 1];
+                if (CK) ha[k] = ha[k + 1];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) sp[(k * 4 + c) * 32 + lane] = sp[((k + 1) * 4 + c) * 32 + lane];
             }
@@ -191,6 +212,7 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
             if (b + 1 < nb) load_block_words(qb, b + 1, qn);
 #pragma unroll
             for (int c = 0; c < 4; ++c) sp[((P - 1) * 4 + c) * 32 + lane] = e[c];
+            keep_planes(b, e);
             next_shift += 64;
         }
         const int jj = j - 1;
@@ -201,6 +223,8 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
 #pragma unroll
         for (int k = 0; k < P; ++k) {
             const uint64_t eq = eqp[k * 128];
+            if (CK)   // +1 enters the window's top block
+                ha[k] = k == 0 ? (ha[0] << 2) | 2u : __funnelshift_l(ma, __funnelshift_l(pa, ha[k], 1), 1);
             const uint64_t ph = k == 0 ? advance_block<true>(vp[0], vn[0], eq, pa, ma)
                                        : advance_block<false>(vp[k], vn[k], eq, pa, ma);
             if (!CK)
@@ -213,6 +237,11 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
 #pragma unroll
             for (int k = 0; k < P; ++k)
                 *reinterpret_cast<uint4*>(c + k * 512) = make_uint4(lo32(vp[k]), hi32(vp[k]), lo32(vn[k]), hi32(vn[k]));
+        }
+        if (CK && ((j % kSegCols) == 0 || j == g.n_max)) {   // warp-uniform
+            uint8_t* h = hin + hin_off<P>((j - 1) / kSegCols, 0, lane);
+#pragma unroll
+            for (int k = 0; k < P; ++k) *reinterpret_cast<uint16_t*>(h + k * 64) = static_cast<uint16_t>(ha[k]);
         }
     }
 }
@@ -366,145 +395,164 @@ __device__ __forceinline__ bool lane_trace(const uint32_t* __restrict__ qb, cons
     return ok;
 }
 
-// Shared memory of one warp in checkpoint mode: the Peq ring (kLaneMaxSlots + 1 blocks,
-// [block % (P + 1)][base][lane], 64-bit masks). The forward pass's Peq ([slot][base]
-// [lane]) reuses its start. The segment's records live in the warp's scratch slot: each
-// lane writes and reads back only its own, a few KB per warp that stay in L1/L2, and
-// shared memory stays small enough for two blocks per SM.
-constexpr int kRingBytes = (kLaneMaxSlots + 1) * 4 * 32 * 8;
-constexpr int kCkWarpBytes = kRingBytes;
+// Shared memory of one warp in checkpoint mode. Traceback: the records of the two blocks each
+// lane's path is in over one segment ([column][block & 1][lane]). The forward pass's Peq
+// ([slot][base][lane]) has the same space.
+constexpr int kTraceRecBytes = kSegCols * 2 * 32 * 16;
+constexpr int kLanePeqWarpBytes = kLaneMaxSlots * 4 * 32 * 8;  // Peq (and record mode's traceback buffers) per warp
+constexpr int kCkWarpBytes = kTraceRecBytes > kLanePeqWarpBytes ? kTraceRecBytes : kLanePeqWarpBytes;
 
-// Peq of query block b (zero past the query) into ring slot b % (P + 1).
-template <int P>
-__device__ __forceinline__ void ring_fill(uint64_t* ring, const uint32_t* __restrict__ qb, int b, int nb, int lane) {
-    uint64_t e[4] = {0, 0, 0, 0};
-    if (b < nb) {
-        uint32_t qw[4];
-        load_block_words(qb, b, qw);
-        peq_words(qw, e);
-    }
-    uint64_t* r = ring + (b % (P + 1)) * 128 + lane;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) r[c * 32] = e[c];
-}
-
-// Traceback of one lane's pair from (m, n) over segments of kSegCols columns, top
-// segment first. For each segment the warp recomputes its columns from the forward
-// pass's checkpoint (the same window, shifts and block updates, so the same bits), keeps
-// their {VP, HP} records in shared memory, and every lane whose walk is inside the
-// segment moves through it one event at a time (D run, I move or diagonal cell, with
-// the precedence of myers_backtrace_flat) until it leaves the segment's columns. Returns
-// false when the walk left the band or cost more than E (the pair is then redone).
+// Traceback of one lane's pair from (m, n) over segments of kSegCols columns, top segment
+// first. In a segment a lane's path stays in the 64-row block it enters by the last column
+// and the one above (a longer D run takes another round), so only those two are
+// recomputed, from the segment's checkpoint and the horizontal deltas the forward pass
+// kept for every block: the same block updates on the same inputs, hence the same bits,
+// without the other blocks of the window and without one block waiting for the other's
+// carry. Then every lane moves through its records one event at a time (D run, I move or
+// diagonal cell, with the precedence of myers_backtrace_flat). Recomputing the whole window
+// (3.6 blocks on average in the 64-2048 bp set) made the traceback as long as the forward
+// pass: 13.4 ms per 1,000,000 pairs against 9.6 now. Returns false when the walk left
+// the band or cost more than E (the pair is then redone).
 template <int P>
 __device__ __forceinline__ bool lane_trace_ck(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb,
                                               int m, int n, int nb, const LaneBand& band, const LaneGeom& g, bool act,
-                                              uint8_t* ck, uint8_t* smem, RunWriter& rw, int* ed_out) {
+                                              const uint8_t* ck, const uint8_t* hin, const uint4* planes, uint8_t* smem,
+                                              RunWriter& rw,
+                                              int* ed_out) {
     const int lane = lane_id();
-    uint64_t* ring = reinterpret_cast<uint64_t*>(smem);
-    uint4* seg = reinterpret_cast<uint4*>(ck + lane_ckpt_bytes(g.n_max, P));
+    uint4* seg = reinterpret_cast<uint4*>(smem) + lane;
     int i = act ? m : 0, j = act ? n : 0, cost = 0;
     bool ok = act;
-    int q_idx = -1;       // query word held in q_word (the walk's row moves slowly)
-    uint32_t q_word = 0;
-    if (g.n_max > 0) {
-        const int S = (g.n_max - 1) / kSegCols;
-        int ring_lo = lane_blo(g, S * kSegCols);  // the ring holds blocks [ring_lo, ring_lo + P]
+    int held[2] = {-1, -1};   // blocks whose bit planes the lane holds, by parity
+    uint4 pl[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    for (int sgi = (g.n_max - 1) / kSegCols; sgi >= 0 && g.n_max > 0; --sgi) {
+        const int j0 = sgi * kSegCols;
+        const int jend = min(j0 + kSegCols, g.n_max), cols = jend - j0;
+        const int blo0 = lane_blo(g, j0), blo_end = lane_blo(g, jend);
+        // target symbols j0 .. j0 + kSegCols - 1 share one 16-symbol word (kSegCols divides 16)
+        const int wj = j0 >> 4;
+        const uint32_t tw = wj * 16 < n ? __ldg(tb + wj) : 0u;
+        for (;;) {
+            const bool in = ok && i > 0 && j > j0;
+            if (!__any_sync(PHR_FULL_MASK, in)) break;
+            // ---- recompute the path's block and the one above ----
+            const int b1 = in ? (i - 1) >> 6 : -1;
+            uint64_t vp[2], vn[2];   // by parity of the block
+            uint32_t ha[2];
+            int blk[2];
 #pragma unroll
-        for (int k = 0; k <= P; ++k) ring_fill<P>(ring, qb, ring_lo + k, nb, lane);
-        for (int sgi = S; sgi >= 0; --sgi) {
-            const int j0 = sgi * kSegCols;
-            const int blo0 = lane_blo(g, j0);
-            if (blo0 < ring_lo) {  // one block enters the ring at the top (in the slot of ring_lo + P)
-                ring_lo = blo0;
-                ring_fill<P>(ring, qb, ring_lo, nb, lane);
-            }
-            // ---- recompute columns j0 + 1 .. min(j0 + kSegCols, n_max) ----
-            uint64_t vp[P], vn[P];
-            if (sgi == 0) {
-#pragma unroll
-                for (int k = 0; k < P; ++k) {
-                    vp[k] = ~0ull;
-                    vn[k] = 0;
-                }
-            } else {
-                const uint8_t* c = ck + ck_off<P>(sgi - 1, 0, lane);
-#pragma unroll
-                for (int k = 0; k < P; ++k) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(c + k * 512);
-                    vp[k] = mk64(x.x, x.y);
-                    vn[k] = mk64(x.z, x.w);
-                }
-            }
-            int blo = blo0;
-            const int jend = min(j0 + kSegCols, g.n_max);
-            // target symbols j0 .. j0 + kSegCols - 1 share one 16-symbol word (kSegCols divides 16)
-            const int wj = j0 >> 4;
-            const uint32_t tw = wj * 16 < n ? __ldg(tb + wj) : 0u;
-            // (each lane reads back only the records it wrote: no barrier is needed)
-            for (int jj = j0 + 1; jj <= jend; ++jj) {  // warp-uniform
-                if (g.slide && lane_blo(g, jj) > blo) {  // the window moves down one block
-#pragma unroll
-                    for (int k = 0; k + 1 < P; ++k) {
-                        vp[k] = vp[k + 1];
-                        vn[k] = vn[k + 1];
+            for (int par = 0; par < 2; ++par) {
+                const int b = (b1 & 1) == par ? b1 : b1 - 1;
+                blk[par] = b;
+                vp[par] = ~0ull;
+                vn[par] = 0;
+                ha[par] = 0xAAAAu;   // +1 in every column: the window's top block
+                if (in && b >= 0) {
+                    const int s0 = b - blo0, se = b - blo_end;
+                    if (sgi > 0 && s0 >= 0 && s0 < P) {
+                        const uint4 x = *reinterpret_cast<const uint4*>(ck + ck_off<P>(sgi - 1, s0, lane));
+                        vp[par] = mk64(x.x, x.y);
+                        vn[par] = mk64(x.z, x.w);
                     }
-                    vp[P - 1] = ~0ull;
-                    vn[P - 1] = 0;
-                    ++blo;
+                    if (se >= 0 && se < P) ha[par] = *reinterpret_cast<const uint16_t*>(hin + hin_off<P>(sgi, se, lane));
+                    if (held[par] != b) {
+                        held[par] = b;
+                        pl[par] = planes[b * 32 + lane];
+                    }
                 }
-                const uint32_t c = (tw >> (((jj - 1) & 15) * 2)) & 3u;
-                uint4* out = seg + (jj - j0 - 1) * (P * 32) + lane;
-                uint32_t pa = 0, ma = 0;
-#pragma unroll
-                for (int k = 0; k < P; ++k) {
-                    int rs = (blo + k) % (P + 1);
-                    const uint64_t eq = ring[(rs * 4 + c) * 32 + lane];
-                    const uint64_t ph = k == 0 ? advance_block<true>(vp[0], vn[0], eq, pa, ma)
-                                               : advance_block<false>(vp[k], vn[k], eq, pa, ma);
-                    out[k * 32] = make_uint4(lo32(vp[k]), hi32(vp[k]), lo32(ph), hi32(ph));
-                }
+                ha[par] <<= 2 * (kSegCols - cols);   // the first column's bits highest
             }
-            __syncwarp();
-            // ---- walk every lane through this segment's columns ----
+            // column at which the window slides within the segment: a block entering there starts
+            // anew (its updates before are never read)
+            const int t_slide = blo_end > blo0 ? g.dmax + 1 + 64 * blo_end - (j0 + 1) : -1;
+            // (rolled: two block updates are the body. Unrolled eight times, warps at different
+            // places of the trace evicted one another's instructions: 7 of 12 cycles between two
+            // issues of a warp were waits for instructions, 12.6 ms against 9.6)
+            uint4* out = seg;
+            uint32_t syms = tw >> ((j0 & 15) * 2);
+#pragma unroll 1
+            for (int t = 0; t < cols; ++t) {   // warp-uniform
+                if (t == t_slide) {
+#pragma unroll
+                    for (int par = 0; par < 2; ++par)
+                        if (blk[par] - blo0 >= P) {
+                            vp[par] = ~0ull;
+                            vn[par] = 0;
+                        }
+                }
+                const uint32_t n0 = (syms & 1u) - 1u, n1 = ((syms >> 1) & 1u) - 1u;   // ~0 where the symbol's bit is 0
+#pragma unroll
+                for (int par = 0; par < 2; ++par) {
+                    const uint64_t eq = mk64((pl[par].x ^ n0) & (pl[par].z ^ n1), (pl[par].y ^ n0) & (pl[par].w ^ n1));
+                    uint32_t pa = ha[par] << 16, ma = ha[par] << 17;   // bit 15: +1, bit 14: -1
+                    const uint64_t ph = advance_block<false>(vp[par], vn[par], eq, pa, ma);
+                    out[par * 32] = make_uint4(lo32(vp[par]), hi32(vp[par]), lo32(vp[par] | ph), hi32(vp[par] | ph));
+                    ha[par] <<= 2;
+                }
+                out += 64;
+                syms >>= 2;
+            }
+            // (each lane reads back only the records it wrote: no barrier is needed)
+            // ---- walk every lane through its two blocks of this segment ----
+            const uint8_t* st = reinterpret_cast<const uint8_t*>(seg) + 8;   // VP | HP of column 0, even block
             for (;;) {
-                const bool want = ok && i > 0 && j > j0;
+                const int b = (i - 1) >> 6;
+                const bool want = ok && i > 0 && j > j0 && b1 - b < 2;
                 if (!__any_sync(PHR_FULL_MASK, want)) break;
                 if (!want) continue;
-                const int kb = ((i - 1) >> 6) - lane_blo(g, j);
-                if (kb < 0 || kb >= P) {
-                    ok = false;
-                    continue;
-                }
-                const uint4 R = seg[((j - j0 - 1) * P + kb) * 32 + lane];
-                const uint64_t vpb = mk64(R.x, R.y), hpb = mk64(R.z, R.w);
-                const int bit = (i - 1) & 63;
-                if ((vpb >> bit) & 1ull) {
-                    // D run: consecutive VP bits upward from row i within this block
-                    const int run = __clzll(~(vpb << (63 - bit)));
-                    rw.push(3, static_cast<uint32_t>(run));
-                    i -= run;
-                    cost += run;
-                } else if ((hpb >> bit) & 1ull) {
-                    rw.push(2, 1);
-                    j -= 1;
-                    cost += 1;
+                const int kb = b - lane_blo(g, j);
+                const int t = j - 1 - j0, r = i - 1, bit = r & 63;
+                const uint4 R = seg[(t * 2 + (b & 1)) * 32];
+                const uint64_t vpb = mk64(R.x, R.y);
+                const uint32_t sw = bit & 32 ? R.w : R.z;
+                uint32_t op, count, neq = 0;   // first run of this step; differences of the cells after it
+                int done = 0, run = 0;         // diagonal cells pushed, of `run`
+                if ((sw >> (bit & 31)) & 1u) {
+                    // D run: consecutive VP bits upward from row i within this block; else I
+                    const int up = static_cast<int>(__clzll(~(vpb << (63 - bit))));
+                    op = up > 0 ? 3u : 2u;
+                    count = static_cast<uint32_t>(max(up, 1));
+                    cost += max(up, 1);
+                    i -= up;
+                    j -= up > 0 ? 0 : 1;
                 } else {
-                    // target symbol j - 1 from the segment's word; query word cached
-                    const int qwi = (i - 1) >> 4;
-                    if (qwi != q_idx) {
-                        q_idx = qwi;
-                        q_word = __ldg(qb + qwi);
+                    // diagonal stretch: up to the first cell with a VP or HP bit, or out of the
+                    // segment (eight rows up at most: still in the two blocks)
+                    const int most = min(t + 1, i);
+                    uint32_t stop = ~0u << most;
+#pragma unroll
+                    for (int u = 1; u < kSegCols; ++u) {
+                        const int ru = r - u;
+                        uint32_t w = 0;
+                        if (u <= t)
+                            w = *reinterpret_cast<const uint32_t*>(st + (t - u) * 1024 + ((ru << 3) & 512) + ((ru >> 3) & 4));
+                        stop |= ((w >> (ru & 31)) & 1u) << u;
                     }
-                    const uint32_t qs = (q_word >> (((i - 1) & 15) * 2)) & 3u;
-                    const uint32_t ts = (tw >> (((j - 1) & 15) * 2)) & 3u;
-                    const uint32_t x = qs != ts ? 1u : 0u;
-                    rw.push(x, 1);
-                    cost += static_cast<int>(x);
-                    i -= 1;
-                    j -= 1;
+                    run = __ffs(stop) - 1;   // >= 1: cell 0 is diagonal
+                    // M / X: cell u compares query symbol i - 1 - u with target symbol j - 1 - u, both
+                    // at index 7 - u of their windows
+                    const int pos = (j - 1) & 15;
+                    const uint32_t tsym = static_cast<uint32_t>((static_cast<uint64_t>(tw) << 14) >> (2 * pos));
+                    const uint32_t x = diag_window(qb, i) ^ tsym;
+                    const uint32_t nz = (x | (x >> 1)) & 0x5555u;
+                    neq = even_bits(__brev(nz) >> 17) & ((1u << run) - 1u);   // bit u: cell u differs
+                    cost += __popc(neq);
+                    i -= run;
+                    j -= run;
+                    op = 0;
+                    count = neq ? __ffs(neq) - 1 : run;
+                    done = static_cast<int>(count);
+                }
+                for (;;) {   // one push in the code: matches and differences in turn
+                    rw.push(op, count);
+                    if (done >= run) break;
+                    op ^= 1u;
+                    const uint32_t rest = (op ? ~neq : neq) >> done;   // bit 0: the run ends here (never)
+                    count = static_cast<uint32_t>(min(rest ? __ffs(rest) - 1 : 32, run - done));
+                    done += static_cast<int>(count);
                 }
                 const int d = j - i;
-                if (d < band.dmin || d > band.dmax || cost > band.E) ok = false;
+                if (kb < 0 || kb >= P || d < band.dmin || d > band.dmax || cost > band.E) ok = false;
             }
         }
     }
@@ -536,12 +584,14 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     const int nb = (m + 63) >> 6;
     const uint32_t* qb = Pm.packed2 + (act ? d.q_word : 0);
     const uint32_t* tb = Pm.packed2 + (act ? d.t_word : 0);
-    lane_forward<P, CK>(qb, tb, n, nb, g, sp, slot);
+    uint8_t* hin = slot + lane_ckpt_bytes(g.n_max, P);   // checkpoint mode
+    uint4* planes = reinterpret_cast<uint4*>(hin + lane_hin_bytes(g.n_max, P));
+    lane_forward<P, CK>(qb, tb, n, nb, g, sp, slot, hin, planes);
     // work counter: block-columns this task evaluated for its pairs
     const unsigned long long cols = __reduce_add_sync(PHR_FULL_MASK, act ? static_cast<unsigned>(n) * P : 0u);
     if (lane == 0) atomicAdd(Pm.work, cols);
     __syncwarp();  // the traceback reuses the Peq shared memory
-    const uint64_t rec_bytes = lane_rec_bytes(g.n_max, P, CK ? 1 : 0);
+    const uint64_t rec_bytes = lane_rec_bytes(g.n_max, g.m_max, P, CK ? 1 : 0);
     const uint32_t cap = static_cast<uint32_t>(g.m_max + g.n_max + 2);
     uint32_t* runs = reinterpret_cast<uint32_t*>(slot + rec_bytes) + static_cast<uint64_t>(lane) * cap;
     RunWriter rw;
@@ -549,7 +599,7 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     int ed = 0;
     bool ok;
     if (CK)
-        ok = lane_trace_ck<P>(qb, tb, m, n, nb, band, g, act, slot, reinterpret_cast<uint8_t*>(sp), rw, &ed);
+        ok = lane_trace_ck<P>(qb, tb, m, n, nb, band, g, act, slot, hin, planes, reinterpret_cast<uint8_t*>(sp), rw, &ed);
     else
         ok = lane_trace<P>(qb, tb, m, n, band, g, act, slot, reinterpret_cast<uint4*>(sp) + lane, rw, &ed);
     // work counter: pairs sent to redo
@@ -638,9 +688,6 @@ __device__ __forceinline__ void lane_tasks(const ExtendParams& Pm, uint64_t* sp)
         __syncwarp();
     }
 }
-
-constexpr int kLanePeqWarpBytes = kLaneMaxSlots * 4 * 32 * 8;  // Peq (and traceback buffers) per warp
-static_assert(kLanePeqWarpBytes <= kCkWarpBytes, "the forward pass's Peq must fit the checkpoint-mode area");
 
 __global__ void __launch_bounds__(kLaneThreads, 2) myers_lane_kernel(ExtendParams Pm) {
     extern __shared__ uint64_t lane_smem[];
