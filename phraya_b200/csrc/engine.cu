@@ -148,10 +148,8 @@ struct PrepParams {
     uint64_t* tb;      // text bound per pair
 };
 
-// Suffix lengths, seed validation, arena sizes. One thread per pair.
-__global__ void prep_sizes_kernel(PrepParams P) {
-    const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    if (i >= P.in.n) return;
+// Suffix lengths, seed validation, arena sizes of pair i.
+__device__ __forceinline__ void prep_pair(const PrepParams& P, uint64_t i) {
     const uint32_t ql = P.in.q_len[i], tl = P.in.t_len[i];
     uint32_t qs = P.in.q_seed ? P.in.q_seed[i] : 0, ts = P.in.t_seed ? P.in.t_seed[i] : 0;
     if (P.engine == PHR_ENGINE_MYERS_GLOBAL) qs = ts = 0;
@@ -171,6 +169,11 @@ __global__ void prep_sizes_kernel(PrepParams P) {
     P.w2[i] = d.trivial ? 0 : (qn + 15) / 16 + 4 + (tn + 15) / 16 + 4;
     P.wb[i] = d.trivial ? 0 : (qn + 3) / 4 + 4 + (tn + 3) / 4 + 4;
     P.tb[i] = 2 * (qn + tn) + 16;
+}
+
+__global__ void prep_sizes_kernel(PrepParams P) {
+    const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    if (i < P.in.n) prep_pair(P, i);
 }
 
 __device__ __forceinline__ uint32_t code2(uint8_t b, bool& pure) {
@@ -233,11 +236,7 @@ struct PackParams {
 // 2-bit packing (16 bases per word) of both suffixes; a pair holding any byte other
 // than A/C/G/T is also copied word-aligned to the byte arena and runs the byte path.
 // Trivial pairs (an empty suffix) get their final result here. One warp per pair.
-__global__ void pack_kernel(PackParams P) {
-    const uint64_t warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= P.in.n) return;
-    const uint64_t i = warp;
+__device__ __forceinline__ void pack_pair(const PackParams& P, uint64_t i, int lane) {
     PairDesc d = P.desc[i];
     if (d.trivial) {
         if (lane == 0) {
@@ -372,6 +371,11 @@ __global__ void pack_kernel(PackParams P) {
     }
 }
 
+__global__ void pack_kernel(PackParams P) {
+    const uint64_t warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
+    if (warp < P.in.n) pack_pair(P, warp, threadIdx.x & 31);
+}
+
 struct TaskBuild {
     const uint32_t* keys;      // sorted
     const uint32_t* order;     // sorted pair ids
@@ -428,8 +432,8 @@ __device__ __forceinline__ uint64_t myers_need_est(int m, int n, int G, int band
     return need;
 }
 
-__global__ void task_fill_kernel(TaskBuild T) {
-    const uint64_t p = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+// Task of sorted position p; called by whole warps.
+__device__ __forceinline__ void task_fill(const TaskBuild& T, uint64_t p) {
     // every lane stays to the warp-level reductions at the end; lanes without a task
     // contribute nothing to them
     const bool has_task = p < T.n && T.flag[p];
@@ -512,14 +516,17 @@ __global__ void task_fill_kernel(TaskBuild T) {
     }
 }
 
-__global__ void task_finalize_kernel(TaskBuild T) {
-    uint32_t nt = 0;
-    if (T.n > 0) nt = T.tidx[T.n - 1] + T.flag[T.n - 1];
-    const uint32_t split = min(*T.split_min, nt);
+__global__ void task_fill_kernel(TaskBuild T) {
+    task_fill(T, blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x);
+}
+
+// Task ranges from the number of tasks and the reduced first tasks. One thread.
+__device__ __forceinline__ void task_ranges(const TaskBuild& T, uint32_t nt) {
+    const uint32_t split = min(__ldcg(T.split_min), nt);
     // segments of each mode in key order: warp groups, one-warp tiles, CTA tiles
     for (int m = 0; m < 2; ++m) {
         const uint32_t begin = m ? split : 0, end = m ? nt : split;
-        const uint32_t cta = min(T.tile_min[2 + m], end), warp = min(T.tile_min[m], cta);
+        const uint32_t cta = min(__ldcg(T.tile_min + 2 + m), end), warp = min(__ldcg(T.tile_min + m), cta);
         T.ranges[2 * m] = begin;
         T.ranges[2 * m + 1] = warp;
         T.tile_ranges[2 * m] = warp;
@@ -528,11 +535,142 @@ __global__ void task_finalize_kernel(TaskBuild T) {
         T.tile_ranges[4 + 2 * m + 1] = end;
     }
     // lane-kernel range {0, g1} and warp-group 2-bit range {g1, split} (global Myers)
-    const uint32_t g1 = min(*T.g1_min, split);
+    const uint32_t g1 = min(__ldcg(T.g1_min), split);
     T.ranges[28] = 0;
     T.ranges[29] = g1;
     T.ranges[30] = g1;
     T.ranges[31] = split;
+}
+
+__global__ void task_finalize_kernel(TaskBuild T) {
+    task_ranges(T, T.n > 0 ? T.tidx[T.n - 1] + T.flag[T.n - 1] : 0);
+}
+
+// ---------------------------------------------------------------------------
+// Small batches: one CTA does what the scans, the sort and the task build do for a large
+// one, a thread per pair. A call on a few pairs is bound by its launches, copies and
+// waits: 31 launches and 8 copies of 0.1 ms of kernels took 0.25 ms.
+// ---------------------------------------------------------------------------
+constexpr int kSmallPairs = 1024;
+constexpr int kTinyPairs = 32;      // few enough to be packed by the same CTA, a warp each
+
+// Exclusive sum over the CTA's kSmallPairs threads; `sh` holds a value per warp.
+__device__ __forceinline__ uint64_t cta_excl_sum(uint64_t v, uint64_t* sh, uint64_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t up = __shfl_up_sync(PHR_FULL_MASK, incl, o);
+        if (lane >= o) incl += up;
+    }
+    __syncthreads();   // sh may still be read from the last call
+    if (lane == 31) sh[warp] = incl;
+    __syncthreads();
+    uint64_t before = 0, all = 0;
+    for (int w = 0; w < kSmallPairs / 32; ++w) {
+        const uint64_t x = sh[w];
+        if (w < warp) before += x;
+        all += x;
+    }
+    *total = all;
+    return before + incl - v;
+}
+
+// Sorts the keys (stable: pair ids break ties) and builds the task list.
+__device__ void small_tasks(const TaskBuild& T, const uint32_t* keys_in, uint32_t* keys_out, uint32_t* order_out,
+                            uint64_t* sh_sort, uint64_t* sh_sum) {
+    const int t = threadIdx.x, n = static_cast<int>(T.n);
+    int m = 32;
+    while (m < n) m <<= 1;
+    sh_sort[t] = t < n ? static_cast<uint64_t>(keys_in[t]) << 32 | static_cast<uint32_t>(t) : ~0ull;
+    __syncthreads();
+    for (int k = 2; k <= m; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const int o = t ^ j;
+            if (t < m && o > t) {
+                const uint64_t a = sh_sort[t], b = sh_sort[o];
+                if ((a > b) == ((t & k) == 0)) {
+                    sh_sort[t] = b;
+                    sh_sort[o] = a;
+                }
+            }
+            __syncthreads();
+        }
+    const uint32_t key = static_cast<uint32_t>(sh_sort[t] >> 32);
+    const uint32_t id = static_cast<uint32_t>(sh_sort[t]);
+    const bool first = t < n && (t == 0 || key_seg(static_cast<uint32_t>(sh_sort[t > 0 ? t - 1 : 0] >> 32)) != key_seg(key));
+    if (t < n) {
+        keys_out[t] = key;
+        order_out[t] = id;
+    }
+    // start of this position's segment: the last `first` at or before it
+    int head = first ? t : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) head = max(head, __shfl_up_sync(PHR_FULL_MASK, head, o));
+    __syncthreads();
+    if ((t & 31) == 31) sh_sum[t >> 5] = static_cast<uint64_t>(head);
+    __syncthreads();
+    for (int w = 0; w < t >> 5; ++w) head = max(head, static_cast<int>(sh_sum[w]));
+    const uint32_t per = 32 / key_group(key);
+    const bool task = t < n && key != kInvalidKey && ((t - head) % per) == 0;
+    uint64_t nt = 0;
+    const uint64_t at = cta_excl_sum(task ? 1 : 0, sh_sum, &nt);
+    if (t < n) {
+        T.flag[t] = task ? 1u : 0u;
+        T.tidx[t] = static_cast<uint32_t>(at);
+    }
+    __syncthreads();
+    task_fill(T, t);
+    __syncthreads();
+    if (t == 0) task_ranges(T, static_cast<uint32_t>(nt));
+}
+
+struct SmallBuild {
+    PrepParams prep;
+    PackParams pack;
+    TaskBuild tasks;
+    uint64_t *w2o, *wbo, *tbo;
+    uint32_t* cnt;       // counter block, set up here
+    uint32_t *keys_s, *order;
+};
+
+// Counter block, pair descriptors and arena offsets; tiny batches are packed and their
+// tasks built as well.
+__global__ void __launch_bounds__(kSmallPairs) small_build_kernel(SmallBuild B, bool tiny) {
+    __shared__ uint64_t sh_sort[kSmallPairs];
+    __shared__ uint64_t sh_sum[32];
+    const int t = threadIdx.x, n = static_cast<int>(B.prep.in.n);
+    if (t < 64) {   // the "first task" counters start at their maximum
+        const bool is_min = t == 4 || t == 20 || (t >= 40 && t < 44);
+        B.cnt[t] = is_min ? 0xFFFFFFFFu : 0u;
+        B.tasks.need_hist[t] = 0;
+    }
+    uint64_t w2 = 0, wb = 0, tb = 0, total;
+    if (t < n) {
+        prep_pair(B.prep, t);
+        w2 = B.prep.w2[t];
+        wb = B.prep.wb[t];
+        tb = B.prep.tb[t];
+    }
+    w2 = cta_excl_sum(w2, sh_sum, &total);
+    wb = cta_excl_sum(wb, sh_sum, &total);
+    tb = cta_excl_sum(tb, sh_sum, &total);
+    if (t < n) {
+        B.w2o[t] = w2;
+        B.wbo[t] = wb;
+        B.tbo[t] = tb;
+    }
+    if (!tiny) return;
+    __syncthreads();
+    if ((t >> 5) < n) pack_pair(B.pack, t >> 5, t & 31);
+    __syncthreads();
+    small_tasks(B.tasks, B.pack.keys, B.keys_s, B.order, sh_sort, sh_sum);
+}
+
+__global__ void __launch_bounds__(kSmallPairs) small_tasks_kernel(SmallBuild B) {
+    __shared__ uint64_t sh_sort[kSmallPairs];
+    __shared__ uint64_t sh_sum[32];
+    small_tasks(B.tasks, B.pack.keys, B.keys_s, B.order, sh_sort, sh_sum);
 }
 
 // Redo pass task list: one pair per task, in redo order.
@@ -576,6 +714,8 @@ struct FinishParams {
     uint32_t* error_flag;
     uint64_t cigar_base;
     int per_warp;            // pairs a warp writes (1..32)
+    const uint32_t* redo_count;
+    uint64_t* total;         // text bytes of all pairs
 };
 
 __global__ void text_len_kernel(const PairOut* out, uint64_t n, uint64_t* len) {
@@ -616,11 +756,7 @@ __device__ __forceinline__ void copy_text(char* dst, const char* src, uint32_t l
 // contiguous), then the lanes copy the pairs' texts one pair after the other. 32 pairs per
 // warp in a large batch; fewer when there are few pairs, whose texts then are copied side
 // by side (500 texts of ~3 kB: 0.60 ms with 32 per warp and byte copies, below 0.01 ms now).
-__global__ void finish_kernel(FinishParams F) {
-    const uint64_t first =
-        ((blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5) * static_cast<uint64_t>(F.per_warp);
-    const int lane = threadIdx.x & 31;
-    if (first >= F.n) return;
+__device__ __forceinline__ void finish_pairs(const FinishParams& F, uint64_t first, int lane) {
     const uint64_t i = first + lane;
     uint64_t off = 0, toff = 0;
     uint32_t len = 0;
@@ -668,6 +804,42 @@ __global__ void finish_kernel(FinishParams F) {
     }
 }
 
+// Launched before the host knows how the pass went: nothing is written when pairs are to be
+// redone or the text does not fit (the host looks at both next).
+__device__ __forceinline__ bool finish_blocked(const FinishParams& F) {
+    return __ldcg(F.redo_count) != 0 || __ldcg(F.total) > F.cigar_capacity;
+}
+
+__global__ void finish_kernel(FinishParams F) {
+    const uint64_t first =
+        ((blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5) * static_cast<uint64_t>(F.per_warp);
+    if (first >= F.n || finish_blocked(F)) return;
+    finish_pairs(F, first, threadIdx.x & 31);
+}
+
+// The tail of a small batch in one CTA: text offsets and total, and with `texts` the records
+// and texts too.
+__global__ void __launch_bounds__(kSmallPairs) small_tail_kernel(FinishParams F, uint64_t* tlen, bool texts) {
+    __shared__ uint64_t sh_sum[32];
+    const int t = threadIdx.x;
+    uint64_t len = 0, total = 0;
+    if (t < static_cast<int>(F.n)) {
+        const PairOut o = F.out[t];
+        len = o.status == PHR_OK ? o.text_len : 0;
+    }
+    const uint64_t off = cta_excl_sum(len, sh_sum, &total);
+    if (t < static_cast<int>(F.n)) {
+        tlen[t] = len;
+        F.cig_off[t] = off;
+    }
+    if (t == 0) *F.total = total;
+    __threadfence_block();
+    __syncthreads();
+    if (!texts || *F.redo_count != 0 || total > F.cigar_capacity) return;
+    const uint64_t first = static_cast<uint64_t>(t >> 5) * F.per_warp;   // per_warp covers n with 32 warps
+    if (first < F.n) finish_pairs(F, first, t & 31);
+}
+
 __global__ void total_kernel(const uint64_t* off, const uint64_t* len, uint64_t n, uint64_t* total) {
     *total = n ? off[n - 1] + len[n - 1] : 0;
 }
@@ -685,6 +857,20 @@ __global__ void sum_lengths_kernel(const uint32_t* a, const uint32_t* b, uint64_
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(PHR_FULL_MASK, acc, o);
     if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
 }
+
+// The same for few lengths, one CTA: no counter to clear first.
+__global__ void sum_lengths_small_kernel(const uint32_t* a, const uint32_t* b, uint32_t n, unsigned long long* out) {
+    __shared__ unsigned long long sh[32];
+    unsigned long long acc = 0;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) acc += static_cast<unsigned long long>(a[i]) + b[i];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(PHR_FULL_MASK, acc, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (unsigned w = 1; w < blockDim.x / 32; ++w) acc += sh[w];
+        *out = acc;
+    }
+}
 }  // namespace
 
 uint64_t device_length_sum(Ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, cudaError_t* err) {
@@ -694,15 +880,18 @@ uint64_t device_length_sum(Ctx* ctx, const uint32_t* a, const uint32_t* b, uint6
         if (*err != cudaSuccess) return 0;
     }
     if (!ctx->h_pinned) {
-        *err = cudaMallocHost(&ctx->h_pinned, 256);
+        *err = cudaMallocHost(&ctx->h_pinned, kPinnedBytes);
         if (*err != cudaSuccess) return 0;
     }
     unsigned long long* d = reinterpret_cast<unsigned long long*>(ctx->d_counters);
     unsigned long long* h = static_cast<unsigned long long*>(ctx->h_pinned);
     cudaStream_t st = ctx->stream;
-    if ((*err = cudaMemsetAsync(d, 0, 8, st)) != cudaSuccess) return 0;
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 4ull * ctx->sm_count));
-    {
+    if (n <= 16384) {
+        KernelScope ks(ctx, "sum_lengths");
+        sum_lengths_small_kernel<<<1, 1024, 0, st>>>(a, b, static_cast<uint32_t>(n), d);
+    } else {
+        if ((*err = cudaMemsetAsync(d, 0, 8, st)) != cudaSuccess) return 0;
         KernelScope ks(ctx, "sum_lengths");
         sum_lengths_kernel<<<std::max(1u, grid), 256, 0, st>>>(a, b, n, d);
     }
@@ -774,7 +963,6 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     unsigned long long* redo_need = static_cast<unsigned long long*>(take(n * 8));
     uint64_t* rtask_off = static_cast<uint64_t*>(take(n * 8));
     uint64_t* rtask_len = static_cast<uint64_t*>(take(n * 8));
-    unsigned int* need_hist = static_cast<unsigned int*>(take(64 * 4));
     // counters: [0..3] ranges, [4] split_min, [5] queue head 0, [6] queue head 1,
     // [7] redo count, [8..9] need max (u64), [10] error flag, [12..13] total (u64), [14..17] redo ranges,
     // [20] first multi-lane 2-bit task, [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
@@ -782,89 +970,115 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // [40..43] first register-tile task of each kind (one warp 2-bit / bytes, CTA 2-bit / bytes),
     // [44..51] their ranges, [52..55] their scratch need: sum, largest (u64), [56..59] their queue
     // heads, [60..61] pool bytes taken (u64), [62] deferred register-tile pairs, [63] their queue head
-    uint32_t* cnt = static_cast<uint32_t*>(take(256));
+    // The histogram of the tasks' needs follows, so that one copy brings both back.
+    uint32_t* cnt = static_cast<uint32_t*>(take(512));
     if (!cnt) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted");
+    unsigned int* need_hist = cnt + 64;
+    if (!ctx->h_pinned) PHR_CUDA_TRY(ctx, cudaMallocHost(&ctx->h_pinned, kPinnedBytes));
+    const uint32_t* h_cnt = static_cast<const uint32_t*>(ctx->h_pinned);   // the host's copy of both
+    auto read_counters = [&](size_t bytes) -> cudaError_t {
+        const cudaError_t e = cudaMemcpyAsync(ctx->h_pinned, cnt, bytes, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    };
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
     uint64_t* total = reinterpret_cast<uint64_t*>(cnt + 12);
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 256, st));
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 4, 0xFF, 4, st));
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 20, 0xFF, 4, st));
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 40, 0xFF, 16, st));
-
-    // CUB temp sizes
-    size_t t_sort = 0, t_scan = 0, t_max = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, t_sort, keys, keys_s, vals, order, static_cast<int>(n), 0, 32, st);
-    cub::DeviceScan::ExclusiveSum(nullptr, t_scan, w2, w2o, static_cast<int>(n), st);
-    cub::DeviceScan::InclusiveScan(nullptr, t_max, head, head_s, cub::Max(), static_cast<int>(n), st);
-    size_t t_scan32 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, t_scan32, flag, tidx, static_cast<int>(n), st);
-    const size_t t_need = std::max({t_sort, t_scan, t_max, t_scan32});
-    void* tmp = take(t_need);
-    if (!tmp) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted (cub)");
-
     const unsigned T = 256;
+    const bool small = n <= kSmallPairs;
     // lanes per short WFA pair: affine and linear tune separately
     const int g_short = engine == PHR_ENGINE_WFA_AFFINE ? ctx->tune.wfa_affine_group_short : ctx->tune.wfa_group_short;
-    PrepParams pp{in, engine, costs, desc, pout, w2, wb, tb};
-    {
-        KernelScope ks(ctx, "prep_sizes");
-        prep_sizes_kernel<<<blocks_for(n, T), T, 0, st>>>(pp);
-    }
-    size_t tn_ = t_need;
-    cub::DeviceScan::ExclusiveSum(tmp, tn_, w2, w2o, static_cast<int>(n), st);
-    tn_ = t_need;
-    cub::DeviceScan::ExclusiveSum(tmp, tn_, wb, wbo, static_cast<int>(n), st);
-    tn_ = t_need;
-    cub::DeviceScan::ExclusiveSum(tmp, tn_, tb, tbo, static_cast<int>(n), st);
-
-    PackParams pk{in, engine, costs, desc, pout, w2o, wbo, tbo, arena2, arenab, text, keys, vals,
-                  g_short, ctx->tune.wfa_group_long, ctx->tune.wfa_long_min,
-                  ctx->tune.myers_band_base, ctx->tune.wfa_big_min};
-    {
-        KernelScope ks(ctx, "pack");
-        pack_kernel<<<blocks_for(n * 32, T), T, 0, st>>>(pk);
-    }
-    tn_ = t_need;
-    cub::DeviceRadixSort::SortPairs(tmp, tn_, keys, keys_s, vals, order, static_cast<int>(n), 0, 32, st);
-
-    PHR_CUDA_TRY(ctx, cudaMemsetAsync(need_hist, 0, 64 * 4, st));
-    TaskBuild tbp{keys_s, order, n, head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4, cnt + 20, desc,
-                  engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
+    const PrepParams pp{in, engine, costs, desc, pout, w2, wb, tb};
+    const PackParams pk{in, engine, costs, desc, pout, w2o, wbo, tbo, arena2, arenab, text, keys, vals,
+                        g_short, ctx->tune.wfa_group_long, ctx->tune.wfa_long_min,
+                        ctx->tune.myers_band_base, ctx->tune.wfa_big_min};
+    TaskBuild tbp{keys_s, order, n, small ? head_s : head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4,
+                  cnt + 20, desc, engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
                   ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt,
                   cnt + 40, cnt + 44, reinterpret_cast<unsigned long long*>(cnt + 52)};
-    {
-        KernelScope ks(ctx, "task_head");
-        task_head_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
-    }
-    tn_ = t_need;
-    cub::DeviceScan::InclusiveScan(tmp, tn_, head, head_s, cub::Max(), static_cast<int>(n), st);
-    tbp.head = head_s;
-    {
-        KernelScope ks(ctx, "task_flag");
-        task_flag_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
-    }
-    tn_ = t_need;
-    cub::DeviceScan::ExclusiveSum(tmp, tn_, flag, tidx, static_cast<int>(n), st);
-    {
-        KernelScope ks(ctx, "task_fill");
-        task_fill_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
-    }
-    {
-        KernelScope ks(ctx, "task_finalize");
-        task_finalize_kernel<<<1, 1, 0, st>>>(tbp);
+    size_t t_need = 0, tn_ = 0;
+    void* tmp = nullptr;
+    if (small) {
+        const SmallBuild sb{pp, pk, tbp, w2o, wbo, tbo, cnt, keys_s, order};
+        const bool tiny = n <= kTinyPairs;
+        {
+            KernelScope ks(ctx, "small_build");
+            small_build_kernel<<<1, kSmallPairs, 0, st>>>(sb, tiny);
+        }
+        if (!tiny) {
+            {
+                KernelScope ks(ctx, "pack");
+                pack_kernel<<<blocks_for(n * 32, T), T, 0, st>>>(pk);
+            }
+            KernelScope ks(ctx, "small_tasks");
+            small_tasks_kernel<<<1, kSmallPairs, 0, st>>>(sb);
+        }
+    } else {
+        PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 512, st));   // the histogram follows the counters
+        PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 4, 0xFF, 4, st));
+        PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 20, 0xFF, 4, st));
+        PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 40, 0xFF, 16, st));
+        // CUB temp sizes
+        size_t t_sort = 0, t_scan = 0, t_max = 0, t_scan32 = 0;
+        cub::DeviceRadixSort::SortPairs(nullptr, t_sort, keys, keys_s, vals, order, static_cast<int>(n), 0, 32, st);
+        cub::DeviceScan::ExclusiveSum(nullptr, t_scan, w2, w2o, static_cast<int>(n), st);
+        cub::DeviceScan::InclusiveScan(nullptr, t_max, head, head_s, cub::Max(), static_cast<int>(n), st);
+        cub::DeviceScan::ExclusiveSum(nullptr, t_scan32, flag, tidx, static_cast<int>(n), st);
+        t_need = std::max({t_sort, t_scan, t_max, t_scan32});
+        tmp = take(t_need);
+        if (!tmp) return set_error(ctx, PHR_ERR_OOM, "device arena exhausted (cub)");
+        {
+            KernelScope ks(ctx, "prep_sizes");
+            prep_sizes_kernel<<<blocks_for(n, T), T, 0, st>>>(pp);
+        }
+        tn_ = t_need;
+        cub::DeviceScan::ExclusiveSum(tmp, tn_, w2, w2o, static_cast<int>(n), st);
+        tn_ = t_need;
+        cub::DeviceScan::ExclusiveSum(tmp, tn_, wb, wbo, static_cast<int>(n), st);
+        tn_ = t_need;
+        cub::DeviceScan::ExclusiveSum(tmp, tn_, tb, tbo, static_cast<int>(n), st);
+        {
+            KernelScope ks(ctx, "pack");
+            pack_kernel<<<blocks_for(n * 32, T), T, 0, st>>>(pk);
+        }
+        tn_ = t_need;
+        cub::DeviceRadixSort::SortPairs(tmp, tn_, keys, keys_s, vals, order, static_cast<int>(n), 0, 32, st);
+        {
+            KernelScope ks(ctx, "task_head");
+            task_head_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
+        }
+        tn_ = t_need;
+        cub::DeviceScan::InclusiveScan(tmp, tn_, head, head_s, cub::Max(), static_cast<int>(n), st);
+        tbp.head = head_s;
+        {
+            KernelScope ks(ctx, "task_flag");
+            task_flag_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
+        }
+        tn_ = t_need;
+        cub::DeviceScan::ExclusiveSum(tmp, tn_, flag, tidx, static_cast<int>(n), st);
+        {
+            KernelScope ks(ctx, "task_fill");
+            task_fill_kernel<<<blocks_for(n, T), T, 0, st>>>(tbp);
+        }
+        {
+            KernelScope ks(ctx, "task_finalize");
+            task_finalize_kernel<<<1, 1, 0, st>>>(tbp);
+        }
     }
 
     // Main-pass slot: the smallest power of two that covers 99.5 % of the tasks (and no
     // less than the largest task when that still fits a full grid); tasks needing more
     // are deferred to the redo passes, which size scratch per task.
+    PHR_CUDA_TRY(ctx, read_counters(512));
     uint64_t h_need = 0;
+    std::memcpy(&h_need, h_cnt + 8, 8);
     unsigned int h_hist[64];
-    uint32_t h_cnt[56];   // the counter block up to the register-tile need
-    const uint32_t* h_ranges = h_cnt;
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_need, need_max, 8, cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_hist, need_hist, sizeof(h_hist), cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    std::memcpy(h_hist, h_cnt + 64, sizeof(h_hist));
+    uint32_t h_ranges[4];
+    std::memcpy(h_ranges, h_cnt, sizeof(h_ranges));
+    const uint32_t n_lane = h_cnt[29] - h_cnt[28], n_group2 = engine == PHR_ENGINE_MYERS_GLOBAL
+                                                                  ? h_cnt[31] - h_cnt[30]
+                                                                  : h_ranges[1] - h_ranges[0];
+    const uint32_t n_groupb = h_ranges[3] - h_ranges[2];
+    const bool any_2bit = h_ranges[2] > 0, any_bytes = h_cnt[51] > h_ranges[2];
     PHR_CUDA_TRY(ctx, cudaGetLastError());
     hs_setup.stop();
     uint32_t n_tile[4], n_tiles = 0;
@@ -951,7 +1165,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         P.tasks.task_first = tfirst;
         P.tasks.task_count = tcount;
         P.tasks.task_group = tgroup;
-        PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 5, 0, 8, st));
+        // the queue heads start at zero with the counter block
+        if (per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 5, 0, 8, st));
         static const char* const names[2][3][2] = {
             {{"myers", "myers_bytes"}, {"wfa_linear", "wfa_linear_bytes"}, {"wfa_affine", "wfa_affine_bytes"}},
             {{"myers_redo", "myers_bytes_redo"}, {"wfa_linear_redo", "wfa_linear_bytes_redo"},
@@ -959,24 +1174,23 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         const int ek = is_myers ? 0 : engine == PHR_ENGINE_WFA_LINEAR ? 1 : 2;
         const char* kname = names[per_task][ek][0];
         const char* kname_b = names[per_task][ek][1];
-        if (!per_task && engine == PHR_ENGINE_MYERS_GLOBAL) {
+        if (!per_task && engine == PHR_ENGINE_MYERS_GLOBAL) range0 = cnt + 30;
+        if (!per_task && engine == PHR_ENGINE_MYERS_GLOBAL && n_lane > 0) {
             // global 2-bit pairs of one lane each (tasks [0, g1)); the warp-group kernel
             // below takes the remaining 2-bit tasks [g1, split)
             const uint64_t lane_grid =
                 std::min<uint64_t>(grid * warps_per_block / (kLaneThreads / 32),
                                    static_cast<uint64_t>(ctx->sm_count) * myers_lane_blocks_per_sm(P.lane_ckpt));
-            PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 26, 0, 4, st));
             P.tasks.range = cnt + 28;
             P.queue_head = cnt + 26;
             {
                 KernelScope ks(ctx, "myers_lane");
                 launch_myers_lane(P, static_cast<int>(std::max<uint64_t>(lane_grid, 1)), st);
             }
-            range0 = cnt + 30;
         }
         P.tasks.range = range0;
         P.queue_head = cnt + 5;
-        {
+        if (per_task ? any_2bit : n_group2 > 0) {
             KernelScope ks(ctx, kname);
             if (is_myers)
                 launch_myers(P, static_cast<int>(grid), block, st);
@@ -987,7 +1201,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         }
         P.tasks.range = range1;
         P.queue_head = cnt + 6;
-        {
+        if (per_task ? any_bytes : n_groupb > 0) {
             KernelScope ks(ctx, kname_b);
             if (is_myers)
                 launch_myers_bytes(P, static_cast<int>(grid), block, st);
@@ -1000,13 +1214,13 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                            (engine == PHR_ENGINE_WFA_AFFINE && aff_tile_open(costs) != 0);
         if (tiles && P.big_min > 0 && (per_task ? n_tasks_hint : n_tiles) > 0) {
             // register tiles: long pairs one CTA each (one per SM), the others a warp each
-            PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 56, 0, 16, st));
+            if (per_task) PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 56, 0, 16, st));
             static const char* const tile_names[2][4] = {
                 {"wfa_linear_tile", "wfa_linear_tile_bytes", "wfa_linear_big", "wfa_linear_big_bytes"},
                 {"wfa_affine_tile", "wfa_affine_tile_bytes", "wfa_affine_big", "wfa_affine_big_bytes"}};
             const bool affine = engine == PHR_ENGINE_WFA_AFFINE;
             for (int i = 3; i >= 0; --i) {   // the longest first
-                const uint64_t nt = per_task ? n_tasks_hint : n_tile[i];
+                const uint64_t nt = per_task ? (((i & 1) ? any_bytes : any_2bit) ? n_tasks_hint : 0) : n_tile[i];
                 if (nt == 0) continue;
                 const bool cta = i >= 2;
                 const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 60), pool,
@@ -1034,6 +1248,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 n_tasks_hint, ctx->sm_count * static_cast<uint64_t>(kBigAffineThreads / aff_threads)));
             PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 24, 0, 8, st));
             for (int mode = 0; mode < 2; ++mode) {
+                if (!(mode ? any_bytes : any_2bit)) continue;
                 P.tasks.range = mode ? range1 : range0;
                 P.queue_head = cnt + 24 + mode;
                 KernelScope ks(ctx, mode ? "wfa_affine_big_bytes" : "wfa_affine_big");
@@ -1048,9 +1263,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     if (s != PHR_OK) return s;
     if (n_tile[2] + n_tile[3] > 0) {
         // long pairs left by the CTA kernels when most SMs had run out of pairs: a cluster each
-        uint32_t h_defer = 0;
-        PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_defer, cnt + 62, 4, cudaMemcpyDeviceToHost, st));
-        PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        PHR_CUDA_TRY(ctx, read_counters(256));
+        const uint32_t h_defer = h_cnt[62];
         if (h_defer > 0) {
             const TileLaunch tl{reinterpret_cast<unsigned long long*>(cnt + 60), tile_pool, kTileChunk, 0, ctx->sm_count, cnt + 62,
                                 reinterpret_cast<unsigned long long*>(rtask_off)};
@@ -1081,11 +1295,44 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // other pairs of the call go on)
     static const PairOut kOomOut = {PHR_ERR_OOM, 0, 0, 0, 0, 0};
     uint64_t n_oom = 0;
+    // Text offsets, their total, the records and texts; nothing is written while pairs wait for
+    // a redo pass or when the text does not fit.
+    FinishParams F{n, engine, desc, pout, tbo, text, cigoff, res->aln, res->cigar, res->cigar_capacity, cnt + 10,
+                   res->cigar_base, 32, cnt + 7, total};
+    auto launch_tail = [&]() {
+        const bool texts = small && sum_qt <= (64u << 10);   // little enough for one CTA to copy
+        if (small) {
+            FinishParams f = F;
+            f.per_warp = static_cast<int>((n + 31) / 32);
+            KernelScope ks(ctx, "small_tail");
+            small_tail_kernel<<<1, kSmallPairs, 0, st>>>(f, tlen, texts);
+        } else {
+            {
+                KernelScope ks(ctx, "text_len");
+                text_len_kernel<<<blocks_for(n, T), T, 0, st>>>(pout, n, tlen);
+            }
+            tn_ = t_need;
+            cub::DeviceScan::ExclusiveSum(tmp, tn_, tlen, cigoff, static_cast<int>(n), st);
+            KernelScope ks(ctx, "total");
+            total_kernel<<<1, 1, 0, st>>>(cigoff, tlen, n, total);
+        }
+        if (texts) return;
+        FinishParams f = F;
+        // at least 16 warps per SM before a warp takes more than one pair
+        while (f.per_warp > 1 && (n + f.per_warp - 1) / f.per_warp < 16ull * ctx->sm_count) f.per_warp /= 2;
+        KernelScope ks(ctx, "finish");
+        finish_kernel<<<blocks_for((n + f.per_warp - 1) / f.per_warp * 32, T), T, 0, st>>>(f);
+    };
+    // a batch this small is finished before the host knows whether pairs are to be redone: one
+    // wait less when there are none, a few microseconds of work in vain otherwise
+    const bool ahead = n <= (1u << 16);
+    bool tail_done = false;
     HostScope hs_redo(ctx, "host:redo");
     for (int round = 0; round < 12; ++round) {
-        uint32_t h_redo = 0;
-        PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_redo, cnt + 7, 4, cudaMemcpyDeviceToHost, st));
-        PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        if (ahead) launch_tail();
+        PHR_CUDA_TRY(ctx, read_counters(256));
+        const uint32_t h_redo = h_cnt[7];
+        tail_done = ahead && h_redo == 0;
         if (h_redo == 0) break;
         if (round == 11) return set_error(ctx, PHR_ERR_CAPACITY, "extension did not fit after repeated redo passes");
         h_list.resize(h_redo);
@@ -1190,35 +1437,17 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         }
     }
     HostScope hs_tail(ctx, "host:extend_tail");
-    // pack CIGAR text
-    {
-        KernelScope ks(ctx, "text_len");
-        text_len_kernel<<<blocks_for(n, T), T, 0, st>>>(pout, n, tlen);
-    }
-    tn_ = t_need;
-    cub::DeviceScan::ExclusiveSum(tmp, tn_, tlen, cigoff, static_cast<int>(n), st);
-    {
-        KernelScope ks(ctx, "total");
-        total_kernel<<<1, 1, 0, st>>>(cigoff, tlen, n, total);
+    if (!tail_done) {
+        launch_tail();
+        PHR_CUDA_TRY(ctx, read_counters(256));
     }
     uint64_t h_total = 0;
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_total, total, 8, cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    std::memcpy(&h_total, h_cnt + 12, 8);
     if (h_total > res->cigar_capacity)
         return set_error(ctx, PHR_ERR_CAPACITY, "CIGAR arena too small: need " + std::to_string(h_total) + " bytes");
-    FinishParams F{n,           engine,     desc,       pout,    tbo, text, cigoff, res->aln, res->cigar,
-                   res->cigar_capacity, cnt + 10, res->cigar_base, 32};
-    // at least 16 warps per SM before a warp takes more than one pair
-    while (F.per_warp > 1 && (n + F.per_warp - 1) / F.per_warp < 16ull * ctx->sm_count) F.per_warp /= 2;
-    {
-        KernelScope ks(ctx, "finish");
-        finish_kernel<<<blocks_for((n + F.per_warp - 1) / F.per_warp * 32, T), T, 0, st>>>(F);
-    }
-    uint32_t h_err = 0;
-    unsigned long long h_work[4] = {0, 0, 0, 0};
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(&h_err, cnt + 10, 4, cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaMemcpyAsync(h_work, cnt + 32, sizeof(h_work), cudaMemcpyDeviceToHost, st));
-    PHR_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    const uint32_t h_err = h_cnt[10];
+    unsigned long long h_work[4];
+    std::memcpy(h_work, h_cnt + 32, sizeof(h_work));
     if (h_work[0]) ctx->counters["myers_lane_block_columns"] += h_work[0];
     if (h_work[1]) ctx->counters["myers_lane_redo_pairs"] += h_work[1];
     if (h_work[2] || h_work[3]) {

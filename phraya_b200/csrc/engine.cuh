@@ -49,6 +49,8 @@ struct EngineTune {
                                      // or store every column's records (0)
 };
 
+constexpr size_t kPinnedBytes = 512;
+
 struct Ctx {
     int device = 0;
     int sm_count = 0;
@@ -68,7 +70,7 @@ struct Ctx {
     bool tune_file_enable = false;
     std::mutex mu;
     uint32_t* d_counters = nullptr;   // small device scratch for counters (pinned size)
-    void* h_pinned = nullptr;         // small pinned host buffer for D2H of counters
+    void* h_pinned = nullptr;         // small pinned host buffer (kPinnedBytes) for D2H of counters
     // kernel timing (phr_ctx_set_timing)
     bool timing = false;
     struct Pending {
