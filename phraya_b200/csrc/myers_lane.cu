@@ -408,10 +408,10 @@ constexpr int kCkWarpBytes = kTraceRecBytes > kLanePeqWarpBytes ? kTraceRecBytes
 // recomputed, from the segment's checkpoint and the horizontal deltas the forward pass
 // kept for every block: the same block updates on the same inputs, hence the same bits,
 // without the other blocks of the window and without one block waiting for the other's
-// carry. Then every lane moves through its records one event at a time (D run, I move or
-// diagonal cell, with the precedence of myers_backtrace_flat). Recomputing the whole window
+// carry. Then the lanes walk down the segment's columns together, each column's move (with
+// the precedence of myers_backtrace_flat: D, I, diagonal) two bits of its record. Recomputing the whole window
 // (3.6 blocks on average in the 64-2048 bp set) made the traceback as long as the forward
-// pass: 13.4 ms per 1,000,000 pairs against 9.6 now. Returns false when the walk left
+// pass: 13.4 ms per 1,000,000 pairs against 8.45 now. Returns false when the walk left
 // the band or cost more than E (the pair is then redone).
 template <int P>
 __device__ __forceinline__ bool lane_trace_ck(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb,
@@ -486,74 +486,52 @@ __device__ __forceinline__ bool lane_trace_ck(const uint32_t* __restrict__ qb, c
                     const uint64_t eq = mk64((pl[par].x ^ n0) & (pl[par].z ^ n1), (pl[par].y ^ n0) & (pl[par].w ^ n1));
                     uint32_t pa = ha[par] << 16, ma = ha[par] << 17;   // bit 15: +1, bit 14: -1
                     const uint64_t ph = advance_block<false>(vp[par], vn[par], eq, pa, ma);
-                    out[par * 32] = make_uint4(lo32(vp[par]), hi32(vp[par]), lo32(vp[par] | ph), hi32(vp[par] | ph));
+                    // a cell's move in two bits: ST = VP | HP and B = VP, or a mismatch where neither is
+                    // set: 3 D, 2 I, 1 X, 0 M
+                    const uint64_t st = vp[par] | ph, mv = vp[par] | ~(st | eq);
+                    out[par * 32] = make_uint4(lo32(st), hi32(st), lo32(mv), hi32(mv));
                     ha[par] <<= 2;
                 }
                 out += 64;
                 syms >>= 2;
             }
             // (each lane reads back only the records it wrote: no barrier is needed)
-            // ---- walk every lane through its two blocks of this segment ----
-            const uint8_t* st = reinterpret_cast<const uint8_t*>(seg) + 8;   // VP | HP of column 0, even block
-            for (;;) {
-                const int b = (i - 1) >> 6;
-                const bool want = ok && i > 0 && j > j0 && b1 - b < 2;
-                if (!__any_sync(PHR_FULL_MASK, want)) break;
-                if (!want) continue;
-                const int kb = b - lane_blo(g, j);
-                const int t = j - 1 - j0, r = i - 1, bit = r & 63;
-                const uint4 R = seg[(t * 2 + (b & 1)) * 32];
-                const uint64_t vpb = mk64(R.x, R.y);
-                const uint32_t sw = bit & 32 ? R.w : R.z;
-                uint32_t op, count, neq = 0;   // first run of this step; differences of the cells after it
-                int done = 0, run = 0;         // diagonal cells pushed, of `run`
-                if ((sw >> (bit & 31)) & 1u) {
-                    // D run: consecutive VP bits upward from row i within this block; else I
-                    const int up = static_cast<int>(__clzll(~(vpb << (63 - bit))));
-                    op = up > 0 ? 3u : 2u;
-                    count = static_cast<uint32_t>(max(up, 1));
-                    cost += max(up, 1);
-                    i -= up;
-                    j -= up > 0 ? 0 : 1;
-                } else {
-                    // diagonal stretch: up to the first cell with a VP or HP bit, or out of the
-                    // segment (eight rows up at most: still in the two blocks)
-                    const int most = min(t + 1, i);
-                    uint32_t stop = ~0u << most;
-#pragma unroll
-                    for (int u = 1; u < kSegCols; ++u) {
-                        const int ru = r - u;
-                        uint32_t w = 0;
-                        if (u <= t)
-                            w = *reinterpret_cast<const uint32_t*>(st + (t - u) * 1024 + ((ru << 3) & 512) + ((ru >> 3) & 4));
-                        stop |= ((w >> (ru & 31)) & 1u) << u;
-                    }
-                    run = __ffs(stop) - 1;   // >= 1: cell 0 is diagonal
-                    // M / X: cell u compares query symbol i - 1 - u with target symbol j - 1 - u, both
-                    // at index 7 - u of their windows
-                    const int pos = (j - 1) & 15;
-                    const uint32_t tsym = static_cast<uint32_t>((static_cast<uint64_t>(tw) << 14) >> (2 * pos));
-                    const uint32_t x = diag_window(qb, i) ^ tsym;
-                    const uint32_t nz = (x | (x >> 1)) & 0x5555u;
-                    neq = even_bits(__brev(nz) >> 17) & ((1u << run) - 1u);   // bit u: cell u differs
-                    cost += __popc(neq);
-                    i -= run;
-                    j -= run;
-                    op = 0;
-                    count = neq ? __ffs(neq) - 1 : run;
-                    done = static_cast<int>(count);
+            // ---- walk down the columns, all lanes together: a D run where one starts, then the
+            // column's I, X or M. A lane whose D run leaves its two blocks waits for another round.
+            const uint8_t* cells = reinterpret_cast<const uint8_t*>(seg);
+            int lo_d = j - i, hi_d = j - i;   // diagonals visited
+#pragma unroll 1
+            for (int t = cols - 1; t >= 0; --t) {
+                auto move_at = [&](int r) -> uint32_t {   // row r of column j0 + 1 + t
+                    const uint8_t* p = cells + t * 1024 + ((r << 3) & 512) + ((r >> 3) & 4);
+                    const uint32_t st = *reinterpret_cast<const uint32_t*>(p) >> (r & 31);
+                    const uint32_t mv = *reinterpret_cast<const uint32_t*>(p + 8) >> (r & 31);
+                    return (st & 1u) * 2 + (mv & 1u);
+                };
+                const bool at = in && i > 0 && j - 1 - j0 == t;
+                if (!at || b1 - ((i - 1) >> 6) > 1) continue;
+                uint32_t mv = move_at(i - 1);
+                if (mv == 3) {
+                    uint32_t run = 0;
+                    do {
+                        ++run;
+                        --i;
+                        mv = i > 0 && b1 - ((i - 1) >> 6) <= 1 ? move_at(i - 1) : 4u;
+                    } while (mv == 3);
+                    rw.push(3, run);
+                    cost += static_cast<int>(run);
+                    hi_d = max(hi_d, j - i);
+                    if (mv == 4) continue;
                 }
-                for (;;) {   // one push in the code: matches and differences in turn
-                    rw.push(op, count);
-                    if (done >= run) break;
-                    op ^= 1u;
-                    const uint32_t rest = (op ? ~neq : neq) >> done;   // bit 0: the run ends here (never)
-                    count = static_cast<uint32_t>(min(rest ? __ffs(rest) - 1 : 32, run - done));
-                    done += static_cast<int>(count);
-                }
-                const int d = j - i;
-                if (kb < 0 || kb >= P || d < band.dmin || d > band.dmax || cost > band.E) ok = false;
+                rw.push(mv, 1);
+                cost += mv != 0;
+                i -= mv < 2 ? 1 : 0;
+                --j;
+                lo_d = min(lo_d, j - i);
             }
+            // (the band is convex and a step moves one diagonal: outside it anywhere is outside
+            // here, and rows outside the window were read as they were left)
+            if (in && (lo_d < band.dmin || hi_d > band.dmax || cost > band.E)) ok = false;
         }
     }
     if (ok) {
@@ -694,15 +672,16 @@ __global__ void __launch_bounds__(kLaneThreads, 2) myers_lane_kernel(ExtendParam
     lane_tasks<false>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kLanePeqWarpBytes / 8));
 }
 
-// Checkpoint mode: kCkWarpBytes of shared memory per warp, two blocks per SM.
-__global__ void __launch_bounds__(kLaneThreads, 2) myers_lane_ck_kernel(ExtendParams Pm) {
+// Checkpoint mode: kCkWarpBytes of shared memory per warp, three blocks per SM at 80 registers
+// (two at 128: 8.9 ms per 1,000,000 pairs of 64-2048 bp, three 8.45 in spite of spills).
+__global__ void __launch_bounds__(kLaneThreads, 3) myers_lane_ck_kernel(ExtendParams Pm) {
     extern __shared__ uint64_t lane_smem[];
     lane_tasks<true>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kCkWarpBytes / 8));
 }
 
 }  // namespace
 
-int myers_lane_blocks_per_sm(int) { return 2; }
+int myers_lane_blocks_per_sm(int ckpt) { return ckpt ? 3 : 2; }
 
 void launch_myers_lane(const ExtendParams& p, int grid, cudaStream_t st) {
     if (p.lane_ckpt) {
