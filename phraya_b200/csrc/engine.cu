@@ -231,6 +231,7 @@ struct PackParams {
     int wfa_long_min;   // qn + tn from which a WFA pair gets wfa_g_long lanes
     int band_base;      // Myers band half-width base
     int big_min;        // qn + tn from which a linear WFA pair runs in register tiles
+    int lane_ckpt;      // mode of the lane-per-pair Myers kernel
 };
 
 // 2-bit packing (16 bases per word) of both suffixes; a pair holding any byte other
@@ -357,7 +358,12 @@ __device__ __forceinline__ void pack_pair(const PackParams& P, uint64_t i, int l
                 const LaneBand b = lane_band(d.qn, d.tn, P.band_base);
                 if (lane_slots(b.dmin, b.dmax, (d.qn + 63) / 64) <= kLaneMaxSlots - 2) G = 1;
             }
-            len = static_cast<uint32_t>(d.tn) * (static_cast<uint32_t>((d.qn + 63) / 64));
+            const uint32_t nb = static_cast<uint32_t>((d.qn + 63) / 64);
+            len = static_cast<uint32_t>(d.tn) * nb;
+            if (fit_lanes(P.engine, P.in.n, P.lane_ckpt) && d.mode == 0 && nb <= kLaneMaxSlots) {
+                G = 1;   // a warp's pairs of one block count, for the last block's score
+                len = nb << 22 | min(static_cast<uint32_t>(d.tn), (1u << 22) - 1u);
+            }
         } else {
             G = (d.qn + d.tn < P.wfa_long_min) ? P.wfa_g_short : P.wfa_g_long;
             len = static_cast<uint32_t>(d.qn + d.tn);
@@ -446,7 +452,8 @@ __device__ __forceinline__ void task_fill(const TaskBuild& T, uint64_t p) {
         uint32_t cnt = 0;
         uint64_t region = 0;
         // lane-kernel tasks (global Myers, 2-bit, one lane per pair): window over the union band
-        const bool lane_task = T.engine == PHR_ENGINE_MYERS_GLOBAL && G == 1 && !((k >> 31) & 1);
+        const bool fit = fit_lanes(T.engine, T.n, T.lane_ckpt);
+        const bool lane_task = (T.engine == PHR_ENGINE_MYERS_GLOBAL || fit) && G == 1 && !((k >> 31) & 1);
         int dmin = 0x7fffffff, dmax = static_cast<int>(0x80000000), n_max = 0, m_max = 0;
         for (uint32_t c = 0; c < per && p + c < T.n; ++c) {
             const uint32_t kc = T.keys[p + c];
@@ -470,7 +477,10 @@ __device__ __forceinline__ void task_fill(const TaskBuild& T, uint64_t p) {
             ++cnt;
         }
         if (T.engine != PHR_ENGINE_MYERS_FIT && T.engine != PHR_ENGINE_MYERS_GLOBAL) need = region * per;
-        if (lane_task && cnt) need = lane_task_need(n_max, m_max, lane_slots(dmin, dmax, (m_max + 63) >> 6), T.lane_ckpt);
+        if (lane_task && cnt) {
+            const int nb = (m_max + 63) >> 6;
+            need = lane_task_need(n_max, m_max, fit ? nb : lane_slots(dmin, dmax, nb), T.lane_ckpt);
+        }
         const uint32_t t = T.tidx[p];
         T.task_first[t] = static_cast<uint32_t>(p);
         T.task_count[t] = static_cast<uint8_t>(cnt);
@@ -989,7 +999,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     const PrepParams pp{in, engine, costs, desc, pout, w2, wb, tb};
     const PackParams pk{in, engine, costs, desc, pout, w2o, wbo, tbo, arena2, arenab, text, keys, vals,
                         g_short, ctx->tune.wfa_group_long, ctx->tune.wfa_long_min,
-                        ctx->tune.myers_band_base, ctx->tune.wfa_big_min};
+                        ctx->tune.myers_band_base, ctx->tune.wfa_big_min, ctx->tune.myers_lane_ckpt};
     TaskBuild tbp{keys_s, order, n, small ? head_s : head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4,
                   cnt + 20, desc, engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
                   ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt,
@@ -1074,9 +1084,9 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     std::memcpy(h_hist, h_cnt + 64, sizeof(h_hist));
     uint32_t h_ranges[4];
     std::memcpy(h_ranges, h_cnt, sizeof(h_ranges));
-    const uint32_t n_lane = h_cnt[29] - h_cnt[28], n_group2 = engine == PHR_ENGINE_MYERS_GLOBAL
-                                                                  ? h_cnt[31] - h_cnt[30]
-                                                                  : h_ranges[1] - h_ranges[0];
+    const bool lanes = engine == PHR_ENGINE_MYERS_GLOBAL || fit_lanes(engine, n, ctx->tune.myers_lane_ckpt);
+    const uint32_t n_lane = lanes ? h_cnt[29] - h_cnt[28] : 0;
+    const uint32_t n_group2 = lanes ? h_cnt[31] - h_cnt[30] : h_ranges[1] - h_ranges[0];
     const uint32_t n_groupb = h_ranges[3] - h_ranges[2];
     const bool any_2bit = h_ranges[2] > 0, any_bytes = h_cnt[51] > h_ranges[2];
     PHR_CUDA_TRY(ctx, cudaGetLastError());
@@ -1174,9 +1184,9 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         const int ek = is_myers ? 0 : engine == PHR_ENGINE_WFA_LINEAR ? 1 : 2;
         const char* kname = names[per_task][ek][0];
         const char* kname_b = names[per_task][ek][1];
-        if (!per_task && engine == PHR_ENGINE_MYERS_GLOBAL) range0 = cnt + 30;
-        if (!per_task && engine == PHR_ENGINE_MYERS_GLOBAL && n_lane > 0) {
-            // global 2-bit pairs of one lane each (tasks [0, g1)); the warp-group kernel
+        if (!per_task && lanes) range0 = cnt + 30;
+        if (!per_task && n_lane > 0) {
+            // 2-bit pairs of one lane each (tasks [0, g1)); the warp-group kernel
             // below takes the remaining 2-bit tasks [g1, split)
             const uint64_t lane_grid =
                 std::min<uint64_t>(grid * warps_per_block / (kLaneThreads / 32),

@@ -1,6 +1,7 @@
 // myers_lane.cu -- banded Myers edit distance with CIGAR, one pair per lane (sm_100a).
 //
-// Serves the global engine (myers_edit_distance, phraya-align/src/lib.rs:94-96 ->
+// Serves large fitting batches (myers_extend, every block in the window) and the global
+// engine (myers_edit_distance, phraya-align/src/lib.rs:94-96 ->
 // myers_edit_distance_impl, wfa_simd.rs:3657-3673) for 2-bit pairs: distance plus the
 // traceback of myers_backtrace_flat (wfa_simd.rs:3702-3781: precedence D, I, diagonal).
 //
@@ -92,7 +93,7 @@ __device__ __forceinline__ uint64_t shl1_in(uint64_t x, uint32_t above_hi) {
 // is hin = +1 / -1); replaced by this block's on return. TOP: hin = +1.
 template <bool TOP>
 __device__ __forceinline__ uint64_t advance_block(uint64_t& vp, uint64_t& vn, uint64_t eq, uint32_t& pa,
-                                                  uint32_t& ma) {
+                                                  uint32_t& ma, uint64_t* mh_out = nullptr) {
     const uint32_t a_p = TOP ? 0x80000000u : pa;
     const uint32_t a_m = TOP ? 0u : ma;
     const uint64_t xv = eq | vn;
@@ -106,6 +107,7 @@ __device__ __forceinline__ uint64_t advance_block(uint64_t& vp, uint64_t& vn, ui
     vn = phs & xv;
     pa = hi32(ph);
     ma = hi32(mh);
+    if (mh_out) *mh_out = mh;
     return ph;
 }
 
@@ -146,11 +148,20 @@ __device__ __forceinline__ uint64_t hin_off(int sg, int k, int lane) {
 // n_max, and per segment of kSegCols columns the horizontal deltas (two bits a column,
 // the latest lowest) that entered each block of the window at the segment's end, to
 // `hin`. The traceback recomputes from those the two blocks a lane's path is in.
-template <int P, bool CK>
+// FIT: `fit` is the lane's search for the best end column (myers_fitting_impl), and the pass
+// ends early once every lane's is over.
+struct FitEnd {
+    bool on;                   // a fitting pair (its target runs on past the query)
+    int m, best, best_col, score;
+    bool stopped;
+};
+template <int P, bool CK, bool FIT>
 __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb, int n,
                                              int nb, const LaneGeom& g, uint64_t* sp, uint8_t* rec, uint8_t* hin,
-                                             uint4* planes) {
+                                             uint4* planes, FitEnd& fit) {
     const int lane = lane_id();
+    const bool upper = ((fit.m - 1) & 32) != 0;   // half of its block that holds the last row
+    const int nb_min = FIT ? static_cast<int>(__reduce_min_sync(PHR_FULL_MASK, static_cast<unsigned>(nb > 0 ? nb : P))) : 0;
     // a block's two bit planes, from its match masks, for the traceback
     auto keep_planes = [&](int b, const uint64_t e[4]) {
         if (CK && b < nb) {
@@ -225,8 +236,14 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
             const uint64_t eq = eqp[k * 128];
             if (CK)   // +1 enters the window's top block
                 ha[k] = k == 0 ? (ha[0] << 2) | 2u : __funnelshift_l(ma, __funnelshift_l(pa, ha[k], 1), 1);
-            const uint64_t ph = k == 0 ? advance_block<true>(vp[0], vn[0], eq, pa, ma)
-                                       : advance_block<false>(vp[k], vn[k], eq, pa, ma);
+            uint64_t mh = 0;
+            const uint64_t ph = k == 0 ? advance_block<true>(vp[0], vn[0], eq, pa, ma, FIT ? &mh : nullptr)
+                                       : advance_block<false>(vp[k], vn[k], eq, pa, ma, FIT ? &mh : nullptr);
+            if (FIT && k >= nb_min - 1) {   // warp-uniform: only the last block in most warps
+                const uint32_t p = upper ? hi32(ph) : lo32(ph), q = upper ? hi32(mh) : lo32(mh);
+                if (k == nb - 1) fit.score += static_cast<int>((p >> ((fit.m - 1) & 31)) & 1u) -
+                                              static_cast<int>((q >> ((fit.m - 1) & 31)) & 1u);
+            }
             if (!CK)
                 *reinterpret_cast<uint4*>(r + k * (512 * kLaneColGroup) + sub * 16) =
                     make_uint4(lo32(vp[k]), hi32(vp[k]), lo32(ph), hi32(ph));
@@ -238,10 +255,22 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
             for (int k = 0; k < P; ++k)
                 *reinterpret_cast<uint4*>(c + k * 512) = make_uint4(lo32(vp[k]), hi32(vp[k]), lo32(vn[k]), hi32(vn[k]));
         }
+        if (FIT && j <= n) {
+            fit.score = max(fit.score, 0);
+            if (fit.on && !fit.stopped) {
+                if (fit.score < fit.best) {
+                    fit.best = fit.score;
+                    fit.best_col = j;
+                }
+                fit.stopped = fit.score > fit.best + fit.m / 10 + 1;
+            }
+        }
         if (CK && ((j % kSegCols) == 0 || j == g.n_max)) {   // warp-uniform
             uint8_t* h = hin + hin_off<P>((j - 1) / kSegCols, 0, lane);
 #pragma unroll
             for (int k = 0; k < P; ++k) *reinterpret_cast<uint16_t*>(h + k * 64) = static_cast<uint16_t>(ha[k]);
+            // no lane reads a column past its best end (or its target's end)
+            if (FIT && !__any_sync(PHR_FULL_MASK, j < n && !(fit.on && fit.stopped))) break;
         }
     }
 }
@@ -402,7 +431,7 @@ constexpr int kTraceRecBytes = kSegCols * 2 * 32 * 16;
 constexpr int kLanePeqWarpBytes = kLaneMaxSlots * 4 * 32 * 8;  // Peq (and record mode's traceback buffers) per warp
 constexpr int kCkWarpBytes = kTraceRecBytes > kLanePeqWarpBytes ? kTraceRecBytes : kLanePeqWarpBytes;
 
-// Traceback of one lane's pair from (m, n) over segments of kSegCols columns, top segment
+// Traceback of one lane's pair from (m, j_end) over segments of kSegCols columns, top segment
 // first. In a segment a lane's path stays in the 64-row block it enters by the last column
 // and the one above (a longer D run takes another round), so only those two are
 // recomputed, from the segment's checkpoint and the horizontal deltas the forward pass
@@ -417,11 +446,11 @@ template <int P>
 __device__ __forceinline__ bool lane_trace_ck(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb,
                                               int m, int n, int nb, const LaneBand& band, const LaneGeom& g, bool act,
                                               const uint8_t* ck, const uint8_t* hin, const uint4* planes, uint8_t* smem,
-                                              RunWriter& rw,
+                                              int j_end, RunWriter& rw,
                                               int* ed_out) {
     const int lane = lane_id();
     uint4* seg = reinterpret_cast<uint4*>(smem) + lane;
-    int i = act ? m : 0, j = act ? n : 0, cost = 0;
+    int i = act ? m : 0, j = act ? j_end : 0, cost = 0;
     bool ok = act;
     int held[2] = {-1, -1};   // blocks whose bit planes the lane holds, by parity
     uint4 pl[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -554,7 +583,7 @@ __device__ __forceinline__ bool lane_trace_ck(const uint32_t* __restrict__ qb, c
 // separate traceback kernel with more resident warps measured slower on B200: the 32
 // lanes' walks diverge, so a traceback warp executes about as many instructions as the
 // forward pass whatever hides its latency.)
-template <int P, bool CK>
+template <int P, bool CK, bool FIT>
 __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& d, bool act, const LaneBand& band,
                           const LaneGeom& g, uint64_t* sp, uint8_t* slot) {
     const int lane = lane_id();
@@ -564,7 +593,9 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     const uint32_t* tb = Pm.packed2 + (act ? d.t_word : 0);
     uint8_t* hin = slot + lane_ckpt_bytes(g.n_max, P);   // checkpoint mode
     uint4* planes = reinterpret_cast<uint4*>(hin + lane_hin_bytes(g.n_max, P));
-    lane_forward<P, CK>(qb, tb, n, nb, g, sp, slot, hin, planes);
+    FitEnd fit = {FIT && act && n > m + m / 2 + 10, m, m, 0, m, false};
+    lane_forward<P, CK, FIT>(qb, tb, n, nb, g, sp, slot, hin, planes, fit);
+    const int j_end = FIT && fit.on ? fit.best_col : n;
     // work counter: block-columns this task evaluated for its pairs
     const unsigned long long cols = __reduce_add_sync(PHR_FULL_MASK, act ? static_cast<unsigned>(n) * P : 0u);
     if (lane == 0) atomicAdd(Pm.work, cols);
@@ -577,7 +608,7 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     int ed = 0;
     bool ok;
     if (CK)
-        ok = lane_trace_ck<P>(qb, tb, m, n, nb, band, g, act, slot, hin, planes, reinterpret_cast<uint8_t*>(sp), rw, &ed);
+        ok = lane_trace_ck<P>(qb, tb, m, n, nb, band, g, act, slot, hin, planes, reinterpret_cast<uint8_t*>(sp), j_end, rw, &ed);
     else
         ok = lane_trace<P>(qb, tb, m, n, band, g, act, slot, reinterpret_cast<uint4*>(sp) + lane, rw, &ed);
     // work counter: pairs sent to redo
@@ -607,7 +638,7 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
         PairOut o;
         o.status = PHR_OK;
         o.ed = ed;
-        o.t_consumed = n;
+        o.t_consumed = j_end;
         o.affine_score = 0;
         o.n_runs = rw.n;
         o.text_len = tl;
@@ -615,7 +646,7 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     }
 }
 
-template <bool CK>
+template <bool CK, bool FIT>
 __device__ __forceinline__ void lane_tasks(const ExtendParams& Pm, uint64_t* sp) {
     const int lane = lane_id();
     const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -631,7 +662,9 @@ __device__ __forceinline__ void lane_tasks(const ExtendParams& Pm, uint64_t* sp)
         PairDesc d = {};
         if (act) d = Pm.desc[pid];
         const int m = act ? d.qn : 0, n = act ? d.tn : 0;
-        const LaneBand band = lane_band(m, n, Pm.band_base);
+        // fitting batches: every block in the window, no band
+        constexpr int kFar = 1 << 28;
+        const LaneBand band = FIT ? LaneBand{kFar, -kFar, kFar} : lane_band(m, n, Pm.band_base);
         LaneGeom g;
         g.dmin = __reduce_min_sync(PHR_FULL_MASK, act ? band.dmin : 0x7fffffff);
         g.dmax = __reduce_max_sync(PHR_FULL_MASK, act ? band.dmax : static_cast<int>(0x80000000));
@@ -654,14 +687,14 @@ __device__ __forceinline__ void lane_tasks(const ExtendParams& Pm, uint64_t* sp)
             continue;
         }
         switch (g.P) {
-            case 1: lane_task<1, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 2: lane_task<2, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 3: lane_task<3, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 4: lane_task<4, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 5: lane_task<5, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 6: lane_task<6, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            case 7: lane_task<7, CK>(Pm, pid, d, act, band, g, sp, slot); break;
-            default: lane_task<8, CK>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 1: lane_task<1, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 2: lane_task<2, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 3: lane_task<3, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 4: lane_task<4, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 5: lane_task<5, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 6: lane_task<6, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            case 7: lane_task<7, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
+            default: lane_task<8, CK, FIT>(Pm, pid, d, act, band, g, sp, slot); break;
         }
         __syncwarp();
     }
@@ -669,14 +702,19 @@ __device__ __forceinline__ void lane_tasks(const ExtendParams& Pm, uint64_t* sp)
 
 __global__ void __launch_bounds__(kLaneThreads, 2) myers_lane_kernel(ExtendParams Pm) {
     extern __shared__ uint64_t lane_smem[];
-    lane_tasks<false>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kLanePeqWarpBytes / 8));
+    lane_tasks<false, false>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kLanePeqWarpBytes / 8));
 }
 
 // Checkpoint mode: kCkWarpBytes of shared memory per warp, three blocks per SM at 80 registers
 // (two at 128: 8.9 ms per 1,000,000 pairs of 64-2048 bp, three 8.45 in spite of spills).
 __global__ void __launch_bounds__(kLaneThreads, 3) myers_lane_ck_kernel(ExtendParams Pm) {
     extern __shared__ uint64_t lane_smem[];
-    lane_tasks<true>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kCkWarpBytes / 8));
+    lane_tasks<true, false>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kCkWarpBytes / 8));
+}
+
+__global__ void __launch_bounds__(kLaneThreads, 3) myers_lane_fit_kernel(ExtendParams Pm) {
+    extern __shared__ uint64_t lane_smem[];
+    lane_tasks<true, true>(Pm, lane_smem + static_cast<uint64_t>(threadIdx.x >> 5) * (kCkWarpBytes / 8));
 }
 
 }  // namespace
@@ -686,6 +724,11 @@ int myers_lane_blocks_per_sm(int ckpt) { return ckpt ? 3 : 2; }
 void launch_myers_lane(const ExtendParams& p, int grid, cudaStream_t st) {
     if (p.lane_ckpt) {
         const int smem = kLaneWarps * kCkWarpBytes;
+        if (p.engine == PHR_ENGINE_MYERS_FIT) {
+            cudaFuncSetAttribute(myers_lane_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            myers_lane_fit_kernel<<<grid, kLaneThreads, smem, st>>>(p);
+            return;
+        }
         cudaFuncSetAttribute(myers_lane_ck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         myers_lane_ck_kernel<<<grid, kLaneThreads, smem, st>>>(p);
         return;
