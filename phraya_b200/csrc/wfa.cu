@@ -23,9 +23,9 @@
 // later scores) and the pre-extension candidate `raw` with its op code. In both
 // tracebacks the match-run start is exactly `raw` (linear: edit_start = pred_pos+1 for
 // ops 1/2 and pred_pos for op 3 == the winning candidate; affine: raw of each m_op).
-#include <type_traits>
 
 #include "kernels.cuh"
+#include "wfa_tile.cuh"
 
 namespace phr {
 namespace {
@@ -603,7 +603,7 @@ __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int
 template <class S>
 __device__ void wfa_affine_group(const ExtendParams& P, const PairDesc& d, uint32_t pid, bool act, int G,
                                  uint8_t* region, uint64_t region_bytes, SDir* ring, uint32_t* sseq,
-                                 int sseq_words) {
+                                 int sseq_words, unsigned long long* work) {
     const int gl = lane_id() & (G - 1);
     const int qn = act ? d.qn : 0, tn = act ? d.tn : 0;
     const bool fitting = act && tn > qn + qn / 2 + 10;
@@ -856,9 +856,9 @@ __device__ void wfa_affine_group(const ExtendParams& P, const PairDesc& d, uint3
     }
     {
         const unsigned cw = __reduce_add_sync(PHR_FULL_MASK, wf_cells), lw = __reduce_add_sync(PHR_FULL_MASK, lcp_words);
-        if (lane_id() == 0 && P.work) {
-            atomicAdd(P.work + 2, static_cast<unsigned long long>(cw));
-            atomicAdd(P.work + 3, static_cast<unsigned long long>(lw));
+        if (lane_id() == 0) {
+            work[0] += cw;
+            work[1] += lw;
         }
     }
     const bool failed = act && !done && !overflow;
@@ -1183,271 +1183,256 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
 }
 
 // ===========================================================================
-// Gap-affine WFA, one pair per warp, wavefronts in registers
+// Gap-affine WFA, one short pair per warp, wavefronts in registers
 // ===========================================================================
-// Every reachable cell of score s lies on a diagonal |k| <= (s - O) / E (a gap of length
-// L costs O + L E), so a window of kRegWin diagonals (slots of 32, lane = offset in the
-// slot) holds whole wavefronts while that bound stays inside it. Each lane keeps the M,
-// I and D values of its diagonals for the last scores the recurrence looks back to
-// (X, O + E and E, in steps of g = gcd(X, O, E)) in shift registers; neighbour diagonals
-// k - 1 and k + 1 come from the adjacent lane by shuffle. Cells are computed exactly as
-// in wfa_affine_group (candidate order, strict >, validity), so values, ops and the end
-// cell are identical; only the traceback's aux words go to memory, in the same history
-// layout (one row of kRegWin words per layer and score), so the same traceback runs.
-// A pair whose reachable band would leave the window stops and is redone by
-// wfa_affine_group.
-// Slots of 32 diagonals, centred on diagonal 0 so that the band of the early scores (and
-// of most pairs' whole search) is one slot: 0 = [-16, 15], 1 = [-48, -17], 2 = [16, 47],
-// 3 = [-80, -49], 4 = [48, 79].
-constexpr int kRegSlots = 5;
-constexpr int kRegMaxLen = 1024;  // qlen + tlen below which a pair tries the register kernel
-constexpr int kRegWin = 32 * kRegSlots;
+// Every reachable cell of score s lies on a diagonal |k| <= (s - O) / E (a gap of length L
+// costs O + L E), so 32 R lanes hold whole wavefronts while that bound stays inside them: R
+// is 1 for diagonals -16..15, then 2, 4 and 8. A lane keeps M of the last (O + E) / g steps and
+// I and D of the last one, as in wfa_affine_tile.cu (X / g = 2, E / g = 1): the larger of
+// "open" and "extend" is formed on its source diagonal and crosses lanes as one value, tie
+// tags in the two low bits decide as the reference's candidate order does, and an offset at
+// a sequence's end is the only one with an invalid successor. What a step costs is
+// instructions (about 60 and the longest match run); the cells are computed exactly as in
+// wfa_affine_group, so values, ops and the end cell are identical. Only the traceback's aux
+// words are stored, one row per step. A pair whose band would leave the window runs through
+// wfa_affine_group in the same warp.
+// Before, four values crossed lanes per cell, validity was a range test per candidate and
+// wide bands stepped five slots of which some lay outside: 1,000,000 pairs of 100-300 bp at
+// 0-5 %, costs (4, 6, 2), 8.57 -> 6.12 ms (6,213 -> about 4,100 warp instructions a pair);
+// 300,000 at 0-10 % 6.88 -> 4.99, at 0-20 % 27.1 -> 18.3, of 300-480 bp 6.62 -> 5.04.
+// With 4 slots at most, pairs whose band passes 128 diagonals are done twice: 7.97 at 0-10 %.
+constexpr int kRegMaxLen = 1024;  // qlen + tlen below which a pair tries the register path
+constexpr int kRegMaxSlots = 8;   // most diagonals per lane
+constexpr int kRegWin = 32 * kRegMaxSlots;   // history words of a step's row, from diagonal kRegLo on
 constexpr int kRegLo = -kRegWin / 2;
-__host__ __device__ constexpr int reg_slot_lo(int h) { return h == 0 ? -16 : h == 1 ? -48 : h == 2 ? 16 : h == 3 ? -80 : 48; }
-__host__ __device__ constexpr int reg_left(int h) { return h == 0 ? 1 : h == 1 ? 3 : h == 2 ? 0 : h == 4 ? 2 : -1; }
-__host__ __device__ constexpr int reg_right(int h) { return h == 0 ? 2 : h == 1 ? 0 : h == 2 ? 4 : h == 3 ? 1 : -1; }
+// History rows of diagonals -16..15 kept in the warp's shared memory: those of the first
+// kRegShRows steps, which hold the whole history of most short pairs.
+constexpr int kRegShRows = 32;
+// A short pair's sequences as overlapping word pairs, each with room for reads from
+// diagonals outside the pair.
+constexpr int kRegSeqPad = kRegWin / 32 + 4;
+constexpr int kRegSeqEntries = kRegMaxLen / 16 + 2 + 2 * kRegSeqPad;
+constexpr int kRegWarpSmem = kRegShRows * 128 + kRegSeqEntries * 8;
 
-// value at diagonal k - 1 (UP) or k + 1 of slot h, across lanes and into the adjacent slot;
-// SOLO: the band has never left slot h, so the adjacent slot holds UNSET everywhere
-template <bool UP, bool SOLO>
-__device__ __forceinline__ int32_t reg_neighbor(const int32_t (&v)[kRegSlots], int h) {
+// What the steps of a pair share.
+struct RegPair {
+    int qn, tn;
+    bool fitting;
+    int64_t max_t;
+    uint32_t* rows;       // global history
+    uint64_t row_cap;
+    uint32_t* sh_hist;
+    uint32_t extra;       // word compares beyond a cell's first
+    uint32_t cells;       // diagonals of the bands
+    int t;                // last step done
+    int end_k, end_layer; // end cell, end_layer < 0: none yet
+};
+
+// Steps of a pair while its band stays inside 32 R lanes; false when it would leave them.
+template <class S, int R, int OES>
+__device__ __forceinline__ bool reg_steps(const PairSeq<S, true>& sq, RegPair& C, int (&M)[OES][R], int (&I)[R],
+                                          int (&D)[R]) {
+    constexpr int kUnset = kNeg;
     const int lane = lane_id();
-    if (UP) {
-        const int32_t a = __shfl_up_sync(PHR_FULL_MASK, v[h], 1);
-        const int32_t b =
-            SOLO ? UNSET : __shfl_sync(PHR_FULL_MASK, reg_left(h) >= 0 ? v[reg_left(h)] : UNSET, 31);
-        return lane == 0 ? b : a;
+    const int qn = C.qn, tn = C.tn;
+    const int k0 = lane - 16 * R;
+    const int kend = qn - tn;
+    const int q_last = (qn << 2) | 3;
+    const int up_src = (lane + 31) & 31, dn_src = (lane + 1) & 31;
+#pragma unroll 1
+    while (C.t < C.max_t) {
+        const int t = C.t + 1;
+        const int half = max(t - OES + 1, 0);
+        const int blo = max(-tn, -half), bhi = min(qn, half);
+        if (blo < -16 * R || bhi > 16 * R - 1 || static_cast<uint64_t>(t) >= C.row_cap) return false;
+        C.cells += static_cast<uint32_t>(bhi - blo + 1);
+        int to_up[R], to_dn[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            // [open from M, extend], open first on a tie
+            int a = M[OES - 1][r] + 4 + 1, e = I[r] + 4;
+            int c = max(a, e);
+            if (c > q_last) c = max(a > q_last ? kUnset : a, e > q_last ? kUnset : e);
+            to_up[r] = c;
+            const int t_last = ((tn + k0 + 32 * r - 1) << 2) | 3;
+            a = M[OES - 1][r] + 1, e = D[r];
+            c = max(a, e);
+            if (c > t_last) c = max(a > t_last ? kUnset : a, e > t_last ? kUnset : e);
+            to_dn[r] = c;
+        }
+        uint32_t more = 0;
+        int nM[R];
+        uint32_t aux[R];
+        int prev_up = kUnset;
+        int dn = __shfl_sync(PHR_FULL_MASK, to_dn[0], dn_src);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            constexpr int kLast = R - 1;
+            const int up_rot = __shfl_sync(PHR_FULL_MASK, to_up[r], up_src);
+            const int dn_next = r < kLast ? __shfl_sync(PHR_FULL_MASK, to_dn[r < kLast ? r + 1 : r], dn_src) : kUnset;
+            const int ins = lane == 0 ? prev_up : up_rot;
+            const int del = lane == 31 ? dn_next : dn;
+            prev_up = up_rot;
+            dn = dn_next;
+            I[r] = ins & ~3;
+            D[r] = del & ~3;
+            // [mismatch, close I, close D], the first on a tie
+            const int k = k0 + 32 * r;
+            const int hi = min(qn, tn + k);
+            int mis = M[1][r] + 4 + 3;
+            if (mis > ((hi << 2) | 3)) mis = kUnset;
+            const int m = __viaddmax_s32(I[r], 2, __viaddmax_s32(D[r], 1, mis));
+            const int pos = m >> 2;
+            const int lim = m >= 0 ? hi - pos : -1;
+            const int p = max(pos, max(k, 0));   // an unset cell reads within the staged padding
+            const int n = min(first_diff<S>(sq.diff(p, p - k)), lim);
+            nM[r] = (m & ~3) + (n << 2);         // an unset cell stays negative
+            if (n == S::kPerWord) more |= 1u << r;
+            // raw << 4 | D extends << 3 | I extends << 2 | M's source (0 mismatch, 1 I, 2 D)
+            aux[r] = (static_cast<uint32_t>(m & ~3) << 2) | (static_cast<uint32_t>(~m) & 3u) |
+                     ((static_cast<uint32_t>(~ins) & 1u) << 2) | ((static_cast<uint32_t>(~del) & 1u) << 3);
+        }
+        while (more) {   // match runs longer than one word
+            const int r = __ffs(more) - 1;
+            more &= more - 1;
+            int v = nM[0];
+#pragma unroll
+            for (int i = 1; i < R; ++i) v = r == i ? nM[i] : v;
+            const int k = k0 + 32 * r;
+            v = extend_run<S, true>(sq, v >> 2, k, min(qn, tn + k), C.extra) << 2;
+#pragma unroll
+            for (int i = 0; i < R; ++i) nM[i] = r == i ? v : nM[i];
+        }
+        // end cell: value == qn in layer order M, I, D; smallest k (largest t_end)
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int k = k0 + 32 * r;
+            any |= max(nM[r], max(I[r], D[r])) >= (qn << 2) && (C.fitting ? k >= kend : k == kend);
+        }
+        if (__any_sync(PHR_FULL_MASK, any)) {
+            int best = INT32_MAX;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int k = k0 + 32 * r;
+                const int layer = nM[r] >= (qn << 2) ? 0 : I[r] >= (qn << 2) ? 1 : D[r] >= (qn << 2) ? 2 : 3;
+                if (layer < 3 && (C.fitting ? k >= kend : k == kend)) best = min(best, (k + tn) * 4 + layer);
+            }
+            best = __reduce_min_sync(PHR_FULL_MASK, best);
+            C.end_k = (best >> 2) - tn;
+            C.end_layer = best & 3;
+        }
+        uint32_t* row = C.rows + static_cast<uint64_t>(t) * kRegWin - kRegLo;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int k = k0 + 32 * r;
+            if (t < kRegShRows && static_cast<unsigned>(k + 16) < 32u)
+                C.sh_hist[t * 32 + k + 16] = aux[r];
+            else
+                row[k] = aux[r];
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int a = OES - 1; a > 0; --a) M[a][r] = M[a - 1][r];
+            M[0][r] = nM[r];
+        }
+        C.t = t;
+        if (C.end_layer >= 0) return true;
     }
-    const int32_t a = __shfl_down_sync(PHR_FULL_MASK, v[h], 1);
-    const int32_t b = SOLO ? UNSET : __shfl_sync(PHR_FULL_MASK, reg_right(h) >= 0 ? v[reg_right(h)] : UNSET, 0);
-    return lane == 31 ? b : a;
+    return true;
 }
 
-// History rows of slot 0 (diagonals -16..15) kept in the warp's shared memory: rows of
-// scores 0 .. (kRegShRows - 1) g, which hold the whole history of most short pairs, so
-// their traceback reads shared memory.
-constexpr int kRegShRows = 32;
-// Words of a short pair's two staged sequences (qlen + tlen < kRegMaxLen, each followed by
-// one padding word for the 32-bit windows that read one word ahead).
-constexpr int kRegSeqWords = 1024 / 16 + 4;
-// Shared memory of one warp on the register path: the history rows, then the staged
-// sequences of its pair.
-constexpr int kRegWarpSmem = kRegShRows * 128 + kRegSeqWords * 4;
+// A row of 32 A lanes as one of 32 B (both centred on diagonal 0).
+template <int A, int B>
+__device__ __forceinline__ void reg_widen(const int (&x)[A], int (&y)[B]) {
+    if constexpr (A == 1) {
+        const int lane = lane_id();
+        const int a = __shfl_sync(PHR_FULL_MASK, x[0], (lane + 16) & 31);
+#pragma unroll
+        for (int i = 0; i < B; ++i) y[i] = (i == B / 2 - 1 && lane >= 16) || (i == B / 2 && lane < 16) ? a : kNeg;
+    } else {
+        constexpr int kOff = (B - A) / 2;
+#pragma unroll
+        for (int i = 0; i < B; ++i) y[i] = kNeg;
+#pragma unroll
+        for (int i = 0; i < A; ++i) y[kOff + i] = x[i];
+    }
+}
 
-// Copies a short 2-bit pair's words into `dst` (q first, then t) with the W lanes of
-// its segment; the caller synchronises the warp before reading them. Match extension
-// then reads shared memory instead of L1/L2.
-template <int W>
-__device__ __forceinline__ void stage_pair_words(uint32_t* dst, const uint32_t* q, int qn, const uint32_t* t, int tn,
-                                                 int ls, const uint32_t** sq, const uint32_t** st) {
-    const int qw = (qn + 15) / 16 + 1, tw = (tn + 15) / 16 + 1;
-    for (int i = ls; i < qw; i += W) dst[i] = __ldg(q + i);
-    for (int i = ls; i < tw; i += W) dst[qw + i] = __ldg(t + i);
-    *sq = dst;
-    *st = dst + qw;
+// The steps of a pair from a state of 32 R lanes on, widened as the band grows.
+template <class S, int R, int OES>
+__device__ __forceinline__ bool reg_search(const PairSeq<S, true>& sq, RegPair& C, int (&M)[OES][R], int (&I)[R],
+                                           int (&D)[R]) {
+    if (reg_steps<S, R, OES>(sq, C, M, I, D)) return true;
+    if constexpr (R < kRegMaxSlots) {
+        constexpr int N = R == 1 ? 2 : 2 * R;
+        int Mn[OES][N], In[N], Dn[N];
+#pragma unroll
+        for (int a = 0; a < OES; ++a) reg_widen<R, N>(M[a], Mn[a]);
+        reg_widen<R, N>(I, In);
+        reg_widen<R, N>(D, Dn);
+        return reg_search<S, N, OES>(sq, C, Mn, In, Dn);
+    } else {
+        return false;
+    }
 }
 
 // Returns true when the pair's band left the window: nothing is written for it and the
 // caller runs it through wfa_affine_group.
-template <class S, int XS, int OES, int ES>
+template <class S, int OES>
 __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
-                               uint64_t region_bytes, uint32_t* sh_hist) {
-    constexpr int RM = (XS > OES ? XS : OES);  // M values kept: steps 1..RM back
+                               uint64_t region_bytes, uint32_t sm_off, unsigned long long* work) {
     const int lane = lane_id();
     const int qn = d.qn, tn = d.tn;
-    const bool fitting = tn > qn + qn / 2 + 10;
     const int X = P.costs.mismatch, O = P.costs.gap_open, E = P.costs.gap_extend;
-    const int g = X / XS;  // the step of reachable scores
-    const uint32_t *qb, *tb;
-    stage_pair_words<32>(sh_hist + kRegShRows * 32, seq_base<S>(P, d.q_word), qn, seq_base<S>(P, d.t_word), tn, lane,
-                         &qb, &tb);
+    const int g = E;   // score of a step
+    const int qw = (qn + 15) / 16, tw = (tn + 15) / 16;
+    uint64_t* q2 = reinterpret_cast<uint64_t*>(tile_sm + sm_off + kRegShRows * 128);
+    uint64_t* t2 = q2 + qw + kRegSeqPad;
+    stage_pairs(q2, seq_base<S>(P, d.q_word), qw, lane, 32);
+    stage_pairs(t2, seq_base<S>(P, d.t_word), tw, lane, 32);
     __syncwarp();
-    const int64_t hard_max_s = static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4;
+    const PairSeq<S, true> sq{sm_off + kRegShRows * 128, sm_off + kRegShRows * 128 + (qw + kRegSeqPad) * 8, nullptr, nullptr};
 
-    // region: [runs][aux rows: kRegWin words per visited score, each word the M, I and D
-    // history of one diagonal]; row r holds score r * g, so the traceback needs no
-    // directory
+    // region: [runs][history rows: kRegWin words per step]; row r holds step r, so the
+    // traceback needs no directory
     uint32_t* runs = reinterpret_cast<uint32_t*>(region);
     const uint64_t runs_bytes = align16(static_cast<uint64_t>(qn + tn + 2) * 4);
     const uint64_t rest = region_bytes > runs_bytes ? region_bytes - runs_bytes : 0;
-    const uint64_t row_cap = rest / (kRegWin * 4);
-    uint32_t* auxs = reinterpret_cast<uint32_t*>(region + runs_bytes);
-    const int wlo = max(kRegLo, -tn), whi = min(kRegLo + kRegWin - 1, qn);  // window clipped to [-tn, qn]
-
-    int32_t M[RM][kRegSlots], I[ES][kRegSlots], D[ES][kRegSlots];
+    RegPair C = {};
+    C.qn = qn;
+    C.tn = tn;
+    C.fitting = tn > qn + qn / 2 + 10;
+    C.max_t = (static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4) / g;
+    C.rows = reinterpret_cast<uint32_t*>(region + runs_bytes);
+    C.row_cap = rest / (kRegWin * 4);
+    C.sh_hist = reinterpret_cast<uint32_t*>(tile_sm + sm_off);
+    C.end_layer = -1;
+    // ---- s = 0: M[0][0] = extend(0, 0) ----
+    const int v0 = warp_lcp<S, true>(sq, 0, 0, min(qn, tn));
+    if (v0 == qn && (C.fitting ? qn <= tn : qn == tn)) C.end_layer = 0;
+    if (lane == 0) C.sh_hist[16] = 0;   // row 0, diagonal 0
+    bool inside = C.row_cap >= 2;
+    if (inside && C.end_layer < 0) {
+        int M[OES][1], I[1] = {kNeg}, D[1] = {kNeg};
 #pragma unroll
-    for (int h = 0; h < kRegSlots; ++h) {
-#pragma unroll
-        for (int r = 0; r < RM; ++r) M[r][h] = UNSET;
-#pragma unroll
-        for (int r = 0; r < ES; ++r) {
-            I[r][h] = UNSET;
-            D[r][h] = UNSET;
-        }
-    }
-    uint32_t wf_cells = 0, lcp_words = 0;
-    bool done = false, overflow = row_cap < 2;
-    int s_end = 0, t_end = 0, k_end = 0, layer_end = 0;
-    // ---- s = 0: M[0][0] = extend(0, 0), at slot -kRegLo / 32, lane 0 ----
-    int32_t v0 = 0;
-    if (!overflow) {
-        if (lane == 0) v0 = extend_valid<S>(qb, qn, tb, tn, 0, 0, lcp_words);
-        v0 = __shfl_sync(PHR_FULL_MASK, v0, 0);
-        if (lane == 0) sh_hist[16] = 0;  // row 0 = score 0, diagonal 0 (slot 0, lane 16)
-        if (lane == 16) M[0][0] = v0;  // diagonal 0: slot 0, lane 16
-        if (!fitting) {
-            if (qn - tn == 0 && v0 == qn) done = true, t_end = tn;
-        } else if (qn <= tn && v0 == qn) {
-            done = true;
-            t_end = qn;
-        }
-    }
-    uint64_t row = 1;
-    int64_t s = g;
-    // half-width of the reachable band, floor((s - O) / E) from score O + E on, kept
-    // incrementally; `active` marks the slots the band has reached (they stay reached)
-    int hw = 0;
-    int64_t next_hw = static_cast<int64_t>(O) + E;
-    uint32_t active = 1u;
-    for (; !done && !overflow && s <= hard_max_s; s += g) {
-        // reachable diagonals of this score; leaving the window ends this kernel's attempt
-        while (s >= next_hw) {
-            ++hw;
-            next_hw += E;
-        }
-        const int blo = max(-tn, -hw);
-        const int bhi = min(qn, hw);
-        if (blo < wlo || bhi > whi || row >= row_cap) {
-            overflow = true;
-            break;
-        }
-        if (lane == 0) wf_cells += static_cast<uint32_t>(bhi - blo + 1);
-        uint32_t* arow = auxs + row * kRegWin;
-        uint32_t* srow = row < kRegShRows ? sh_hist + row * 32 : nullptr;
-        int32_t nM[kRegSlots], nI[kRegSlots], nD[kRegSlots];
-        int best_k = INT32_MAX, best_l = 0;
-        // one slot of this score; h and SOLO are compile-time
-        auto step_slot = [&](auto hc, auto soloc) {
-            constexpr int h = decltype(hc)::value;
-            constexpr bool solo = decltype(soloc)::value;
-            nM[h] = nI[h] = nD[h] = UNSET;
-            constexpr int klo = reg_slot_lo(h);
-            if (klo + 31 < blo || klo > bhi) return;  // warp-uniform: slot outside the band
-            active |= 1u << h;
-            const int k = klo + lane;
-            // affine_pos_valid for this diagonal as one unsigned range test: pos in
-            // [max(0, k), min(qn, tn + k)] (an empty range admits nothing; UNSET and
-            // UNSET + 1 wrap far above any span)
-            const int vl = max(0, k), vh = min(qn, tn + k);
-            const uint32_t vlo = vh >= vl ? static_cast<uint32_t>(vl) : 0x40000000u;
-            const uint32_t vspan = vh >= vl ? static_cast<uint32_t>(vh - vl) : 0u;
-            auto ok = [&](int32_t pos) { return static_cast<uint32_t>(pos) - vlo <= vspan; };
-            const int32_t mo_dn = reg_neighbor<true, solo>(M[OES - 1], h);   // M[s - O - E][k - 1]
-            const int32_t ie_dn = reg_neighbor<true, solo>(I[ES - 1], h);    // I[s - E][k - 1]
-            const int32_t mo_up = reg_neighbor<false, solo>(M[OES - 1], h);  // M[s - O - E][k + 1]
-            const int32_t de_up = reg_neighbor<false, solo>(D[ES - 1], h);   // D[s - E][k + 1]
-            // I (wfa_simd.rs:682-738): [open from M, extend I], strict >
-            int32_t ins = UNSET;
-            uint32_t iop = 0;
-            if (ok(mo_dn + 1)) ins = mo_dn + 1;
-            if (ok(ie_dn + 1) && ie_dn + 1 > ins) {
-                ins = ie_dn + 1;
-                iop = 1;
-            }
-            int32_t del = UNSET;
-            uint32_t dop = 0;
-            if (ok(mo_up)) del = mo_up;
-            if (ok(de_up) && de_up > del) {
-                del = de_up;
-                dop = 1;
-            }
-            // M (wfa_simd.rs:743-765): [mismatch-extend, ins close, del close], strict >
-            // (ins and del are UNSET or valid already)
-            int32_t best = UNSET;
-            uint32_t mop = 0;
-            if (ok(M[XS - 1][h] + 1)) best = M[XS - 1][h] + 1;
-            if (ins != UNSET && ins > best) {
-                best = ins;
-                mop = 1;
-            }
-            if (del != UNSET && del > best) {
-                best = del;
-                mop = 2;
-            }
-            int32_t mval = UNSET;
-            uint32_t aux = (dop << 3) | (iop << 2);
-            if (best != UNSET) {
-                mval = extend_valid<S>(qb, qn, tb, tn, best, k, lcp_words);
-                aux |= (static_cast<uint32_t>(best) << 4) | mop;
-            }
-            nM[h] = mval;
-            nI[h] = ins;
-            nD[h] = del;
-            if (h == 0 && srow)
-                srow[lane] = aux;
-            else
-                arow[k - kRegLo] = aux;
-            // end cell: value == qn in layer order m, ins, del; smallest k (largest t_end)
-            const int layer = mval == qn ? 0 : ins == qn ? 1 : del == qn ? 2 : -1;
-            const bool cand = layer >= 0 && (fitting ? k >= qn - tn : k == qn - tn);
-            const unsigned bal = __ballot_sync(PHR_FULL_MASK, cand);
-            if (bal) {
-                const int src = __ffs(bal) - 1;
-                const int l = __shfl_sync(PHR_FULL_MASK, layer, src);
-                if (klo + src < best_k) {
-                    best_k = klo + src;
-                    best_l = l;
-                }
-            }
-        };
-        // shift the history of slot h: this score becomes one step back
-        auto shift_slot = [&](int h) {
-#pragma unroll
-            for (int r = RM - 1; r > 0; --r) M[r][h] = M[r - 1][h];
-            M[0][h] = nM[h];
-#pragma unroll
-            for (int r = ES - 1; r > 0; --r) {
-                I[r][h] = I[r - 1][h];
-                D[r][h] = D[r - 1][h];
-            }
-            I[0][h] = nI[h];
-            D[0][h] = nD[h];
-        };
-        if (blo >= -16 && bhi <= 15) {
-            // the band has never left slot 0 (it only grows): one slot, no cross-slot shuffles
-            step_slot(std::integral_constant<int, 0>{}, std::true_type{});
-            shift_slot(0);
-        } else {
-            step_slot(std::integral_constant<int, 0>{}, std::false_type{});
-            step_slot(std::integral_constant<int, 1>{}, std::false_type{});
-            step_slot(std::integral_constant<int, 2>{}, std::false_type{});
-            step_slot(std::integral_constant<int, 3>{}, std::false_type{});
-            step_slot(std::integral_constant<int, 4>{}, std::false_type{});
-            static_assert(kRegSlots == 5, "one step_slot call per slot");
-#pragma unroll
-            for (int h = 0; h < kRegSlots; ++h)
-                if ((active >> h) & 1u) shift_slot(h);
-        }
-        ++row;  // the traceback addresses row s / g directly (no directory)
-        if (best_k != INT32_MAX) {
-            done = true;
-            s_end = static_cast<int>(s);
-            t_end = qn - best_k;
-            k_end = best_k;
-            layer_end = best_l;
-        }
+        for (int a = 0; a < OES; ++a) M[a][0] = kNeg;
+        if (lane == 16) M[0][0] = v0 << 2;
+        inside = reg_search<S, 1, OES>(sq, C, M, I, D);
     }
     {
-        const unsigned lw = __reduce_add_sync(PHR_FULL_MASK, lcp_words);
-        if (lane == 0 && P.work) {
-            atomicAdd(P.work + 2, static_cast<unsigned long long>(wf_cells));
-            atomicAdd(P.work + 3, static_cast<unsigned long long>(lw));
+        const unsigned extra = __reduce_add_sync(PHR_FULL_MASK, C.extra);
+        if (lane == 0) {
+            work[0] += C.cells;
+            work[1] += C.cells + extra + 1;
         }
     }
     __syncwarp();
-    if (overflow) return true;  // wfa_affine_group takes it, which sizes its bands per score
-    affine_finish(P, pid, true, 32, qn, tn, X, O, E, runs, auxs, nullptr, done, !done, s_end, t_end, k_end,
-                  layer_end, g, kRegWin, kRegLo, sh_hist, kRegShRows);
+    if (!inside) return true;   // wfa_affine_group takes it, which sizes its bands per score
+    const bool done = C.end_layer >= 0;
+    affine_finish(P, pid, true, 32, qn, tn, X, O, E, runs, C.rows, nullptr, done, !done, C.t * g, qn - C.end_k, C.end_k,
+                  C.end_layer, g, kRegWin, kRegLo, C.sh_hist, kRegShRows);
     return false;
 }
 
@@ -1455,16 +1440,31 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
 constexpr int kAffGroupSmem = kAffRingGroups * kAffRing * static_cast<int>(sizeof(SDir)) + kWarpSeqWords * 4;
 constexpr int kAffWarpSmem = kAffGroupSmem > kRegWarpSmem ? kAffGroupSmem : kRegWarpSmem;
 
+constexpr uint32_t kTaskGrab = 4;   // tasks a warp takes at a time
+
 template <class S, bool kAffine>
 __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams P) {
     extern __shared__ __align__(16) uint8_t wfa_smem[];
     const int lane = lane_id();
     const uint64_t warp_global = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    for (;;) {
-        uint32_t task = 0;
-        if (lane == 0) task = P.tasks.range[0] + atomicAdd(P.queue_head, 1u);
-        task = __shfl_sync(PHR_FULL_MASK, task, 0);
-        if (task >= P.tasks.range[1]) break;
+    // One counter hands out every task, and an addition to one address costs about a
+    // nanosecond (300,000 equal pairs of 100-300 bp with three of them a pair: 1.00 ms; with
+    // one a four tasks, and the work counters' sums kept per warp: 0.45). Gap-affine tasks of
+    // a pair each are taken by fours where a warp gets 128 or more, so that the last ones of
+    // the launch wait for little; linear tasks hold up to 16 pairs and lose 4 % by the same.
+    __shared__ unsigned long long sh_work[kAffine ? 8 : 1][2];
+    unsigned long long* work = sh_work[kAffine ? threadIdx.x >> 5 : 0];
+    if (kAffine && lane == 0) work[0] = work[1] = 0;
+    const uint32_t grab =
+        kAffine && P.tasks.range[1] - P.tasks.range[0] >= 32 * kTaskGrab * (gridDim.x * blockDim.x / 32) ? kTaskGrab : 1;
+    uint32_t task = 0, batch_end = 0;
+    for (;; ++task) {
+        if (!kAffine || task == batch_end) {
+            if (lane == 0) task = P.tasks.range[0] + atomicAdd(P.queue_head, grab);
+            task = __shfl_sync(PHR_FULL_MASK, task, 0);
+            if (task >= P.tasks.range[1]) break;
+            batch_end = min(task + grab, P.tasks.range[1]);
+        }
         uint8_t* slot = P.task_off ? P.scratch + P.task_off[task] : P.scratch + warp_global * P.slot_bytes;
         const uint64_t slot_bytes = P.task_off ? P.task_len[task] : P.slot_bytes;
         const uint8_t tg = P.tasks.task_group[task];
@@ -1498,13 +1498,11 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
             // short 2-bit pairs of one warp each, costs with a register specialisation:
             // wavefronts in registers (redo passes and wide bands take the group kernel)
             if (G == 32 && !P.task_off && act && d.qn + d.tn < kRegMaxLen) {
-                const int X = P.costs.mismatch, O = P.costs.gap_open, E = P.costs.gap_extend;
-                uint32_t* sh_hist = reinterpret_cast<uint32_t*>(wfa_smem + static_cast<size_t>(threadIdx.x >> 5) *
-                                                                                  kAffWarpSmem);
+                const uint32_t sm_off = (threadIdx.x >> 5) * static_cast<uint32_t>(kAffWarpSmem);
+                const int open = aff_tile_open(P.costs);
                 bool wide = true;  // the band left the register window (or no specialisation)
-                if (X == 4 && O == 6 && E == 2) wide = wfa_affine_reg<S, 2, 4, 1>(P, d, pid, region, region_bytes, sh_hist);
-                else if (X == 2 && O == 4 && E == 1)
-                    wide = wfa_affine_reg<S, 2, 5, 1>(P, d, pid, region, region_bytes, sh_hist);
+                if (open == 4) wide = wfa_affine_reg<S, 4>(P, d, pid, region, region_bytes, sm_off, work);
+                else if (open == 5) wide = wfa_affine_reg<S, 5>(P, d, pid, region, region_bytes, sm_off, work);
                 if (!wide) continue;
                 // otherwise the group kernel below takes the pair in place (no redo pass)
             }
@@ -1517,10 +1515,14 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
             uint32_t* sseq = seq_words > 0 ? reinterpret_cast<uint32_t*>(wsm + kAffRingGroups * kAffRing * sizeof(SDir)) +
                                                  grp * seq_words
                                            : nullptr;
-            wfa_affine_group<S>(P, d, pid, act, G, region, region_bytes, ring, sseq, seq_words);
+            wfa_affine_group<S>(P, d, pid, act, G, region, region_bytes, ring, sseq, seq_words, work);
         }
         else
             wfa_linear_group<S>(P, d, pid, act, G, region, region_bytes);
+    }
+    if (kAffine && lane == 0 && P.work) {
+        atomicAdd(P.work + 2, work[0]);
+        atomicAdd(P.work + 3, work[1]);
     }
 }
 
