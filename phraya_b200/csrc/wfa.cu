@@ -477,6 +477,39 @@ __device__ __forceinline__ bool pos_ok(int32_t pos, int k, int qn, int tn) {
            static_cast<uint32_t>(pos) - static_cast<uint32_t>(k) <= static_cast<uint32_t>(tn);
 }
 
+// CIGAR text and record of a pair whose group leader has walked its runs into `rw`.
+__device__ __forceinline__ void affine_result(const ExtendParams& P, uint32_t pid, bool act, int G, bool trace, bool failed,
+                                              const RunWriter& rw, const uint32_t* runs, uint32_t n_edit, int s_end,
+                                              int t_end) {
+    const int gl = lane_id() & (G - 1);
+    const int leader = lane_id() & ~(G - 1);
+    const uint32_t nr = __shfl_sync(PHR_FULL_MASK, rw.n, leader);
+    const bool ovf = __shfl_sync(PHR_FULL_MASK, rw.overflow ? 1 : 0, leader) != 0;
+    const uint32_t ned = __shfl_sync(PHR_FULL_MASK, n_edit, leader);
+    __syncwarp();
+    const uint32_t nr_fmt = (trace && !ovf) ? nr : 0;
+    char* out = act ? P.text + P.text_off[pid] : nullptr;
+    const uint32_t tl = format_group(runs, nr_fmt, out, G);
+    if (act && gl == 0) {
+        if (trace && !ovf) {
+            PairOut o;
+            o.status = PHR_OK;
+            o.ed = static_cast<int32_t>(ned);  // levenshtein_from_cigar: X + I/D lengths
+            o.t_consumed = t_end;
+            o.affine_score = s_end;
+            o.n_runs = nr;
+            o.text_len = tl;
+            P.out[pid] = o;
+        } else if (failed) {
+            PairOut o = {};
+            o.status = PHR_ALIGNMENT_FAILED;
+            P.out[pid] = o;
+        } else if (trace && ovf) {
+            atomicOr(P.error_flag, 2u);
+        }
+    }
+}
+
 // Traceback (wfa_simd.rs:785-886) of a finished affine wavefront and the pair's result:
 // history in `auxs` through the score directory below `dir_top`. Called by all lanes of
 // the warp; the leader of each group of G lanes walks its pair.
@@ -487,9 +520,7 @@ __device__ __forceinline__ bool pos_ok(int32_t pos, int k, int qn, int tn) {
 // kernel).
 __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int G, int qn, int tn, int X, int O,
                               int E, uint32_t* runs, const uint32_t* auxs, const AffDir* dir_top, bool done,
-                              bool failed, int s_end, int t_end, int k_end, int layer_end, int row_g = 0,
-                              int row_w = 0, int row_lo = 0, const uint32_t* sh_hist = nullptr, int sh_rows = 0,
-                              bool folded = false) {
+                              bool failed, int s_end, int t_end, int k_end, int layer_end, bool folded = false) {
     const int gl = lane_id() & (G - 1);
     auto dir_at = [&](int64_t sc) -> const AffDir& { return dir_top[-1 - sc]; };
     auto aux_at = [&](int ss, int layer, int k) -> uint32_t {
@@ -497,15 +528,6 @@ __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int
             // one word per diagonal of the score's M band (the CTA kernel's layout)
             const LayerBand& b = dir_at(ss).L[0];
             const uint32_t w = auxs[b.base + (k - b.lo)];
-            return layer == 0 ? (((w >> 4) << 2) | (w & 3u)) : (w >> (layer + 1)) & 1u;
-        }
-        if (row_g > 0) {
-            // rows below sh_rows of diagonals -16..15 live in shared memory
-            // row of score ss (a multiple of g; g is 1 or 2 for the specialised costs)
-            const int rr = row_g == 1 ? ss : row_g == 2 ? (ss >> 1) : ss / row_g;
-            const uint32_t w = (rr < sh_rows && static_cast<unsigned>(k + 16) < 32u)
-                                   ? sh_hist[rr * 32 + (k + 16)]
-                                   : auxs[static_cast<uint64_t>(rr) * row_w + (k - row_lo)];
             return layer == 0 ? (((w >> 4) << 2) | (w & 3u)) : (w >> (layer + 1)) & 1u;
         }
         const LayerBand& b = dir_at(ss).L[layer];
@@ -572,32 +594,7 @@ __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int
         if (guard < 0) atomicOr(P.error_flag, 4u);
         rw.flush();
     }
-    const int leader = lane_id() & ~(G - 1);
-    const uint32_t nr = __shfl_sync(PHR_FULL_MASK, rw.n, leader);
-    const bool ovf = __shfl_sync(PHR_FULL_MASK, rw.overflow ? 1 : 0, leader) != 0;
-    const uint32_t ned = __shfl_sync(PHR_FULL_MASK, n_edit, leader);
-    __syncwarp();
-    const uint32_t nr_fmt = (trace && !ovf) ? nr : 0;
-    char* out = act ? P.text + P.text_off[pid] : nullptr;
-    const uint32_t tl = format_group(runs, nr_fmt, out, G);
-    if (act && gl == 0) {
-        if (trace && !ovf) {
-            PairOut o;
-            o.status = PHR_OK;
-            o.ed = static_cast<int32_t>(ned);  // levenshtein_from_cigar: X + I/D lengths
-            o.t_consumed = t_end;
-            o.affine_score = s_end;
-            o.n_runs = nr;
-            o.text_len = tl;
-            P.out[pid] = o;
-        } else if (failed) {
-            PairOut o = {};
-            o.status = PHR_ALIGNMENT_FAILED;
-            P.out[pid] = o;
-        } else if (trace && ovf) {
-            atomicOr(P.error_flag, 2u);
-        }
-    }
+    affine_result(P, pid, act, G, trace, failed, rw, runs, n_edit, s_end, t_end);
 }
 
 template <class S>
@@ -1154,7 +1151,7 @@ __device__ void wfa_affine_cta(const ExtendParams& P, const PairDesc& d, uint32_
     __syncthreads();
     if (tid < 32)
         affine_finish(P, pid, true, 32, qn, tn, X, O, E, runs, auxs, dir_top, done, failed, s_end, t_end, k_end,
-                      layer_end, 0, 0, 0, nullptr, 0, true);
+                      layer_end, true);
     __syncthreads();
 }
 
@@ -1198,19 +1195,19 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
 // wfa_affine_group in the same warp.
 // Before, four values crossed lanes per cell, validity was a range test per candidate and
 // wide bands stepped five slots of which some lay outside: 1,000,000 pairs of 100-300 bp at
-// 0-5 %, costs (4, 6, 2), 8.57 -> 6.12 ms (6,213 -> about 4,100 warp instructions a pair);
-// 300,000 at 0-10 % 6.88 -> 4.99, at 0-20 % 27.1 -> 18.3, of 300-480 bp 6.62 -> 5.04.
+// 0-5 %, costs (4, 6, 2), 8.57 -> 5.72 ms (6,213 -> about 3,950 warp instructions a pair),
+// and 4.43 in wfa_affine_short_kernel; 300,000 at 0-10 % 6.88 -> 4.24, at 0-20 %
+// 27.1 -> 17.7, of 300-480 bp 6.62 -> 4.14.
 // With 4 slots at most, pairs whose band passes 128 diagonals are done twice: 7.97 at 0-10 %.
 constexpr int kRegMaxLen = 1024;  // qlen + tlen below which a pair tries the register path
-constexpr int kRegMaxSlots = 8;   // most diagonals per lane
-constexpr int kRegWin = 32 * kRegMaxSlots;   // history words of a step's row, from diagonal kRegLo on
-constexpr int kRegLo = -kRegWin / 2;
+constexpr int kRegSlots = 8;      // most diagonals per lane here
+constexpr int kRegFewSlots = 4;   // and in the kernel for short pairs alone
 // History rows of diagonals -16..15 kept in the warp's shared memory: those of the first
 // kRegShRows steps, which hold the whole history of most short pairs.
 constexpr int kRegShRows = 32;
 // A short pair's sequences as overlapping word pairs, each with room for reads from
 // diagonals outside the pair.
-constexpr int kRegSeqPad = kRegWin / 32 + 4;
+constexpr int kRegSeqPad = kRegSlots + 4;
 constexpr int kRegSeqEntries = kRegMaxLen / 16 + 2 + 2 * kRegSeqPad;
 constexpr int kRegWarpSmem = kRegShRows * 128 + kRegSeqEntries * 8;
 
@@ -1219,7 +1216,8 @@ struct RegPair {
     int qn, tn;
     bool fitting;
     int64_t max_t;
-    uint32_t* rows;       // global history
+    uint32_t* rows;       // global history: `win` words a step, diagonals -win / 2 on
+    int win;
     uint64_t row_cap;
     uint32_t* sh_hist;
     uint32_t extra;       // word compares beyond a cell's first
@@ -1322,7 +1320,7 @@ __device__ __forceinline__ bool reg_steps(const PairSeq<S, true>& sq, RegPair& C
             C.end_k = (best >> 2) - tn;
             C.end_layer = best & 3;
         }
-        uint32_t* row = C.rows + static_cast<uint64_t>(t) * kRegWin - kRegLo;
+        uint32_t* row = C.rows + static_cast<uint64_t>(t) * C.win + C.win / 2;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int k = k0 + 32 * r;
@@ -1361,26 +1359,77 @@ __device__ __forceinline__ void reg_widen(const int (&x)[A], int (&y)[B]) {
 }
 
 // The steps of a pair from a state of 32 R lanes on, widened as the band grows.
-template <class S, int R, int OES>
+template <class S, int R, int RMAX, int OES>
 __device__ __forceinline__ bool reg_search(const PairSeq<S, true>& sq, RegPair& C, int (&M)[OES][R], int (&I)[R],
                                            int (&D)[R]) {
     if (reg_steps<S, R, OES>(sq, C, M, I, D)) return true;
-    if constexpr (R < kRegMaxSlots) {
-        constexpr int N = R == 1 ? 2 : 2 * R;
+    if constexpr (R < RMAX) {
+        constexpr int N = 2 * R;
         int Mn[OES][N], In[N], Dn[N];
 #pragma unroll
         for (int a = 0; a < OES; ++a) reg_widen<R, N>(M[a], Mn[a]);
         reg_widen<R, N>(I, In);
         reg_widen<R, N>(D, Dn);
-        return reg_search<S, N, OES>(sq, C, Mn, In, Dn);
+        return reg_search<S, N, RMAX, OES>(sq, C, Mn, In, Dn);
     } else {
         return false;
     }
 }
 
+// Path of a finished pair from its history (lane 0), its text and record.
+template <int OES>
+__device__ __forceinline__ void reg_finish(const ExtendParams& P, uint32_t pid, const RegPair& C, uint32_t* runs, int g) {
+    RunWriter rw;
+    rw.init(runs, static_cast<uint32_t>(C.qn + C.tn + 2));
+    const bool trace = C.end_layer >= 0;
+    uint32_t n_edit = 0;
+    if (trace && lane_id() == 0) {
+        int qi = C.qn, ti = C.qn - C.end_k, k = C.end_k, t = C.t, layer = C.end_layer;
+        int guard = 4 * (C.qn + C.tn) + 16;
+        while ((qi > 0 || ti > 0) && guard-- > 0) {
+            if (t == 0) {
+                const int mm = min(qi, ti);
+                rw.push(0, static_cast<uint32_t>(mm));
+                qi -= mm;
+                ti -= mm;
+                break;
+            }
+            const uint32_t w = t < kRegShRows && static_cast<unsigned>(k + 16) < 32u
+                                   ? C.sh_hist[t * 32 + k + 16]
+                                   : C.rows[static_cast<uint64_t>(t) * C.win + C.win / 2 + k];
+            if (layer == 0) {
+                const int mc = max(qi - static_cast<int>(w >> 4), 0);
+                rw.push(0, static_cast<uint32_t>(mc));
+                qi -= mc;
+                ti -= mc;
+                layer = static_cast<int>(w & 3u);
+                if (layer == 0) {
+                    rw.push(1, 1);
+                    --qi;
+                    --ti;
+                    ++n_edit;
+                    t -= 2;
+                    continue;
+                }
+            }
+            ++n_edit;
+            const bool ins = layer == 1;   // query-extra -> 'D'; target-extra -> 'I'
+            const bool open = ((w >> (layer + 1)) & 1u) == 0;
+            rw.push(ins ? 3 : 2, 1);
+            if (ins) --qi, --k;
+            else --ti, ++k;
+            t -= open ? OES : 1;
+            if (open) layer = 0;
+        }
+        if (guard < 0) atomicOr(P.error_flag, 4u);
+        rw.flush();
+    }
+    affine_result(P, pid, true, 32, trace, !trace, rw, runs, n_edit, C.t * g, C.qn - C.end_k);
+}
+
 // Returns true when the pair's band left the window: nothing is written for it and the
-// caller runs it through wfa_affine_group.
-template <class S, int OES>
+// caller runs it another way.
+template <class S, int RMAX, int OES>
 __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
                                uint64_t region_bytes, uint32_t sm_off, unsigned long long* work) {
     const int lane = lane_id();
@@ -1395,7 +1444,7 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
     __syncwarp();
     const PairSeq<S, true> sq{sm_off + kRegShRows * 128, sm_off + kRegShRows * 128 + (qw + kRegSeqPad) * 8, nullptr, nullptr};
 
-    // region: [runs][history rows: kRegWin words per step]; row r holds step r, so the
+    // region: [runs][history rows: a word per diagonal of the window]; row r holds step r, so the
     // traceback needs no directory
     uint32_t* runs = reinterpret_cast<uint32_t*>(region);
     const uint64_t runs_bytes = align16(static_cast<uint64_t>(qn + tn + 2) * 4);
@@ -1406,7 +1455,8 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
     C.fitting = tn > qn + qn / 2 + 10;
     C.max_t = (static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4) / g;
     C.rows = reinterpret_cast<uint32_t*>(region + runs_bytes);
-    C.row_cap = rest / (kRegWin * 4);
+    C.win = 32 * RMAX;
+    C.row_cap = rest / (C.win * 4);
     C.sh_hist = reinterpret_cast<uint32_t*>(tile_sm + sm_off);
     C.end_layer = -1;
     // ---- s = 0: M[0][0] = extend(0, 0) ----
@@ -1419,7 +1469,7 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
 #pragma unroll
         for (int a = 0; a < OES; ++a) M[a][0] = kNeg;
         if (lane == 16) M[0][0] = v0 << 2;
-        inside = reg_search<S, 1, OES>(sq, C, M, I, D);
+        inside = reg_search<S, 1, RMAX, OES>(sq, C, M, I, D);
     }
     {
         const unsigned extra = __reduce_add_sync(PHR_FULL_MASK, C.extra);
@@ -1429,10 +1479,8 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
         }
     }
     __syncwarp();
-    if (!inside) return true;   // wfa_affine_group takes it, which sizes its bands per score
-    const bool done = C.end_layer >= 0;
-    affine_finish(P, pid, true, 32, qn, tn, X, O, E, runs, C.rows, nullptr, done, !done, C.t * g, qn - C.end_k, C.end_k,
-                  C.end_layer, g, kRegWin, kRegLo, C.sh_hist, kRegShRows);
+    if (!inside) return true;
+    reg_finish<OES>(P, pid, C, runs, g);
     return false;
 }
 
@@ -1457,14 +1505,15 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
     if (kAffine && lane == 0) work[0] = work[1] = 0;
     const uint32_t grab =
         kAffine && P.tasks.range[1] - P.tasks.range[0] >= 32 * kTaskGrab * (gridDim.x * blockDim.x / 32) ? kTaskGrab : 1;
-    uint32_t task = 0, batch_end = 0;
-    for (;; ++task) {
-        if (!kAffine || task == batch_end) {
-            if (lane == 0) task = P.tasks.range[0] + atomicAdd(P.queue_head, grab);
-            task = __shfl_sync(PHR_FULL_MASK, task, 0);
-            if (task >= P.tasks.range[1]) break;
-            batch_end = min(task + grab, P.tasks.range[1]);
+    uint32_t next = 0, batch_end = 0;
+    for (;; ++next) {
+        if (!kAffine || next == batch_end) {
+            if (lane == 0) next = P.tasks.range[0] + atomicAdd(P.queue_head, grab);
+            next = __shfl_sync(PHR_FULL_MASK, next, 0);
+            if (next >= P.tasks.range[1]) break;
+            batch_end = min(next + grab, P.tasks.range[1]);
         }
+        const uint32_t task = kAffine && P.task_list ? P.task_list[next] : next;
         uint8_t* slot = P.task_off ? P.scratch + P.task_off[task] : P.scratch + warp_global * P.slot_bytes;
         const uint64_t slot_bytes = P.task_off ? P.task_len[task] : P.slot_bytes;
         const uint8_t tg = P.tasks.task_group[task];
@@ -1501,8 +1550,8 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
                 const uint32_t sm_off = (threadIdx.x >> 5) * static_cast<uint32_t>(kAffWarpSmem);
                 const int open = aff_tile_open(P.costs);
                 bool wide = true;  // the band left the register window (or no specialisation)
-                if (open == 4) wide = wfa_affine_reg<S, 4>(P, d, pid, region, region_bytes, sm_off, work);
-                else if (open == 5) wide = wfa_affine_reg<S, 5>(P, d, pid, region, region_bytes, sm_off, work);
+                if (open == 4) wide = wfa_affine_reg<S, kRegSlots, 4>(P, d, pid, region, region_bytes, sm_off, work);
+                else if (open == 5) wide = wfa_affine_reg<S, kRegSlots, 5>(P, d, pid, region, region_bytes, sm_off, work);
                 if (!wide) continue;
                 // otherwise the group kernel below takes the pair in place (no redo pass)
             }
@@ -1521,6 +1570,58 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
             wfa_linear_group<S>(P, d, pid, act, G, region, region_bytes);
     }
     if (kAffine && lane == 0 && P.work) {
+        atomicAdd(P.work + 2, work[0]);
+        atomicAdd(P.work + 3, work[1]);
+    }
+}
+
+// Bytes of a warp's region in the kernel below: runs and rows of its widest band's steps.
+constexpr uint64_t kShortSlot = ((kRegMaxLen + 2) * 4 + 15) / 16 * 16 + (16 * kRegFewSlots + 16) * (32 * kRegFewSlots * 4);
+
+// The register path alone, for batches that fill the chip: without the group path's registers
+// and code three CTAs fit an SM where wfa_kernel has two, which the stalls on the steps' own
+// dependences need (general kernel: an instruction in 52 % of the cycles). A task whose pair
+// is too long or too wide goes to wfa_kernel by `left`. 1,000,000 pairs of 100-300 bp at
+// 0-5 %: 5.72 -> 4.43 ms; four CTAs, with spills, 4.54.
+template <int OES>
+__global__ void __launch_bounds__(256, 3) wfa_affine_short_kernel(ExtendParams P, uint32_t* left, uint32_t* n_left) {
+    __shared__ unsigned long long sh_work[8][2];
+    const int lane = lane_id();
+    unsigned long long* work = sh_work[threadIdx.x >> 5];
+    if (lane == 0) work[0] = work[1] = 0;
+    const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    uint8_t* region = P.scratch + warp * kShortSlot;
+    const uint32_t sm_off = (threadIdx.x >> 5) * static_cast<uint32_t>(kRegWarpSmem);
+    const uint32_t end = P.tasks.range[1];
+    for (;;) {
+        uint32_t base = 0;
+        if (lane == 0) base = P.tasks.range[0] + atomicAdd(P.queue_head, kTaskGrab);
+        base = __shfl_sync(PHR_FULL_MASK, base, 0);
+        if (base >= end) break;
+        const uint32_t n = min(kTaskGrab, end - base);
+        // the batch's pairs, a lane each
+        uint32_t pid_l = 0;
+        bool ok_l = false;
+        PairDesc d_l = {};
+        if (static_cast<uint32_t>(lane) < n && P.tasks.task_group[base + lane] == 32) {
+            pid_l = P.tasks.order[P.tasks.task_first[base + lane]];
+            d_l = P.desc[pid_l];
+            ok_l = d_l.mode == 0 && d_l.qn + d_l.tn < kRegMaxLen &&
+                   !big_pair(P.engine, P.big_min, P.big_smem, d_l.qn, d_l.tn, d_l.mode);
+        }
+        for (uint32_t i = 0; i < n; ++i) {
+            PairDesc d = {};
+            d.qn = __shfl_sync(PHR_FULL_MASK, d_l.qn, i);
+            d.tn = __shfl_sync(PHR_FULL_MASK, d_l.tn, i);
+            d.q_word = __shfl_sync(PHR_FULL_MASK, d_l.q_word, i);
+            d.t_word = __shfl_sync(PHR_FULL_MASK, d_l.t_word, i);
+            const uint32_t pid = __shfl_sync(PHR_FULL_MASK, pid_l, i);
+            bool wide = __shfl_sync(PHR_FULL_MASK, ok_l ? 0 : 1, i) != 0;
+            if (!wide) wide = wfa_affine_reg<Seq2, kRegFewSlots, OES>(P, d, pid, region, kShortSlot, sm_off, work);
+            if (wide && lane == 0) left[atomicAdd(n_left, 1u)] = base + i;
+        }
+    }
+    if (lane == 0 && P.work) {
         atomicAdd(P.work + 2, work[0]);
         atomicAdd(P.work + 3, work[1]);
     }
@@ -1546,6 +1647,17 @@ void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mod
     }
 }
 
+int launch_wfa_affine_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int blocks_per_sm, uint32_t* left,
+                            uint32_t* n_left, cudaStream_t st) {
+    const int smem = 8 * kRegWarpSmem;
+    const uint64_t fit = scratch_bytes / (8 * kShortSlot);
+    const int grid = static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(sms) * std::min(blocks_per_sm, 3), fit));
+    if (grid == 0) return 0;
+    auto* kernel = aff_tile_open(p.costs) == 4 ? wfa_affine_short_kernel<4> : wfa_affine_short_kernel<5>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kernel<<<grid, 256, smem, st>>>(p, left, n_left);
+    return grid;
+}
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st) {
     const int smem = (block / 32) * kAffWarpSmem;
     cudaFuncSetAttribute(wfa_kernel<Seq2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

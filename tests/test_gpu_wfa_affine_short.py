@@ -45,9 +45,10 @@ def pairs_of(rng):
 
 
 @pytest.mark.parametrize("costs", [(2, 4, 1), (4, 6, 2), (6, 12, 3), (4, 8, 2), (1, 3, 1)])
-@pytest.mark.parametrize("copies", [1, 40])
+@pytest.mark.parametrize("copies", [1, 40, 540])
 def test_short_affine(costs, copies):
-    """One batch of a few hundred pairs, and one of more than the small-batch limit."""
+    """Batches of a few hundred pairs, of more than the small-batch limit, and of enough for
+    the kernel for short pairs alone, which leaves the wide ones to the general one."""
     rng = np.random.default_rng(71)
     packed = O.PackedPairs(pairs_of(rng) * copies)
     oa, oc = O.extend_packed(A.ENGINE_WFA_AFFINE, O.PackedPairs(pairs_of(np.random.default_rng(71))), costs)
