@@ -975,8 +975,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     uint64_t* rtask_len = static_cast<uint64_t*>(take(n * 8));
     // counters: [0..3] ranges, [4] split_min, [5] queue head 0, [6] queue head 1,
     // [7] redo count, [8..9] need max (u64), [10] error flag, [12..13] total (u64), [14..17] redo ranges,
-    // [20] first multi-lane 2-bit task, [21] queue head of the short gap-affine kernel, [22..23] range of
-    // the tasks it left (from 0), [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
+    // [20] first multi-lane 2-bit task, [21] queue head of the kernel for short WFA pairs, [22..23] range of
+    // the pairs it left (from 0), [24..25] CTA-kernel queue heads, [26] lane-kernel queue head,
     // [28..31] lane-kernel and warp-group 2-bit ranges (global Myers), [32..39] work counters (u64),
     // [40..43] first register-tile task of each kind (one warp 2-bit / bytes, CTA 2-bit / bytes),
     // [44..51] their ranges, [52..55] their scratch need: sum, largest (u64), [56..59] their queue
@@ -1200,15 +1200,16 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             }
         }
         P.tasks.range = range0;
-        if (!per_task && engine == PHR_ENGINE_WFA_AFFINE && aff_tile_open(costs) != 0 &&
-            n_group2 > kShortAffineMin * static_cast<uint32_t>(ctx->sm_count)) {
-            // more short pairs than the warps of the general kernel: most end in the kernel for
-            // them alone, the rest follow below from its list
+        const uint32_t short_min = engine == PHR_ENGINE_WFA_LINEAR ? kShortLinearMin : kShortAffineMin;
+        if (!per_task && (engine == PHR_ENGINE_WFA_LINEAR || (engine == PHR_ENGINE_WFA_AFFINE && aff_tile_open(costs) != 0)) &&
+            P.big_min > 0 && n_group2 > short_min * static_cast<uint32_t>(ctx->sm_count)) {
+            // most short pairs of a large batch end in the kernel for them alone, the rest
+            // follow below from its list
             P.queue_head = cnt + 21;
             KernelScope ks(ctx, kname);
-            if (launch_wfa_affine_short(P, grid * warps_per_block * slot, ctx->sm_count, ctx->tune.max_blocks_per_sm, head,
-                                        cnt + 23, st) > 0) {
-                P.task_list = head;
+            if (launch_wfa_short(P, grid * warps_per_block * slot, ctx->sm_count, ctx->tune.max_blocks_per_sm, head, cnt + 23,
+                                 st) > 0) {
+                P.pair_list = head;
                 P.tasks.range = cnt + 22;
             }
         }
@@ -1222,7 +1223,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             else
                 launch_wfa_affine(P, static_cast<int>(grid), block, st);
         }
-        P.task_list = nullptr;
+        P.pair_list = nullptr;
         P.tasks.range = range1;
         P.queue_head = cnt + 6;
         if (per_task ? any_bytes : n_groupb > 0) {

@@ -34,7 +34,7 @@ struct ExtendParams {
     const uint64_t* task_off;   // when set: task t uses scratch + task_off[t] ...
     const uint64_t* task_len;   // ... with task_len[t] bytes (redo passes); else per-warp slots
     const uint64_t* task_need;  // estimated scratch need per task (main pass), may be NULL
-    const uint32_t* task_list;  // when set: the launch's tasks are task_list[range], not the range itself
+    const uint32_t* pair_list;  // when set: the launch's tasks are these pairs, 32 lanes each
     int32_t engine;             // phr_engine
     int32_t full_band;          // Myers: store every block (no band)
     int32_t band_base;          // Myers: band half-width base
@@ -309,11 +309,14 @@ void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t 
 // it / without, 20,000 0.23 / 0.14 ms, 60,000 0.38 / 0.37, 90,000 0.52 / 0.55, 150,000
 // 0.79 / 0.91, 1,000,000 4.43 / 5.72.
 constexpr uint32_t kShortAffineMin = 512;
-// Short gap-affine pairs of the launch's tasks (costs aff_tile_open knows) in `blocks_per_sm`
-// CTAs a SM at most; the tasks it leaves go to left[0 .. *n_left). 0 CTAs: no room in
-// `scratch_bytes` of p.scratch, nothing launched.
-int launch_wfa_affine_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int blocks_per_sm, uint32_t* left,
-                            uint32_t* n_left, cudaStream_t st);
+// The same for linear pairs (four a task): with it / without, 20,000 0.10 / 0.17 ms, 100,000
+// 0.25 / 0.36, 1,000,000 2.08 / 3.01; below, the warps of one launch hold every task.
+constexpr uint32_t kShortLinearMin = 16;
+// The launch's linear or (costs aff_tile_open knows) gap-affine pairs, those of few symbols and
+// edits, in `blocks_per_sm` CTAs a SM at most; the pairs it leaves go to left[0 .. *n_left).
+// 0 CTAs: no room in the `scratch_bytes` of p.scratch, nothing launched.
+int launch_wfa_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int blocks_per_sm, uint32_t* left,
+                     uint32_t* n_left, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 // Deferred pairs of both symbol modes' launches, `ctas` (4, 8 or 16) CTAs per pair.

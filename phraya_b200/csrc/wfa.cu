@@ -478,7 +478,7 @@ __device__ __forceinline__ bool pos_ok(int32_t pos, int k, int qn, int tn) {
 }
 
 // CIGAR text and record of a pair whose group leader has walked its runs into `rw`.
-__device__ __forceinline__ void affine_result(const ExtendParams& P, uint32_t pid, bool act, int G, bool trace, bool failed,
+__device__ __forceinline__ void wfa_result(const ExtendParams& P, uint32_t pid, bool act, int G, bool trace, bool failed,
                                               const RunWriter& rw, const uint32_t* runs, uint32_t n_edit, int s_end,
                                               int t_end) {
     const int gl = lane_id() & (G - 1);
@@ -594,7 +594,7 @@ __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int
         if (guard < 0) atomicOr(P.error_flag, 4u);
         rw.flush();
     }
-    affine_result(P, pid, act, G, trace, failed, rw, runs, n_edit, s_end, t_end);
+    wfa_result(P, pid, act, G, trace, failed, rw, runs, n_edit, s_end, t_end);
 }
 
 template <class S>
@@ -1180,9 +1180,9 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
 }
 
 // ===========================================================================
-// Gap-affine WFA, one short pair per warp, wavefronts in registers
+// WFA, one short pair per warp, wavefronts in registers
 // ===========================================================================
-// Every reachable cell of score s lies on a diagonal |k| <= (s - O) / E (a gap of length L
+// Gap-affine: every reachable cell of score s lies on a diagonal |k| <= (s - O) / E (a gap of length L
 // costs O + L E), so 32 R lanes hold whole wavefronts while that bound stays inside them: R
 // is 1 for diagonals -16..15, then 2, 4 and 8. A lane keeps M of the last (O + E) / g steps and
 // I and D of the last one, as in wfa_affine_tile.cu (X / g = 2, E / g = 1): the larger of
@@ -1196,7 +1196,7 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
 // Before, four values crossed lanes per cell, validity was a range test per candidate and
 // wide bands stepped five slots of which some lay outside: 1,000,000 pairs of 100-300 bp at
 // 0-5 %, costs (4, 6, 2), 8.57 -> 5.72 ms (6,213 -> about 3,950 warp instructions a pair),
-// and 4.43 in wfa_affine_short_kernel; 300,000 at 0-10 % 6.88 -> 4.24, at 0-20 %
+// and 4.43 in wfa_short_kernel; 300,000 at 0-10 % 6.88 -> 4.24, at 0-20 %
 // 27.1 -> 17.7, of 300-480 bp 6.62 -> 4.14.
 // With 4 slots at most, pairs whose band passes 128 diagonals are done twice: 7.97 at 0-10 %.
 constexpr int kRegMaxLen = 1024;  // qlen + tlen below which a pair tries the register path
@@ -1341,6 +1341,83 @@ __device__ __forceinline__ bool reg_steps(const PairSeq<S, true>& sq, RegPair& C
     return true;
 }
 
+// Linear scores of a pair while its band stays inside 32 R lanes: a step is a score, the band
+// of score s |k| <= s; candidates [mismatch, I, D], the LAST maximal one wins, and a cell whose
+// winner lies outside the sequences is invalid, as in wfa_linear_group.
+template <class S, int R>
+__device__ __forceinline__ bool lin_steps(const PairSeq<S, true>& sq, RegPair& C, int (&x)[R]) {
+    const int lane = lane_id();
+    const int qn = C.qn, tn = C.tn;
+    const int k0 = lane - 16 * R;
+    const int kend = qn - tn;
+    const int up_src = (lane + 31) & 31, dn_src = (lane + 1) & 31;
+#pragma unroll 1
+    while (C.t < C.max_t) {
+        const int t = C.t + 1;
+        const int blo = -min(t, tn), bhi = min(t, qn);
+        if (blo < -16 * R || bhi > 16 * R - 1 || static_cast<uint64_t>(t) >= C.row_cap) return false;
+        C.cells += static_cast<uint32_t>(bhi - blo + 1);
+        uint32_t more = 0;
+        int nx[R];
+        int prev_up = kNeg;
+        int dn = __shfl_sync(PHR_FULL_MASK, x[0], dn_src);
+        uint32_t* row = C.rows + static_cast<uint64_t>(t) * C.win + C.win / 2;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            constexpr int kLast = R - 1;
+            const int up_rot = __shfl_sync(PHR_FULL_MASK, x[r], up_src);
+            const int dn_next = r < kLast ? __shfl_sync(PHR_FULL_MASK, x[r < kLast ? r + 1 : r], dn_src) : kNeg;
+            const int up = lane == 0 ? prev_up : up_rot;
+            const int down = lane == 31 ? dn_next : dn;
+            prev_up = up_rot;
+            dn = dn_next;
+            const int m = __viaddmax_s32(up, 4 + 2, __viaddmax_s32(x[r], 4 + 1, down + 3));   // raw << 2 | op
+            const int k = k0 + 32 * r;
+            const int pos = m >> 2;
+            const int lim = m >= 0 ? min(qn, tn + k) - pos : -1;
+            const int p = lim >= 0 ? pos : max(k, 0);   // an unset cell reads within the staged padding
+            const int n = min(first_diff<S>(sq.diff(p, p - k)), lim);
+            nx[r] = lim >= 0 ? (m & ~3) + (n << 2) : kNeg;
+            if (n == S::kPerWord) more |= 1u << r;
+            if (t < kRegShRows && static_cast<unsigned>(k + 16) < 32u)
+                C.sh_hist[t * 32 + k + 16] = static_cast<uint32_t>(m);
+            else
+                row[k] = static_cast<uint32_t>(m);
+        }
+        while (more) {   // match runs longer than one word
+            const int r = __ffs(more) - 1;
+            more &= more - 1;
+            int v = nx[0];
+#pragma unroll
+            for (int i = 1; i < R; ++i) v = r == i ? nx[i] : v;
+            const int k = k0 + 32 * r;
+            v = extend_run<S, true>(sq, v >> 2, k, min(qn, tn + k), C.extra) << 2;
+#pragma unroll
+            for (int i = 0; i < R; ++i) nx[i] = r == i ? v : nx[i];
+        }
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            x[r] = nx[r];
+            const int k = k0 + 32 * r;
+            any |= x[r] >= (qn << 2) && (C.fitting ? k >= kend : k == kend);
+        }
+        C.t = t;
+        if (__any_sync(PHR_FULL_MASK, any)) {   // smallest k (largest t_end)
+            int best = INT32_MAX;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int k = k0 + 32 * r;
+                if (x[r] >= (qn << 2) && (C.fitting ? k >= kend : k == kend)) best = min(best, k);
+            }
+            C.end_k = __reduce_min_sync(PHR_FULL_MASK, best);
+            C.end_layer = 0;
+            return true;
+        }
+    }
+    return true;
+}
+
 // A row of 32 A lanes as one of 32 B (both centred on diagonal 0).
 template <int A, int B>
 __device__ __forceinline__ void reg_widen(const int (&x)[A], int (&y)[B]) {
@@ -1376,7 +1453,19 @@ __device__ __forceinline__ bool reg_search(const PairSeq<S, true>& sq, RegPair& 
     }
 }
 
-// Path of a finished pair from its history (lane 0), its text and record.
+template <class S, int R, int RMAX>
+__device__ __forceinline__ bool lin_search(const PairSeq<S, true>& sq, RegPair& C, int (&x)[R]) {
+    if (lin_steps<S, R>(sq, C, x)) return true;
+    if constexpr (R < RMAX) {
+        int y[2 * R];
+        reg_widen<R, 2 * R>(x, y);
+        return lin_search<S, 2 * R, RMAX>(sq, C, y);
+    } else {
+        return false;
+    }
+}
+
+// Path of a finished pair from its history (lane 0), its text and record. OES 0: linear.
 template <int OES>
 __device__ __forceinline__ void reg_finish(const ExtendParams& P, uint32_t pid, const RegPair& C, uint32_t* runs, int g) {
     RunWriter rw;
@@ -1397,6 +1486,19 @@ __device__ __forceinline__ void reg_finish(const ExtendParams& P, uint32_t pid, 
             const uint32_t w = t < kRegShRows && static_cast<unsigned>(k + 16) < 32u
                                    ? C.sh_hist[t * 32 + k + 16]
                                    : C.rows[static_cast<uint64_t>(t) * C.win + C.win / 2 + k];
+            if constexpr (OES == 0) {
+                const int mc = max(qi - static_cast<int>(w >> 2), 0);
+                rw.push(0, static_cast<uint32_t>(mc));
+                qi -= mc;
+                ti -= mc;
+                const uint32_t op = w & 3u;   // 1 mismatch, 2 I (query-extra -> 'D'), 3 D (target-extra -> 'I')
+                rw.push(op == 1 ? 1 : op == 2 ? 3 : 2, 1);
+                if (op != 3) --qi;
+                if (op != 2) --ti;
+                k += op == 2 ? -1 : op == 3 ? 1 : 0;
+                --t;
+                continue;
+            }
             if (layer == 0) {
                 const int mc = max(qi - static_cast<int>(w >> 4), 0);
                 rw.push(0, static_cast<uint32_t>(mc));
@@ -1424,18 +1526,19 @@ __device__ __forceinline__ void reg_finish(const ExtendParams& P, uint32_t pid, 
         if (guard < 0) atomicOr(P.error_flag, 4u);
         rw.flush();
     }
-    affine_result(P, pid, true, 32, trace, !trace, rw, runs, n_edit, C.t * g, C.qn - C.end_k);
+    wfa_result(P, pid, true, 32, trace, !trace, rw, runs, OES == 0 ? static_cast<uint32_t>(C.t) : n_edit, C.t * g,
+                  C.qn - C.end_k);
 }
 
 // Returns true when the pair's band left the window: nothing is written for it and the
 // caller runs it another way.
 template <class S, int RMAX, int OES>
-__device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
+__device__ bool wfa_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
                                uint64_t region_bytes, uint32_t sm_off, unsigned long long* work) {
     const int lane = lane_id();
     const int qn = d.qn, tn = d.tn;
     const int X = P.costs.mismatch, O = P.costs.gap_open, E = P.costs.gap_extend;
-    const int g = E;   // score of a step
+    const int g = OES == 0 ? 0 : E;   // affine score of a step
     const int qw = (qn + 15) / 16, tw = (tn + 15) / 16;
     uint64_t* q2 = reinterpret_cast<uint64_t*>(tile_sm + sm_off + kRegShRows * 128);
     uint64_t* t2 = q2 + qw + kRegSeqPad;
@@ -1453,7 +1556,8 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
     C.qn = qn;
     C.tn = tn;
     C.fitting = tn > qn + qn / 2 + 10;
-    C.max_t = (static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4) / g;
+    C.max_t = qn + tn;
+    if constexpr (OES != 0) C.max_t = (static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4) / E;
     C.rows = reinterpret_cast<uint32_t*>(region + runs_bytes);
     C.win = 32 * RMAX;
     C.row_cap = rest / (C.win * 4);
@@ -1465,11 +1569,16 @@ __device__ bool wfa_affine_reg(const ExtendParams& P, const PairDesc& d, uint32_
     if (lane == 0) C.sh_hist[16] = 0;   // row 0, diagonal 0
     bool inside = C.row_cap >= 2;
     if (inside && C.end_layer < 0) {
-        int M[OES][1], I[1] = {kNeg}, D[1] = {kNeg};
+        if constexpr (OES == 0) {
+            int x[1] = {lane == 16 ? v0 << 2 : kNeg};
+            inside = lin_search<S, 1, RMAX>(sq, C, x);
+        } else {
+            int M[OES][1], I[1] = {kNeg}, D[1] = {kNeg};
 #pragma unroll
-        for (int a = 0; a < OES; ++a) M[a][0] = kNeg;
-        if (lane == 16) M[0][0] = v0 << 2;
-        inside = reg_search<S, 1, RMAX, OES>(sq, C, M, I, D);
+            for (int a = 0; a < OES; ++a) M[a][0] = kNeg;
+            if (lane == 16) M[0][0] = v0 << 2;
+            inside = reg_search<S, 1, RMAX, OES>(sq, C, M, I, D);
+        }
     }
     {
         const unsigned extra = __reduce_add_sync(PHR_FULL_MASK, C.extra);
@@ -1513,16 +1622,16 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
             if (next >= P.tasks.range[1]) break;
             batch_end = min(next + grab, P.tasks.range[1]);
         }
-        const uint32_t task = kAffine && P.task_list ? P.task_list[next] : next;
+        const uint32_t task = next;   // (of one pair and 32 lanes with a pair list)
         uint8_t* slot = P.task_off ? P.scratch + P.task_off[task] : P.scratch + warp_global * P.slot_bytes;
         const uint64_t slot_bytes = P.task_off ? P.task_len[task] : P.slot_bytes;
-        const uint8_t tg = P.tasks.task_group[task];
+        const uint8_t tg = P.pair_list ? 32 : P.tasks.task_group[task];
         if (tg & kOtherKernel) continue;  // a redo task of another kernel
         const int G = tg;
-        const int count = P.tasks.task_count[task];
+        const int count = P.pair_list ? 1 : P.tasks.task_count[task];
         const int grp = lane / G;
         bool act = grp < count;
-        const uint32_t pid = act ? P.tasks.order[P.tasks.task_first[task] + grp] : 0;
+        const uint32_t pid = P.pair_list ? P.pair_list[task] : act ? P.tasks.order[P.tasks.task_first[task] + grp] : 0;
         PairDesc d = {};
         if (act) d = P.desc[pid];
         // pairs of the other symbol mode run in the other instantiation
@@ -1539,7 +1648,7 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
         const uint64_t region_bytes = (P.task_off ? slot_bytes : slot_bytes / (32 / G)) & ~15ull;
         uint8_t* region = slot + static_cast<uint64_t>(grp) * region_bytes;
         // a task whose estimated need exceeds the slot goes straight to a redo pass
-        if (!P.task_off && P.task_need && P.task_need[task] > slot_bytes) {
+        if (!P.task_off && !P.pair_list && P.task_need && P.task_need[task] > slot_bytes) {
             if (act && (lane & (G - 1)) == 0) report_redo(P, pid, P.task_need[task] / (32 / G));
             continue;
         }
@@ -1550,8 +1659,8 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
                 const uint32_t sm_off = (threadIdx.x >> 5) * static_cast<uint32_t>(kAffWarpSmem);
                 const int open = aff_tile_open(P.costs);
                 bool wide = true;  // the band left the register window (or no specialisation)
-                if (open == 4) wide = wfa_affine_reg<S, kRegSlots, 4>(P, d, pid, region, region_bytes, sm_off, work);
-                else if (open == 5) wide = wfa_affine_reg<S, kRegSlots, 5>(P, d, pid, region, region_bytes, sm_off, work);
+                if (open == 4) wide = wfa_reg<S, kRegSlots, 4>(P, d, pid, region, region_bytes, sm_off, work);
+                else if (open == 5) wide = wfa_reg<S, kRegSlots, 5>(P, d, pid, region, region_bytes, sm_off, work);
                 if (!wide) continue;
                 // otherwise the group kernel below takes the pair in place (no redo pass)
             }
@@ -1577,14 +1686,20 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
 
 // Bytes of a warp's region in the kernel below: runs and rows of its widest band's steps.
 constexpr uint64_t kShortSlot = ((kRegMaxLen + 2) * 4 + 15) / 16 * 16 + (16 * kRegFewSlots + 16) * (32 * kRegFewSlots * 4);
+__host__ __device__ constexpr int short_blocks(int oes) { return oes == 0 ? 4 : 3; }
 
 // The register path alone, for batches that fill the chip: without the group path's registers
 // and code three CTAs fit an SM where wfa_kernel has two, which the stalls on the steps' own
-// dependences need (general kernel: an instruction in 52 % of the cycles). A task whose pair
-// is too long or too wide goes to wfa_kernel by `left`. 1,000,000 pairs of 100-300 bp at
-// 0-5 %: 5.72 -> 4.43 ms; four CTAs, with spills, 4.54.
+// dependences need (general kernel: an instruction in 52 % of the cycles). A pair that is too
+// long or too wide goes to wfa_kernel by `left`. 1,000,000 pairs of 100-300 bp at 0-5 %:
+// gap-affine 5.72 -> 4.45 ms; four CTAs, with spills, 4.54.
+// OES 0: linear pairs, whose tasks hold several pairs; the warp takes one after the other.
+// wfa_linear_group's lanes waited for the longest of four pairs and kept frames in global
+// memory (12 of 32 lanes busy): 3.01 -> 2.08 ms; 300,000 at 0-10 % 2.06 -> 1.28, of
+// 300-480 bp 2.19 -> 1.35, of 20-60 bp 0.30 -> 0.28.
 template <int OES>
-__global__ void __launch_bounds__(256, 3) wfa_affine_short_kernel(ExtendParams P, uint32_t* left, uint32_t* n_left) {
+__global__ void __launch_bounds__(256, short_blocks(OES)) wfa_short_kernel(ExtendParams P, uint32_t* left, uint32_t* n_left) {
+    constexpr uint32_t kGrab = OES == 0 ? 1 : kTaskGrab;
     __shared__ unsigned long long sh_work[8][2];
     const int lane = lane_id();
     unsigned long long* work = sh_work[threadIdx.x >> 5];
@@ -1595,30 +1710,34 @@ __global__ void __launch_bounds__(256, 3) wfa_affine_short_kernel(ExtendParams P
     const uint32_t end = P.tasks.range[1];
     for (;;) {
         uint32_t base = 0;
-        if (lane == 0) base = P.tasks.range[0] + atomicAdd(P.queue_head, kTaskGrab);
+        if (lane == 0) base = P.tasks.range[0] + atomicAdd(P.queue_head, kGrab);
         base = __shfl_sync(PHR_FULL_MASK, base, 0);
         if (base >= end) break;
-        const uint32_t n = min(kTaskGrab, end - base);
-        // the batch's pairs, a lane each
-        uint32_t pid_l = 0;
-        bool ok_l = false;
-        PairDesc d_l = {};
-        if (static_cast<uint32_t>(lane) < n && P.tasks.task_group[base + lane] == 32) {
-            pid_l = P.tasks.order[P.tasks.task_first[base + lane]];
-            d_l = P.desc[pid_l];
-            ok_l = d_l.mode == 0 && d_l.qn + d_l.tn < kRegMaxLen &&
-                   !big_pair(P.engine, P.big_min, P.big_smem, d_l.qn, d_l.tn, d_l.mode);
-        }
-        for (uint32_t i = 0; i < n; ++i) {
-            PairDesc d = {};
-            d.qn = __shfl_sync(PHR_FULL_MASK, d_l.qn, i);
-            d.tn = __shfl_sync(PHR_FULL_MASK, d_l.tn, i);
-            d.q_word = __shfl_sync(PHR_FULL_MASK, d_l.q_word, i);
-            d.t_word = __shfl_sync(PHR_FULL_MASK, d_l.t_word, i);
-            const uint32_t pid = __shfl_sync(PHR_FULL_MASK, pid_l, i);
-            bool wide = __shfl_sync(PHR_FULL_MASK, ok_l ? 0 : 1, i) != 0;
-            if (!wide) wide = wfa_affine_reg<Seq2, kRegFewSlots, OES>(P, d, pid, region, kShortSlot, sm_off, work);
-            if (wide && lane == 0) left[atomicAdd(n_left, 1u)] = base + i;
+        // the pairs of the tasks taken (consecutive in `order`), a lane each
+        uint32_t first = P.tasks.task_first[base];
+        const uint32_t last = min(base + kGrab, end) - 1;
+        const uint32_t stop = P.tasks.task_first[last] + P.tasks.task_count[last];
+        for (; first < stop; first += 32) {
+            const uint32_t n = min(stop - first, 32u);
+            uint32_t pid_l = 0;
+            bool ok_l = false;
+            PairDesc d_l = {};
+            if (static_cast<uint32_t>(lane) < n) {
+                pid_l = P.tasks.order[first + lane];
+                d_l = P.desc[pid_l];
+                ok_l = d_l.mode == 0 && d_l.qn + d_l.tn < kRegMaxLen;
+            }
+            for (uint32_t i = 0; i < n; ++i) {
+                PairDesc d = {};
+                d.qn = __shfl_sync(PHR_FULL_MASK, d_l.qn, i);
+                d.tn = __shfl_sync(PHR_FULL_MASK, d_l.tn, i);
+                d.q_word = __shfl_sync(PHR_FULL_MASK, d_l.q_word, i);
+                d.t_word = __shfl_sync(PHR_FULL_MASK, d_l.t_word, i);
+                const uint32_t pid = __shfl_sync(PHR_FULL_MASK, pid_l, i);
+                bool wide = __shfl_sync(PHR_FULL_MASK, ok_l ? 0 : 1, i) != 0;
+                if (!wide) wide = wfa_reg<Seq2, kRegFewSlots, OES>(P, d, pid, region, kShortSlot, sm_off, work);
+                if (wide && lane == 0) left[atomicAdd(n_left, 1u)] = pid;
+            }
         }
     }
     if (lane == 0 && P.work) {
@@ -1647,13 +1766,14 @@ void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mod
     }
 }
 
-int launch_wfa_affine_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int blocks_per_sm, uint32_t* left,
-                            uint32_t* n_left, cudaStream_t st) {
+int launch_wfa_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int blocks_per_sm, uint32_t* left,
+                     uint32_t* n_left, cudaStream_t st) {
     const int smem = 8 * kRegWarpSmem;
+    const int oes = p.engine == PHR_ENGINE_WFA_LINEAR ? 0 : aff_tile_open(p.costs);
     const uint64_t fit = scratch_bytes / (8 * kShortSlot);
-    const int grid = static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(sms) * std::min(blocks_per_sm, 3), fit));
+    const int grid = static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(sms) * std::min(blocks_per_sm, short_blocks(oes)), fit));
     if (grid == 0) return 0;
-    auto* kernel = aff_tile_open(p.costs) == 4 ? wfa_affine_short_kernel<4> : wfa_affine_short_kernel<5>;
+    auto* kernel = oes == 0 ? wfa_short_kernel<0> : oes == 4 ? wfa_short_kernel<4> : wfa_short_kernel<5>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     kernel<<<grid, 256, smem, st>>>(p, left, n_left);
     return grid;

@@ -1,4 +1,4 @@
-"""Short gap-affine pairs, wavefronts in one warp's registers, against the oracle where the
+"""Short gap-affine and linear pairs, wavefronts in one warp's registers, against the oracle where the
 path can go wrong: bands that end at, cross and leave 32, 64 and 128 diagonals, both end
 rules, gaps at either sequence's end, matches longer than a word, lengths around words."""
 import numpy as np
@@ -44,18 +44,22 @@ def pairs_of(rng):
     return pairs
 
 
-@pytest.mark.parametrize("costs", [(2, 4, 1), (4, 6, 2), (6, 12, 3), (4, 8, 2), (1, 3, 1)])
+ENGINES = [(A.ENGINE_WFA_AFFINE, c) for c in ((2, 4, 1), (4, 6, 2), (6, 12, 3), (4, 8, 2), (1, 3, 1))]
+
+
+@pytest.mark.parametrize("engine,costs", ENGINES + [(A.ENGINE_WFA_LINEAR, (2, 4, 1))])
 @pytest.mark.parametrize("copies", [1, 40, 540])
-def test_short_affine(costs, copies):
+def test_short(engine, costs, copies):
     """Batches of a few hundred pairs, of more than the small-batch limit, and of enough for
     the kernel for short pairs alone, which leaves the wide ones to the general one."""
     rng = np.random.default_rng(71)
     packed = O.PackedPairs(pairs_of(rng) * copies)
-    oa, oc = O.extend_packed(A.ENGINE_WFA_AFFINE, O.PackedPairs(pairs_of(np.random.default_rng(71))), costs)
+    oa, oc = O.extend_packed(engine, O.PackedPairs(pairs_of(np.random.default_rng(71))), costs)
     want = P.unpack(oa, oc) * copies
     with P.Engine(0) as eng:
-        ga, gc = eng.extend_packed(A.ENGINE_WFA_AFFINE, packed, P.AffineCosts(*costs))
+        ga, gc = eng.extend_packed(engine, packed, P.AffineCosts(*costs))
     got = P.unpack(ga, gc)
     bad = [i for i in range(packed.n) if got[i] != want[i]]
     assert not bad, (len(bad), got[bad[0]], want[bad[0]])
-    assert np.array_equal(ga["affine_score"], np.tile(oa["affine_score"], copies))
+    if engine == A.ENGINE_WFA_AFFINE:
+        assert np.array_equal(ga["affine_score"], np.tile(oa["affine_score"], copies))
