@@ -54,8 +54,8 @@ constexpr uint8_t kBigTask = 0x80;
 constexpr uint8_t kCtaTileTask = 0xC0;
 constexpr uint8_t kWarpTileTask = 0x40;
 constexpr uint8_t kOtherKernel = 0xC0;   // mask of the three
-constexpr int kBigThreads = 512;         // threads of the linear CTA-per-pair kernel (two CTAs per SM)
-// most threads per CTA of the gap-affine CTA-per-pair kernel, and its default (one CTA
+constexpr int kBigThreads = 512;         // threads of a register-tile CTA (one CTA per SM)
+// most threads per CTA of wfa.cu's gap-affine CTA-per-pair kernel, and its default (one CTA
 // per SM; the "wfa_affine_big_threads" setting launches 512 or 256, two or four per SM)
 constexpr int kBigAffineThreads = 1024;
 constexpr uint32_t kBigMinFrameCells = 4096;  // smallest shared frame pair worth staging
@@ -224,7 +224,8 @@ struct TileHead {
 };
 constexpr uint64_t kTileHeadBytes = 256;
 
-__host__ __device__ __forceinline__ uint64_t tile_align(uint64_t v) { return (v + 255) & ~255ull; }
+constexpr uint64_t kRecordAlign = 256;
+__host__ __device__ __forceinline__ uint64_t tile_align(uint64_t v) { return (v + kRecordAlign - 1) & ~(kRecordAlign - 1); }
 __host__ __device__ __forceinline__ uint64_t tile_runs_bytes(int qn, int tn) {
     return tile_align(4 * (static_cast<uint64_t>(qn) + tn + 2));
 }
@@ -240,7 +241,7 @@ __host__ __device__ __forceinline__ uint64_t tile_fixed_bytes(int qn, int tn) {
 // small bands.
 __host__ __device__ __forceinline__ uint64_t tile_hist_bytes(int64_t s) {
     const uint64_t u = static_cast<uint64_t>(s) / kTileSteps + 1;
-    return u * 3200 + 54 * u * (u + 1);
+    return u * 3328 + 54 * u * (u + 1);
 }
 // The gap-affine tiles' counterparts. Steps are scores over g = gcd of the costs; an edit
 // costs at least one, a mismatch two.
@@ -256,7 +257,7 @@ __host__ __device__ __forceinline__ uint64_t aff_tile_fixed_bytes(int qn, int tn
 // Block u: up to 16 (u + 1) diagonals at 28 bytes of values and at most 8 of ops.
 __host__ __device__ __forceinline__ uint64_t aff_tile_hist_bytes(int64_t steps) {
     const uint64_t u = static_cast<uint64_t>(steps) / kTileSteps + 1;
-    return u * 8192 + 288 * u * (u + 1);
+    return u * 8320 + 288 * u * (u + 1);
 }
 // Costs the gap-affine tiles are specialised for, as (O + E) / g; 0: none. (2, 4, 1) gives 5,
 // (4, 6, 2) gives 4.

@@ -227,22 +227,23 @@ __device__ __forceinline__ TileMin* team_min(TileCtl* sh, uint8_t* region, uint6
         return reinterpret_cast<TileMin*>(region + fixed - kTileHeadBytes / 2);
 }
 
-// Record block u of a pair: where it starts, in units of 128 bytes of P.scratch, and log2 of
-// its tiles' diagonals per lane.
+// Record block u of a pair: where it starts, in units of kRecordAlign bytes of P.scratch (30
+// bits: any offset in a GPU's memory), and log2 of its tiles' diagonals per lane (1..8).
 __device__ __forceinline__ uint32_t table_entry(uint64_t base, int R) {
-    return static_cast<uint32_t>(base / 128) << 3 | static_cast<uint32_t>(31 - __clz(R));
+    return static_cast<uint32_t>(base / kRecordAlign) << 2 | static_cast<uint32_t>(31 - __clz(R));
 }
-__device__ __forceinline__ uint64_t entry_base(uint32_t e) { return static_cast<uint64_t>(e >> 3) * 128; }
-__device__ __forceinline__ int entry_regs(uint32_t e) { return 1 << (e & 7u); }
+__device__ __forceinline__ uint64_t entry_base(uint32_t e) { return static_cast<uint64_t>(e >> 2) * kRecordAlign; }
+__device__ __forceinline__ int entry_regs(uint32_t e) { return 1 << (e & 3u); }
 
 // Record space for `bytes`, kNoBase when there is none (one thread of the team). New chunks
 // double from A.chunk up to 256 times that.
 __device__ __forceinline__ unsigned long long grab_records(const TileLaunch& A, TileCtl* sh, uint64_t bytes) {
+    bytes = tile_align(bytes);   // table_entry's unit
     while (sh->cursor + bytes > sh->chunk_end) {
         const int i = sh->cur_chunk + 1;
         if (!A.pool_used || i >= kMaxChunks) return kNoBase;
         if (i >= sh->n_chunks) {
-            const uint64_t size = max(static_cast<uint64_t>(A.chunk) << min(i, 8), tile_align(bytes));
+            const uint64_t size = max(static_cast<uint64_t>(A.chunk) << min(i, 8), bytes);
             const uint64_t o = atomicAdd(A.pool_used, static_cast<unsigned long long>(size));
             if (o + size > A.pool_end) return kNoBase;
             sh->chunk[i] = o;
