@@ -96,7 +96,9 @@ __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>&
             to_up[r] = c;
             a = M[OES - 1][r] + (2 << 8) - 1, e = D[r] - 1;
             c = max(a, e);
-            const int t_last = ((tn + k0 + 32 * r - 1) << 10) | 1023;   // no offset beyond the target's end
+            // no offset beyond the target's end; none is beyond the query's, which keeps the
+            // bound within a value word whatever the target's length
+            const int t_last = (__viaddmin_s32(tn + k0, 32 * r - 1, qn) << 10) | 1023;
             if (c > t_last) {
                 if (a > t_last) a = kUnset;
                 if (e > t_last) e = kUnset;
