@@ -401,8 +401,8 @@ struct TaskBuild {
     unsigned long long* need_max;
     uint64_t* task_need;          // per task
     unsigned int* need_hist;      // 64 buckets by bit length of the need
-    int32_t big_min;              // linear WFA pairs for the CTA-per-pair kernel (not in the
-    uint32_t big_smem;            // main pass, so not in its slot statistics)
+    int32_t big_min;              // WFA pairs for wfa.cu's CTA-per-pair kernels (not in the main
+                                  // pass, so not in its slot statistics)
     int32_t lane_ckpt;            // lane kernel mode (its scratch need)
     uint32_t* tile_min;           // [4] first one-warp register-tile task of each symbol mode, first CTA one
     uint32_t* tile_ranges;        // {begin, end} of each of the four
@@ -472,7 +472,7 @@ __device__ __forceinline__ void task_fill(const TaskBuild& T, uint64_t p) {
                                 ? aff_tile_fixed_bytes(d.qn, d.tn) +
                                       tile_align(aff_tile_hist_bytes(tile_score_est(d.qn, d.mode)))
                                 : tile_fixed_bytes(d.qn, d.tn) + tile_align(tile_hist_bytes(tile_score_est(d.qn, d.mode)));
-            else if (!big_pair(T.engine, T.big_min, T.big_smem, d.qn, d.tn, d.mode))
+            else if (!big_pair(T.engine, T.big_min, d.qn, d.tn))
                 region = max(region, wfa_region_est(d.qn, d.tn, T.engine == PHR_ENGINE_WFA_AFFINE));
             ++cnt;
         }
@@ -686,8 +686,8 @@ __global__ void __launch_bounds__(kSmallPairs) small_tasks_kernel(SmallBuild B) 
 // Redo pass task list: one pair per task, in redo order.
 __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* redo_count, const PairDesc* desc,
                                   int32_t engine, int aff_open, int wfa_g_short, int wfa_g_long, int wfa_long_min, int32_t big_min,
-                                  uint32_t big_smem, uint32_t* task_first, uint8_t* task_count,
-                                  uint8_t* task_group, uint32_t* ranges) {
+                                  uint32_t* task_first, uint8_t* task_count, uint8_t* task_group,
+                                  uint32_t* ranges) {
     const uint32_t n = *redo_count;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) {
@@ -707,7 +707,7 @@ __global__ void redo_tasks_kernel(const uint32_t* redo_list, const uint32_t* red
     const int tw = tile_warps(engine, aff_open, big_min, wfa_long_min, d.qn, d.tn, d.mode);
     if (tw > 1) task_group[t] = kCtaTileTask | 32;
     else if (tw == 1) task_group[t] = kWarpTileTask | 32;
-    else if (big_pair(engine, big_min, big_smem, d.qn, d.tn, d.mode)) task_group[t] = kBigTask | 32;
+    else if (big_pair(engine, big_min, d.qn, d.tn)) task_group[t] = kBigTask | 32;
 }
 
 struct FinishParams {
@@ -1003,8 +1003,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                         ctx->tune.myers_band_base, ctx->tune.wfa_big_min, ctx->tune.myers_lane_ckpt};
     TaskBuild tbp{keys_s, order, n, small ? head_s : head, flag, tidx, task_first, task_count, task_group, cnt, cnt + 4,
                   cnt + 20, desc, engine, ctx->tune.myers_band_base, need_max, task_need, need_hist,
-                  ctx->tune.wfa_big_min, static_cast<uint32_t>(ctx->tune.wfa_big_smem), ctx->tune.myers_lane_ckpt,
-                  cnt + 40, cnt + 44, reinterpret_cast<unsigned long long*>(cnt + 52)};
+                  ctx->tune.wfa_big_min, ctx->tune.myers_lane_ckpt, cnt + 40, cnt + 44, reinterpret_cast<unsigned long long*>(cnt + 52)};
     size_t t_need = 0, tn_ = 0;
     void* tmp = nullptr;
     if (small) {
@@ -1270,19 +1269,28 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                     (cta ? launch_wfa_linear_big : launch_wfa_linear_tile)(P, tl, tile_grid, i & 1, st);
             }
         }
-        if (per_task && engine == PHR_ENGINE_WFA_AFFINE && P.big_min > 0 && n_tasks_hint > 0) {
-            // long gap-affine pairs the register tiles do not take, one CTA each:
-            // kBigAffineThreads / wfa_affine_big_threads CTAs per SM
+        // (no linear pair is beyond the tiles in a batch of fewer symbols than their limit)
+        const bool aff = engine == PHR_ENGINE_WFA_AFFINE;
+        if (per_task && (aff || (engine == PHR_ENGINE_WFA_LINEAR && sum_qt >= static_cast<uint64_t>(kTileMaxQuery))) &&
+            P.big_min > 0 && n_tasks_hint > 0) {
+            // long pairs the register tiles do not take, one CTA each. Gap-affine:
+            // kBigAffineThreads / wfa_affine_big_threads CTAs per SM; linear: two (one when the
+            // tune keeps fewer blocks resident)
             const int aff_threads = ctx->tune.wfa_affine_big_threads;
-            const int big_grid = static_cast<int>(std::min<uint64_t>(
-                n_tasks_hint, ctx->sm_count * static_cast<uint64_t>(kBigAffineThreads / aff_threads)));
+            const uint64_t per_sm = aff ? kBigAffineThreads / aff_threads : ctx->tune.max_blocks_per_sm >= 4 ? 2 : 1;
+            const int big_grid = static_cast<int>(std::min<uint64_t>(n_tasks_hint, ctx->sm_count * per_sm));
             PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 24, 0, 8, st));
             for (int mode = 0; mode < 2; ++mode) {
                 if (!(mode ? any_bytes : any_2bit)) continue;
                 P.tasks.range = mode ? range1 : range0;
                 P.queue_head = cnt + 24 + mode;
-                KernelScope ks(ctx, mode ? "wfa_affine_big_bytes" : "wfa_affine_big");
-                launch_wfa_affine_big(P, big_grid, aff_threads, mode, st);
+                if (aff) {
+                    KernelScope ks(ctx, mode ? "wfa_affine_big_bytes" : "wfa_affine_big");
+                    launch_wfa_affine_big(P, big_grid, aff_threads, mode, st);
+                } else {
+                    KernelScope ks(ctx, mode ? "wfa_linear_long_bytes" : "wfa_linear_long");
+                    launch_wfa_linear_long(P, big_grid, mode, st);
+                }
             }
         }
         PHR_CUDA_TRY(ctx, cudaGetLastError());
@@ -1430,8 +1438,8 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 redo_tasks_kernel<<<blocks_for(m, T), T, 0, st>>>(rlist2, cnt + 18, desc, engine,
                                                                  aff_tile_open(costs), g_short, ctx->tune.wfa_group_long,
                                                                  ctx->tune.wfa_long_min,
-                                                                 P.big_min, P.big_smem, task_first, task_count,
-                                                                 task_group, cnt + 14);
+                                                                 P.big_min, task_first, task_count, task_group,
+                                                                 cnt + 14);
             }
             // byte-mode and 2-bit pairs share this list: both launches walk all of it
             PHR_CUDA_TRY(ctx, cudaMemcpyAsync(cnt + 16, cnt + 14, 8, cudaMemcpyDeviceToDevice, st));

@@ -70,17 +70,14 @@ __host__ __device__ __forceinline__ uint64_t big_seq_words(int qn, int tn, int m
     return static_cast<uint64_t>((qn + per - 1) / per) + static_cast<uint64_t>((tn + per - 1) / per) + 16;
 }
 
-// A gap-affine WFA pair long enough that one warp would be latency-bound on it: it runs
-// one per CTA of wfa.cu's kernel unless the register tiles take it (tile_warps below).
-__host__ __device__ __forceinline__ bool big_pair(int32_t engine, int32_t big_min, uint32_t big_smem, int qn, int tn,
-                                                  int mode) {
-    (void)big_smem;
-    (void)mode;
-    return big_min > 0 && engine == PHR_ENGINE_WFA_AFFINE && qn + tn >= big_min;
+// A WFA pair long enough that one warp would be latency-bound on it: unless the register
+// tiles take it (tile_warps below), it runs one per CTA of wfa.cu's kernels, in a redo pass.
+__host__ __device__ __forceinline__ bool big_pair(int32_t engine, int32_t big_min, int qn, int tn) {
+    return big_min > 0 && (engine == PHR_ENGINE_WFA_LINEAR || engine == PHR_ENGINE_WFA_AFFINE) && qn + tn >= big_min;
 }
 
-// Whether the CTA kernel stages a big pair's sequences in its shared memory (with room
-// left for the linear kernel's first frames); longer ones are read from global memory.
+// Whether the gap-affine CTA kernel stages a big pair's sequences in its shared memory;
+// longer ones are read from global memory.
 __host__ __device__ __forceinline__ bool big_staged(uint32_t big_smem, int qn, int tn, int mode) {
     return (big_seq_words(qn, tn, mode) + 2ull * kBigMinFrameCells) * 4 <= big_smem;
 }
@@ -284,14 +281,16 @@ constexpr uint32_t kWarpTileSmem = 12 << 10;    // shared memory of a one-warp t
 // the warp-group kernel's frames in global memory cost more than a warp per pair: 5,000
 // protein pairs of 200-800 at 30 % measured 1.9 + 1.6 ms (two passes) before and 0.78 ms
 // now (linear). `open` is aff_tile_open for gap-affine pairs. Offsets are kept times 256
-// (linear) or 1024 in 32 bits, hence the upper limits; longer queries stay where they were.
+// (linear) or 1024 in 32 bits, hence the upper limits; longer pairs run one per CTA of
+// wfa.cu's kernels (big_pair).
 constexpr int kWarpTileBytesMin = 128;
+constexpr int kTileMaxQuery = 1 << 22;   // a linear pair's query is shorter, its target below 2^27
 __host__ __device__ __forceinline__ int tile_warps(int32_t engine, int open, int32_t big_min, int32_t long_min, int qn,
                                                    int tn, int mode) {
     const int64_t len = static_cast<int64_t>(qn) + tn;
     if (big_min <= 0 || tn >= (1 << 27)) return 0;
     if (engine == PHR_ENGINE_WFA_LINEAR) {
-        if (qn >= (1 << 22)) return 0;
+        if (qn >= kTileMaxQuery) return 0;
     } else if (engine != PHR_ENGINE_WFA_AFFINE || open == 0 || qn >= (1 << 20)) {
         return 0;
     }
@@ -326,6 +325,7 @@ void launch_wfa_affine_resume(const ExtendParams& p, const TileLaunch& a, int pa
 void launch_wfa_affine_cta_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_warp_tiles(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
 void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+void launch_wfa_linear_long(const ExtendParams& p, int grid, int mode, cudaStream_t st);
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st);
 
 }  // namespace phr

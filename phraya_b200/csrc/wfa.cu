@@ -113,6 +113,47 @@ __device__ __forceinline__ uint64_t lin_base(int64_t s, int64_t qn, int64_t tn) 
     return static_cast<uint64_t>(s) + tri_min(s, qn) + tri_min(s, tn);
 }
 
+// Traceback (wfa_simd.rs:959-1041) from (qn, t_end) over the history words raw << 2 | op of
+// every score's band, into reverse-order runs. One thread.
+__device__ __forceinline__ void lin_trace(RunWriter& rw, const uint32_t* hr, int qn, int tn, int t_end, int s_end) {
+    int qi = qn, ti = t_end, k = qi - ti, ss = s_end;
+    while (qi > 0 || ti > 0) {
+        if (ss < 0) break;
+        if (ss == 0) {
+            const int mm = min(qi, ti);
+            rw.push(0, static_cast<uint32_t>(mm));
+            qi -= mm;
+            ti -= mm;
+            break;
+        }
+        const int lo = -min(ss, tn);
+        const uint32_t aux = hr[lin_base(ss, qn, tn) + (k - lo)];
+        const uint32_t op = aux & 3;
+        const int32_t edit_start = static_cast<int32_t>(aux >> 2);
+        const int mc = qi - edit_start;
+        if (mc > 0) {
+            rw.push(0, static_cast<uint32_t>(mc));
+            qi -= mc;
+            ti -= mc;
+        }
+        if (op == 1) {
+            rw.push(1, 1);
+            --qi;
+            --ti;
+        } else if (op == 2) {
+            rw.push(3, 1);  // 'D': query advances
+            --qi;
+            k -= 1;
+        } else if (op == 3) {
+            rw.push(2, 1);  // 'I': target advances
+            --ti;
+            k += 1;
+        }
+        --ss;
+    }
+    rw.flush();
+}
+
 template <class S>
 __device__ void wfa_linear_group(const ExtendParams& P, const PairDesc& d, uint32_t pid, bool act, int G,
                                  uint8_t* region, uint64_t region_bytes) {
@@ -278,52 +319,11 @@ __device__ void wfa_linear_group(const ExtendParams& P, const PairDesc& d, uint3
         report_redo(P, pid, need);
     }
 
-    // ---- traceback (wfa_simd.rs:959-1041), one walk per group ----
+    // ---- traceback, one walk per group ----
     RunWriter rw;
     rw.init(runs, static_cast<uint32_t>(qn + tn + 2));
     const bool trace = act && done;
-    uint32_t n_x = 0, n_gap = 0;
-    if (trace && gl == 0) {
-        int qi = qn, ti = t_end, k = qi - ti, ss = s_end;
-        while (qi > 0 || ti > 0) {
-            if (ss < 0) break;
-            if (ss == 0) {
-                const int mm = min(qi, ti);
-                rw.push(0, static_cast<uint32_t>(mm));
-                qi -= mm;
-                ti -= mm;
-                break;
-            }
-            const int lo = -min(ss, tn);
-            const uint32_t aux = hr[lin_base(ss, qn, tn) + (k - lo)];
-            const uint32_t op = aux & 3;
-            const int32_t edit_start = static_cast<int32_t>(aux >> 2);
-            const int mc = qi - edit_start;
-            if (mc > 0) {
-                rw.push(0, static_cast<uint32_t>(mc));
-                qi -= mc;
-                ti -= mc;
-            }
-            if (op == 1) {
-                rw.push(1, 1);
-                --qi;
-                --ti;
-                ++n_x;
-            } else if (op == 2) {
-                rw.push(3, 1);  // 'D': query advances
-                --qi;
-                ++n_gap;
-                k -= 1;
-            } else if (op == 3) {
-                rw.push(2, 1);  // 'I': target advances
-                --ti;
-                ++n_gap;
-                k += 1;
-            }
-            --ss;
-        }
-        rw.flush();
-    }
+    if (trace && gl == 0) lin_trace(rw, hr, qn, tn, t_end, s_end);
     const uint32_t nr = __shfl_sync(PHR_FULL_MASK, rw.n, lane_id() & ~(G - 1));
     const bool ovf = __shfl_sync(PHR_FULL_MASK, rw.overflow ? 1 : 0, lane_id() & ~(G - 1)) != 0;
     __syncwarp();
@@ -1180,6 +1180,179 @@ __global__ void __launch_bounds__(kBigAffineThreads, 1) wfa_affine_big_kernel(Ex
 }
 
 // ===========================================================================
+// Linear WFA, one CTA per pair (pairs beyond the register tiles' offsets)
+// ===========================================================================
+// Queries of 2^22 symbols and targets of 2^27 do not fit the value words of wfa_tile.cu. Such
+// a pair is latency-bound on one warp (every cell is a chain of dependent loads), so
+// kBigThreads threads share its diagonals. The sequences are read in place; the two value
+// frames live in shared memory while they fit, then in the region's global frames, the
+// layout of wfa_linear_group, so scratch needs and the redo rule are identical.
+// What bounds it is the match runs, a thread's word compares one after the other: 4.2 Mb
+// pairs of 4, 200 and 2,000 mismatches 23.7, 25.0 and 31.7 ms (with the sequences' staging
+// code in the same kernel, which pairs of this size never took, 23.3, 24.3 and 31.5).
+template <class S>
+__device__ void wfa_linear_cta(const ExtendParams& P, const PairDesc& d, uint32_t pid, uint8_t* region,
+                               uint64_t region_bytes, int32_t* sfr, uint32_t fcap, int* sh_end) {
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int qn = d.qn, tn = d.tn;
+    const bool fitting = tn > qn + qn / 2 + 10;
+    const uint32_t* sq = seq_base<S>(P, d.q_word);
+    const uint32_t* st = seq_base<S>(P, d.t_word);
+
+    // ---- region layout, as in wfa_linear_group ----
+    uint32_t* runs = reinterpret_cast<uint32_t*>(region);
+    const uint64_t runs_bytes = align16(static_cast<uint64_t>(qn + tn + 2) * 4);
+    const uint64_t frame_bytes = align16(static_cast<uint64_t>(qn + tn + 1) * 4);
+    const uint64_t fixed = runs_bytes + 2 * frame_bytes;
+    const uint64_t cell_cap = region_bytes > fixed ? (region_bytes - fixed) / 4 : 0;
+    int32_t* gfr = reinterpret_cast<int32_t*>(region + runs_bytes);
+    uint32_t* hr = reinterpret_cast<uint32_t*>(region + fixed);
+    bool global_frames = false;
+    auto frame = [&](int sc) -> int32_t* {
+        return global_frames ? gfr + (sc & 1) * (frame_bytes / 4) : sfr + (sc & 1) * fcap;
+    };
+
+    if (tid < 3) sh_end[tid] = INT32_MAX;
+    const int max_s = qn + tn;
+    bool done = false, overflow = lin_base(1, qn, tn) > cell_cap;
+    uint64_t wf_cells = 0;   // band diagonals of the scores computed
+    uint32_t lcp_words = 0;  // this thread's word compares of match extension
+    int s_end = 0, t_end = 0, s = 1;
+    __syncthreads();
+    if (!overflow) {
+        if (tid == 0) {
+            frame(0)[0] = extend_valid<S>(sq, qn, st, tn, 0, 0, lcp_words);
+            hr[0] = 0;
+        }
+        __syncthreads();
+        const int32_t v0 = frame(0)[0];
+        if (!fitting) {
+            if (qn - tn == 0 && v0 == qn) {  // wfa_simd.rs:277-283
+                done = true;
+                t_end = tn;
+            }
+        } else if (qn <= tn && v0 >= qn) {
+            done = true;
+            t_end = qn;
+        }
+        for (; !done && s <= max_s; ++s) {
+            const int lo = -min(s, tn), hi = min(s, qn);
+            const int plo = -min(s - 1, tn), phi = min(s - 1, qn);
+            const uint64_t base = lin_base(s, qn, tn);
+            const int width = hi - lo + 1;
+            if (base + static_cast<uint64_t>(width) > cell_cap) {
+                overflow = true;
+                break;
+            }
+            wf_cells += static_cast<uint64_t>(width);
+            if (!global_frames && static_cast<uint32_t>(width) > fcap) {
+                // frames outgrow shared memory: continue on the region's global frames
+                const int32_t* src = frame(s - 1);
+                int32_t* dst = gfr + ((s - 1) & 1) * (frame_bytes / 4);
+                for (int i = tid; i < phi - plo + 1; i += nthr) dst[i] = src[i];
+                global_frames = true;
+                __syncthreads();
+            }
+            const int32_t* pv_frame = frame(s - 1);
+            int32_t* cur_frame = frame(s);
+            if (tid == 0) sh_end[(s + 1) % 3] = INT32_MAX;
+            int my_end = INT32_MAX;
+            for (int k = lo + tid; k <= hi; k += nthr) {
+                // candidates in order [mismatch, ins, del]; the LAST maximal one wins
+                auto prev = [&](int pk) { return pk >= plo && pk <= phi ? pv_frame[pk - plo] : UNSET; };
+                const int32_t mis = prev(k), ins = k > -tn ? prev(k - 1) : UNSET, del = k < qn ? prev(k + 1) : UNSET;
+                int32_t best_pos = UNSET;
+                uint32_t best_op = 0;
+                if (mis != UNSET) best_pos = mis + 1, best_op = 1;
+                if (ins != UNSET && ins + 1 >= best_pos) best_pos = ins + 1, best_op = 2;
+                if (del != UNSET && del >= best_pos) best_pos = del, best_op = 3;
+                int32_t val = UNSET;
+                uint32_t aux = 0;
+                const int32_t j = best_pos - k;
+                if (best_op != 0 && best_pos <= qn && j >= 0 && j <= tn) {
+                    val = extend_valid<S>(sq, qn, st, tn, best_pos, k, lcp_words);
+                    aux = (static_cast<uint32_t>(best_pos) << 2) | best_op;
+                }
+                cur_frame[k - lo] = val;
+                hr[base + (k - lo)] = aux;
+                if (val >= qn && (fitting ? k >= qn - tn : k == qn - tn)) my_end = min(my_end, k);
+            }
+            my_end = __reduce_min_sync(PHR_FULL_MASK, my_end);
+            if ((tid & 31) == 0 && my_end != INT32_MAX) atomicMin(&sh_end[s % 3], my_end);
+            __syncthreads();
+            const int kk = sh_end[s % 3];
+            if (kk != INT32_MAX) {
+                done = true;
+                s_end = s;
+                t_end = qn - kk;
+            }
+        }
+    }
+    if (P.work) {  // work counters: band diagonals (the same in every thread), LCP word compares
+        if (tid == 0) atomicAdd(P.work + 2, static_cast<unsigned long long>(wf_cells));
+        if (lcp_words) atomicAdd(P.work + 3, static_cast<unsigned long long>(lcp_words));
+    }
+    if (overflow) {  // CTA-uniform
+        // Scratch for the redo: extrapolate the final score from the furthest query offset
+        // of the last score (the wavefront advances about in proportion to the score) plus a
+        // quarter; at least twice the scores reached, at most the whole search.
+        int vm = 0;
+        if (s >= 2) {
+            const int32_t* pf = frame(s - 1);
+            const int plo = -min(s - 1, tn), phi = min(s - 1, qn);
+            for (int k = plo + tid; k <= phi; k += nthr) vm = max(vm, pf[k - plo]);
+        }
+        vm = __reduce_max_sync(PHR_FULL_MASK, vm);
+        __syncthreads();  // every thread is done with the end flags
+        if (tid == 0) sh_end[0] = 0;
+        __syncthreads();
+        if ((tid & 31) == 0) atomicMax(&sh_end[0], vm);
+        __syncthreads();
+        if (tid == 0) {
+            const int64_t reach = sh_end[0];
+            int64_t s2 = 2LL * s + 64;
+            if (reach > 0) {
+                int64_t est = static_cast<int64_t>(s) * qn / reach;
+                est += est / 4 + 64;
+                s2 = ::max(s2, est);
+            }
+            s2 = ::min(static_cast<int64_t>(max_s) + 1, s2);
+            report_redo(P, pid, fixed + lin_base(s2, qn, tn) * 4 + 64);
+        }
+    }
+
+    // ---- traceback by thread 0, formatting by warp 0 ----
+    if (tid < 32) {
+        RunWriter rw;
+        rw.init(runs, static_cast<uint32_t>(qn + tn + 2));
+        if (done && tid == 0) lin_trace(rw, hr, qn, tn, t_end, s_end);
+        wfa_result(P, pid, true, 32, done, !done && !overflow, rw, runs, static_cast<uint32_t>(s_end), 0,
+                   t_end);
+    }
+    __syncthreads();  // shared memory and the task slot are reused by the next pair
+}
+
+template <class S>
+__global__ void __launch_bounds__(kBigThreads, 2) wfa_linear_long_kernel(ExtendParams P) {
+    extern __shared__ __align__(16) int32_t long_frames[];
+    __shared__ uint32_t sh_task;
+    __shared__ int sh_end[3];
+    for (;;) {
+        if (threadIdx.x == 0) sh_task = P.tasks.range[0] + atomicAdd(P.queue_head, 1u);
+        __syncthreads();
+        const uint32_t task = sh_task;
+        __syncthreads();
+        if (task >= P.tasks.range[1]) break;
+        if ((P.tasks.task_group[task] & kOtherKernel) != kBigTask) continue;
+        const uint32_t pid = P.tasks.order[P.tasks.task_first[task]];
+        const PairDesc d = P.desc[pid];
+        if (d.mode != (S::kBits == 2 ? 0 : 1)) continue;
+        wfa_linear_cta<S>(P, d, pid, P.scratch + P.task_off[task], P.task_len[task] & ~15ull, long_frames, P.big_smem / 8,
+                          sh_end);
+    }
+}
+
+// ===========================================================================
 // WFA, one short pair per warp, wavefronts in registers
 // ===========================================================================
 // Gap-affine: every reachable cell of score s lies on a diagonal |k| <= (s - O) / E (a gap of length L
@@ -1636,9 +1809,9 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
         if (act) d = P.desc[pid];
         // pairs of the other symbol mode run in the other instantiation
         act = act && d.mode == (S::kBits == 2 ? 0 : 1);
-        // long pairs run one per CTA: deferred from the main pass to the redo passes,
-        // where wfa_linear_big_kernel / wfa_affine_big_kernel take them
-        if (act && !P.task_off && big_pair(P.engine, P.big_min, P.big_smem, d.qn, d.tn, d.mode)) {
+        // long pairs that the register tiles do not take run one per CTA: deferred from the main
+        // pass to the redo passes, where wfa_linear_long_kernel / wfa_affine_big_kernel take them
+        if (act && !P.task_off && big_pair(P.engine, P.big_min, d.qn, d.tn)) {
             if ((lane & (G - 1)) == 0)
                 report_redo(P, pid, wfa_region_est(d.qn, d.tn, kAffine));
             act = false;
@@ -1753,6 +1926,13 @@ void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t 
 }
 void launch_wfa_linear_bytes(const ExtendParams& p, int grid, int block, cudaStream_t st) {
     wfa_kernel<SeqB, false><<<grid, block, 0, st>>>(p);
+}
+void launch_wfa_linear_long(const ExtendParams& p, int grid, int mode, cudaStream_t st) {
+    auto go = [&](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.big_smem));
+        kernel<<<grid, kBigThreads, p.big_smem, st>>>(p);
+    };
+    mode == 0 ? go(wfa_linear_long_kernel<Seq2>) : go(wfa_linear_long_kernel<SeqB>);
 }
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st) {
     if (mode == 0) {

@@ -41,3 +41,27 @@ def test_long_targets(engine, costs, alphabet, big_min):
     # (the oracle keeps full-width wavefronts: the pair of the fewest score steps)
     oa, oc = O.extend_packed(engine, O.PackedPairs([whole[len(cut) // 2]]), costs)
     assert [got[0][len(cut) // 2]] == P.unpack(oa, oc)
+
+
+@pytest.mark.parametrize("n", [(1 << 22) - 1, 1 << 22, (1 << 22) + 333])
+@pytest.mark.parametrize("company", [0, 1500], ids=["alone", "among_short"])
+def test_long_linear_queries(n, company):
+    """Near-identical linear pairs on both sides of the register tiles' longest query, both end
+    rules and symbol modes, alone and in a batch of short pairs, in a small workspace."""
+    rng = np.random.default_rng(92)
+    base = rng.choice(np.frombuffer(DNA, np.uint8), 2 * n).tobytes()
+    q = base[:n]
+    near = q[:70_000] + q[70_002:2_000_000] + (b"C" if q[2_000_000:2_000_001] != b"C" else b"G") + q[2_000_001:] + b"ACG"
+    window = near + base[n: n + n // 2 + 20]
+    pairs = [(q, near), (q, window), (q[:100_000] + b"N" + q[100_001:], near)]
+    for _ in range(company):
+        s = int(rng.integers(0, n - 300))
+        pairs.append((base[s:s + 150], base[s:s + 70] + base[s + 72:s + 160]))
+    packed = O.PackedPairs(pairs)
+    with P.Engine(0, workspace_bytes=256 << 20) as eng:
+        eng.set_timing(True)
+        ga, gc = eng.extend_packed(A.ENGINE_WFA_LINEAR, packed)
+        ran = eng.kernel_times()
+    assert ("wfa_linear_long" in ran) == (n >= 1 << 22)
+    oa, oc = O.extend_packed(A.ENGINE_WFA_LINEAR, packed, (2, 4, 1))
+    assert P.unpack(ga, gc) == P.unpack(oa, oc)
