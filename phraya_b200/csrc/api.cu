@@ -384,6 +384,7 @@ int* tune_field(phr::EngineTune& t, const char* key) {
     if (!std::strcmp(key, "host_chunks")) return &t.host_chunks;
     if (!std::strcmp(key, "myers_lane_ckpt")) return &t.myers_lane_ckpt;
     if (!std::strcmp(key, "wfa_affine_big_threads")) return &t.wfa_affine_big_threads;
+    if (!std::strcmp(key, "wfa_cluster_max")) return &t.wfa_cluster_max;
     return nullptr;
 }
 bool tune_valid(const char* key, int64_t v) {
@@ -399,6 +400,7 @@ bool tune_valid(const char* key, int64_t v) {
     if (!std::strcmp(key, "host_chunks")) return v >= 2 && v <= 32;
     if (!std::strcmp(key, "myers_lane_ckpt")) return v == 0 || v == 1;
     if (!std::strcmp(key, "wfa_affine_big_threads")) return v == 256 || v == 512 || v == 1024;
+    if (!std::strcmp(key, "wfa_cluster_max")) return v == 1 || v == 4 || v == 8 || v == 16;
     return false;
 }
 }  // namespace

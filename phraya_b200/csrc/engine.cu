@@ -1234,11 +1234,6 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             else
                 launch_wfa_affine_bytes(P, static_cast<int>(grid), block, st);
         }
-        // A context that leaves room on the SMs (a server's worker for long reads) shares the GPU:
-        // other contexts have work for SMs idle here, which clusters would hold or wait for.
-        // 150 bp reads served beside long ones at 10^6 reads/s offered: p99 74-116 ms with
-        // clusters (three runs), 6-9 ms without (five of six; one 77).
-        const bool shared_gpu = ctx->tune.max_blocks_per_sm < EngineTune{}.max_blocks_per_sm;
         const bool tiles = engine == PHR_ENGINE_WFA_LINEAR ||
                            (engine == PHR_ENGINE_WFA_AFFINE && aff_tile_open(costs) != 0);
         if (tiles && P.big_min > 0 && (per_task ? n_tasks_hint : n_tiles) > 0) {
@@ -1254,7 +1249,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 const bool cta = i >= 2;
                 const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 60), pool,
                                     cta ? kTileChunk : kWarpTileChunk,
-                                    per_task || !cta || shared_gpu ? 0 : kTileDeferStep, ctx->sm_count,
+                                    per_task || !cta || ctx->tune.wfa_cluster_max == 1 ? 0 : kTileDeferStep, ctx->sm_count,
                                     cnt + 62, reinterpret_cast<unsigned long long*>(rtask_off)};
                 const uint64_t most = static_cast<uint64_t>(ctx->sm_count) *
                                       (cta ? 1 : std::min(ctx->tune.max_blocks_per_sm, 2));
@@ -1307,7 +1302,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
             const TileLaunch tl{reinterpret_cast<unsigned long long*>(cnt + 60), tile_pool, kTileChunk, 0, ctx->sm_count, cnt + 62,
                                 reinterpret_cast<unsigned long long*>(rtask_off)};
             const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
-            const int ctas = h_defer <= sms / 16 ? 16 : h_defer <= sms / 8 ? 8 : 4;
+            const int ctas = std::min(h_defer <= sms / 16 ? 16 : h_defer <= sms / 8 ? 8 : 4, ctx->tune.wfa_cluster_max);
             for (int mode = 0; mode < 2; ++mode) {
                 if (n_tile[2 + mode] == 0) continue;
                 PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 63, 0, 4, st));

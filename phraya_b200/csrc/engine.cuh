@@ -45,6 +45,8 @@ struct EngineTune {
     int host_chunks = 4;             // chunks a large host batch is copied and aligned in (overlapped)
     int wfa_affine_big_threads = kBigAffineThreads;  // threads per CTA of the gap-affine
                                      // CTA-per-pair kernel (256, 512 or 1024; 1024 / this CTAs per SM)
+    int wfa_cluster_max = 16;        // most CTAs that a long pair left alone on the GPU is given (1: its one
+                                     // CTA keeps it; else 4, 8 or 16)
     int myers_lane_ckpt = 1;         // banded Myers lane kernel: recompute segments from checkpoints (1)
                                      // or store every column's records (0)
 };

@@ -1,0 +1,84 @@
+"""Long WFA pairs that the CTA kernels leave to clusters of CTAs once most SMs have run out of
+pairs (wfa_tile.cuh): when that happens, and that the results stay the oracle's."""
+import time
+
+import numpy as np
+import pytest
+
+import oracle as O
+from phraya_b200 import _abi as A
+from phraya_b200 import api as P
+from phraya_b200 import casegen as G
+
+pytestmark = pytest.mark.gpu
+
+DNA, AA = b"ACGT", b"ACDEFGHIKLMNPQRSTVWY"
+ENGINES = [(A.ENGINE_WFA_LINEAR, (2, 4, 1)), (A.ENGINE_WFA_AFFINE, (2, 4, 1)), (A.ENGINE_WFA_AFFINE, (4, 6, 2))]
+engines = pytest.mark.parametrize("engine,costs", ENGINES, ids=["linear", "2-4-1", "4-6-2"])
+RESUME = {A.ENGINE_WFA_LINEAR: "wfa_linear_resume", A.ENGINE_WFA_AFFINE: "wfa_affine_resume"}
+
+
+def divergent(rng, n, length, alphabet=DNA, rate=0.15):
+    """Pairs of about `length` symbols whose score passes the step at which a pair is left."""
+    pairs = []
+    for i in range(n):
+        q = rng.choice(np.frombuffer(alphabet, np.uint8), length + 17 * i)
+        t = q.copy()
+        hit = rng.random(t.size) < rate
+        t[hit] = rng.choice(np.frombuffer(alphabet, np.uint8), int(hit.sum()))
+        t = np.delete(t, np.flatnonzero(rng.random(t.size) < rate / 4))
+        pairs.append((q.tobytes(), t.tobytes()))
+    return pairs
+
+
+def run(eng, engine, costs, pairs):
+    """The pairs' results, the oracle's, and how often each kernel ran."""
+    packed = O.PackedPairs(pairs)
+    eng._lib.phr_ctx_reset_timing(eng.handle)
+    eng.set_timing(True)
+    ga, gc = eng.extend_packed(engine, packed, P.AffineCosts(*costs))
+    ran = {k: v[0] for k, v in eng.kernel_times().items()}
+    eng.set_timing(False)
+    oa, oc = O.extend_packed(engine, packed, costs)
+    if engine == A.ENGINE_WFA_AFFINE:
+        assert np.array_equal(ga["affine_score"], oa["affine_score"])
+    return P.unpack(ga, gc), P.unpack(oa, oc), ran
+
+
+@engines
+def test_resident_blocks_do_not_decide(engine, costs):
+    """"max_blocks_per_sm" is about resident blocks only; "wfa_cluster_max" 1 keeps every pair on
+    its CTA."""
+    pairs = divergent(np.random.default_rng(61), 3, 3000)
+    with P.Engine(0) as eng:
+        for blocks in (4, 3, 2, 1):
+            eng.set_tune("max_blocks_per_sm", blocks)
+            got, want, ran = run(eng, engine, costs, pairs)
+            assert got == want and ran.get(RESUME[engine], 0) == 1, (blocks, ran)
+        eng.set_tune("wfa_cluster_max", 1)
+        got, want, ran = run(eng, engine, costs, pairs)
+        assert got == want and RESUME[engine] not in ran
+
+
+@pytest.mark.parametrize("streams,short_lane,blocks,clusters", [(1, -1, 4, True), (2, -1, 4, False), (2, 1, 4, False)])
+def test_server_workers(streams, short_lane, blocks, clusters, tmp_path, monkeypatch):
+    """Workers that share the GPU with others leave their long pairs on single CTAs, whatever the
+    lanes and the blocks per SM; one worker alone uses clusters."""
+    trace = tmp_path / "trace.txt"
+    monkeypatch.setenv("PHRAYA_SERVER_TRACE", str(trace))
+    ref = G.repeat_reference(2_000_000, 20, seed=62)
+    packed, _, _ = G.long_reads(ref, 60, seed=63, error=0.12)
+    reads = [bytes(packed.seq[o:o + n]) for o, n in zip(packed.off.tolist(), packed.len.tolist())]
+    with P.Engine(0) as eng:
+        idx = eng.index(ref)
+        batched, _ = eng.align_reads(idx, reads, A.BALANCED)
+        srv = eng.server(idx, strategy=A.BALANCED, max_batch_reads=64, max_wait_us=20000, n_streams=streams,
+                         short_lane=short_lane, long_blocks_per_sm=blocks)
+        ids = srv.submit_many(reads)
+        got, until = {}, time.time() + 120
+        while len(got) < len(reads) and time.time() < until:
+            for rid, res, _ in srv.poll(4096, wait_us=20000):
+                got[rid] = res
+        srv.close()
+    assert [got[i] for i in ids] == batched
+    assert ("wfa_linear_resume" in trace.read_text()) == clusters
