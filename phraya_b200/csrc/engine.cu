@@ -994,6 +994,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
     uint64_t* total = reinterpret_cast<uint64_t*>(cnt + 12);
     const unsigned T = 256;
+    const uint64_t pass_budget = std::min(ctx->scratch_budget, ctx->pass_budget);
     const bool small = n <= kSmallPairs;
     // lanes per short WFA pair: affine and linear tune separately
     const int g_short = engine == PHR_ENGINE_WFA_AFFINE ? ctx->tune.wfa_affine_group_short : ctx->tune.wfa_group_short;
@@ -1160,7 +1161,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 const uint64_t teams = n_tile[0] + n_tile[1] > 0 ? 16ull * ctx->sm_count : ctx->sm_count;
                 pool = std::min<uint64_t>(2 * tile_need[0], 2 * teams * tile_need[1]);
                 pool = std::max<uint64_t>(pool, std::min<uint64_t>(16 * tile_need[0], 1ull << 30)) + (1 << 20);
-                pool = std::min<uint64_t>(pool, ctx->scratch_budget);
+                pool = std::min<uint64_t>(pool, pass_budget);
                 tile_pool = pool;
             }
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
@@ -1413,7 +1414,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                     clamp = true;
                     need = ctx->scratch_budget & ~255ull;
                 }
-                if (!pl.empty() && tot + need > ctx->scratch_budget) break;  // this pair opens the next pass
+                if (!pl.empty() && tot + need > pass_budget) break;  // this pair opens the next pass
                 // the whole-budget try is spent only once the pair is placed in a pass
                 if (clamp) clamped.insert(h_list[idx[pos]]);
                 pl.push_back(h_list[idx[pos]]);

@@ -65,6 +65,8 @@ struct Ctx {
     DeviceArena pipe;        // align_read pipeline state (kept across its extension calls)
     DeviceArena seeds;       // per-seed arrays of seeding/chaining, sized from the exact seed count
     size_t scratch_budget = 8ull << 30;
+    size_t pass_budget = ~0ull;   // what the long pairs of one pass share of it (a pair alone may take all):
+                                  // a server's worker keeps to the scratch it has
     std::string last_error;
     std::atomic<uint64_t> launches{0};
     EngineTune tune;

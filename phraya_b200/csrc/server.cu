@@ -449,7 +449,15 @@ phr_status phr_server_create(phr_ctx* c, const phr_index* idx, const phr_server_
             W->ctx.seeds.reserve(nb * 40 + (16ull << 20));
             W->ctx.io.reserve(nb * 16 + nr * 1024 + (16ull << 20));
             W->ctx.arena.reserve(nb * 24 + nr * 2048 + (96ull << 20));
-            W->ctx.scratch.reserve(std::min<uint64_t>(W->ctx.scratch_budget, W->short_only ? (512ull << 20) : (4ull << 30)));
+            const uint64_t scratch = std::min<uint64_t>(W->ctx.scratch_budget, W->short_only ? (512ull << 20) : (4ull << 30));
+            W->ctx.scratch.reserve(scratch);
+            // Linear pairs keep to it: the records of those in flight fit, where room for every
+            // pair of a batch (what a batched call takes) made the buffer grow from batch to
+            // batch, to 12 GB and more. 2,000 long and 2,000 short reads at once, balanced:
+            // 3,100-12,500 reads/s, p99 of the long ones 0.3-1.3 s, 63 GiB in use; with the
+            // limit 50,000-64,000 reads/s, 46-66 ms, 26 GiB. Gap-affine pairs hold five times
+            // the records: 150 reads/s with the limit, 850 without.
+            if (!W->short_only && S->cfg.align.strategy != PHR_SENSITIVE) W->ctx.pass_budget = scratch;
             cudaGetLastError();
             const uint32_t K = S->cfg.align.strategy == PHR_FAST ? 1 : S->cfg.align.strategy == PHR_BALANCED ? 2 : 50;
             W->seq.ensure(nb + 64);
