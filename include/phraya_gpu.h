@@ -141,9 +141,7 @@ void phr_ctx_destroy(phr_ctx* ctx);
  *                                        kernel: 1024 (default, one CTA per SM), 512 or 256
  *   "wfa_cluster_max"                    most SMs that the last long WFA pairs of a batch are
  *                                        given once most SMs have run out of pairs: 16
- *                                        (default), 8, 4 or 1 (each stays on its one SM). A
- *                                        server of several streams uses 1: its other streams
- *                                        have work for those SMs.
+ *                                        (default), 8, 4 or 1 (each stays on its one SM)
  *   "max_blocks_per_sm"                  resident blocks per SM of the persistent extension
  *                                        kernels (1..4)
  *   "host_chunks"                        chunks a host batch of more than 128 MiB of sequence

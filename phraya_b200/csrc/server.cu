@@ -426,9 +426,6 @@ phr_status phr_server_create(phr_ctx* c, const phr_index* idx, const phr_server_
         if (S->short_lane && w > 0)
             W->ctx.tune.max_blocks_per_sm = std::min<int>(W->ctx.tune.max_blocks_per_sm,
                                                           static_cast<int>(S->cfg.long_blocks_per_sm));
-        // SMs idle in one worker have another's reads to run, which clusters of CTAs would hold
-        // up or wait for.
-        if (S->cfg.n_streams > 1) W->ctx.tune.wfa_cluster_max = 1;
         const int prio = W->short_only ? prio_high : prio_low;
         if (cudaStreamCreateWithPriority(&W->ctx.stream, cudaStreamNonBlocking, prio) != cudaSuccess) {
             delete W;

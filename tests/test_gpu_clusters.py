@@ -60,16 +60,17 @@ def test_resident_blocks_do_not_decide(engine, costs):
         assert got == want and RESUME[engine] not in ran
 
 
-@pytest.mark.parametrize("streams,short_lane,blocks,clusters", [(1, -1, 4, True), (2, -1, 4, False), (2, 1, 4, False)])
+@pytest.mark.parametrize("streams,short_lane,blocks", [(1, -1, 4), (2, -1, 4), (2, 1, 4), (2, 1, 2)])
+@pytest.mark.parametrize("clusters", [16, 1])
 def test_server_workers(streams, short_lane, blocks, clusters, tmp_path, monkeypatch):
-    """Workers that share the GPU with others leave their long pairs on single CTAs, whatever the
-    lanes and the blocks per SM; one worker alone uses clusters."""
+    """A server's workers follow its context's setting, whatever the lanes and blocks per SM."""
     trace = tmp_path / "trace.txt"
     monkeypatch.setenv("PHRAYA_SERVER_TRACE", str(trace))
     ref = G.repeat_reference(2_000_000, 20, seed=62)
     packed, _, _ = G.long_reads(ref, 60, seed=63, error=0.12)
     reads = [bytes(packed.seq[o:o + n]) for o, n in zip(packed.off.tolist(), packed.len.tolist())]
     with P.Engine(0) as eng:
+        eng.set_tune("wfa_cluster_max", clusters)
         idx = eng.index(ref)
         batched, _ = eng.align_reads(idx, reads, A.BALANCED)
         srv = eng.server(idx, strategy=A.BALANCED, max_batch_reads=64, max_wait_us=20000, n_streams=streams,
@@ -81,4 +82,4 @@ def test_server_workers(streams, short_lane, blocks, clusters, tmp_path, monkeyp
                 got[rid] = res
         srv.close()
     assert [got[i] for i in ids] == batched
-    assert ("wfa_linear_resume" in trace.read_text()) == clusters
+    assert ("wfa_linear_resume" in trace.read_text()) == (clusters > 1)
