@@ -1141,6 +1141,11 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     // scratch (P.task_off / P.task_len set by the caller, `per_task_total` bytes in all,
     // `n_tasks_hint` tasks)
     uint64_t tile_pool = 0;   // of the main pass
+    int cluster_max = 1;      // most CTAs that a long pair left by its own is given
+    if (n_tile[2] + n_tile[3] > 0 && ctx->tune.wfa_cluster_max > 1) {
+        if (ctx->cluster_fit == 0) ctx->cluster_fit = wfa_cluster_fit(P.big_smem);
+        cluster_max = std::min(ctx->cluster_fit, ctx->tune.wfa_cluster_max);
+    }
     auto launch_pass = [&](const uint32_t* ord, const uint32_t* tfirst, const uint8_t* tcount, const uint8_t* tgroup,
                            const uint32_t* range0, const uint32_t* range1, uint64_t slot, int full_band,
                            bool per_task = false, uint64_t per_task_total = 0,
@@ -1250,7 +1255,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 const bool cta = i >= 2;
                 const TileLaunch tl{per_task ? nullptr : reinterpret_cast<unsigned long long*>(cnt + 60), pool,
                                     cta ? kTileChunk : kWarpTileChunk,
-                                    per_task || !cta || ctx->tune.wfa_cluster_max == 1 ? 0 : kTileDeferStep, ctx->sm_count,
+                                    per_task || !cta || cluster_max == 1 ? 0 : kTileDeferStep, ctx->sm_count,
                                     cnt + 62, reinterpret_cast<unsigned long long*>(rtask_off)};
                 const uint64_t most = static_cast<uint64_t>(ctx->sm_count) *
                                       (cta ? 1 : std::min(ctx->tune.max_blocks_per_sm, 2));
@@ -1302,8 +1307,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         if (h_defer > 0) {
             const TileLaunch tl{reinterpret_cast<unsigned long long*>(cnt + 60), tile_pool, kTileChunk, 0, ctx->sm_count, cnt + 62,
                                 reinterpret_cast<unsigned long long*>(rtask_off)};
-            const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
-            const int ctas = std::min(h_defer <= sms / 16 ? 16 : h_defer <= sms / 8 ? 8 : 4, ctx->tune.wfa_cluster_max);
+            const int ctas = wfa_cluster_size(h_defer, ctx->sm_count, cluster_max);
             for (int mode = 0; mode < 2; ++mode) {
                 if (n_tile[2 + mode] == 0) continue;
                 PHR_CUDA_TRY(ctx, cudaMemsetAsync(cnt + 63, 0, 4, st));

@@ -67,6 +67,7 @@ struct Ctx {
     size_t scratch_budget = 8ull << 30;
     size_t pass_budget = ~0ull;   // what the long pairs of one pass share of it (a pair alone may take all):
                                   // a server's worker keeps to the scratch it has
+    int cluster_fit = 0;          // wfa_cluster_fit of the device, 0: not asked yet
     std::string last_error;
     std::atomic<uint64_t> launches{0};
     EngineTune tune;

@@ -319,6 +319,16 @@ int launch_wfa_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int
                      uint32_t* n_left, cudaStream_t st);
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st);
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st);
+// The largest cluster of the resume kernels that the device can hold: 16 (not a portable size),
+// 8, 4, or 1 for none. All of them are CTAs of kBigThreads threads, one per SM.
+int wfa_cluster_fit(uint32_t smem);
+// The size for `pairs` deferred pairs where up to `most` CTAs are allowed: the fewer the pairs,
+// the more SMs each.
+__host__ __forceinline__ int wfa_cluster_size(uint32_t pairs, int sm_count, int most) {
+    const uint32_t sms = static_cast<uint32_t>(sm_count);
+    const int want = pairs <= sms / 16 ? 16 : pairs <= sms / 8 ? 8 : 4;
+    return want < most ? want : most;
+}
 // Deferred pairs of both symbol modes' launches, `ctas` (4, 8 or 16) CTAs per pair.
 void launch_wfa_linear_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st);
 void launch_wfa_affine_resume(const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, int mode, cudaStream_t st);

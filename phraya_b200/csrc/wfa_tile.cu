@@ -548,6 +548,12 @@ void launch_wfa_linear_resume(const ExtendParams& p, const TileLaunch& a, int pa
     else
         ctas == 16 ? go(wfa_linear_resume_kernel<SeqB, 16>) : ctas == 8 ? go(wfa_linear_resume_kernel<SeqB, 8>) : go(wfa_linear_resume_kernel<SeqB, 4>);
 }
+int wfa_cluster_fit(uint32_t smem) {
+    return cluster_fits(wfa_linear_resume_kernel<Seq2, 16>, 16, smem)  ? 16
+           : cluster_fits(wfa_linear_resume_kernel<Seq2, 8>, 8, smem) ? 8
+           : cluster_fits(wfa_linear_resume_kernel<Seq2, 4>, 4, smem) ? 4
+                                                                      : 1;
+}
 void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
     constexpr int smem = kWarpTileThreads / 32 * static_cast<int>(kWarpTileSmem);
     if (mode == 0) {

@@ -456,24 +456,43 @@ __device__ __forceinline__ void tile_defer(const ExtendParams& P, const TileLaun
     sh->n_chunks = 0;
 }
 
+// Launch of `teams` clusters of `ctas` CTAs each.
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    template <class K>
+    ClusterLaunch(K kernel, int teams, int ctas, uint32_t smem, cudaStream_t st) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (ctas > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cfg.gridDim = dim3(static_cast<unsigned>(teams * ctas));
+        cfg.blockDim = dim3(kBigThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+    ClusterLaunch(const ClusterLaunch&) = delete;
+};
+
 // Launches a cluster kernel, `ctas` CTAs per team, at most as many teams as fit at once.
 template <class K>
 inline void launch_clusters(K kernel, const ExtendParams& p, const TileLaunch& a, int pairs, int ctas, cudaStream_t st) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.big_smem));
-    if (ctas > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaLaunchConfig_t cfg = {};
     const int most = a.sm_count / ctas > 0 ? a.sm_count / ctas : 1;
-    cfg.gridDim = dim3(static_cast<unsigned>((pairs < most ? pairs : most) * ctas));
-    cfg.blockDim = dim3(kBigThreads);
-    cfg.dynamicSmemBytes = p.big_smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(ctas);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, p, a);
+    ClusterLaunch l(kernel, pairs < most ? pairs : most, ctas, p.big_smem, st);
+    cudaLaunchKernelEx(&l.cfg, kernel, p, a);
+}
+
+// Whether the device can hold one such cluster.
+template <class K>
+inline bool cluster_fits(K kernel, int ctas, uint32_t smem) {
+    ClusterLaunch l(kernel, 1, ctas, smem, nullptr);
+    int n = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();   // a size the device does not know is an answer, not a failure
+    return ok;
 }
 
 }  // namespace

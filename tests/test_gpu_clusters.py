@@ -83,3 +83,32 @@ def test_server_workers(streams, short_lane, blocks, clusters, tmp_path, monkeyp
         srv.close()
     assert [got[i] for i in ids] == batched
     assert ("wfa_linear_resume" in trace.read_text()) == (clusters > 1)
+
+
+@engines
+@pytest.mark.parametrize("alphabet", [DNA, AA], ids=["2bit", "bytes"])
+@pytest.mark.parametrize("clusters,n", [(16, 4), (16, 14), (16, 30), (8, 4), (4, 4)])
+def test_cluster_sizes(engine, costs, alphabet, clusters, n):
+    """16, 8 and 4 CTAs a pair: by the number of pairs left (148 SMs) and by the setting, which a
+    device without room for the larger ones has too."""
+    pairs = divergent(np.random.default_rng(64), n, 2200, alphabet)
+    with P.Engine(0) as eng:
+        eng.set_tune("wfa_cluster_max", clusters)
+        got, want, ran = run(eng, engine, costs, pairs)
+    assert got == want and ran.get(RESUME[engine], 0) == 1, ran
+
+
+@engines
+@pytest.mark.parametrize("clusters", [16, 4, 1])
+def test_records_run_out(engine, costs, clusters):
+    """A workspace that the pair's records outgrow: on its cluster, after the hand-over, or on its
+    one CTA. Either way a redo pass follows and fits."""
+    pairs = divergent(np.random.default_rng(65), 1, 3000)
+    # (record chunks double from 64 KiB: a CTA's first three end at 448, its first seven at 8,128)
+    budget = 8000 if engine == A.ENGINE_WFA_AFFINE else 550 if clusters > 1 else 430
+    with P.Engine(0, workspace_bytes=budget << 10) as eng:
+        eng.set_tune("wfa_cluster_max", clusters)
+        got, want, ran = run(eng, engine, costs, pairs)
+        assert eng.counter("scratch_oom_pairs") == 0
+    # (one pair: were it redone before the hand-over, no cluster would have run)
+    assert got == want and ran.get(RESUME[engine], 0) == (1 if clusters > 1 else 0) and ran["redo_tasks"] >= 1, ran
