@@ -1194,14 +1194,12 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
         if (!per_task && n_lane > 0) {
             // 2-bit pairs of one lane each (tasks [0, g1)); the warp-group kernel
             // below takes the remaining 2-bit tasks [g1, split)
-            const uint64_t lane_grid =
-                std::min<uint64_t>(grid * warps_per_block / (kLaneThreads / 32),
-                                   static_cast<uint64_t>(ctx->sm_count) * myers_lane_blocks_per_sm(P.lane_ckpt));
+            const LaneGrid lg = lane_grid(grid * warps_per_block, ctx->sm_count, myers_lane_blocks_per_sm(P.lane_ckpt));
             P.tasks.range = cnt + 28;
             P.queue_head = cnt + 26;
             {
                 KernelScope ks(ctx, "myers_lane");
-                launch_myers_lane(P, static_cast<int>(std::max<uint64_t>(lane_grid, 1)), st);
+                launch_myers_lane(P, lg, st);
             }
         }
         P.tasks.range = range0;

@@ -299,10 +299,20 @@ __host__ __device__ __forceinline__ int tile_warps(int32_t engine, int open, int
 }
 
 void launch_myers(const ExtendParams& p, int grid, int block, cudaStream_t st);
-void launch_myers_lane(const ExtendParams& p, int grid, cudaStream_t st);
+constexpr int kLaneThreads = 256;   // most threads per block of the lane kernel
+// Launch of the lane kernel over `warps` scratch slots, one per warp: never more warps than
+// slots, whatever the block size of the other kernels.
+struct LaneGrid {
+    int blocks, threads;
+};
+__host__ __forceinline__ LaneGrid lane_grid(uint64_t warps, int sm_count, int blocks_per_sm) {
+    const uint64_t per_block = warps < kLaneThreads / 32 ? warps : kLaneThreads / 32;
+    const uint64_t most = static_cast<uint64_t>(sm_count) * blocks_per_sm, want = warps / per_block;
+    return LaneGrid{static_cast<int>(want < most ? want : most), static_cast<int>(32 * per_block)};
+}
+void launch_myers_lane(const ExtendParams& p, LaneGrid g, cudaStream_t st);
 // Resident blocks per SM of the lane kernel in each mode (its shared memory per warp).
 int myers_lane_blocks_per_sm(int ckpt);
-constexpr int kLaneThreads = 256;
 void launch_wfa_linear(const ExtendParams& p, int grid, int block, cudaStream_t st);
 // Tasks per SM above which they run first in the kernel for short pairs alone, whose second
 // launch and tail of the longest pairs need time to pay: pairs of 100-300 bp at 0-5 %, with

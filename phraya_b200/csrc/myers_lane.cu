@@ -721,21 +721,21 @@ __global__ void __launch_bounds__(kLaneThreads, 3) myers_lane_fit_kernel(ExtendP
 
 int myers_lane_blocks_per_sm(int ckpt) { return ckpt ? 3 : 2; }
 
-void launch_myers_lane(const ExtendParams& p, int grid, cudaStream_t st) {
+void launch_myers_lane(const ExtendParams& p, LaneGrid g, cudaStream_t st) {
     if (p.lane_ckpt) {
         const int smem = kLaneWarps * kCkWarpBytes;
         if (p.engine == PHR_ENGINE_MYERS_FIT) {
             cudaFuncSetAttribute(myers_lane_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            myers_lane_fit_kernel<<<grid, kLaneThreads, smem, st>>>(p);
+            myers_lane_fit_kernel<<<g.blocks, g.threads, smem, st>>>(p);
             return;
         }
         cudaFuncSetAttribute(myers_lane_ck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        myers_lane_ck_kernel<<<grid, kLaneThreads, smem, st>>>(p);
+        myers_lane_ck_kernel<<<g.blocks, g.threads, smem, st>>>(p);
         return;
     }
     const int smem = kLaneWarps * kLanePeqWarpBytes;
     cudaFuncSetAttribute(myers_lane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    myers_lane_kernel<<<grid, kLaneThreads, smem, st>>>(p);
+    myers_lane_kernel<<<g.blocks, g.threads, smem, st>>>(p);
 }
 
 }  // namespace phr
