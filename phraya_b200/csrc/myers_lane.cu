@@ -149,14 +149,14 @@ __device__ __forceinline__ uint64_t hin_off(int sg, int k, int lane) {
 // the latest lowest) that entered each block of the window at the segment's end, to
 // `hin`. The traceback recomputes from those the two blocks a lane's path is in.
 // FIT: `fit` is the lane's search for the best end column (myers_fitting_impl), and the pass
-// ends early once every lane's is over.
+// ends early once every lane's is over. Returns the last column advanced.
 struct FitEnd {
     bool on;                   // a fitting pair (its target runs on past the query)
     int m, best, best_col, score;
     bool stopped;
 };
 template <int P, bool CK, bool FIT>
-__device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb, int n,
+__device__ __forceinline__ int lane_forward(const uint32_t* __restrict__ qb, const uint32_t* __restrict__ tb, int n,
                                              int nb, const LaneGeom& g, uint64_t* sp, uint8_t* rec, uint8_t* hin,
                                              uint4* planes, FitEnd& fit) {
     const int lane = lane_id();
@@ -270,9 +270,10 @@ __device__ __forceinline__ void lane_forward(const uint32_t* __restrict__ qb, co
 #pragma unroll
             for (int k = 0; k < P; ++k) *reinterpret_cast<uint16_t*>(h + k * 64) = static_cast<uint16_t>(ha[k]);
             // no lane reads a column past its best end (or its target's end)
-            if (FIT && !__any_sync(PHR_FULL_MASK, j < n && !(fit.on && fit.stopped))) break;
+            if (FIT && !__any_sync(PHR_FULL_MASK, j < n && !(fit.on && fit.stopped))) return j;
         }
     }
+    return g.n_max;
 }
 
 // Issues asynchronous global -> shared copies of the records of the kTraceBatch cells
@@ -594,10 +595,10 @@ __device__ void lane_task(const ExtendParams& Pm, uint32_t pid, const PairDesc& 
     uint8_t* hin = slot + lane_ckpt_bytes(g.n_max, P);   // checkpoint mode
     uint4* planes = reinterpret_cast<uint4*>(hin + lane_hin_bytes(g.n_max, P));
     FitEnd fit = {FIT && act && n > m + m / 2 + 10, m, m, 0, m, false};
-    lane_forward<P, CK, FIT>(qb, tb, n, nb, g, sp, slot, hin, planes, fit);
+    const int last = lane_forward<P, CK, FIT>(qb, tb, n, nb, g, sp, slot, hin, planes, fit);
     const int j_end = FIT && fit.on ? fit.best_col : n;
     // work counter: block-columns this task evaluated for its pairs
-    const unsigned long long cols = __reduce_add_sync(PHR_FULL_MASK, act ? static_cast<unsigned>(n) * P : 0u);
+    const unsigned long long cols = __reduce_add_sync(PHR_FULL_MASK, act ? static_cast<unsigned>(min(n, last)) * P : 0u);
     if (lane == 0) atomicAdd(Pm.work, cols);
     __syncwarp();  // the traceback reuses the Peq shared memory
     const uint64_t rec_bytes = lane_rec_bytes(g.n_max, g.m_max, P, CK ? 1 : 0);
