@@ -394,7 +394,7 @@ bool tune_valid(const char* key, int64_t v) {
     if (!std::strcmp(key, "myers_band_base")) return v >= 0 && v <= (1 << 20);
     if (!std::strcmp(key, "block_threads")) return v >= 32 && v <= 256 && v % 32 == 0;
     if (!std::strcmp(key, "wfa_big_min")) return v >= 0 && v <= INT32_MAX;
-    if (!std::strcmp(key, "wfa_big_smem")) return v >= (16 << 10) && v <= (200 << 10) && v % 16 == 0;
+    if (!std::strcmp(key, "wfa_big_smem")) return v >= (16 << 10) && v <= phr::kBigSmemMax && v % 16 == 0;
     if (!std::strcmp(key, "max_blocks_per_sm")) return v >= 1 && v <= 4;
     if (!std::strcmp(key, "wfa_long_min")) return v >= 0 && v <= INT32_MAX;
     if (!std::strcmp(key, "host_chunks")) return v >= 2 && v <= 32;

@@ -58,6 +58,10 @@ constexpr int kBigThreads = 512;         // threads of a register-tile CTA (one 
 // most threads per CTA of wfa.cu's gap-affine CTA-per-pair kernel, and its default (one CTA
 // per SM; the "wfa_affine_big_threads" setting launches 512 or 256, two or four per SM)
 constexpr int kBigAffineThreads = 1024;
+// Largest "wfa_big_smem". A kernel's limit of dynamic shared memory belongs to the process, so
+// every launch sets this one, whatever the context's own size: contexts of different sizes set
+// and launched side by side otherwise.
+constexpr int kBigSmemMax = 200 << 10;
 constexpr uint32_t kBigMinFrameCells = 4096;  // smallest shared frame pair worth staging
 
 // Shared-memory words the CTA-per-pair kernel needs for the two sequences of a pair:

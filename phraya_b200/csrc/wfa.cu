@@ -1769,6 +1769,7 @@ __device__ bool wfa_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, 
 // Persistent kernel: warps pull tasks; each task's groups split the warp's slot evenly.
 constexpr int kAffGroupSmem = kAffRingGroups * kAffRing * static_cast<int>(sizeof(SDir)) + kWarpSeqWords * 4;
 constexpr int kAffWarpSmem = kAffGroupSmem > kRegWarpSmem ? kAffGroupSmem : kRegWarpSmem;
+constexpr int kAffBlockSmem = 8 * kAffWarpSmem;   // of the largest block (the limit set for every size, as kBigSmemMax)
 
 constexpr uint32_t kTaskGrab = 4;   // tasks a warp takes at a time
 
@@ -1929,19 +1930,17 @@ void launch_wfa_linear_bytes(const ExtendParams& p, int grid, int block, cudaStr
 }
 void launch_wfa_linear_long(const ExtendParams& p, int grid, int mode, cudaStream_t st) {
     auto go = [&](auto kernel) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.big_smem));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         kernel<<<grid, kBigThreads, p.big_smem, st>>>(p);
     };
     mode == 0 ? go(wfa_linear_long_kernel<Seq2>) : go(wfa_linear_long_kernel<SeqB>);
 }
 void launch_wfa_affine_big(const ExtendParams& p, int grid, int threads, int mode, cudaStream_t st) {
     if (mode == 0) {
-        cudaFuncSetAttribute(wfa_affine_big_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
+        cudaFuncSetAttribute(wfa_affine_big_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         wfa_affine_big_kernel<Seq2><<<grid, threads, p.big_smem, st>>>(p);
     } else {
-        cudaFuncSetAttribute(wfa_affine_big_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
+        cudaFuncSetAttribute(wfa_affine_big_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         wfa_affine_big_kernel<SeqB><<<grid, threads, p.big_smem, st>>>(p);
     }
 }
@@ -1960,12 +1959,12 @@ int launch_wfa_short(const ExtendParams& p, uint64_t scratch_bytes, int sms, int
 }
 void launch_wfa_affine(const ExtendParams& p, int grid, int block, cudaStream_t st) {
     const int smem = (block / 32) * kAffWarpSmem;
-    cudaFuncSetAttribute(wfa_kernel<Seq2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(wfa_kernel<Seq2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAffBlockSmem);
     wfa_kernel<Seq2, true><<<grid, block, smem, st>>>(p);
 }
 void launch_wfa_affine_bytes(const ExtendParams& p, int grid, int block, cudaStream_t st) {
     const int smem = (block / 32) * kAffWarpSmem;
-    cudaFuncSetAttribute(wfa_kernel<SeqB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(wfa_kernel<SeqB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAffBlockSmem);
     wfa_kernel<SeqB, true><<<grid, block, smem, st>>>(p);
 }
 

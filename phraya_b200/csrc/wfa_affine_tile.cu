@@ -582,8 +582,7 @@ __global__ void __launch_bounds__(kWarpTileThreads, 2) wfa_affine_tile_kernel(Ex
 
 template <class S, int OES>
 void launch_cta(const ExtendParams& p, const TileLaunch& a, int grid, cudaStream_t st) {
-    cudaFuncSetAttribute(wfa_affine_big_tile_kernel<S, OES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(p.big_smem));
+    cudaFuncSetAttribute(wfa_affine_big_tile_kernel<S, OES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
     wfa_affine_big_tile_kernel<S, OES><<<grid, kBigThreads, p.big_smem, st>>>(p, a);
 }
 

@@ -567,12 +567,10 @@ void launch_wfa_linear_tile(const ExtendParams& p, const TileLaunch& a, int grid
 
 void launch_wfa_linear_big(const ExtendParams& p, const TileLaunch& a, int grid, int mode, cudaStream_t st) {
     if (mode == 0) {
-        cudaFuncSetAttribute(wfa_linear_big_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
+        cudaFuncSetAttribute(wfa_linear_big_kernel<Seq2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         wfa_linear_big_kernel<Seq2><<<grid, kBigThreads, p.big_smem, st>>>(p, a);
     } else {
-        cudaFuncSetAttribute(wfa_linear_big_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(p.big_smem));
+        cudaFuncSetAttribute(wfa_linear_big_kernel<SeqB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         wfa_linear_big_kernel<SeqB><<<grid, kBigThreads, p.big_smem, st>>>(p, a);
     }
 }

@@ -462,7 +462,7 @@ struct ClusterLaunch {
     cudaLaunchAttribute attr = {};
     template <class K>
     ClusterLaunch(K kernel, int teams, int ctas, uint32_t smem, cudaStream_t st) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBigSmemMax);
         if (ctas > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cfg.gridDim = dim3(static_cast<unsigned>(teams * ctas));
         cfg.blockDim = dim3(kBigThreads);
