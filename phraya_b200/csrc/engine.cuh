@@ -39,8 +39,8 @@ struct EngineTune {
     int wfa_long_min = 1024;     // bucket edge: qn+tn from which WFA pairs get wfa_group_long lanes
     int myers_band_base = 64;
     int block_threads = 256;
-    int wfa_big_min = 4096;          // linear WFA pairs with qn+tn >= this run one per CTA (0: off)
-    int wfa_big_smem = 100 << 10;    // shared memory of that kernel, bytes (two CTAs per SM)
+    int wfa_big_min = 4096;          // WFA pairs with qn+tn >= this run one per CTA (0: off, register tiles too)
+    int wfa_big_smem = 100 << 10;    // shared memory of those CTAs, bytes
     int max_blocks_per_sm = 4;       // resident blocks per SM of the persistent extension kernels
     int host_chunks = 4;             // chunks a large host batch is copied and aligned in (overlapped)
     int wfa_affine_big_threads = kBigAffineThreads;  // threads per CTA of the gap-affine

@@ -466,10 +466,6 @@ struct SDir {
 };
 constexpr int kAffRing = 16;          // scores per ring (power of two)
 constexpr int kAffRingGroups = 4;     // rings per warp: groups of 8 or more lanes
-// Shared sequence words per warp, split among its groups. Zero: the sequences are read
-// through L1, which keeps more of the recent wavefront cells when shared memory is small
-// (staging both sequences measured slower: it took L1 capacity from the cells).
-constexpr int kWarpSeqWords = 0;
 
 // affine_pos_valid (wfa_simd.rs:563-569); UNSET and UNSET + 1 are negative, so invalid.
 __device__ __forceinline__ bool pos_ok(int32_t pos, int k, int qn, int tn) {
@@ -599,8 +595,7 @@ __device__ void affine_finish(const ExtendParams& P, uint32_t pid, bool act, int
 
 template <class S>
 __device__ void wfa_affine_group(const ExtendParams& P, const PairDesc& d, uint32_t pid, bool act, int G,
-                                 uint8_t* region, uint64_t region_bytes, SDir* ring, uint32_t* sseq,
-                                 int sseq_words, unsigned long long* work) {
+                                 uint8_t* region, uint64_t region_bytes, SDir* ring, unsigned long long* work) {
     const int gl = lane_id() & (G - 1);
     const int qn = act ? d.qn : 0, tn = act ? d.tn : 0;
     const bool fitting = act && tn > qn + qn / 2 + 10;
@@ -608,22 +603,7 @@ __device__ void wfa_affine_group(const ExtendParams& P, const PairDesc& d, uint3
     const uint32_t* qb = seq_base<S>(P, d.q_word);
     const uint32_t* tb = seq_base<S>(P, d.t_word);
     const int64_t hard_max_s = static_cast<int64_t>(qn + tn) * max(X, 1) + O + E + 4;
-    // both sequences into the group's shared words when they fit (one extra word each:
-    // windows read one word past the last symbol; the arena pads every sequence)
-    {
-        const int qw = act ? (qn + S::kPerWord - 1) / S::kPerWord + 1 : 0;
-        const int tw = act ? (tn + S::kPerWord - 1) / S::kPerWord + 1 : 0;
-        const bool stage = sseq != nullptr && qw + tw <= sseq_words;
-        if (stage) {
-            for (int i = gl; i < qw; i += G) sseq[i] = qb[i];
-            for (int i = gl; i < tw; i += G) sseq[qw + i] = tb[i];
-        }
-        __syncwarp();
-        if (stage) {
-            qb = sseq;
-            tb = sseq + qw;
-        }
-    }
+    __syncwarp();
     const bool use_ring = ring != nullptr && O + E < kAffRing && X < kAffRing;
 
     // region: [runs][values: cap int32][aux: cap uint32][... directory growing down]
@@ -1767,7 +1747,7 @@ __device__ bool wfa_reg(const ExtendParams& P, const PairDesc& d, uint32_t pid, 
 }
 
 // Persistent kernel: warps pull tasks; each task's groups split the warp's slot evenly.
-constexpr int kAffGroupSmem = kAffRingGroups * kAffRing * static_cast<int>(sizeof(SDir)) + kWarpSeqWords * 4;
+constexpr int kAffGroupSmem = kAffRingGroups * kAffRing * static_cast<int>(sizeof(SDir));
 constexpr int kAffWarpSmem = kAffGroupSmem > kRegWarpSmem ? kAffGroupSmem : kRegWarpSmem;
 constexpr int kAffBlockSmem = 8 * kAffWarpSmem;   // of the largest block (the limit set for every size, as kBigSmemMax)
 
@@ -1840,14 +1820,10 @@ __global__ void __launch_bounds__(256, kAffine ? 2 : 4) wfa_kernel(ExtendParams 
             }
         }
         if (kAffine) {
-            // per warp: one directory ring per group of >= 4 lanes, then the sequence words
+            // per warp: one directory ring per group of >= 4 lanes
             uint8_t* wsm = wfa_smem + static_cast<size_t>(threadIdx.x >> 5) * kAffWarpSmem;
             SDir* ring = 32 / G <= kAffRingGroups ? reinterpret_cast<SDir*>(wsm) + grp * kAffRing : nullptr;
-            const int seq_words = kWarpSeqWords / (32 / G);
-            uint32_t* sseq = seq_words > 0 ? reinterpret_cast<uint32_t*>(wsm + kAffRingGroups * kAffRing * sizeof(SDir)) +
-                                                 grp * seq_words
-                                           : nullptr;
-            wfa_affine_group<S>(P, d, pid, act, G, region, region_bytes, ring, sseq, seq_words, work);
+            wfa_affine_group<S>(P, d, pid, act, G, region, region_bytes, ring, work);
         }
         else
             wfa_linear_group<S>(P, d, pid, act, G, region, region_bytes);
