@@ -58,6 +58,9 @@ __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>&
     const int lane = lane_id();
     const int qn = G.qn, tn = G.tn;
     const int k0 = G.first(g) - kTileSteps + lane;   // this lane's first diagonal
+    // where this lane's diagonal ends in the target: no offset is beyond the query's end, and
+    // a bound just past that stays within a value word whatever the target's length
+    const int tk0 = min(tn + k0, qn + 1);
     int M[RM][R], I[R], D[R];
     uint32_t ops[R];
 #pragma unroll
@@ -96,9 +99,7 @@ __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>&
             to_up[r] = c;
             a = M[OES - 1][r] + (2 << 8) - 1, e = D[r] - 1;
             c = max(a, e);
-            // no offset beyond the target's end; none is beyond the query's, which keeps the
-            // bound within a value word whatever the target's length
-            const int t_last = (__viaddmin_s32(tn + k0, 32 * r - 1, qn) << 10) | 1023;
+            const int t_last = ((tk0 + 32 * r - 1) << 10) | 1023;   // no offset beyond the target's end
             if (c > t_last) {
                 if (a > t_last) a = kUnset;
                 if (e > t_last) e = kUnset;
@@ -123,7 +124,7 @@ __device__ __forceinline__ unsigned long long aff_tile(const PairSeq<S, STAGED>&
             D[r] = del & ~kTag;
             // [mismatch, close I, close D], the first on a tie
             const int k = k0 + 32 * r;
-            const int hi = __viaddmin_s32(tn + k0, 32 * r, qn);
+            const int hi = __viaddmin_s32(tk0, 32 * r, qn);
             int mis = M[XS - 1][r] + kOne + (3 << 8);
             if (mis > ((hi << 10) | 1023)) mis = kUnset;
             const int m = __viaddmax_s32(I[r], 2 << 8, __viaddmax_s32(D[r], 1 << 8, mis));
