@@ -139,8 +139,8 @@ __host__ __device__ __forceinline__ int lane_slots(int dmin, int dmax, int nb) {
 // Whether a fitting-mode batch of n pairs gives its 2-bit pairs of up to kLaneMaxSlots blocks
 // a lane each (every block in the window: nothing is banded) instead of a group of lanes.
 // A lane takes the latency of its whole pair, so the batch has to fill the chip's lanes:
-// windows of 150-300 bp, lanes against groups: 12,000 0.46 / 0.43 ms, 20,000 0.47 / 0.50,
-// 50,000 0.60 / 0.99, 200,000 1.33 / 3.22.
+// windows of 100-300 bp, lanes against groups: 20,000 0.47 / 0.51 ms, 50,000 0.59 / 1.00,
+// 200,000 1.12 / 3.21 (12,000, with lanes 20 % slower on large batches than now, 0.46 / 0.43).
 constexpr uint64_t kFitLaneMin = 16384;
 __host__ __device__ __forceinline__ bool fit_lanes(int32_t engine, uint64_t n, int32_t lane_ckpt) {
     return engine == PHR_ENGINE_MYERS_FIT && n >= kFitLaneMin && lane_ckpt;

@@ -6,10 +6,12 @@
 //
 // What bounds it: a score's cells are a short dependent chain (three neighbours, one
 // compare of 16 bases), so a pair is bound by that chain's latency while its wavefront is
-// narrow and by the integer pipes once it is wide (about 45 instructions per cell, one SM
-// per pair). 500 pairs of 4-16 kb at up to 10 % divergence: 2.6 ms, 160 G diagonals/s; the
-// kernel before it (one barrier per score, ~200 instructions per cell, frames and history
-// of 32-bit words, a second pass for every pair that outgrew its first scratch): 14.5 ms.
+// narrow and by the integer pipes once it is wide, one SM per pair. 200 pairs of 4-16 kb at
+// up to 10 % divergence: 165 M band diagonals in 2.1 ms, 84 instructions a diagonal with the
+// tiles' overlap, idle lanes and the traceback (issue 49 % on single CTAs, 27 % on
+// clusters). 500 such pairs: 2.5 ms a call; with the kernel before it (one barrier per score,
+// ~200 instructions per cell, frames and history of 32-bit words, a second pass for every
+// pair that outgrew its first scratch) 15.2 ms.
 //
 // Tiles. A warp holds 32 R consecutive diagonals, lane l the diagonals l, l + 32, ... of
 // the tile (neighbours are then one lane away, and the 32 lanes' sequence reads of one

@@ -112,3 +112,15 @@ def test_records_run_out(engine, costs, clusters):
         assert eng.counter("scratch_oom_pairs") == 0
     # (one pair: were it redone before the hand-over, no cluster would have run)
     assert got == want and ran.get(RESUME[engine], 0) == (1 if clusters > 1 else 0) and ran["redo_tasks"] >= 1, ran
+
+
+@engines
+def test_one_warp_records_run_out(engine, costs):
+    """Six unrelated pairs, a warp each, in a workspace for the records of about one."""
+    rng = np.random.default_rng(66)
+    pairs = [(rng.choice(np.frombuffer(DNA, np.uint8), 900).tobytes(), rng.choice(np.frombuffer(DNA, np.uint8), 950).tobytes())
+             for _ in range(6)]
+    with P.Engine(0, workspace_bytes=10 << 20 if engine == A.ENGINE_WFA_AFFINE else 512 << 10) as eng:
+        got, want, ran = run(eng, engine, costs, pairs)
+        assert eng.counter("scratch_oom_pairs") == 0
+    assert got == want and ran["redo_tasks"] >= 1, ran
