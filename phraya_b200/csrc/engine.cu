@@ -994,7 +994,7 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
     unsigned long long* need_max = reinterpret_cast<unsigned long long*>(cnt + 8);
     uint64_t* total = reinterpret_cast<uint64_t*>(cnt + 12);
     const unsigned T = 256;
-    const uint64_t pass_budget = std::min(ctx->scratch_budget, ctx->pass_budget);
+    uint64_t pass_budget = std::min(ctx->scratch_budget, ctx->pass_budget);
     const bool small = n <= kSmallPairs;
     // lanes per short WFA pair: affine and linear tune separately
     const int g_short = engine == PHR_ENGINE_WFA_AFFINE ? ctx->tune.wfa_affine_group_short : ctx->tune.wfa_group_short;
@@ -1167,9 +1167,18 @@ phr_status run_extend(Ctx* ctx, phr_engine engine, const DevPairs& in, phr_affin
                 pool = std::min<uint64_t>(2 * tile_need[0], 2 * teams * tile_need[1]);
                 pool = std::max<uint64_t>(pool, std::min<uint64_t>(16 * tile_need[0], 1ull << 30)) + (1 << 20);
                 pool = std::min<uint64_t>(pool, pass_budget);
-                tile_pool = pool;
             }
-            PHR_CUDA_TRY(ctx, ctx->scratch.reserve(std::max(grid * warps_per_block * slot, pool)));
+            const uint64_t slots = grid * warps_per_block * slot;
+            cudaError_t e = ctx->scratch.reserve(std::max(slots, pool));
+            // the pool is what is wanted, not what is needed: where the device has less to give,
+            // pairs that do not fit follow in redo passes, which then keep to the same
+            while (e == cudaErrorMemoryAllocation && pool > std::max<uint64_t>(slots, 64 << 20)) {
+                cudaGetLastError();
+                pass_budget = pool /= 2;
+                e = ctx->scratch.reserve(std::max(slots, pool));
+            }
+            PHR_CUDA_TRY(ctx, e);
+            tile_pool = pool;
         } else {
             grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, (n_tasks_hint + warps_per_block - 1) / warps_per_block));
             PHR_CUDA_TRY(ctx, ctx->scratch.reserve(per_task_total));
