@@ -452,7 +452,7 @@ phr_status phr_server_create(phr_ctx* c, const phr_index* idx, const phr_server_
             // pair of a batch (what a batched call takes) made the buffer grow from batch to
             // batch, to 12 GB and more. 2,000 long and 2,000 short reads at once, balanced:
             // 3,100-12,500 reads/s, p99 of the long ones 0.3-1.3 s, 63 GiB in use; with the
-            // limit 50,000-64,000 reads/s, 46-66 ms, 26 GiB. Gap-affine pairs hold five times
+            // limit 48,000-67,000 reads/s, 46-69 ms, 26 GiB. Gap-affine pairs hold five times
             // the records: 150 reads/s with the limit, 850 without.
             if (!W->short_only && S->cfg.align.strategy != PHR_SENSITIVE) W->ctx.pass_budget = scratch;
             cudaGetLastError();
